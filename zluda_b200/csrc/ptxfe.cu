@@ -168,145 +168,6 @@ __global__ void __launch_bounds__(256) staged_kernel(size_t n, uint32_t* table, 
     for (uint32_t k = 0; k < r.n; k++) row[k] = stage[k * STAGE_STRIDE + threadIdx.x];
 }
 
-// ---- one thread per item of a segmented range: a block takes 256 consecutive segments, whose items are contiguous,
-// and every thread finds the segment of its item by binary search over the block's offsets in shared memory
-// Record emission (PtxEmitStep): a block takes 256 consecutive units, whose words are contiguous, loads what a word
-// needs of its unit into shared memory once, and then goes over the words with EMIT_ILP words per thread at a time:
-// all their reads are issued before the first of them is written, so that several chains of dependent loads (unit ->
-// template -> token) are in flight per thread.  The literals are collected and converted in a second round with the
-// warps full.
-#define SEG_DEFER_CAP 2048u
-#define EMIT_ILP 4
-__global__ void __launch_bounds__(256, 6) emit_records_kernel(uint32_t n_units, const PtxPair* off, PtxEmitStep e) {
-    __shared__ uint32_t so[257];
-    __shared__ PtxEmitUnit su[256];
-    __shared__ uint32_t later[SEG_DEFER_CAP];
-    __shared__ uint32_t n_later;
-    const uint32_t u0 = blockIdx.x * 256;
-    const uint32_t nu = n_units - u0 < 256u ? n_units - u0 : 256u;
-    for (uint32_t k = threadIdx.x; k <= nu; k += 256) so[k] = off[u0 + k].a;
-    if (threadIdx.x < nu) su[threadIdx.x] = e.unit(u0 + threadIdx.x);
-    if (threadIdx.x == 0) n_later = 0;
-    __syncthreads();
-    const uint32_t first = so[0], total = so[nu] - so[0];
-    // Every warp takes a contiguous eighth of the block's words, 32 at a time.  The unit of a word: `ua` is the unit of
-    // the window's first word; the lanes read the next 32 unit offsets, those inside the window mark their place in a
-    // 32-bit mask, and a lane's unit is ua + the number of marks at or below it.  (Units without words put two marks on
-    // one place: such a window searches, as does the first of a warp.)
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t per_warp = ((total + 255u) / 256u) * 32u;
-    const uint32_t wbeg = warp * per_warp, wend = wbeg + per_warp < total ? wbeg + per_warp : total;
-    uint32_t ua = 0;
-    if (wbeg < wend) {
-        const uint32_t o = first + wbeg;
-        uint32_t lo = 0, hi = nu;              // last k with so[k] <= o
-        while (hi - lo > 1) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (so[mid] <= o) lo = mid; else hi = mid;
-        }
-        ua = lo;
-    }
-    for (uint32_t jb = wbeg; jb < wend; jb += 32 * EMIT_ILP) {
-        uint32_t x[EMIT_ILP], unit[EMIT_ILP];
-        int what[EMIT_ILP];
-#pragma unroll
-        for (int q = 0; q < EMIT_ILP; q++) {
-            const uint32_t j0 = jb + q * 32, j = j0 + lane;       // j0 is the same for the whole warp
-            what[q] = PtxEmitStep::NOTHING;
-            unit[q] = 0;
-            if (j0 >= wend) continue;
-            const uint32_t o0 = first + j0, o = o0 + lane;
-            while (ua + 1 < nu && so[ua + 1] <= o0) ua++;        // the unit of the window's first word (a step or none)
-            const uint32_t k = ua + 1 + lane;
-            const uint32_t rel = k <= nu ? so[k] - o0 : 0xFFFFFFFFu;
-            const bool inside = rel < 32u;
-            const uint32_t n_in = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, inside));
-            const uint32_t marks = __reduce_or_sync(0xFFFFFFFFu, inside ? 1u << rel : 0u);
-            uint32_t lo;
-            if ((uint32_t)__popc(marks) == n_in) {
-                lo = ua + (uint32_t)__popc(marks & (0xFFFFFFFFu >> (31u - lane)));
-            } else {
-                uint32_t hi = nu;
-                lo = ua;
-                while (hi - lo > 1) {
-                    uint32_t mid = (lo + hi) >> 1;
-                    if (so[mid] <= o) lo = mid; else hi = mid;
-                }
-            }
-            ua = ua + n_in < nu - 1u ? ua + n_in : nu - 1u;     // the marks are all in front of the next window
-            if (j >= wend) continue;
-            unit[q] = lo;
-            what[q] = e.word(su[lo], (size_t)(u0 + lo), o - so[lo], x[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < EMIT_ILP; q++) {
-            const uint32_t j = jb + q * 32 + lane;
-            if (what[q] == PtxEmitStep::WRITE) {
-                e.words[first + j] = x[q];
-            } else if (what[q] == PtxEmitStep::SECOND_ROUND) {
-                const uint32_t slot = atomicAdd(&n_later, 1u);
-                if (slot < SEG_DEFER_CAP && j < (1u << 24)) later[slot] = j | (unit[q] << 24);
-                else e.literal(su[unit[q]], first + j - so[unit[q]], first + j);
-            }
-        }
-    }
-    __syncthreads();
-    const uint32_t nl = n_later < SEG_DEFER_CAP ? n_later : SEG_DEFER_CAP;
-    for (uint32_t x = threadIdx.x; x < nl; x += 256) {
-        const uint32_t j = later[x] & 0xFFFFFFu, lo = later[x] >> 24, o = first + j;
-        e.literal(su[lo], o - so[lo], o);
-    }
-}
-template <class F>
-__global__ void __launch_bounds__(256) segments_kernel(uint32_t n_units, const PtxPair* off, F f) {
-    __shared__ uint32_t so[257];
-    const uint32_t u0 = blockIdx.x * 256;
-    const uint32_t nu = n_units - u0 < 256u ? n_units - u0 : 256u;
-    for (uint32_t k = threadIdx.x; k <= nu; k += 256) so[k] = off[u0 + k].a;
-    __syncthreads();
-    const uint32_t first = so[0], total = so[nu] - so[0];
-    for (uint32_t j = threadIdx.x; j < total; j += 256) {
-        uint32_t o = first + j;
-        uint32_t lo = 0, hi = nu;          // last k with so[k] <= o
-        while (hi - lo > 1) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (so[mid] <= o) lo = mid; else hi = mid;
-        }
-        f((size_t)(u0 + lo), o - so[lo], o);
-    }
-}
-
-__global__ void copy_words_kernel(uint32_t* dst, const uint32_t* src, uint32_t n) {
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
-    __threadfence_system();
-}
-
-// ---- text that arrived as one host-contiguous run: move every module to its chunk-aligned slot
-// One thread per 16 bytes of destination.  `raw_off` of a module is where its first byte lies in `raw`.
-struct RepackModule {
-    uint32_t chunk_begin, raw_off, len;
-};
-__global__ void __launch_bounds__(256) repack_text_kernel(uint32_t n_pieces, uint32_t n_modules, const RepackModule* mods, const uint32_t* mcb,
-                                                          const uint8_t* raw, uint8_t* text) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_pieces) return;
-    uint32_t chunk = i >> 3;
-    uint32_t m = ptx_upper_bound_u32(mcb, n_modules, chunk) - 1;
-    uint32_t o = (chunk - mods[m].chunk_begin) * PTX_CHUNK + (i & 7u) * 16;   // offset inside the module
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (o < mods[m].len) {
-        size_t a = (size_t)mods[m].raw_off + o;
-        const uint32_t* w = (const uint32_t*)(raw + (a & ~(size_t)3));       // the raw buffer has 32 spare bytes at its end
-        uint32_t sh = (uint32_t)(a & 3) * 8;
-        uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
-        v.x = __funnelshift_r(w0, w1, sh);
-        v.y = __funnelshift_r(w1, w2, sh);
-        v.z = __funnelshift_r(w2, w3, sh);
-        v.w = __funnelshift_r(w3, w4, sh);
-    }
-    ((uint4*)text)[i] = v;
-}
-
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
@@ -355,6 +216,140 @@ __device__ inline void block_scan(T v, Op op, T identity, T* warp_tot, T& incl, 
     for (int w = 0; w < warp; w++) wp = op(wp, warp_tot[w]);
     incl = op(wp, x);
     excl = op(wp, prev);
+}
+
+// ---- record emission (PtxEmitStep): a block takes 256 consecutive units, loads what a word needs of its unit into
+// shared memory once, and then goes over their words with EMIT_ILP words per thread at a time: all their reads are
+// issued before the first of them is written, so that several chains of dependent loads (unit -> template -> token)
+// are in flight per thread.  The literals are collected and converted in a second round with the warps full.
+// The words counted are those of staged and templated units only (at most PTX_TMP_STRIDE each): a unit that the second
+// decode pass writes can have millions of words - an array with its initialiser - and one block that stepped over them
+// word by word took 16.3 of 19.5 ms of a 41 MB module of constant tables (0.1 ms without them).
+#define SEG_DEFER_CAP 2048u
+#define EMIT_ILP 4
+__global__ void __launch_bounds__(256, 6) emit_records_kernel(uint32_t n_units, const PtxPair* off, PtxEmitStep e) {
+    __shared__ uint32_t so[257];              // words of the units in front of unit k that this kernel writes
+    __shared__ PtxEmitUnit su[256];
+    __shared__ uint32_t warp_tot[8];
+    __shared__ uint32_t later[SEG_DEFER_CAP];
+    __shared__ uint32_t n_later;
+    const uint32_t u0 = blockIdx.x * 256;
+    const uint32_t nu = n_units - u0 < 256u ? n_units - u0 : 256u;
+    uint32_t mine = 0;
+    if (threadIdx.x < nu) {
+        const uint32_t begin = off[u0 + threadIdx.x].a, end = off[u0 + threadIdx.x + 1].a;
+        PtxEmitUnit eu = e.unit(u0 + threadIdx.x);
+        eu.first = begin;
+        su[threadIdx.x] = eu;
+        if (eu.flag == PTX_UNIT_STAGED || eu.flag == PTX_UNIT_TEMPLATED) mine = end - begin;
+    }
+    if (threadIdx.x == 0) n_later = 0;
+    {
+        uint32_t incl, excl;
+        block_scan(mine, AddOp(), 0u, warp_tot, incl, excl);
+        so[threadIdx.x] = excl;
+        if (threadIdx.x == 255) so[256] = incl;
+    }
+    __syncthreads();
+    const uint32_t total = so[nu];
+    // Every warp takes a contiguous eighth of the block's words, 32 at a time.  The unit of a word: `ua` is the unit of
+    // the window's first word; the lanes read the next 32 unit offsets, those inside the window mark their place in a
+    // 32-bit mask, and a lane's unit is ua + the number of marks at or below it.  (Units without words put two marks on
+    // one place: such a window searches, as does the first of a warp.)
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t per_warp = ((total + 255u) / 256u) * 32u;
+    const uint32_t wbeg = warp * per_warp, wend = wbeg + per_warp < total ? wbeg + per_warp : total;
+    uint32_t ua = 0;
+    if (wbeg < wend) {
+        const uint32_t o = wbeg;
+        uint32_t lo = 0, hi = nu;              // last k with so[k] <= o
+        while (hi - lo > 1) {
+            uint32_t mid = (lo + hi) >> 1;
+            if (so[mid] <= o) lo = mid; else hi = mid;
+        }
+        ua = lo;
+    }
+    for (uint32_t jb = wbeg; jb < wend; jb += 32 * EMIT_ILP) {
+        uint32_t x[EMIT_ILP], unit[EMIT_ILP];
+        int what[EMIT_ILP];
+#pragma unroll
+        for (int q = 0; q < EMIT_ILP; q++) {
+            const uint32_t j0 = jb + q * 32, j = j0 + lane;       // j0 is the same for the whole warp
+            what[q] = PtxEmitStep::NOTHING;
+            unit[q] = 0;
+            if (j0 >= wend) continue;
+            const uint32_t o0 = j0, o = o0 + lane;
+            while (ua + 1 < nu && so[ua + 1] <= o0) ua++;        // the unit of the window's first word (a step or none)
+            const uint32_t k = ua + 1 + lane;
+            const uint32_t rel = k <= nu ? so[k] - o0 : 0xFFFFFFFFu;
+            const bool inside = rel < 32u;
+            const uint32_t n_in = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, inside));
+            const uint32_t marks = __reduce_or_sync(0xFFFFFFFFu, inside ? 1u << rel : 0u);
+            uint32_t lo;
+            if ((uint32_t)__popc(marks) == n_in) {
+                lo = ua + (uint32_t)__popc(marks & (0xFFFFFFFFu >> (31u - lane)));
+            } else {
+                uint32_t hi = nu;
+                lo = ua;
+                while (hi - lo > 1) {
+                    uint32_t mid = (lo + hi) >> 1;
+                    if (so[mid] <= o) lo = mid; else hi = mid;
+                }
+            }
+            ua = ua + n_in < nu - 1u ? ua + n_in : nu - 1u;     // the marks are all in front of the next window
+            if (j >= wend) continue;
+            unit[q] = lo;
+            what[q] = e.word(su[lo], (size_t)(u0 + lo), o - so[lo], x[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < EMIT_ILP; q++) {
+            const uint32_t j = jb + q * 32 + lane;
+            if (what[q] == PtxEmitStep::WRITE) {
+                e.words[su[unit[q]].first + (j - so[unit[q]])] = x[q];
+            } else if (what[q] == PtxEmitStep::SECOND_ROUND) {
+                const uint32_t slot = atomicAdd(&n_later, 1u);
+                const uint32_t i = j - so[unit[q]];
+                if (slot < SEG_DEFER_CAP) later[slot] = i | (unit[q] << 24);
+                else e.literal(su[unit[q]], i, su[unit[q]].first + i);
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t nl = n_later < SEG_DEFER_CAP ? n_later : SEG_DEFER_CAP;
+    for (uint32_t x = threadIdx.x; x < nl; x += 256) {
+        const uint32_t i = later[x] & 0xFFFFFFu, lo = later[x] >> 24;
+        e.literal(su[lo], i, su[lo].first + i);
+    }
+}
+__global__ void copy_words_kernel(uint32_t* dst, const uint32_t* src, uint32_t n) {
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
+    __threadfence_system();
+}
+
+// ---- text that arrived as one host-contiguous run: move every module to its chunk-aligned slot
+// One thread per 16 bytes of destination.  `raw_off` of a module is where its first byte lies in `raw`.
+struct RepackModule {
+    uint32_t chunk_begin, raw_off, len;
+};
+__global__ void __launch_bounds__(256) repack_text_kernel(uint32_t n_pieces, uint32_t n_modules, const RepackModule* mods, const uint32_t* mcb,
+                                                          const uint8_t* raw, uint8_t* text) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_pieces) return;
+    uint32_t chunk = i >> 3;
+    uint32_t m = ptx_upper_bound_u32(mcb, n_modules, chunk) - 1;
+    uint32_t o = (chunk - mods[m].chunk_begin) * PTX_CHUNK + (i & 7u) * 16;   // offset inside the module
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (o < mods[m].len) {
+        size_t a = (size_t)mods[m].raw_off + o;
+        const uint32_t* w = (const uint32_t*)(raw + (a & ~(size_t)3));       // the raw buffer has 32 spare bytes at its end
+        uint32_t sh = (uint32_t)(a & 3) * 8;
+        uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+        v.x = __funnelshift_r(w0, w1, sh);
+        v.y = __funnelshift_r(w1, w2, sh);
+        v.z = __funnelshift_r(w2, w3, sh);
+        v.w = __funnelshift_r(w3, w4, sh);
+    }
+    ((uint4*)text)[i] = v;
 }
 
 template <class T, class Op, class Ld>
@@ -827,13 +822,6 @@ struct CudaBackend {
         // more shared memory than a kernel gets by default: opt in (cheap, so done at every launch)
         cudaFuncSetAttribute(staged_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STAGED_SMEM_BYTES);
         staged_kernel<<<(unsigned)((n + 255) / 256), 256, STAGED_SMEM_BYTES, ctx->stream>>>(n, table, row_words, f);
-        prof_end();
-        ctx->launches++;
-    }
-    template <class F> void pf_segments(const char* name, size_t n, const PtxPair* off, F f) {
-        if (ctx->failed || n == 0) return;
-        prof_begin(name);
-        segments_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>((uint32_t)n, off, f);
         prof_end();
         ctx->launches++;
     }

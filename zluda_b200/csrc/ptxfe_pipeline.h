@@ -318,11 +318,7 @@ struct AddOp {
 //   template <class F> void pf_staged(const char* name, size_t n, uint32_t* table, uint32_t row_words, F f);
 //        PtxStaged r = f(i, scratch) for i in [0, n), scratch a PtxScratch of the backend's;
 //        afterwards the backend copies the first r.n staged words to table[r.unit * row_words ...]
-//   template <class F> void pf_segments(const char* name, size_t n, const PtxPair* off, F f);
-//        segment s owns the items [off[s].a, off[s + 1].a): f(s, i, off[s].a + i) for every s < n and every item i of s
 //   void emit_records(const char* name, size_t n_units, const PtxPair* off, const PtxEmitStep& e);   C5, see PtxEmitStep
-//        the same in two rounds: an item for which f returns true is handled by g(s, i, off[s].a + i) afterwards, the
-//        items put off packed together (work that few scattered items need)
 //   PtxClassStore class_store(bool reset);   the batch's class store (device memory that outlives the arena), emptied if asked
 //   const PtxLexTables* lex_tables();   the constant tables of ptx_lex_tile.h where the steps can read them (filled by lt_fill_tables)
 //   void lex_mark(const char* name, size_t n_tiles, const PtxLexTileArgs& a);   the phases of ptx_lex_tile.h's mark step, one block per tile
@@ -550,7 +546,7 @@ inline void ptx_stage_structure(BK& bk, PtxWork& w, PtxCounters& host_counters, 
 // the backend); word() only reads and says what to do with the word, so that a backend can have several words in flight
 // per thread; literal() is the second round (one literal per call, written in place).
 struct PtxEmitUnit {
-    uint32_t tmpl, start, flag;
+    uint32_t tmpl, start, flag, first;      // first: its first word in the record stream (filled in by the backend)
 };
 struct PtxEmitStep {
     const uint8_t* uflag;
@@ -567,6 +563,7 @@ struct PtxEmitStep {
         e.flag = uflag[u];
         e.tmpl = e.flag == PTX_UNIT_TEMPLATED ? utmpl[u] : 0u;
         e.start = ustart[u];
+        e.first = 0;
         return e;
     }
     PTX_HD int word(const PtxEmitUnit& e, size_t u, uint32_t i, uint32_t& x) const {
