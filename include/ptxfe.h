@@ -134,6 +134,9 @@ int ptxfe_module_records(const ptxfe_batch* batch, uint32_t i, const uint32_t** 
 /* Canonical text dump of module i: the tree printed as if every ptx_parser AST type derived Debug (floats as bit
  * patterns), followed by the ordered error list.  malloc'ed; release with ptxfe_free. */
 int ptxfe_module_dump(const ptxfe_batch* batch, uint32_t i, char** out, uint64_t* out_len);
+/* The ordered error list of module i alone: the lines of the dump behind its last "errors: N" line.  malloc'ed; release
+ * with ptxfe_free. */
+int ptxfe_module_errors(const ptxfe_batch* batch, uint32_t i, char** out, uint64_t* out_len);
 /* Materialiser: builds, for every module of the batch, the tree a caller of the reference holds - module, directives,
  * functions, statements with nested blocks, variables with their padded initialisers, instructions with typed data and
  * operands, names as slices of the caller's text (zluda_b200/csrc/ptx_ast.h mirrors ptx_parser/src/ast.rs:14-19,

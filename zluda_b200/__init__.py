@@ -70,6 +70,7 @@ def lib():
         L.ptxfe_profile.restype = ctypes.c_char_p
         L.ptxfe_module_records.argtypes = [vp, u32, ctypes.POINTER(ctypes.POINTER(u32)), ctypes.POINTER(u64), ctypes.POINTER(u64)]
         L.ptxfe_module_dump.argtypes = [vp, u32, ctypes.POINTER(vp), ctypes.POINTER(u64)]
+        L.ptxfe_module_errors.argtypes = [vp, u32, ctypes.POINTER(vp), ctypes.POINTER(u64)]
         L.ptxfe_module_dump_hash.argtypes = [vp, u32, ctypes.POINTER(u64)]
         L.ptxfe_free.argtypes = [vp]
         L.ptxfe_lex_module.argtypes = [vp, ctypes.c_char_p, u64, ctypes.POINTER(vp), ctypes.POINTER(u64), ctypes.POINTER(u64)]
@@ -85,6 +86,12 @@ def lib():
         L.ptxfe_multi_part_of.argtypes = [vp, u32]
         _lib = L
     return _lib
+
+
+# bytes at an address -> str without a bytes object in between
+_decode_utf8 = ctypes.pythonapi.PyUnicode_DecodeUTF8
+_decode_utf8.restype = ctypes.py_object
+_decode_utf8.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t, ctypes.c_char_p]
 
 
 class Texts:
@@ -154,13 +161,16 @@ class Batch:
     def error_count(self, i):
         return lib().ptxfe_module_error_count(self._h, i)
 
-    def dump(self, i):
+    def _text(self, fn, i):
         p = ctypes.c_void_p()
         n = ctypes.c_uint64()
-        self._ctx._check(lib().ptxfe_module_dump(self._h, i, ctypes.byref(p), ctypes.byref(n)))
-        s = ctypes.string_at(p, n.value).decode("utf-8", "replace")
+        self._ctx._check(fn(self._h, i, ctypes.byref(p), ctypes.byref(n)))
+        s = _decode_utf8(p, n.value, b"replace")
         lib().ptxfe_free(p)
         return s
+
+    def dump(self, i):
+        return self._text(lib().ptxfe_module_dump, i)
 
     def dump_hash(self, i):
         h = ctypes.c_uint64()
@@ -178,9 +188,7 @@ class Batch:
         return np.ctypeslib.as_array(p, shape=(n.value,)).copy(), base.value
 
     def errors(self, i):
-        lines = self.dump(i).split("\n")
-        k = max(j for j, l in enumerate(lines) if l.startswith("errors: "))
-        return [l for l in lines[k + 1:] if l]
+        return [l for l in self._text(lib().ptxfe_module_errors, i).split("\n") if l]
 
 
 class Context:
@@ -328,7 +336,7 @@ def _ctx():
 
 def _single(text, mode):
     b = _ctx().parse_batch([text], mode)
-    r = ParseResult(b.status(0) == 0, b.dump(0), b.errors(0))
+    r = ParseResult(b.status(0) == 0, b.dump(0), b.errors(0) if b.error_count(0) else [])
     b.free()
     return r
 
@@ -345,4 +353,7 @@ def parse_module_unchecked(text):
 
 def parse_for_errors(text):
     """Only the ordered error list; keeps parsing after lex errors (lib.rs:392-411)."""
-    return _single(text, ERRORS_ONLY).errors
+    b = _ctx().parse_batch([text], ERRORS_ONLY)
+    errors = b.errors(0) if b.error_count(0) else []
+    b.free()
+    return errors

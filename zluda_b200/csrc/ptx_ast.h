@@ -94,6 +94,8 @@ struct Function {
     std::vector<Variable> rets, inputs;
     std::vector<Tuning> tuning;
     std::vector<Statement> body;
+    const uint32_t* body_rec = nullptr;     // materialised without bodies: the body's records instead
+    const uint32_t* body_end = nullptr;
 };
 struct Directive {
     bool is_method = false;
@@ -151,6 +153,7 @@ struct Builder {
     const uint32_t* operand(const uint32_t* w, Operand* o) const {
         const uint32_t kind = w[0] & 0xF, aux = (w[0] >> 4) & 0xF;
         o->kind = (uint8_t)kind;
+        o->absent = false;
         m.nodes++;
         switch (kind) {
         case OPK_REG: o->name = name(w[0], w[1]); return w + 2;
@@ -236,6 +239,7 @@ struct Builder {
         const uint32_t w0 = rec[0];
         const uint32_t* w = rec + 1;
         const uint32_t w1 = (w0 & 0xFF) == U_INSTR ? (((w0 >> 29) & 3u) | (((w0 >> 22) & 0x7Fu) << 16)) : rec[ptxdump::rec_len(w0)];
+        o->data.clear();
         o->variant = (uint16_t)(w1 >> 16);
         o->has_pred = (w1 & 1) != 0;
         o->pred_not = (w1 & 2) != 0;
@@ -252,6 +256,10 @@ struct Builder {
             std::vector<Operand> inputs(n_inputs);
             for (uint32_t i = 0; i < n_inputs; i++) p = operand(p, &inputs[i]);
             o->resolved = *p != 0;
+            o->args.clear();
+            o->callee_rets.clear();
+            o->callee_inputs.clear();
+            o->call_rets.clear();
             if (o->resolved) {
                 const uint32_t* f = r.v.words + callee;      // the callee's U_FUNC record
                 const uint32_t cr = f[4], ci = f[5];
@@ -283,6 +291,7 @@ struct Builder {
         o->parameterized = w[0] != 0;
         o->count = w[1];
         info(names + 2 * n_names, &o->info);
+        o->names.clear();
         if (o->parameterized) o->name = str(names[0], names[1]);
         else
             for (uint32_t i = 0; i < n_names; i++) o->names.push_back(str(names[2 * i], names[2 * i + 1]));
@@ -331,24 +340,42 @@ struct Builder {
     }
 };
 
-// module `mi` of a fetched batch as a tree
-inline void materialize(const PtxBatchView& v, uint32_t mi, Module* out) {
+// the ordered error list of module `mi`; false: the module was given up or refused, it has none
+inline bool materialize_errors(const PtxBatchView& v, uint32_t mi, Module* out) {
+    const PtxModuleResult& res = v.results[mi];
+    const bool skip_parse = res.lexerr_end != res.lexerr_begin && v.mode != 2;
+    if (res.sequential && ((res.status & US_MASK) == US_DIVERGE || (res.status & US_MASK) == US_REFUSED) && !skip_parse) return false;
+    for (uint32_t i = res.lexerr_begin; i < res.lexerr_end; i++) {
+        Error e;
+        e.lexer = true;
+        e.lex_start = v.lexerrs[2 * (size_t)i] - v.layout[mi].text_off;
+        out->errors.push_back(e);
+    }
+    if (skip_parse) return true;
+    for (uint32_t i = res.err_begin; i < res.err_end; i++) {
+        const PtxErrRec& er = v.errs[i];
+        if ((er.w0 & 0xFFFF) == E_NONE) continue;
+        Error e;
+        e.w0 = er.w0;
+        e.a = er.a;
+        e.b = er.b;
+        out->errors.push_back(e);
+    }
+    out->implicit_parser_error = res.word_begin == res.word_end;      // a module without tokens: its header does not parse
+    return true;
+}
+
+// module `mi` of a fetched batch as a tree; without bodies: a function keeps the place of its body's records instead
+// (a reader that goes over the statements once, like the printer, takes them one at a time)
+inline void materialize(const PtxBatchView& v, uint32_t mi, Module* out, bool bodies = true) {
     ptxdump::Reader r(v, mi);
     Module& m = *out;
     Builder b{r, m};
     const PtxModuleResult& res = v.results[mi];
     const uint32_t n_lex = res.lexerr_end - res.lexerr_begin;
-    const uint64_t base = v.layout[mi].text_off;
     const bool skip_parse = n_lex != 0 && v.mode != 2;
-    for (uint32_t i = res.lexerr_begin; i < res.lexerr_end; i++) {
-        Error e;
-        e.lexer = true;
-        e.lex_start = v.lexerrs[2 * (size_t)i] - base;
-        m.errors.push_back(e);
-    }
-    if (res.sequential && ((res.status & US_MASK) == US_DIVERGE || (res.status & US_MASK) == US_REFUSED) && !skip_parse) {
+    if (!materialize_errors(v, mi, out)) {
         m.verdict = (res.status & US_MASK) == US_DIVERGE ? V_DIVERGES : V_REFUSED;
-        m.errors.clear();
         return;
     }
     struct Dir {
@@ -393,15 +420,9 @@ inline void materialize(const PtxBatchView& v, uint32_t mi, Module* out) {
             const PtxErrRec& er = v.errs[e];
             if ((er.w0 & 0xFFFF) == E_NONE) continue;
             n_parse_errs++;
-            Error x;
-            x.w0 = er.w0;
-            x.a = er.a;
-            x.b = er.b;
-            m.errors.push_back(x);
             while (di + 1 < dirs.size() && dirs[di + 1].start_off <= er.pos) di++;
             if (!dirs.empty() && dirs[di].start_off <= er.pos) dirs[di].n_errors++;
         }
-        m.implicit_parser_error = !parsed_ok && res.word_begin == res.word_end;
     }
     uint64_t invalid = 0;
     for (const Dir& d : dirs) invalid += d.n_errors ? 1 : 0;
@@ -462,7 +483,8 @@ inline void materialize(const PtxBatchView& v, uint32_t mi, Module* out) {
             const uint32_t* q = p + 1 + ptxdump::rec_len(p[0]);
             const uint32_t* end = d.end;
             // d.end lies behind the U_FUNC_END record: the body's records stop in front of it
-            b.body(q, end, &f.body);
+            if (bodies) b.body(q, end, &f.body);
+            else { f.body_rec = q; f.body_end = end; }
         }
     }
 }
@@ -478,9 +500,9 @@ struct Printer {
     void operand(const Operand& p) {
         switch (p.kind) {
         case OPK_REG: o.put("Reg("); str(p.name); o.put(")"); break;
-        case OPK_REG_OFFSET: o.put("RegOffset("); str(p.name); o.putf(", %d)", p.offset); break;
+        case OPK_REG_OFFSET: o.put("RegOffset("); str(p.name); o.put(", "); o.snum(p.offset); o.put(")"); break;
         case OPK_IMM: o.put("Imm("); ptxdump::imm(o, p.imm.kind, (uint32_t)p.imm.bits, (uint32_t)(p.imm.bits >> 32)); o.put(")"); break;
-        case OPK_VEC_MEMBER: o.put("VecMember("); str(p.name); o.putf(", %u)", p.index); break;
+        case OPK_VEC_MEMBER: o.put("VecMember("); str(p.name); o.put(", "); o.num(p.index); o.put(")"); break;
         default:
             o.put("VecPack([");
             for (size_t i = 0; i < p.pack.size(); i++) {
@@ -532,9 +554,9 @@ struct Printer {
         case 0:
             switch (ty.a) {
             case 0: o.put(*w++ ? "true" : "false"); break;
-            case 3: { uint64_t x = w[0] | ((uint64_t)w[1] << 32); w += 2; o.putf("%llu", (unsigned long long)x); break; }
-            case 4: o.putf("bits=0x%08X", *w++); break;
-            default: o.putf("%u", *w++); break;
+            case 3: { uint64_t x = w[0] | ((uint64_t)w[1] << 32); w += 2; o.num(x); break; }
+            case 4: o.put("bits=0x"); o.hex(*w++, 8); break;
+            default: o.num(*w++); break;
             }
             break;
         case 1: o.put(ptx_enum_names[ty_id][*w++]); break;
@@ -574,7 +596,7 @@ struct Printer {
     void instruction(const Instruction& x) {
         o.put("Instruction(");
         if (x.has_pred) {
-            o.putf("Some(PredAt { not: %s, label: ", x.pred_not ? "true" : "false");
+            o.put(x.pred_not ? "Some(PredAt { not: true, label: " : "Some(PredAt { not: false, label: ");
             str(x.pred);
             o.put(" }), ");
         } else {
@@ -614,7 +636,7 @@ struct Printer {
             if (in.n_args) o.put(", ");
         }
         if (in.n_args) {
-            o.putf("arguments: %sArgs { ", in.name);
+            o.put("arguments: "); o.put(in.name); o.put("Args { ");
             for (int i = 0; i < in.n_args; i++) {
                 if (i) o.put(", ");
                 const PtxArg& a = ptx_args[in.first_arg + i];
@@ -628,26 +650,27 @@ struct Printer {
         }
         o.put(" })\n");
     }
+    void variable_statement(const MultiVariable& v) {
+        if (v.parameterized) {
+            o.put("Variable(Parameterized { info: ");
+            info(v.info);
+            o.put(", name: ");
+            str(v.name);
+            o.putf(", count: %u })\n", v.count);
+        } else {
+            o.put("Variable(Names { info: ");
+            info(v.info);
+            o.put(", names: [");
+            for (size_t i = 0; i < v.names.size(); i++) { if (i) o.put(", "); str(v.names[i]); }
+            o.put("] })\n");
+        }
+    }
     void statements(const std::vector<Statement>& body, int depth) {
         for (const Statement& s : body) {
             o.indent(depth);
             switch (s.kind) {
-            case ST_LABEL: o.put("Label("); str(s.label); o.put(")\n"); break;
-            case ST_VARIABLE:
-                if (s.var.parameterized) {
-                    o.put("Variable(Parameterized { info: ");
-                    info(s.var.info);
-                    o.put(", name: ");
-                    str(s.var.name);
-                    o.putf(", count: %u })\n", s.var.count);
-                } else {
-                    o.put("Variable(Names { info: ");
-                    info(s.var.info);
-                    o.put(", names: [");
-                    for (size_t i = 0; i < s.var.names.size(); i++) { if (i) o.put(", "); str(s.var.names[i]); }
-                    o.put("] })\n");
-                }
-                break;
+            case ST_LABEL: label(s.label); break;
+            case ST_VARIABLE: variable_statement(s.var); break;
             case ST_INSTRUCTION: instruction(s.ins); break;
             default:
                 o.put("Block([\n");
@@ -658,15 +681,54 @@ struct Printer {
             }
         }
     }
+    void label(const Str& s) { o.put("Label("); str(s); o.put(")\n"); }
+    // the statements of a body straight from its records: each is built like a node of the tree, printed, and its memory
+    // goes to the next one
+    void stream(const Builder& b, const uint32_t* q, const uint32_t* end) {
+        Instruction ins;
+        MultiVariable var;
+        int depth = 1;
+        for (; q < end; q += 1 + ptxdump::rec_len(q[0])) {
+            switch (q[0] & 0xFF) {
+            case U_LABEL: o.indent(depth); label(b.str(q[1], q[2])); break;
+            case U_VAR: b.multi_variable(q + 1, &var); o.indent(depth); variable_statement(var); break;
+            case U_INSTR:
+            case U_INSTR_LONG: b.instruction(q, &ins); o.indent(depth); instruction(ins); break;
+            case U_BLOCK_OPEN: o.indent(depth++); o.put("Block([\n"); break;
+            case U_BLOCK_CLOSE:
+                if (depth > 1) { o.indent(--depth); o.put("])\n"); }
+                break;
+            default: break;
+            }
+        }
+        while (depth > 1) { o.indent(--depth); o.put("])\n"); }
+    }
 };
 
-inline std::string print(const PtxBatchView& v, uint32_t mi, const Module& m) {
-    ptxdump::Out o;
+// the ordered list of a module's errors, one per line; returns how many there are
+inline size_t print_errors(const PtxBatchView& v, const ptxdump::Reader& r, ptxdump::Out* o, const Module& m) {
+    const bool skip_parse = !m.errors.empty() && m.errors[0].lexer && v.mode != 2;
+    size_t total = 0;
+    for (const Error& e : m.errors) {
+        if (!e.lexer && skip_parse) continue;
+        total++;
+        if (!o) continue;
+        if (e.lexer) o->putf("Lexer(start=%llu)\n", (unsigned long long)e.lex_start);
+        else ptxdump::error_line(r, *o, e.w0, e.a, e.b);
+    }
+    if (m.implicit_parser_error) {
+        total++;
+        if (o) o->put("Parser(ContextError)\n");
+    }
+    return total;
+}
+
+inline void print_to(ptxdump::Out& o, const PtxBatchView& v, uint32_t mi, Module& m) {
     Printer p{o};
     ptxdump::Reader r(v, mi);
     static const char* const verdicts[] = {"Ok", "Err", "Module", "Empty", "Errors", "ReferencePanics", "ReferenceDiverges", "SequentialPathRefused"};
     o.putf("mode: %s\nstatus: %s\n", v.mode == 0 ? "checked" : v.mode == 1 ? "unchecked" : "errors", verdicts[m.verdict]);
-    if (m.verdict == V_DIVERGES || m.verdict == V_REFUSED) { o.put("errors: 0\n"); return std::move(o.s); }
+    if (m.verdict == V_DIVERGES || m.verdict == V_REFUSED) { o.put("errors: 0\n"); return; }
     if (m.have_module) {
         uint64_t kept = m.directives.size();
         o.putf("Module { ptx_version: (%u, %u), sm_version: %u, address_size: %u, invalid_directives: %llu, directives: %llu }\n", m.major, m.minor,
@@ -699,23 +761,28 @@ inline std::string print(const PtxBatchView& v, uint32_t mi, const Module& m) {
             }
             if (!f.has_body) { o.put("], body: None })\n"); continue; }
             o.put("], body: Some([\n");
-            p.statements(f.body, 1);
+            if (f.body_rec) p.stream(Builder{r, m}, f.body_rec, f.body_end);
+            else p.statements(f.body, 1);
             o.put("]) })\n");
         }
     } else if (v.mode == 1) {
         o.put("Module { ptx_version: (1, 0), sm_version: 0, address_size: 64, invalid_directives: 18446744073709551615, directives: 0 }\n");
     }
-    const bool skip_parse = !m.errors.empty() && m.errors[0].lexer && v.mode != 2;
-    size_t total = 0;
-    for (const Error& e : m.errors) total += (e.lexer || !skip_parse) ? 1 : 0;
-    if (m.implicit_parser_error) total++;
-    o.putf("errors: %u\n", (unsigned)total);
-    for (const Error& e : m.errors) {
-        if (e.lexer) o.putf("Lexer(start=%llu)\n", (unsigned long long)e.lex_start);
-        else if (!skip_parse) ptxdump::error_line(r, o, e.w0, e.a, e.b);
-    }
-    if (m.implicit_parser_error) o.put("Parser(ContextError)\n");
-    return std::move(o.s);
+    o.putf("errors: %u\n", (unsigned)print_errors(v, r, nullptr, m));
+    print_errors(v, r, &o, m);
+}
+
+inline std::string print(const PtxBatchView& v, uint32_t mi, Module& m) {
+    ptxdump::Out o;
+    print_to(o, v, mi, m);
+    return o.take();
+}
+// the error list alone (a module without a verdict of its own - given up or refused - has none)
+inline void print_error_list(ptxdump::Out& o, const PtxBatchView& v, uint32_t mi) {
+    ptxdump::Reader r(v, mi);
+    Module m;
+    materialize_errors(v, mi, &m);
+    print_errors(v, r, &o, m);
 }
 
 }   // namespace ptxast

@@ -22,9 +22,9 @@
 #include <thread>
 
 // host side (ptxfe_dump.cpp)
-std::string ptxfe_dump_module_impl(const PtxBatchView& v, uint32_t m, int* status);
 uint64_t ptxfe_dump_hash_impl(const PtxBatchView& v, uint32_t m, int* status);
-std::string ptxfe_dump_module_tree_impl(const PtxBatchView& v, uint32_t m, int* status);
+char* ptxfe_dump_module_tree_impl(const PtxBatchView& v, uint32_t m, size_t* len);
+char* ptxfe_error_list_impl(const PtxBatchView& v, uint32_t m, size_t* len);
 uint64_t ptxfe_materialize_impl(const PtxBatchView& v, uint32_t m);
 
 #define CUDA_TRY(call)                                                                      \
@@ -1500,14 +1500,19 @@ static PtxBatchView view_of(const ptxfe_batch* b) {
 int ptxfe_module_dump(const ptxfe_batch* b, uint32_t i, char** out, uint64_t* out_len) {
     PTXFE_ROUTE(b, i, ptxfe_module_dump, out, out_len)
     if (!b || !b->ctx || i >= b->n || !out) return PTXFE_ERR_BAD_ARG;
-    int status = 0;
-    // records -> tree -> text (the hash below walks the records directly: both readers must tell the same story)
-    std::string s = ptxfe_dump_module_tree_impl(view_of(b), i, &status);
-    char* r = (char*)malloc(s.size() + 1);
-    if (!r) return PTXFE_ERR_OOM;
-    memcpy(r, s.data(), s.size() + 1);
-    *out = r;
-    if (out_len) *out_len = s.size();
+    size_t len = 0;
+    // records -> nodes -> text (the hash below walks the records directly: both readers must tell the same story)
+    *out = ptxfe_dump_module_tree_impl(view_of(b), i, &len);
+    if (out_len) *out_len = len;
+    return PTXFE_OK;
+}
+
+int ptxfe_module_errors(const ptxfe_batch* b, uint32_t i, char** out, uint64_t* out_len) {
+    PTXFE_ROUTE(b, i, ptxfe_module_errors, out, out_len)
+    if (!b || !b->ctx || i >= b->n || !out) return PTXFE_ERR_BAD_ARG;
+    size_t len = 0;
+    *out = ptxfe_error_list_impl(view_of(b), i, &len);
+    if (out_len) *out_len = len;
     return PTXFE_OK;
 }
 
