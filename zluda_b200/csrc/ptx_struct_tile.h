@@ -34,6 +34,19 @@ struct PtxStructArgs {
     uint32_t* udepth;             // out: scope depth in front of unit u, bit 31 = first unit of a module
     uint32_t* mub;                // out: first unit of module m (modules with tokens only)
     PtxCounters* counters;        // out: n_units
+    // a backend that numbers the top-level units (depth 0: module headers and directives) in the same pass:
+    uint32_t* udir = nullptr;     // out: ordinal (from 1) of the last top-level unit at or before unit u
+    uint32_t* top_unit = nullptr; // out: the unit that is top-level unit number k + 1
+    uint32_t cap_units = 0xFFFFFFFFu;            // rows of the unit table
+    const uint32_t* n_tokens_dev = nullptr;      // the number of tokens is on the device (n_tokens is a bound)
+    PTX_HD void row(uint32_t u, uint32_t token, uint32_t depth, uint32_t& tops) const {
+        ustart[u] = token;
+        udepth[u] = depth;
+        if (udir) {
+            if ((depth & 0x7FFFFFFFu) == 0) top_unit[tops++] = u;
+            udir[u] = tops;
+        }
+    }
 };
 
 // the scan's operator and what a prefix says about the depth
@@ -240,8 +253,10 @@ PTX_HD inline bool sx_continues(uint16_t prev) {      // a directive keyword beh
 // step 2: with the depth in front of the thread's first token: where units start, as a spread mask; the scope depth
 // behind a module's last token goes to mod_final_scope.
 // Token by token from the kinds; with write set, the rows of the unit table are written as well (step 3).
-PTX_HD inline uint32_t sx_walk(const PtxStructArgs& a, const SxThread& t, int32_t depth, bool write, uint32_t units_before) {
+PTX_HD inline uint32_t sx_walk(const PtxStructArgs& a, const SxThread& t, int32_t depth, bool write, uint32_t units_before, uint32_t tops_before = 0,
+                               uint32_t* n_tops = nullptr) {
     int32_t sd = depth;
+    uint32_t tops = tops_before;
     uint32_t starts = 0, u = units_before;
     if (!t.n_valid) return 0;
     SxWindow win;
@@ -265,9 +280,9 @@ PTX_HD inline uint32_t sx_walk(const PtxStructArgs& a, const SxThread& t, int32_
         }
         if (start) {
             starts |= 1u << sx_pos(k);
+            if (n_tops && sd == 0) ++*n_tops;
             if (write) {
-                a.ustart[u] = j;
-                a.udepth[u] = (sd > 0x7FF0 ? 0x7FF0u : (uint32_t)sd) | (first ? 0x80000000u : 0u);
+                a.row(u, j, (sd > 0x7FF0 ? 0x7FF0u : (uint32_t)sd) | (first ? 0x80000000u : 0u), tops);
                 if (first) a.mub[ptx_upper_bound_u32(a.mtb, a.n_modules, j) - 1] = u;
                 u++;
             }
@@ -317,12 +332,33 @@ PTX_HD inline uint32_t sx_decide(const PtxStructArgs& a, const SxThread& t, int3
     return starts;
 }
 
-// step 3: with the number of unit starts in front of the thread's first token: the rows of the unit table
-PTX_HD inline void sx_write(const PtxStructArgs& a, const SxThread& t, int32_t depth, uint32_t starts, uint32_t units_before) {
+// how many of the starts are top-level units (for backends that number those in the same pass)
+PTX_HD inline uint32_t sx_count_tops(const PtxStructArgs& a, const SxThread& t, int32_t depth, uint32_t starts) {
+    uint32_t tops = 0;
     if (!t.fast) {
-        if (t.n_valid) sx_walk(a, t, depth, true, units_before);
+        sx_walk(a, t, depth, false, 0, 0, &tops);
+        return tops;
+    }
+    const uint32_t plus = t.braces & SX_LOW, minus = (t.braces >> 4) & SX_LOW;
+    if (!starts || depth - (int32_t)sx_popc(minus) > 0) return 0;                          // inside a scope all the way
+    if (depth == 0 && !plus) return sx_popc(starts);                                       // top level all the way
+    int32_t sd = depth;
+#pragma unroll 1
+    for (uint32_t k = 0; k < SX_ITEMS; k++) {
+        const uint32_t pos = sx_pos(k);
+        tops += sd == 0 ? (starts >> pos) & 1u : 0u;
+        sd += (int32_t)((plus >> pos) & 1u) - (int32_t)((minus >> pos) & 1u);
+        if (sd < 0) sd = 0;
+    }
+    return tops;
+}
+// step 3: with the number of unit starts in front of the thread's first token: the rows of the unit table
+PTX_HD inline void sx_write(const PtxStructArgs& a, const SxThread& t, int32_t depth, uint32_t starts, uint32_t units_before, uint32_t tops_before = 0) {
+    if (!t.fast) {
+        if (t.n_valid) sx_walk(a, t, depth, true, units_before, tops_before);
         return;
     }
+    uint32_t tops = tops_before;
     uint32_t u = units_before;
     const uint32_t plus = t.braces & SX_LOW, minus = (t.braces >> 4) & SX_LOW;
     if (depth - (int32_t)sx_popc(minus) >= 0) {
@@ -331,8 +367,7 @@ PTX_HD inline void sx_write(const PtxStructArgs& a, const SxThread& t, int32_t d
             const uint32_t pos = sx_lowest(starts), below = (1u << pos) - 1u;
             starts &= starts - 1u;
             const int32_t sd = depth + (int32_t)sx_popc(plus & below) - (int32_t)sx_popc(minus & below);
-            a.ustart[u] = t.tb + (pos >> 3) * 4u + (pos & 3u);
-            a.udepth[u] = sd > 0x7FF0 ? 0x7FF0u : (uint32_t)sd;
+            a.row(u, t.tb + (pos >> 3) * 4u + (pos & 3u), sd > 0x7FF0 ? 0x7FF0u : (uint32_t)sd, tops);
             u++;
         }
         return;
@@ -342,8 +377,7 @@ PTX_HD inline void sx_write(const PtxStructArgs& a, const SxThread& t, int32_t d
     for (uint32_t k = 0; k < SX_ITEMS; k++) {
         const uint32_t pos = sx_pos(k);
         if ((starts >> pos) & 1u) {
-            a.ustart[u] = t.tb + k;
-            a.udepth[u] = sd > 0x7FF0 ? 0x7FF0u : (uint32_t)sd;
+            a.row(u, t.tb + k, sd > 0x7FF0 ? 0x7FF0u : (uint32_t)sd, tops);
             u++;
         }
         sd += (int32_t)((plus >> pos) & 1u) - (int32_t)((minus >> pos) & 1u);

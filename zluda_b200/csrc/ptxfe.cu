@@ -12,6 +12,7 @@
 #include <atomic>
 #include <string>
 #include <type_traits>
+#include <unordered_map>
 #include <vector>
 
 #define PTX_HD __device__
@@ -37,10 +38,24 @@ uint64_t ptxfe_materialize_impl(const PtxBatchView& v, uint32_t m);
     } while (0)
 
 // ------------------------------------------------------------------------------------------------ kernels
+// How many items a launch has: the host's number, or a bound on it and the number on the device (PtxCount); and the word
+// that stops a slice whose counts outgrew what was prepared for it.
+struct LaunchCount {
+    size_t cap;
+    const uint32_t* dev;
+    const uint32_t* stop;
+    uint32_t plus;
+    __device__ size_t get() const {
+        if (stop && *(const volatile uint32_t*)stop) return 0;
+        if (!dev) return cap;
+        const size_t n = (size_t)*dev + plus;
+        return n < cap ? n : cap;
+    }
+};
 template <class F>
-__global__ void __launch_bounds__(256) pf_kernel(size_t n, F f) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) f(i);
+__global__ void __launch_bounds__(256) pf_kernel(LaunchCount count, F f) {
+    const size_t n = count.get();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) f(i);
 }
 
 // ---- per-chunk lexer steps over a shared-memory tile of the text
@@ -114,7 +129,8 @@ __global__ void __launch_bounds__(256, 8) lex_mark_kernel(PtxLexTileArgs a, uint
         lt_mark_finish(sh, a, tile, tid, 256);
     }
 }
-__global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint32_t n_tiles) {
+__global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint32_t n_tiles, const uint32_t* stop) {
+    if (stop && *(const volatile uint32_t*)stop) return;
     extern __shared__ __align__(16) unsigned char lex_emit_smem[];
     PtxLexEmitShared& sh = *(PtxLexEmitShared*)lex_emit_smem;
     const uint32_t tid = threadIdx.x;
@@ -143,29 +159,29 @@ __global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint
     }
 }
 
-// ---- first decode pass: every thread builds its record in shared memory and copies it to its row of the staging
-// table.  Word k of thread t lives at stage[k * STAGE_STRIDE + t]: threads of a warp decode units of the same shape in
-// lockstep, so they write the same k at the same time (32 consecutive banks).
-#define STAGE_STRIDE 257u
+// ---- decode lists: every active lane builds a record in its share of the block's shared memory.  Word k of slot t lives
+// at stage[k * stride + t]: lanes that decode units of the same shape in lockstep write the same k at the same time.
+// A short list uses few lanes of every warp (down to one): units of different shapes in one warp run one after the other,
+// and what a lone unit waits for is instruction fetches and dependent loads, which other warps of the SM share.  Fewer
+// slots also means longer records and token windows per slot (a function header of eight parameters has 70 words).
+#define STAGE_SLOTS 257u
 #define STAGE_CAP 40u
 #define WIN_CAP 12u
-#define STAGED_SMEM_BYTES (STAGE_CAP * STAGE_STRIDE * 4u + WIN_CAP * STAGE_STRIDE * 8u)
+#define STAGED_SMEM_BYTES (STAGE_CAP * STAGE_SLOTS * 4u + WIN_CAP * STAGE_SLOTS * 8u)
 template <class F>
-__global__ void __launch_bounds__(256) staged_kernel(size_t n, uint32_t* table, uint32_t row_words, F f) {
+__global__ void __launch_bounds__(256) staged_kernel(LaunchCount count, F f) {
     extern __shared__ __align__(16) unsigned char staged_smem[];
-    PtxTokenWord* win = (PtxTokenWord*)staged_smem;                                    // [WIN_CAP][STAGE_STRIDE]
-    uint32_t* stage = (uint32_t*)(staged_smem + WIN_CAP * STAGE_STRIDE * 8u);          // [STAGE_CAP][STAGE_STRIDE]
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    PtxStaged r;
-    r.unit = 0;
-    r.n = 0;
-    if (i < n) r = f(i, PtxScratch{stage + threadIdx.x, STAGE_STRIDE, STAGE_CAP, win + threadIdx.x, STAGE_STRIDE, WIN_CAP});
-    // Every thread copies its own record.  (The copy used to be cooperative, 32 lanes per record behind a __syncwarp and
-    // two __shfl_sync per record.  About one parse in ten of a batch of 3,000 small modules of many shapes, run behind
-    // a large batch, then lost words of a few records: lanes that came late out of long decoders skipped the records of
-    // lanes that were done.  With each thread writing what it staged, 300 such parses in a row come out identical.)
-    uint32_t* row = table + (size_t)r.unit * row_words;
-    for (uint32_t k = 0; k < r.n; k++) row[k] = stage[k * STAGE_STRIDE + threadIdx.x];
+    PtxTokenWord* win = (PtxTokenWord*)staged_smem;
+    uint32_t* stage = (uint32_t*)(staged_smem + WIN_CAP * STAGE_SLOTS * 8u);
+    const uint32_t n = (uint32_t)count.get();
+    const uint32_t warps = gridDim.x * 8u, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t lanes = (n + warps - 1u) / warps;                       // active lanes per warp
+    if (lanes > 32u) lanes = 32u;
+    if (lanes == 0 || lane >= lanes) return;
+    const uint32_t stride = 8u * lanes + 1u, slot = warp * lanes + lane;
+    const PtxScratch scratch{stage + slot, stride, STAGE_CAP * STAGE_SLOTS / stride, win + slot, stride, WIN_CAP * STAGE_SLOTS / stride};
+    // neighbouring entries go to one warp when the lanes are full (they may have the same shape), to different SMs else
+    for (uint32_t i = (blockIdx.x * 8u + warp) * lanes + lane; i < n; i += warps * lanes) f((size_t)i, scratch);
 }
 
 constexpr int SCAN_THREADS = 256;
@@ -227,7 +243,9 @@ __device__ inline void block_scan(T v, Op op, T identity, T* warp_tot, T& incl, 
 // word by word took 16.3 of 19.5 ms of a 41 MB module of constant tables (0.1 ms without them).
 #define SEG_DEFER_CAP 2048u
 #define EMIT_ILP 4
-__global__ void __launch_bounds__(256, 6) emit_records_kernel(uint32_t n_units, const PtxPair* off, PtxEmitStep e) {
+__global__ void __launch_bounds__(256, 6) emit_records_kernel(LaunchCount count, const PtxPair* off, PtxEmitStep e) {
+    const uint32_t n_units = (uint32_t)count.get();
+    if (blockIdx.x * 256u >= n_units) return;
     __shared__ uint32_t so[257];              // words of the units in front of unit k that this kernel writes
     __shared__ PtxEmitUnit su[256];
     __shared__ uint32_t warp_tot[8];
@@ -352,6 +370,112 @@ __global__ void __launch_bounds__(256) repack_text_kernel(uint32_t n_pieces, uin
     ((uint4*)text)[i] = v;
 }
 
+// ---- inclusive scan in one pass.  Tiles are handed out in order by an atomic ticket, so a tile only ever waits for tiles
+// that are running or done; it publishes its aggregate, looks back along the tiles in front of it, 32 at a time, to the
+// nearest known prefix, and publishes its own.  A published word is self-contained: 32 bits of value and the state in the
+// top two bits of 64 (0 nothing yet, 1 the tile's aggregate, 2 the prefix up to and including it); a value of two words
+// counts when both carry the same state.  Waits are bounded: a tile that waits too long sets the abort word, every other
+// waiter sees it and leaves, and the host finds struct_abort among the counters.
+// (As reduce, scan of the tile totals and apply it was three to five launches: 11 us for a few items, 0.35 against 0.27 ms
+// for the 27 million units of a 1 GiB batch.)
+constexpr unsigned long long SXD_AGG = 1ull << 62, SXD_PREFIX = 2ull << 62, SXD_STATE = 3ull << 62;
+constexpr uint32_t SX_WAIT_LIMIT = 1u << 22;
+__device__ inline unsigned long long sx_ld(const unsigned long long* p) { return *(const volatile unsigned long long*)p; }
+__device__ inline void sx_st(unsigned long long* p, unsigned long long v) { *(volatile unsigned long long*)p = v; }
+template <class T> struct ScanDesc {
+    unsigned long long w[sizeof(T) / 4];
+    __device__ void publish(unsigned long long state, T v) {
+        union { T t; uint32_t x[sizeof(T) / 4]; } u;
+        u.t = v;
+#pragma unroll
+        for (size_t i = 0; i < sizeof(T) / 4; i++) sx_st(&w[i], state | u.x[i]);
+    }
+    __device__ unsigned long long look(T& v) const {       // its state, 0 = not there yet
+        union { T t; uint32_t x[sizeof(T) / 4]; } u;
+        unsigned long long q[sizeof(T) / 4];
+#pragma unroll
+        for (size_t i = 0; i < sizeof(T) / 4; i++) q[i] = sx_ld(&w[i]);
+        const unsigned long long state = q[0] & SXD_STATE;
+        bool same = state != 0;
+#pragma unroll
+        for (size_t i = 0; i < sizeof(T) / 4; i++) {
+            same = same && (q[i] & SXD_STATE) == state;
+            u.x[i] = (uint32_t)q[i];
+        }
+        v = u.t;
+        return same ? state : 0ull;
+    }
+};
+template <class T, class Op, class Ld, class St>
+__global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, Ld ld, St st, Op op, T identity, ScanDesc<T>* desc, uint32_t* ctl, uint32_t* aborted) {
+    __shared__ T warp_tot[SCAN_THREADS / 32];
+    __shared__ T s_before;
+    __shared__ uint32_t s_tile, s_ok;
+    const size_t n = count.get();
+    if (threadIdx.x == 0) {
+        s_tile = atomicAdd(&ctl[0], 1u);
+        s_ok = 1;
+    }
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const size_t base = (size_t)tile * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
+    if ((size_t)tile * SCAN_TILE >= n) return;
+    T vals[SCAN_ITEMS];
+    T acc = identity;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; k++) {
+        if (base + k < n) acc = op(acc, ld(base + k));
+        vals[k] = acc;
+    }
+    T incl, excl;
+    block_scan(acc, op, identity, warp_tot, incl, excl);
+    if (threadIdx.x == SCAN_THREADS - 1) s_before = incl;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x;
+        const T agg = s_before;
+        __syncwarp();
+        T before = identity;
+        bool ok = true;
+        if (tile == 0) {
+            if (lane == 0) desc[0].publish(SXD_PREFIX, agg);
+        } else {
+            if (lane == 0) desc[tile].publish(SXD_AGG, agg);
+            for (int64_t back = (int64_t)tile - 1; ok; back -= 32) {
+                const int64_t mine = back - (int64_t)lane;
+                T v = identity;
+                unsigned long long state = SXD_PREFIX;         // in front of tile 0: nothing, and known
+                for (uint32_t spin = 0; mine >= 0; spin++) {
+                    state = desc[mine].look(v);
+                    if (state) break;
+                    if ((spin & 63u) == 63u && *(volatile uint32_t*)&ctl[1]) break;
+                    if (spin >= SX_WAIT_LIMIT) { atomicExch(&ctl[1], 1u); break; }
+                    __nanosleep(20);
+                }
+                if (!__all_sync(0xFFFFFFFFu, state != 0)) { ok = false; break; }
+                const unsigned ends = __ballot_sync(0xFFFFFFFFu, state == SXD_PREFIX);
+                const uint32_t last = ends ? (uint32_t)(__ffs(ends) - 1) : 31u;
+                if (lane > last) v = identity;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {             // ordered: lane 0 ends up with op(v[last], ..., v[1], v[0])
+                    T y = shfl_down_words(v, d);
+                    if (lane + d < 32) v = op(y, v);
+                }
+                before = op(shfl_words(v, 0), before);
+                if (ends) break;
+            }
+            if (ok && lane == 0) desc[tile].publish(SXD_PREFIX, op(before, agg));
+        }
+        if (lane == 0) { s_before = before; if (!ok) { s_ok = 0; *aborted = 1; } }
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    const T prefix = op(s_before, excl);
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; k++)
+        if (base + k < n) st(base + k, op(prefix, vals[k]));
+}
+
 template <class T, class Op, class Ld>
 __global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(size_t n, Ld ld, Op op, T identity, T* partial) {
     __shared__ T warp_tot[SCAN_THREADS / 32];
@@ -397,16 +521,14 @@ struct StructDesc {
     unsigned long long depth0, depth1, count;
     uint32_t has_first, pad;      // has_first: set ahead of the pass (sx_mark_tiles)
 };
-__global__ void structure_mark_kernel(PtxStructArgs a, StructDesc* desc) {
+__global__ void structure_mark_kernel(PtxStructArgs a, StructDesc* desc, const uint32_t* stop) {
+    if (stop && *(const volatile uint32_t*)stop) return;
+    if (a.n_tokens_dev) a.n_tokens = *a.n_tokens_dev;
     uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m < a.n_modules) sx_mark_tiles(a, m, &desc[0].has_first, (uint32_t)(sizeof(StructDesc) / 4));
 }
-constexpr unsigned long long SXD_AGG = 1ull << 62, SXD_PREFIX = 2ull << 62, SXD_STATE = 3ull << 62;
-constexpr uint32_t SX_WAIT_LIMIT = 1u << 22;
 constexpr int SX_DEPTH_PER_LANE = 1, SX_COUNT_PER_LANE = 1;     // tiles a lane of the look-back reads per trip to memory
 
-__device__ inline unsigned long long sx_ld(const unsigned long long* p) { return *(const volatile unsigned long long*)p; }
-__device__ inline void sx_st(unsigned long long* p, unsigned long long v) { *(volatile unsigned long long*)p = v; }
 __device__ inline void sx_publish_depth(StructDesc* d, unsigned long long state, PtxSeg3 v) {
     sx_st(&d->depth0, state | ((unsigned long long)(v.flag ? 1u : 0u) << 32) | (uint32_t)v.scope);
     sx_st(&d->depth1, state | (uint32_t)v.paren);
@@ -427,20 +549,24 @@ __device__ inline bool sx_read_depth(const StructDesc* d, uint32_t* ctl, unsigne
         __nanosleep(20);
     }
 }
-__device__ inline bool sx_read_count(const StructDesc* d, uint32_t* ctl, unsigned long long& state, uint32_t& v) {
+// unit count in bits 0..31, top-level units in bits 32..61
+__device__ inline bool sx_read_count(const StructDesc* d, uint32_t* ctl, unsigned long long& state, unsigned long long& v) {
     for (uint32_t spin = 0;; spin++) {
         unsigned long long a = sx_ld(&d->count);
-        if (a & SXD_STATE) { state = a & SXD_STATE; v = (uint32_t)a; return true; }
+        if (a & SXD_STATE) { state = a & SXD_STATE; v = a & ~SXD_STATE; return true; }
         if ((spin & 63u) == 63u && *(volatile uint32_t*)&ctl[1]) return false;
         if (spin >= SX_WAIT_LIMIT) { atomicExch(&ctl[1], 1u); return false; }
         __nanosleep(20);
     }
 }
 
-__global__ void __launch_bounds__(SX_THREADS) structure_kernel(PtxStructArgs a, uint32_t n_tiles, StructDesc* desc, uint32_t* ctl) {
+__global__ void __launch_bounds__(SX_THREADS) structure_kernel(PtxStructArgs a, StructDesc* desc, uint32_t* ctl, const uint32_t* stop) {
+    if (stop && *(const volatile uint32_t*)stop) return;
+    if (a.n_tokens_dev) a.n_tokens = *a.n_tokens_dev;
+    const uint32_t n_tiles = (uint32_t)(((uint64_t)a.n_tokens + SX_TILE - 1) / SX_TILE);
     __shared__ PtxSeg3 warp_depth[SX_THREADS / 32];
     __shared__ uint32_t warp_count[SX_THREADS / 32];
-    __shared__ uint32_t s_tile, s_has_first, s_units_before, s_ok;
+    __shared__ uint32_t s_tile, s_has_first, s_units_before, s_tops_before, s_tile_units, s_ok;
     __shared__ PtxSeg3 s_before;
     __shared__ uint8_t s_table[512];
     const int lane = threadIdx.x & 31;
@@ -527,14 +653,15 @@ __global__ void __launch_bounds__(SX_THREADS) structure_kernel(PtxStructArgs a, 
         }
         const int32_t before = sx_depth(op(s_before, excl));
         const uint32_t starts = sx_decide(a, t, before);
+        // units in the low half, top-level units in the high half (at most 4,096 of each)
         uint32_t cincl, cexcl;
-        block_scan((uint32_t)__popc(starts), AddOp(), 0u, warp_count, cincl, cexcl);
+        block_scan((uint32_t)__popc(starts) | (sx_count_tops(a, t, before, starts) << 16), AddOp(), 0u, warp_count, cincl, cexcl);
         if (threadIdx.x == SX_THREADS - 1) s_units_before = cincl;
         __syncthreads();
         if (threadIdx.x < 32) {
-            const uint32_t agg = s_units_before;
+            const unsigned long long agg = (unsigned long long)(s_units_before & 0xFFFFu) | ((unsigned long long)(s_units_before >> 16) << 32);
             __syncwarp();
-            uint32_t before = 0;
+            unsigned long long before = 0;
             bool ok = true;
             if (tile == 0) {
                 if (lane == 0) sx_st(&desc[0].count, SXD_PREFIX | agg);
@@ -545,14 +672,14 @@ __global__ void __launch_bounds__(SX_THREADS) structure_kernel(PtxStructArgs a, 
                     unsigned long long w[SX_COUNT_PER_LANE];
 #pragma unroll
                     for (int r = 0; r < SX_COUNT_PER_LANE; r++) w[r] = mine - r >= 0 ? sx_ld(&desc[mine - r].count) : 0ull;
-                    uint32_t v = 0;
+                    unsigned long long v = 0;
                     bool done = false, got = true;
 #pragma unroll
                     for (int r = 0; r < SX_COUNT_PER_LANE; r++) {
                         if (done || !got) continue;
                         if (mine - r < 0) { done = true; continue; }
                         unsigned long long state = w[r] & SXD_STATE;
-                        uint32_t x = (uint32_t)w[r];
+                        unsigned long long x = w[r] & ~SXD_STATE;
                         if (!state) got = sx_read_count(&desc[mine - r], ctl, state, x);
                         if (!got) continue;
                         v += x;
@@ -562,20 +689,30 @@ __global__ void __launch_bounds__(SX_THREADS) structure_kernel(PtxStructArgs a, 
                     unsigned ends = __ballot_sync(0xFFFFFFFFu, done);
                     int last = ends ? __ffs(ends) - 1 : 31;
                     if (lane > last) v = 0;
-                    before += __reduce_add_sync(0xFFFFFFFFu, v);
+                    before += (unsigned long long)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)v) |
+                              ((unsigned long long)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)(v >> 32)) << 32);
                     if (ends) break;
                     back -= 32 * SX_COUNT_PER_LANE;
                 }
-                if (ok && lane == 0) sx_st(&desc[tile].count, SXD_PREFIX | (uint32_t)(before + agg));
+                if (ok && lane == 0) sx_st(&desc[tile].count, SXD_PREFIX | (before + agg));
             }
-            if (lane == 0) { s_units_before = before; if (!ok) s_ok = 0; }
+            if (lane == 0) {
+                s_units_before = (uint32_t)before;
+                s_tops_before = (uint32_t)(before >> 32);
+                s_tile_units = (uint32_t)agg;
+                if (!ok) s_ok = 0;
+            }
         }
         __syncthreads();
         if (!s_ok) {
             if (threadIdx.x == 0) a.counters->struct_abort = 1;
             return;
         }
-        sx_write(a, t, before, starts, s_units_before + cexcl);
+        if ((uint64_t)s_units_before + s_tile_units > a.cap_units) {         // more units than the table has room for
+            if (threadIdx.x == 0) PTX_REDO_SET(a.counters, PTX_REDO_UNITS);
+            continue;
+        }
+        sx_write(a, t, before, starts, s_units_before + (cexcl & 0xFFFFu), s_tops_before + (cexcl >> 16));
     }
 }
 
@@ -698,7 +835,6 @@ struct ptxfe_ctx {
     // staged batch
     std::vector<const char*> texts;
     std::vector<PtxModuleLayout> layout;
-    std::vector<uint32_t> mcb;
     uint64_t text_bytes = 0, padded_bytes = 0;
     uint8_t* d_text = nullptr;
     size_t d_text_cap = 0;
@@ -706,8 +842,14 @@ struct ptxfe_ctx {
     PtxLexTables* d_lex_tables = nullptr; // constant tables of the lexer steps (filled at the first parse)
     uint8_t* d_raw = nullptr;             // host-contiguous runs land here before they are repacked into d_text
     size_t d_raw_cap = 0;
-    PtxWork work;
-    PtxCounters counters;
+    PtxWork works[2];                     // one per arena
+    PtxCounters counters;                 // of the slice that finished last
+    std::unordered_map<const void*, unsigned> resident;      // persistent kernels: blocks that the device holds
+    char* h_meta = nullptr; size_t h_meta_cap = 0;           // pinned: layouts of all slices, as they go to the device
+    char* d_meta = nullptr; size_t d_meta_cap = 0;
+    // What deferred counts prepare for, per byte of text: a little more than the batches so far had (the first guess is
+    // above what real modules have).  A slice beyond it costs a second run, nothing else.
+    double tokens_per_byte = 0.36, units_per_byte = 0.05, words_per_byte = 0.44;
     bool staged = false, ran = false;
     uint32_t mode = 0;
     // pinned result buffers
@@ -728,7 +870,24 @@ struct ptxfe_ctx {
 };
 
 struct CudaBackend {
+    static constexpr bool kStructureTops = true;
     ptxfe_ctx* ctx;
+    const uint32_t* stop = nullptr;        // deferred counts: the word that stops the slice (PtxCounters::redo)
+    uint32_t* aborted = nullptr;           // where a look-back that gave up says so
+    char* zero_base = nullptr;             // a region cleared ahead of the first step, handed out by zalloc
+    size_t zero_size = 0, zero_used = 0;
+    LaunchCount count_of(PtxCount n) const { return LaunchCount{n.cap, n.dev, n.always ? nullptr : stop, n.plus}; }
+    void* zalloc(size_t bytes) {
+        bytes = (bytes + 15) & ~(size_t)15;
+        if (zero_used + bytes <= zero_size) {
+            void* p = zero_base + zero_used;
+            zero_used += bytes;
+            return p;
+        }
+        void* p = alloc(bytes);
+        zero(p, bytes);
+        return p;
+    }
     void* alloc(size_t bytes) {
         bytes = (bytes + 255) & ~(size_t)255;
         for (ArenaBlock& b : ctx->arenas[ctx->cur])
@@ -790,11 +949,14 @@ struct CudaBackend {
         if (!ctx->profile) return;
         cudaEventRecord(ctx->prof_events[ctx->prof_used++], ctx->stream);
     }
-    template <class F> void pf(const char* name, size_t n, F f) {
-        if (ctx->failed || n == 0) return;
-        size_t blocks = (n + 255) / 256;
+    template <class F> void pf(const char* name, PtxCount n, F f) {
+        if (ctx->failed || n.cap == 0) return;
+        // with the count on the device the grid covers a bound that may lie well above it: no more blocks than fill the
+        // GPU a few times over, each taking several rounds
+        size_t blocks = (n.cap + 255) / 256;
+        if (n.dev && blocks > 148 * 64) blocks = 148 * 64;
         prof_begin(name);
-        pf_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(n, f);
+        pf_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(count_of(n), f);
         prof_end();
         ctx->launches++;
     }
@@ -816,19 +978,18 @@ struct CudaBackend {
         }
         return cs;
     }
-    template <class F> void pf_staged(const char* name, size_t n, uint32_t* table, uint32_t row_words, F f) {
-        if (ctx->failed || n == 0) return;
+    template <class F> void pf_staged(const char* name, PtxCount n, uint32_t*, uint32_t, F f) {
+        if (ctx->failed || n.cap == 0) return;
         prof_begin(name);
-        // more shared memory than a kernel gets by default: opt in (cheap, so done at every launch)
-        cudaFuncSetAttribute(staged_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STAGED_SMEM_BYTES);
-        staged_kernel<<<(unsigned)((n + 255) / 256), 256, STAGED_SMEM_BYTES, ctx->stream>>>(n, table, row_words, f);
+        // as many blocks as the device holds, or one list entry per warp
+        staged_kernel<<<resident_blocks((const void*)staged_kernel<F>, STAGED_SMEM_BYTES, (n.cap + 7) / 8), 256, STAGED_SMEM_BYTES, ctx->stream>>>(count_of(n), f);
         prof_end();
         ctx->launches++;
     }
-    void emit_records(const char* name, size_t n, const PtxPair* off, const PtxEmitStep& e) {
-        if (ctx->failed || n == 0) return;
+    void emit_records(const char* name, PtxCount n, const PtxPair* off, const PtxEmitStep& e) {
+        if (ctx->failed || n.cap == 0) return;
         prof_begin(name);
-        emit_records_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>((uint32_t)n, off, e);
+        emit_records_kernel<<<(unsigned)((n.cap + 255) / 256), 256, 0, ctx->stream>>>(count_of(n), off, e);
         prof_end();
         ctx->launches++;
     }
@@ -860,13 +1021,18 @@ struct CudaBackend {
         }
         return ctx->d_lex_tables;
     }
-    // persistent grids: as many blocks as the device holds at once
-    unsigned resident_blocks(const void* kernel, size_t smem, size_t n_tiles) {
-        int per_sm = 0, sms = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-        size_t g = (size_t)(per_sm > 0 ? per_sm : 1) * (size_t)(sms > 0 ? sms : 1);
-        return (unsigned)(g < n_tiles ? g : n_tiles);
+    // persistent grids: as many blocks as the device holds at once (looked up, and the shared memory opted into, once per
+    // kernel and context)
+    unsigned resident_blocks(const void* kernel, size_t smem, size_t n_blocks) {
+        unsigned& g = ctx->resident[kernel];
+        if (!g) {
+            int per_sm = 0, sms = 0;
+            if (smem > 48u << 10) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+            g = (unsigned)(per_sm > 0 ? per_sm : 1) * (unsigned)(sms > 0 ? sms : 1);
+        }
+        return (unsigned)(g < n_blocks ? g : n_blocks);
     }
     void lex_mark(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
@@ -878,8 +1044,7 @@ struct CudaBackend {
     void lex_emit(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
         prof_begin(name);
-        cudaFuncSetAttribute(lex_emit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtxLexEmitShared));
-        lex_emit_kernel<<<resident_blocks((const void*)lex_emit_kernel, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), ctx->stream>>>(a, (uint32_t)n_tiles);
+        lex_emit_kernel<<<resident_blocks((const void*)lex_emit_kernel, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), ctx->stream>>>(a, (uint32_t)n_tiles, stop);
         prof_end();
         ctx->launches++;
     }
@@ -890,16 +1055,14 @@ struct CudaBackend {
     void structure(const char* name, const PtxStructArgs& a) {
         if (ctx->failed || a.n_tokens == 0) return;
         const size_t n_tiles = ((size_t)a.n_tokens + SX_TILE - 1) / SX_TILE;
-        StructDesc* desc = (StructDesc*)alloc(sizeof(StructDesc) * n_tiles + 256);
+        StructDesc* desc = (StructDesc*)zalloc(sizeof(StructDesc) * n_tiles + 256);
         if (!desc) return;
         uint32_t* ctl = (uint32_t*)(desc + n_tiles);      // [0] next tile, [1] abort
         prof_begin(name);
-        cudaMemsetAsync(desc, 0, sizeof(StructDesc) * n_tiles + 256, ctx->stream);
-        structure_mark_kernel<<<(a.n_modules + 255) / 256, 256, 0, ctx->stream>>>(a, desc);
-        const unsigned grid = resident_blocks((const void*)structure_kernel, 0, n_tiles);
-        structure_kernel<<<grid, SX_THREADS, 0, ctx->stream>>>(a, (uint32_t)n_tiles, desc, ctl);
+        structure_mark_kernel<<<(a.n_modules + 255) / 256, 256, 0, ctx->stream>>>(a, desc, stop);
+        structure_kernel<<<resident_blocks((const void*)structure_kernel, 0, n_tiles), SX_THREADS, 0, ctx->stream>>>(a, desc, ctl, stop);
         prof_end();
-        ctx->launches++;
+        ctx->launches += 2;
     }
     void sort_by_key(const char* name, size_t n, const uint16_t* key, uint32_t* order) {
         if (ctx->failed || n == 0) return;
@@ -915,29 +1078,23 @@ struct CudaBackend {
         ArrayLoad<uint32_t> ld{hist};
         ArrayStore<uint32_t> st{begin};
         scan_impl<uint32_t>((size_t)PTX_SORT_BUCKETS, ld, st, AddOp(), 0u);   // inclusive into begin[]
-        pf_kernel<<<(PTX_SORT_BUCKETS + 255) / 256, 256, 0, ctx->stream>>>((size_t)PTX_SORT_BUCKETS, SubtractOwn{begin, hist});
+        pf_kernel<<<(PTX_SORT_BUCKETS + 255) / 256, 256, 0, ctx->stream>>>(LaunchCount{PTX_SORT_BUCKETS, nullptr, nullptr, 0}, SubtractOwn{begin, hist});
         sort_scatter_kernel<<<(unsigned)blocks, SORT_THREADS, 0, ctx->stream>>>(n, key, begin, cursor, order);
         prof_end();
         ctx->launches += 3;
     }
-    template <class T, class Ld, class St, class Op> void scan(const char* name, size_t n, Ld ld, St st, Op op, T identity) {
-        if (ctx->failed || n == 0) return;
+    template <class T, class Ld, class St, class Op> void scan(const char* name, PtxCount n, Ld ld, St st, Op op, T identity) {
+        if (ctx->failed || n.cap == 0) return;
         prof_begin(name);
         scan_impl<T>(n, ld, st, op, identity);
         prof_end();
     }
-    template <class T, class Ld, class St, class Op> void scan_impl(size_t n, Ld ld, St st, Op op, T identity) {
-        if (ctx->failed || n == 0) return;
-        size_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-        T* partial = (T*)alloc(sizeof(T) * (tiles + 1));
-        if (!partial) return;
-        scan_reduce_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(n, ld, op, identity, partial);
-        ctx->launches++;
-        if (tiles > 1) {
-            // scan the tile totals in place (recursively)
-            scan_impl<T>(tiles, ArrayLoad<T>{partial}, ArrayStore<T>{partial}, op, identity);
-        }
-        scan_apply_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(n, ld, st, op, identity, partial);
+    template <class T, class Ld, class St, class Op> void scan_impl(PtxCount n, Ld ld, St st, Op op, T identity) {
+        const size_t tiles = (n.cap + SCAN_TILE - 1) / SCAN_TILE;
+        ScanDesc<T>* desc = (ScanDesc<T>*)zalloc(sizeof(ScanDesc<T>) * tiles + 16);
+        if (!desc) return;
+        uint32_t* ctl = (uint32_t*)(desc + tiles);         // [0] next tile, [1] abort
+        scan_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(count_of(n), ld, st, op, identity, desc, ctl, aborted);
         ctx->launches++;
     }
 };
@@ -997,6 +1154,8 @@ void ptxfe_destroy(ptxfe_ctx* ctx) {
     if (ctx->s_out) cudaStreamDestroy(ctx->s_out);
     if (ctx->d_text) cudaFree(ctx->d_text);
     if (ctx->d_raw) cudaFree(ctx->d_raw);
+    if (ctx->d_meta) cudaFree(ctx->d_meta);
+    if (ctx->h_meta) cudaFreeHost(ctx->h_meta);
     if (ctx->d_class_store) cudaFree(ctx->d_class_store);
     if (ctx->d_lex_tables) cudaFree(ctx->d_lex_tables);
     if (ctx->h_words) cudaFreeHost(ctx->h_words);
@@ -1042,6 +1201,42 @@ static int ensure_text(ptxfe_ctx* ctx, uint64_t bytes) {
     return PTXFE_OK;
 }
 
+// What a slice's kernels know of its modules: layouts, where the modules lie in the raw copy (if the text came as one), and
+// the first chunk of every module.  All slices of a call sit in one pinned buffer and travel in one copy ahead of the text:
+// copies of their own from pageable memory, three per slice in the kernels' stream, each waited behind the text copies
+// that were queued on the same engine.
+static size_t meta_bytes(uint32_t n) {
+    return ((sizeof(PtxModuleLayout) + sizeof(RepackModule)) * (size_t)n + sizeof(uint32_t) * ((size_t)n + 1) + 255) & ~(size_t)255;
+}
+static int grow_pinned(ptxfe_ctx* ctx, void** p, size_t* cap, size_t need, size_t keep);
+static int ensure_meta(ptxfe_ctx* ctx, size_t bytes) {
+    int st = grow_pinned(ctx, (void**)&ctx->h_meta, &ctx->h_meta_cap, bytes, 0);
+    if (st != PTXFE_OK) return st;
+    if (bytes > ctx->d_meta_cap) {
+        if (ctx->d_meta) cudaFree(ctx->d_meta);
+        ctx->d_meta = nullptr;
+        ctx->d_meta_cap = 0;
+        const size_t cap = bytes + bytes / 4 + 4096;
+        CUDA_TRY(cudaMalloc((void**)&ctx->d_meta, cap));
+        ctx->d_meta_cap = cap;
+    }
+    return PTXFE_OK;
+}
+static void write_meta(ptxfe_ctx* ctx, size_t at, uint32_t m0, uint32_t m1, const RepackModule* repack) {
+    const uint32_t n = m1 - m0;
+    PtxModuleLayout* l = (PtxModuleLayout*)(ctx->h_meta + at);
+    RepackModule* r = (RepackModule*)(l + n);
+    uint32_t* mcb = (uint32_t*)(r + n);
+    uint32_t chunks = 0;
+    for (uint32_t m = 0; m < n; m++) {
+        l[m] = ctx->layout[m0 + m];
+        if (repack) r[m] = repack[m0 + m];
+        mcb[m] = l[m].chunk_begin;
+        chunks = l[m].chunk_begin + (uint32_t)((l[m].text_len + PTX_CHUNK - 1) / PTX_CHUNK);
+    }
+    mcb[n] = chunks;
+}
+
 int ptxfe_stage(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, uint32_t n) {
     if (!ctx || (n && (!texts || !lens))) return PTXFE_ERR_BAD_ARG;
     CUDA_TRY(cudaSetDevice(ctx->device));
@@ -1061,6 +1256,9 @@ int ptxfe_stage(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, 
     for (uint32_t m = 0; m < n; m++)
         if (lens[m])
             CUDA_TRY(cudaMemcpyAsync(ctx->d_text + ctx->layout[m].text_off, texts[m], lens[m], cudaMemcpyHostToDevice, ctx->stream));
+    if ((st = ensure_meta(ctx, meta_bytes(n))) != PTXFE_OK) return st;
+    write_meta(ctx, 0, 0, n, nullptr);
+    CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_bytes(n), cudaMemcpyHostToDevice, ctx->stream));
     CUDA_TRY(cudaEventRecord(ctx->ev[1], ctx->stream));
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     CUDA_TRY(cudaEventElapsedTime(&ctx->stats.h2d_ms, ctx->ev[0], ctx->ev[1]));
@@ -1071,53 +1269,97 @@ int ptxfe_stage(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, 
     return PTXFE_OK;
 }
 
-// The three stages over one slice: `text` is the slice's text on the device, `layout` its n module layouts (host).
-// Uses the current arena; leaves the device results in ctx->work and the totals in ctx->counters.  Returns after
-// the kernels have finished.
-static int run_pipeline(ptxfe_ctx* ctx, uint8_t* text, const PtxModuleLayout* layout, uint32_t n, uint32_t mode,
-                        cudaEvent_t ev_begin, cudaEvent_t ev_lex, cudaEvent_t ev_structure, cudaEvent_t ev_end,
-                        const RepackModule* repack = nullptr, const uint8_t* raw = nullptr, bool first_slice = true) {
-    CudaBackend bk{ctx};
+// One slice on its way through the pipeline.
+struct SliceRun {
+    uint8_t* text = nullptr;              // the slice's text on the device
+    size_t meta = 0;                      // where its layouts lie in the metadata buffer
+    uint32_t n = 0, mode = 0;
+    const uint8_t* raw = nullptr;         // text that came as one run of host memory: the first kernel moves it to its slots
+    bool first = true;                    // empties the class store
+    int arena = 0;
+    bool deferred = false;
+    PtxModuleResult* results_out = nullptr;      // pinned host memory the module rows are written to (else they stay on the device)
+    uint32_t* words_out = nullptr;               // pinned host memory the records are written to, words_out_cap words of it
+    uint32_t words_out_cap = 0;
+    cudaEvent_t ev_begin = nullptr, ev_lex = nullptr, ev_structure = nullptr, ev_end = nullptr;
+};
+// Up to this much text in one slice, the last kernels write records straight into the pinned result buffer.
+#define PTXFE_DIRECT_OUT_BYTES (1u << 20)
+#define PTXFE_COUNTERS_SLOT(ctx, arena) ((PtxCounters*)((char*)(ctx)->h_counters + 2048 + 512 * (arena)))
+
+// capacities of a slice that runs with deferred counts: `bytes` of padded text
+static void deferred_caps(const ptxfe_ctx* ctx, uint64_t bytes, PtxWork& w) {
+    auto cap = [&](double per_byte, uint64_t least, uint64_t most) -> uint32_t {
+        uint64_t c = (uint64_t)((double)bytes * per_byte) + 64;
+        if (c < least) c = least;
+        if (c > most) c = most;
+        return (uint32_t)(c < 0xFFFFFF00ull ? c : 0xFFFFFF00ull);
+    };
+    w.cap_tokens = cap(ctx->tokens_per_byte, 4096, bytes);
+    w.cap_units = cap(ctx->units_per_byte, 4096, w.cap_tokens);
+    w.cap_words = cap(ctx->words_per_byte, 16384, 0xFFFFFF00ull);
+    w.cap_list = w.cap_units < PTX_SORT_MIN ? w.cap_units : PTX_SORT_MIN;
+}
+
+// working memory and parameters of a slice, in the current arena
+static int begin_slice(CudaBackend& bk, SliceRun& sl, bool deferred) {
+    ptxfe_ctx* ctx = bk.ctx;
     bk.reset();
-    ctx->mcb.resize((size_t)n + 1);
-    uint32_t chunks = 0;
-    for (uint32_t m = 0; m < n; m++) {
-        ctx->mcb[m] = layout[m].chunk_begin;
-        chunks = layout[m].chunk_begin + (uint32_t)((layout[m].text_len + PTX_CHUNK - 1) / PTX_CHUNK);
-    }
-    ctx->mcb[n] = chunks;
-    PtxWork& w = ctx->work;
+    const uint32_t n = sl.n;
+    PtxWork& w = ctx->works[ctx->cur];
     w = PtxWork();
-    w.first_slice = first_slice;
+    w.deferred = deferred;
+    w.first_slice = sl.first;
     if (const char* e = getenv("PTXFE_SEQ_MAX_TOKENS")) w.seq_max_tokens = (uint32_t)strtoul(e, nullptr, 10);
-    w.text = text;
+    w.text = sl.text;
     w.n_modules = n;
-    w.n_chunks = chunks;
-    w.layout = (PtxModuleLayout*)bk.alloc(sizeof(PtxModuleLayout) * ((size_t)n + 1));
-    w.mod_chunk_begin = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n + 2));
+    const size_t mcb_at = sl.meta + (sizeof(PtxModuleLayout) + sizeof(RepackModule)) * (size_t)n;
+    w.n_chunks = ((const uint32_t*)(ctx->h_meta + mcb_at))[n];
+    w.layout = (PtxModuleLayout*)(ctx->d_meta + sl.meta);
+    w.mod_chunk_begin = (uint32_t*)(ctx->d_meta + mcb_at);
+    if (deferred) deferred_caps(ctx, (uint64_t)w.n_chunks * PTX_CHUNK, w);
+    // everything that the steps want cleared, in one go: per-module words, look-back descriptors, the counters
+    const size_t zero = 8192 + 48 * ((size_t)n + 2) + 24 * ((size_t)w.n_chunks / SCAN_TILE + 2) + 16 * ((size_t)w.cap_units / SCAN_TILE + 2) +
+                        sizeof(StructDesc) * ((size_t)w.cap_tokens / SX_TILE + 2);
+    bk.zero_base = (char*)bk.alloc(zero);
+    bk.zero_size = bk.zero_base ? zero : 0;
+    bk.zero_used = 0;
     w.results = (PtxModuleResult*)bk.alloc(sizeof(PtxModuleResult) * ((size_t)n + 1));
-    w.counters = (PtxCounters*)bk.alloc(sizeof(PtxCounters));
     if (ctx->failed) return PTXFE_ERR_OOM;
-    CUDA_TRY(cudaEventRecord(ev_begin, ctx->stream));
-    if (n) CUDA_TRY(cudaMemcpyAsync(w.layout, layout, sizeof(PtxModuleLayout) * n, cudaMemcpyHostToDevice, ctx->stream));
-    CUDA_TRY(cudaMemcpyAsync(w.mod_chunk_begin, ctx->mcb.data(), sizeof(uint32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, ctx->stream));
-    CUDA_TRY(cudaMemsetAsync(w.counters, 0, sizeof(PtxCounters), ctx->stream));
-    // layout and mcb are pageable host memory: the copies above have consumed them when the calls return
-    if (repack && chunks) {
-        RepackModule* d_mods = (RepackModule*)bk.alloc(sizeof(RepackModule) * (size_t)n);
-        if (ctx->failed) return PTXFE_ERR_OOM;
-        CUDA_TRY(cudaMemcpyAsync(d_mods, repack, sizeof(RepackModule) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
-        uint32_t pieces = chunks * (PTX_CHUNK / 16);
-        repack_text_kernel<<<(pieces + 255) / 256, 256, 0, ctx->stream>>>(pieces, n, d_mods, w.mod_chunk_begin, raw, text);
+    CUDA_TRY(cudaMemsetAsync(bk.zero_base, 0, zero, ctx->stream));
+    w.counters = (PtxCounters*)bk.zalloc(sizeof(PtxCounters));
+    bk.stop = deferred ? &w.counters->redo : nullptr;
+    bk.aborted = &w.counters->struct_abort;
+    w.results_out = sl.results_out;
+    w.counters_out = deferred ? (PtxCounters*)((char*)ctx->d_counters_mapped + ((char*)PTXFE_COUNTERS_SLOT(ctx, ctx->cur) - (char*)ctx->h_counters)) : nullptr;
+    return PTXFE_OK;
+}
+static int run_steps(CudaBackend& bk, SliceRun& sl) {
+    ptxfe_ctx* ctx = bk.ctx;
+    PtxWork& w = ctx->works[ctx->cur];
+    if (sl.raw && w.n_chunks) {
+        const uint32_t pieces = w.n_chunks * (PTX_CHUNK / 16);
+        repack_text_kernel<<<(pieces + 255) / 256, 256, 0, ctx->stream>>>(pieces, sl.n, (const RepackModule*)(ctx->d_meta + sl.meta + sizeof(PtxModuleLayout) * (size_t)sl.n),
+                                                                       w.mod_chunk_begin, sl.raw, sl.text);
         ctx->launches++;
     }
     memset(&ctx->counters, 0, sizeof ctx->counters);
     ptx_stage_lex(bk, w, ctx->counters);
-    if (ev_lex) CUDA_TRY(cudaEventRecord(ev_lex, ctx->stream));
-    if (!ctx->failed) ptx_stage_structure(bk, w, ctx->counters, mode);
-    if (ev_structure) CUDA_TRY(cudaEventRecord(ev_structure, ctx->stream));
+    if (sl.ev_lex) CUDA_TRY(cudaEventRecord(sl.ev_lex, ctx->stream));
+    if (!ctx->failed) ptx_stage_structure(bk, w, ctx->counters, sl.mode);
+    if (sl.ev_structure) CUDA_TRY(cudaEventRecord(sl.ev_structure, ctx->stream));
     if (!ctx->failed) ptx_stage_decode(bk, w, ctx->counters);
-    CUDA_TRY(cudaEventRecord(ev_end, ctx->stream));
+    CUDA_TRY(cudaEventRecord(sl.ev_end, ctx->stream));
+    return PTXFE_OK;
+}
+// the slice with the host reading the counts on the way; returns when its kernels have finished
+static int run_exact(ptxfe_ctx* ctx, SliceRun& sl) {
+    ctx->cur = sl.arena;
+    sl.deferred = false;
+    CudaBackend bk{ctx};
+    int st = begin_slice(bk, sl, false);
+    if (st == PTXFE_OK) st = run_steps(bk, sl);
+    if (st != PTXFE_OK) return st;
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1125,6 +1367,76 @@ static int run_pipeline(ptxfe_ctx* ctx, uint8_t* text, const PtxModuleLayout* la
         return PTXFE_ERR_CUDA;
     }
     if (ctx->failed) return strstr(ctx->err, "cudaMalloc") ? PTXFE_ERR_OOM : PTXFE_ERR_CUDA;
+    return PTXFE_OK;
+}
+// Puts the whole slice into the stream without waiting for any of it (deferred counts); finish_slice waits.
+static int enqueue_slice(ptxfe_ctx* ctx, SliceRun& sl) {
+    sl.arena = ctx->cur;
+    CUDA_TRY(cudaEventRecord(sl.ev_begin, ctx->stream));
+    const uint32_t n_chunks = ((const uint32_t*)(ctx->h_meta + sl.meta + (sizeof(PtxModuleLayout) + sizeof(RepackModule)) * (size_t)sl.n))[sl.n];
+    if (n_chunks == 0) return run_exact(ctx, sl);
+    sl.deferred = true;
+    CudaBackend bk{ctx};
+    int st = begin_slice(bk, sl, true);
+    if (st != PTXFE_OK) return st;
+    PtxWork& w = ctx->works[ctx->cur];
+    if (sl.words_out) {
+        w.words = sl.words_out;
+        if (w.cap_words > sl.words_out_cap) w.cap_words = sl.words_out_cap;
+    } else {
+        w.words = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)w.cap_words + 4));
+    }
+    if (!ctx->failed) st = run_steps(bk, sl);
+    if (ctx->failed) return PTXFE_ERR_OOM;
+    return st;
+}
+// Waits for the slice; what its counters ask for is done here: a second round (lexer errors, damaged modules, units of the
+// second decode pass), or the whole slice again.  Leaves the totals in ctx->counters, the arrays in ctx->works[arena].
+static int finish_slice(ptxfe_ctx* ctx, SliceRun& sl) {
+    PtxWork& w = ctx->works[sl.arena];
+    if (sl.deferred) {
+        cudaError_t e = cudaEventSynchronize(sl.ev_end);
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e != cudaSuccess) {
+            snprintf(ctx->err, sizeof ctx->err, "pipeline failed: %s", cudaGetErrorString(e));
+            return PTXFE_ERR_CUDA;
+        }
+        ctx->counters = *PTXFE_COUNTERS_SLOT(ctx, sl.arena);
+        if (ctx->counters.struct_abort) {
+            snprintf(ctx->err, sizeof ctx->err, "a scan gave up waiting for an earlier tile");
+            return PTXFE_ERR_CUDA;
+        }
+        if (ctx->counters.redo && !(ctx->counters.redo & ~PTX_REDO_DECODE)) {
+            // tokens and units stand: the decode stage alone, with the host reading its counts
+            ctx->cur = sl.arena;
+            CudaBackend bk{ctx};
+            bk.aborted = &w.counters->struct_abort;
+            w.first_slice = true;
+            ptx_stage_decode_anew(bk, w, ctx->counters);
+            CUDA_TRY(cudaEventRecord(sl.ev_end, ctx->stream));
+            CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            if (ctx->failed) return strstr(ctx->err, "cudaMalloc") ? PTXFE_ERR_OOM : PTXFE_ERR_CUDA;
+        } else if (ctx->counters.redo) {
+            sl.first = true;
+            int st = run_exact(ctx, sl);
+            if (st != PTXFE_OK) return st;
+        } else if (ptx_needs_again(ctx->counters)) {
+            ctx->cur = sl.arena;
+            CudaBackend bk{ctx};
+            bk.aborted = &w.counters->struct_abort;
+            ptx_stage_again(bk, w, ctx->counters);
+            CUDA_TRY(cudaEventRecord(sl.ev_end, ctx->stream));
+            CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            if (ctx->failed) return strstr(ctx->err, "cudaMalloc") ? PTXFE_ERR_OOM : PTXFE_ERR_CUDA;
+        }
+    }
+    if (w.n_chunks >= 512) {
+        const double bytes = (double)w.n_chunks * PTX_CHUNK;
+        auto learn = [&](double& ratio, uint32_t n) { if (n * 1.12 / bytes > ratio) ratio = n * 1.12 / bytes; };
+        learn(ctx->tokens_per_byte, ctx->counters.n_tokens);
+        learn(ctx->units_per_byte, ctx->counters.n_units);
+        learn(ctx->words_per_byte, ctx->counters.n_words);
+    }
     return PTXFE_OK;
 }
 
@@ -1150,9 +1462,15 @@ int ptxfe_run(ptxfe_ctx* ctx, uint32_t mode) {
     ctx->prof_names.clear();
     ctx->mode = mode;
     ctx->cur = 0;
-    uint32_t n = (uint32_t)ctx->layout.size();
-    int st = run_pipeline(ctx, ctx->d_text, ctx->layout.data(), n, mode, ctx->ev[2], ctx->ev[3], ctx->ev[4], ctx->ev[5]);
-    if (st != PTXFE_OK) return st;
+    SliceRun sl;
+    sl.text = ctx->d_text;
+    sl.n = (uint32_t)ctx->layout.size();
+    sl.meta = 0;
+    sl.mode = mode;
+    sl.ev_begin = ctx->ev[2]; sl.ev_lex = ctx->ev[3]; sl.ev_structure = ctx->ev[4]; sl.ev_end = ctx->ev[5];
+    int st = enqueue_slice(ctx, sl);
+    if (st == PTXFE_OK) st = finish_slice(ctx, sl);
+    if (st != PTXFE_OK) { cudaStreamSynchronize(ctx->stream); return st; }
     ptxfe_stats& s = ctx->stats;
     cudaEventElapsedTime(&s.kernel_ms, ctx->ev[2], ctx->ev[5]);
     cudaEventElapsedTime(&s.lex_ms, ctx->ev[2], ctx->ev[3]);
@@ -1220,10 +1538,10 @@ int ptxfe_fetch(ptxfe_ctx* ctx, ptxfe_batch** out) {
     if ((st = grow_pinned(ctx, &ctx->h_lexerrs, &ctx->h_lexerrs_cap, lb + 16, 0)) != PTXFE_OK) return st;
     if ((st = grow_pinned(ctx, &ctx->h_results, &ctx->h_results_cap, rb + 16, 0)) != PTXFE_OK) return st;
     CUDA_TRY(cudaEventRecord(ctx->ev[6], ctx->stream));
-    if (wb) CUDA_TRY(cudaMemcpyAsync(ctx->h_words, ctx->work.words, wb, cudaMemcpyDeviceToHost, ctx->stream));
-    if (eb) CUDA_TRY(cudaMemcpyAsync(ctx->h_errs, ctx->work.errs, eb, cudaMemcpyDeviceToHost, ctx->stream));
-    if (lb) CUDA_TRY(cudaMemcpyAsync(ctx->h_lexerrs, ctx->work.lexerrs, lb, cudaMemcpyDeviceToHost, ctx->stream));
-    if (rb) CUDA_TRY(cudaMemcpyAsync(ctx->h_results, ctx->work.results, rb, cudaMemcpyDeviceToHost, ctx->stream));
+    if (wb) CUDA_TRY(cudaMemcpyAsync(ctx->h_words, ctx->works[0].words, wb, cudaMemcpyDeviceToHost, ctx->stream));
+    if (eb) CUDA_TRY(cudaMemcpyAsync(ctx->h_errs, ctx->works[0].errs, eb, cudaMemcpyDeviceToHost, ctx->stream));
+    if (lb) CUDA_TRY(cudaMemcpyAsync(ctx->h_lexerrs, ctx->works[0].lexerrs, lb, cudaMemcpyDeviceToHost, ctx->stream));
+    if (rb) CUDA_TRY(cudaMemcpyAsync(ctx->h_results, ctx->works[0].results, rb, cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_TRY(cudaEventRecord(ctx->ev[7], ctx->stream));
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     CUDA_TRY(cudaEventElapsedTime(&ctx->stats.d2h_ms, ctx->ev[6], ctx->ev[7]));
@@ -1311,8 +1629,29 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
             use_raw[k] = 1;
             raw_base[k] = raw_total;
             raw_total += ((sl.bytes + 15) & ~(uint64_t)15) + 16 * (uint64_t)runs;
+            uint64_t at = 0;     // offset of the current run inside the slice's raw region (multiple of 16)
+            for (uint32_t m = sl.m0; m < sl.m1;) {
+                uint32_t e = m + 1;
+                uint64_t bytes = lens[m];
+                while (e < sl.m1 && texts[e] == texts[e - 1] + lens[e - 1]) bytes += lens[e++];
+                for (uint32_t j = m; j < e; j++) {
+                    repack[j].chunk_begin = ctx->layout[j].chunk_begin;
+                    repack[j].raw_off = (uint32_t)(at + (uint64_t)(texts[j] - texts[m]));
+                    repack[j].len = (uint32_t)lens[j];
+                }
+                at += (bytes + 15) & ~(uint64_t)15;
+                m = e;
+            }
         }
     }
+    size_t meta_total = 0;
+    std::vector<size_t> meta_at(ns);
+    for (size_t k = 0; k < ns; k++) {
+        meta_at[k] = meta_total;
+        meta_total += meta_bytes(slices[k].m1 - slices[k].m0);
+    }
+    if ((st = ensure_meta(ctx, meta_total)) != PTXFE_OK) return st;
+    for (size_t k = 0; k < ns; k++) write_meta(ctx, meta_at[k], slices[k].m0, slices[k].m1, use_raw[k] ? repack.data() : nullptr);
     if (raw_total + 64 > ctx->d_raw_cap) {
         if (ctx->d_raw) cudaFree(ctx->d_raw);
         ctx->d_raw = nullptr;
@@ -1323,20 +1662,16 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     }
     auto submit_text = [&](size_t k) -> int {
         const Slice& sl = slices[k];
-        if (k == 0) CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->s_in));
+        if (k == 0) {
+            CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->s_in));
+            CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_total, cudaMemcpyHostToDevice, ctx->s_in));
+        }
         if (use_raw[k]) {
-            uint64_t at = 0;     // offset of the current run inside the slice's raw region (multiple of 16)
             for (uint32_t m = sl.m0; m < sl.m1;) {
                 uint32_t e = m + 1;
                 uint64_t bytes = lens[m];
                 while (e < sl.m1 && texts[e] == texts[e - 1] + lens[e - 1]) bytes += lens[e++];
-                if (bytes) CUDA_TRY(cudaMemcpyAsync(ctx->d_raw + raw_base[k] + at, texts[m], bytes, cudaMemcpyHostToDevice, ctx->s_in));
-                for (uint32_t j = m; j < e; j++) {
-                    repack[j].chunk_begin = ctx->layout[j].chunk_begin;
-                    repack[j].raw_off = (uint32_t)(at + (uint64_t)(texts[j] - texts[m]));
-                    repack[j].len = (uint32_t)lens[j];
-                }
-                at += (bytes + 15) & ~(uint64_t)15;
+                if (bytes) CUDA_TRY(cudaMemcpyAsync(ctx->d_raw + raw_base[k] + repack[m].raw_off, texts[m], bytes, cudaMemcpyHostToDevice, ctx->s_in));
                 m = e;
             }
         } else {
@@ -1369,7 +1704,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     // ---- host result buffers: sized from the text; grown (after the copies in flight have landed) if a slice needs more
     int rc;
     if ((rc = grow_pinned(ctx, &ctx->h_results, &ctx->h_results_cap, sizeof(PtxModuleResult) * (size_t)n + 16, 0)) != PTXFE_OK) return drain(rc);
-    if ((rc = grow_pinned(ctx, &ctx->h_words, &ctx->h_words_cap, (size_t)(total * 2) + 4096, 0)) != PTXFE_OK) return drain(rc);
+    if ((rc = grow_pinned(ctx, &ctx->h_words, &ctx->h_words_cap, (size_t)(total * 2) + 131072, 0)) != PTXFE_OK) return drain(rc);
     size_t words_done = 0, errs_done = 0, lexerrs_done = 0;
     std::vector<size_t> base_w(ns), base_e(ns), base_l(ns);
     ptxfe_stats& s = ctx->stats;
@@ -1377,19 +1712,41 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     s.n_classes = s.n_untemplated = s.n_signature_words = 0;
     s.n_class_capacity = PTX_MAX_CLASSES;
     s.n_signature_capacity = PTX_SIG_POOL_WORDS;
+    // The kernels of slice k + 1 go into the stream before the host waits for those of slice k: the device does not idle
+    // while the host looks at the counts and sends the results of slice k on their way.
+    std::vector<SliceRun> runs(ns);
+    auto enqueue = [&](size_t k) -> int {
+        const Slice& sl = slices[k];
+        SliceRun& r = runs[k];
+        ctx->cur = (int)(k & 1);
+        // this arena held the results of slice k-2: they leave the device first
+        if (k >= 2) CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->slice_ev[5 * (k - 2) + 4], 0));
+        CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->slice_ev[5 * k], 0));
+        r.text = ctx->d_text + sl.text_off;
+        r.meta = meta_at[k];
+        r.n = sl.m1 - sl.m0;
+        r.mode = mode;
+        r.raw = use_raw[k] ? ctx->d_raw + raw_base[k] : nullptr;
+        r.first = k == 0;
+        r.results_out = (PtxModuleResult*)ctx->h_results + sl.m0;
+        if (ns == 1 && total <= PTXFE_DIRECT_OUT_BYTES) {
+            r.words_out = (uint32_t*)ctx->h_words;
+            r.words_out_cap = (uint32_t)(ctx->h_words_cap / 4 - 4);
+        }
+        r.ev_begin = ctx->slice_ev[5 * k + 1];
+        r.ev_end = ctx->slice_ev[5 * k + 2];
+        return enqueue_slice(ctx, r);
+    };
+    if ((rc = enqueue(0)) != PTXFE_OK) return drain(rc);
     for (size_t k = 0; k < ns; k++) {
         const Slice& sl = slices[k];
-        ctx->cur = (int)(k & 1);
-        // this arena held the results of slice k-2: wait until they have left the device
-        if (k >= 2) DRAIN_TRY(cudaEventSynchronize(ctx->slice_ev[5 * (k - 2) + 4]));
-        DRAIN_TRY(cudaStreamWaitEvent(ctx->stream, ctx->slice_ev[5 * k], 0));
         if (k + 2 < ns && (rc = submit_text(k + 2)) != PTXFE_OK) return drain(rc);
-        rc = run_pipeline(ctx, ctx->d_text + sl.text_off, ctx->layout.data() + sl.m0, sl.m1 - sl.m0, mode,
-                          ctx->slice_ev[5 * k + 1], nullptr, nullptr, ctx->slice_ev[5 * k + 2],
-                          use_raw[k] ? repack.data() + sl.m0 : nullptr, ctx->d_raw + raw_base[k], k == 0);
-        if (rc != PTXFE_OK) return drain(rc);
+        if (k + 1 < ns && (rc = enqueue(k + 1)) != PTXFE_OK) return drain(rc);
+        if ((rc = finish_slice(ctx, runs[k])) != PTXFE_OK) return drain(rc);
         const PtxCounters& c = ctx->counters;
-        size_t nw = c.n_words, ne = c.n_errs, nl = c.n_lexerrs, nm = sl.m1 - sl.m0;
+        const PtxWork& w = ctx->works[k & 1];
+        size_t nw = c.n_words, ne = c.n_errs, nl = c.n_lexerrs;
+        const bool words_there = w.words == (uint32_t*)ctx->h_words;        // the kernels wrote them to the host themselves
         if ((words_done + nw) * sizeof(uint32_t) + 16 > ctx->h_words_cap || (errs_done + ne) * sizeof(PtxErrRec) + 16 > ctx->h_errs_cap ||
             (lexerrs_done + nl) * 8 + 16 > ctx->h_lexerrs_cap) {
             DRAIN_TRY(cudaStreamSynchronize(ctx->s_out));
@@ -1397,16 +1754,15 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
             double done_bytes = 0;
             for (size_t j = 0; j <= k; j++) done_bytes += (double)slices[j].bytes;
             double scale = done_bytes > 0 ? (double)total / done_bytes * 1.1 : 1.0;
-            if ((rc = grow_pinned(ctx, &ctx->h_words, &ctx->h_words_cap, (size_t)((words_done + nw) * scale) * 4 + 4096, words_done * 4)) != PTXFE_OK) return drain(rc);
+            if ((rc = grow_pinned(ctx, &ctx->h_words, &ctx->h_words_cap, (size_t)((words_done + nw) * scale) * 4 + 4096, words_there ? nw * 4 : words_done * 4)) != PTXFE_OK) return drain(rc);
             if ((rc = grow_pinned(ctx, &ctx->h_errs, &ctx->h_errs_cap, (size_t)((errs_done + ne) * scale) * sizeof(PtxErrRec) + 4096, errs_done * sizeof(PtxErrRec))) != PTXFE_OK) return drain(rc);
             if ((rc = grow_pinned(ctx, &ctx->h_lexerrs, &ctx->h_lexerrs_cap, (size_t)((lexerrs_done + nl) * scale) * 8 + 4096, lexerrs_done * 8)) != PTXFE_OK) return drain(rc);
         }
-        // the kernels of this slice have finished (run_pipeline waits for them)
+        // the kernels of this slice have finished
         DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 3], ctx->s_out));
-        if (nw) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_words + words_done, ctx->work.words, nw * 4, cudaMemcpyDeviceToHost, ctx->s_out));
-        if (ne) DRAIN_TRY(cudaMemcpyAsync((PtxErrRec*)ctx->h_errs + errs_done, ctx->work.errs, ne * sizeof(PtxErrRec), cudaMemcpyDeviceToHost, ctx->s_out));
-        if (nl) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_lexerrs + 2 * lexerrs_done, ctx->work.lexerrs, nl * 8, cudaMemcpyDeviceToHost, ctx->s_out));
-        if (nm) DRAIN_TRY(cudaMemcpyAsync((PtxModuleResult*)ctx->h_results + sl.m0, ctx->work.results, nm * sizeof(PtxModuleResult), cudaMemcpyDeviceToHost, ctx->s_out));
+        if (nw && !words_there) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_words + words_done, w.words, nw * 4, cudaMemcpyDeviceToHost, ctx->s_out));
+        if (ne) DRAIN_TRY(cudaMemcpyAsync((PtxErrRec*)ctx->h_errs + errs_done, w.errs, ne * sizeof(PtxErrRec), cudaMemcpyDeviceToHost, ctx->s_out));
+        if (nl) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_lexerrs + 2 * lexerrs_done, w.lexerrs, nl * 8, cudaMemcpyDeviceToHost, ctx->s_out));
         DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 4], ctx->s_out));
         if (words_done + nw > 0xFFFFFFFFull) return drain(PTXFE_ERR_TOO_LARGE);   // module results index words with 32 bits
         base_w[k] = words_done; base_e[k] = errs_done; base_l[k] = lexerrs_done;
@@ -1681,23 +2037,14 @@ int ptxfe_lex_module(ptxfe_ctx* ctx, const char* text, uint64_t len, uint32_t** 
     uint64_t lens[1] = {len};
     int st = ptxfe_stage(ctx, texts, lens, 1);
     if (st != PTXFE_OK) return st;
-    CudaBackend bk{ctx};
-    bk.reset();
     ctx->failed = false;
-    PtxWork& w = ctx->work;
-    w = PtxWork();
-    w.text = ctx->d_text;
-    w.n_modules = 1;
-    ctx->mcb.assign({0u, (uint32_t)((len + PTX_CHUNK - 1) / PTX_CHUNK)});
-    w.n_chunks = ctx->mcb[1];
-    w.layout = (PtxModuleLayout*)bk.alloc(sizeof(PtxModuleLayout) * 2);
-    w.mod_chunk_begin = (uint32_t*)bk.alloc(sizeof(uint32_t) * 3);
-    w.results = (PtxModuleResult*)bk.alloc(sizeof(PtxModuleResult) * 2);
-    w.counters = (PtxCounters*)bk.alloc(sizeof(PtxCounters));
-    if (ctx->failed) return PTXFE_ERR_OOM;
-    CUDA_TRY(cudaMemcpyAsync(w.layout, ctx->layout.data(), sizeof(PtxModuleLayout), cudaMemcpyHostToDevice, ctx->stream));
-    CUDA_TRY(cudaMemcpyAsync(w.mod_chunk_begin, ctx->mcb.data(), sizeof(uint32_t) * 2, cudaMemcpyHostToDevice, ctx->stream));
-    CUDA_TRY(cudaMemsetAsync(w.counters, 0, sizeof(PtxCounters), ctx->stream));
+    ctx->cur = 0;
+    SliceRun sl;
+    sl.text = ctx->d_text;
+    sl.n = 1;
+    CudaBackend bk{ctx};
+    PtxWork& w = ctx->works[0];
+    if ((st = begin_slice(bk, sl, false)) != PTXFE_OK) return st;
     memset(&ctx->counters, 0, sizeof ctx->counters);
     ptx_stage_lex(bk, w, ctx->counters);
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -1795,7 +2142,7 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
     const uint64_t me = len;
     // every scratch word that is read below is written first by this call, so what an earlier call left behind
     // does not matter
-    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>((size_t)n_chunks, [=] __device__(size_t c) {
+    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>(LaunchCount{n_chunks, nullptr, nullptr, 0}, [=] __device__(size_t c) {
         uint64_t cs = (uint64_t)c * PTX_CHUNK;
         uint64_t ce = cs + PTX_CHUNK < me ? cs + PTX_CHUNK : me;
         uint32_t v = cx_chunk_vector(PtxGlobalReader{text, (uint32_t)me}, (uint32_t)cs, (uint32_t)ce);
@@ -1811,7 +2158,7 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
         return cs - q > PTXFE_NOALLOC_MAX_BACK;
     };
     scan_in_scratch<uint32_t>(stream, n_chunks, ArrayLoad<uint32_t>{vec}, ArrayStore<uint32_t>{vec}, ComposeOp(), CX_IDENTITY, partial_u32);
-    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>((size_t)n_chunks, [=] __device__(size_t c) {
+    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>(LaunchCount{n_chunks, nullptr, nullptr, 0}, [=] __device__(size_t c) {
         uint64_t cs = (uint64_t)c * PTX_CHUNK;
         int state = c == 0 ? CX_CODE : (int)(vec[c - 1] & 7u);
         LexCountSink sink;
@@ -1824,7 +2171,7 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
         if (c == 0) { PtxPair z; z.a = z.b = 0; cnt[0] = z; }
     });
     scan_in_scratch<PtxPair>(stream, (size_t)n_chunks + 1, ArrayLoad<PtxPair>{cnt}, ArrayStore<PtxPair>{cnt}, PairAddOp(), PtxPair{0, 0}, partial_pair);
-    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>((size_t)n_chunks, [=] __device__(size_t c) {
+    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>(LaunchCount{n_chunks, nullptr, nullptr, 0}, [=] __device__(size_t c) {
         uint64_t cs = (uint64_t)c * PTX_CHUNK;
         int state = c == 0 ? CX_CODE : (int)(vec[c - 1] & 7u);
         LexCapSink sink;

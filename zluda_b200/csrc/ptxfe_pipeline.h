@@ -51,7 +51,6 @@ struct PtxSeg3 {
 #define PTX_SORT_BUCKETS 4096u
 #define PTX_BULK_MIN_TOKENS 8192u   // statements at least this long get the bulk initialiser path
 #define PTX_MAX_BULK 32u            // per batch slice; further ones are decoded by one thread each
-#define PTX_TMP_STRIDE 48u     // words per unit in the staging table of the first decode pass (192 bytes: sector aligned)
 
 // fast per-thread memory the backend lends to a staged decoder: room for `stage_cap` record words (word k at
 // stage[k * stage_stride]) and for `win_cap` tokens (token k at win[k * win_stride])
@@ -151,7 +150,7 @@ struct PtxClassStore {
     uint32_t* sig_off;          // [PTX_MAX_CLASSES] word offset of the signature in sig_pool
     uint32_t* sig_pool;         // [PTX_SIG_POOL_WORDS]
     uint32_t* rep_unit;         // [PTX_MAX_CLASSES] representative unit (valid for the classes added by the current slice)
-    uint32_t* state;            // [0] classes so far, [1] signature words used, [2] classes before the current slice
+    uint32_t* state;            // [0] classes so far, [1] signature words used, [3] classes were inserted and never decoded
     static size_t bytes() {
         return sizeof(unsigned long long) * PTX_CLASS_SLOTS + 4ull * PTX_CLASS_SLOTS + 4ull * PTX_TMPL_WORDS * PTX_MAX_CLASSES +
                2ull * PTX_TMPL_WORDS * PTX_MAX_CLASSES + sizeof(PtxTemplateInfo) * PTX_MAX_CLASSES + 4ull * PTX_MAX_CLASSES +
@@ -244,12 +243,52 @@ struct PtxCounters {
     uint32_t n_flagged;         // units whose records are written by the second decode pass
     uint32_t n_bulk;            // statements long enough for the bulk initialiser path
     uint32_t n_rest;            // units without a template
-    uint32_t n_listed;
+    uint32_t n_second;          // units that a class promised a template and that have none after all
     uint32_t n_classes;         // statement classes met so far in this batch (all slices)
     uint32_t n_sig_words;       // words of the signature pool in use
     uint32_t struct_abort;      // the structure pass ran into its wait limit (its results are void)
     uint32_t n_skipped;         // modules with tokens that are not parsed (a lexer error, and not the errors-only mode)
+    uint32_t n_first;           // units decoded ahead of the templates: those without a class key, and class representatives
+    uint32_t n_reps;            // ... of which representatives
+    uint32_t n_staged_words;    // words of the staged records so far
+    uint32_t redo;              // PTX_REDO_*: something that the counts-stay-on-the-device flow does not cover
+    uint32_t spare[11];
 };
+// why a slice that was enqueued whole is run again with the host reading the counts on the way
+enum { PTX_REDO_TOKENS = 1, PTX_REDO_SERIAL_LEX = 2, PTX_REDO_UNITS = 4, PTX_REDO_BULK = 8, PTX_REDO_LIST = 16, PTX_REDO_WORDS = 64, PTX_REDO_STORE = 128,
+       PTX_REDO_DECODE = PTX_REDO_BULK | PTX_REDO_LIST | PTX_REDO_WORDS | PTX_REDO_STORE };    // these leave tokens and units as they are
+
+#ifdef __CUDA_ARCH__
+#define PTX_REDO_SET(c, why) atomicOr(&(c)->redo, (uint32_t)(why))
+#define PTX_COUNT_ADD(p, v) atomicAdd((p), (uint32_t)(v))
+#else
+#define PTX_REDO_SET(c, why) ((c)->redo |= (uint32_t)(why))
+#define PTX_COUNT_ADD(p, v) ((*(p) += (uint32_t)(v)) - (uint32_t)(v))
+#endif
+
+// A number of work items: the host's count, or (dev != nullptr) an upper bound on the host and the count on the device
+struct PtxCount {
+    size_t cap;
+    const uint32_t* dev;
+    uint32_t plus;            // items beyond *dev
+    bool always = false;      // also in a slice that stopped itself
+    PtxCount(size_t n, const uint32_t* d = nullptr, uint32_t p = 0) : cap(n), dev(d), plus(p) {}
+    operator size_t() const { return cap; }
+};
+// memory that reads as zero before the first step that uses it: from the region that a backend clears at once, or cleared here
+template <class BK>
+inline auto ptx_zalloc_impl(BK& bk, size_t bytes, int) -> decltype(bk.zalloc(bytes)) { return bk.zalloc(bytes); }
+template <class BK>
+inline void* ptx_zalloc_impl(BK& bk, size_t bytes, long) {
+    void* p = bk.alloc(bytes);
+    bk.zero(p, bytes);
+    return p;
+}
+template <class T, class BK>
+inline T* ptx_zalloc(BK& bk, size_t n) { return (T*)ptx_zalloc_impl(bk, sizeof(T) * n, 0); }
+// a backend whose structure pass numbers the top-level units on the way says so with kStructureTops
+template <class BK, class = void> struct PtxStructureTops { static constexpr bool value = false; };
+template <class BK> struct PtxStructureTops<BK, decltype((void)BK::kStructureTops)> { static constexpr bool value = BK::kStructureTops; };
 
 PTX_HD inline uint32_t ptx_upper_bound_u32(const uint32_t* a, uint32_t n, uint32_t x) {
     // number of entries <= x
@@ -294,7 +333,29 @@ struct PtxWork {
     uint32_t* words = nullptr;             // [n_words]
     PtxErrRec* errs = nullptr;             // [n_errs]
     PtxModuleResult* results = nullptr;    // [n_modules]
+    PtxModuleResult* results_out = nullptr;   // where the finished rows go (nullptr: results)
+    PtxCounters* counters_out = nullptr;   // with results_out: the final counters, as the host reads them
     PtxCounters* counters = nullptr;       // device copy
+    // Deferred counts: the whole slice is enqueued without the host reading anything on the way.  Arrays have the
+    // capacities below, steps take their counts from `counters`, and a slice that does not fit, or that needs a step
+    // that only the host can size (PTX_REDO_*), stops itself and is run again with deferred = false.
+    bool deferred = false;
+    uint32_t cap_tokens = 0, cap_units = 0, cap_words = 0, cap_list = 0;
+    PtxCount tokens_n() const { return deferred ? PtxCount(cap_tokens, &counters->n_tokens) : PtxCount(n_tokens); }
+    PtxCount units_n(uint32_t plus = 0) const { return deferred ? PtxCount((size_t)cap_units + plus, &counters->n_units, plus) : PtxCount((size_t)n_units + plus); }
+    uint32_t n_tokens = 0, n_units = 0;    // the host's copies (not deferred)
+    // what the stages leave for the steps behind them
+    uint32_t* lex_flag = nullptr;          // [n_modules] 1 = lexed by one thread
+    uint32_t* unit_top = nullptr;          // [top-level units] the unit that heads each
+    PtxPair* unit_own = nullptr;           // [n_units] words / errors of the unit itself
+    uint8_t* unit_flag = nullptr;          // [n_units] PTX_UNIT_*
+    uint32_t* unit_tmpl = nullptr;         // [n_units] template, or place of the staged record
+    uint32_t* staged = nullptr;            // staged records
+    uint32_t* list = nullptr;              // [n_first] units decoded first (bit 31: as a class representative)
+    uint32_t* second = nullptr;            // [n_second] units that a class promised a template and that have none
+    PtxClassStore cs;
+    PtxBulkTable bulk;
+    uint32_t bulk_tokens[PTX_MAX_BULK];
 };
 
 struct ComposeOp {
@@ -345,34 +406,16 @@ struct PtxLexChunkInfo {
 struct PtxLexVectorsStep {
     PtxLexChunkInfo info;
     uint32_t* vec;
+    uint32_t* tile_mod;      // module of every tile's first chunk, for the steps that work on tiles
     template <class R> PTX_HD void operator()(size_t c, const R& rd) const {
-        uint32_t ms, me, cs = (uint32_t)c * PTX_CHUNK;
-        bool first;
-        info.locate(c, ms, me, first);
+        uint32_t cs = (uint32_t)c * PTX_CHUNK;
+        const uint32_t m = ptx_upper_bound_u32(info.mcb, info.n_modules, (uint32_t)c) - 1;
+        const uint32_t ms = (uint32_t)info.layout[m].text_off, me = ms + (uint32_t)info.layout[m].text_len;
+        const bool first = c == info.mcb[m];
+        if (c % LT_CHUNKS == 0) tile_mod[c / LT_CHUNKS] = m;
         uint32_t ce = cs + PTX_CHUNK < me ? cs + PTX_CHUNK : me;
         uint32_t v = cx_chunk_vector(rd, cs, ce);
         vec[c] = first ? cx_restart(v) : v;
-    }
-};
-struct PtxLexTokensStep {
-    PtxLexChunkInfo info;
-    const uint8_t* text;
-    const uint32_t* vec;
-    PtxPair* cnt;
-    PtxToken* slots;
-    template <class R> PTX_HD void operator()(size_t c, const R& rd) const {
-        uint32_t ms, me, cs = (uint32_t)c * PTX_CHUNK;
-        bool first;
-        info.locate(c, ms, me, first);
-        int state = first ? CX_CODE : (int)(vec[c - 1] & 7u);
-        LexSlotSink sink;
-        sink.slots = slots + c * PTX_CHUNK;
-        lx_chunk(rd, text, ms, me, cs, cs + PTX_CHUNK, state, sink);
-        PtxPair p;
-        p.a = sink.n_tokens;
-        p.b = sink.n_errors;
-        cnt[c + 1] = p;
-        if (c == 0) { PtxPair z; z.a = z.b = 0; cnt[0] = z; }
     }
 };
 struct PtxLexErrorsStep {
@@ -397,6 +440,67 @@ struct PtxLexErrorsStep {
     }
 };
 
+// rows that depend on the lexer alone: token and error ranges, whether the module is parsed at all
+struct PtxModulesLexed {
+    const uint32_t* mcb;
+    const PtxPair* cnt;
+    uint32_t n_modules, n_chunks, mode;
+    uint32_t* mtb;
+    uint32_t* mod_skip;
+    const uint32_t* mod_flag;     // deferred counts: a module that asks for the one-thread lexer stops the slice
+    PtxModuleResult* results;
+    PtxCounters* counters;
+    PTX_HD void operator()(size_t m) const {
+        const PtxPair none{0, 0};
+        const PtxPair b = n_chunks ? cnt[mcb[m]] : none;
+        mtb[m] = b.a;
+        if (m == n_modules) return;
+        const PtxPair e = n_chunks ? cnt[mcb[m + 1]] : none;
+        PtxModuleResult r;
+        r.tok_begin = b.a;
+        r.tok_end = e.a;
+        r.lexerr_begin = b.b;
+        r.lexerr_end = e.b;
+        r.unit_begin = r.unit_end = r.word_begin = r.word_end = r.err_begin = r.err_end = 0;
+        r.sequential = r.status = r.n_errors = r.seq_tokens = 0;
+        results[m] = r;
+        // a module with a lex error is not parsed unless only its errors are wanted (lib.rs:392-411 vs 447-449, 487-489)
+        const bool lexerr = e.b > b.b && mode != 2;
+        mod_skip[m] = (b.a == e.a || lexerr) ? 1u : 0u;
+        if (b.a != e.a && lexerr) {
+#ifdef __CUDA_ARCH__
+            atomicAdd(&counters->n_skipped, 1u);
+#else
+            counters->n_skipped++;
+#endif
+        }
+        if (mod_flag && mod_flag[m]) PTX_REDO_SET(counters, PTX_REDO_SERIAL_LEX);
+    }
+};
+
+// A6: lexer errors are rare: a second walk, only when there are any, and only over the chunks that have one
+template <class BK>
+inline void ptx_lex_errors(BK& bk, PtxWork& w, uint32_t n_lexerrs) {
+    uint32_t* lexerrs = w.lexerrs = (uint32_t*)bk.alloc(sizeof(uint32_t) * 2 * (size_t)(n_lexerrs + 1));
+    if (!n_lexerrs) return;
+    const uint8_t* text = w.text;
+    const PtxModuleLayout* layout = w.layout;
+    const uint32_t* mcb = w.mod_chunk_begin;
+    const PtxPair* cnt = w.chunk_cnt;
+    const uint32_t* mod_flag = w.lex_flag;
+    bk.pf_text("lex_emit_errors", w.n_chunks, text, PtxLexErrorsStep{PtxLexChunkInfo{layout, mcb, w.n_modules}, text, w.chunk_vec, cnt, lexerrs, mod_flag});
+    // the flagged modules: one thread each, one walk over the module (linear in its length whatever its runs)
+    bk.pf("lex_emit_errors_serial", w.n_modules, [=] PTX_HD(size_t m) {
+        if (!mod_flag[m]) return;
+        const uint32_t c0 = mcb[m], c1 = mcb[m + 1];
+        if (c0 == c1 || cnt[c1].b == cnt[c0].b) return;
+        const uint32_t ms = (uint32_t)layout[m].text_off, me = ms + (uint32_t)layout[m].text_len;
+        LexErrorSink sink;
+        sink.errors = lexerrs + 2 * (size_t)cnt[c0].b;
+        lx_chunk(PtxGlobalReader{text, me}, text, ms, me, ms, me, CX_CODE, sink);
+    });
+}
+
 template <class BK>
 inline void ptx_stage_lex(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     const uint8_t* text = w.text;
@@ -406,75 +510,47 @@ inline void ptx_stage_lex(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     uint32_t* vec = w.chunk_vec = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_chunks + 1));
     PtxPair* cnt = w.chunk_cnt = (PtxPair*)bk.alloc(sizeof(PtxPair) * (n_chunks + 2));
     w.mod_tok_begin = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 2));
-    uint32_t* mod_lexerr_begin = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 2));
     PtxCounters* counters = w.counters;
     const PtxLexChunkInfo info{layout, mcb, n_modules};
 
-    // A1: transition vector of every chunk
-    bk.pf_text("lex_context_vectors", n_chunks, text, PtxLexVectorsStep{info, vec});
+    // A1: transition vector of every chunk, module of every tile
+    const size_t n_tiles = ((size_t)n_chunks + LT_CHUNKS - 1) / LT_CHUNKS;
+    uint32_t* tile_mod = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_tiles + 1));
+    bk.pf_text("lex_context_vectors", n_chunks, text, PtxLexVectorsStep{info, vec, tile_mod});
     // A2: inclusive scan with composition; chunk c starts in state (prefix[c-1])[CODE]
     bk.template scan<uint32_t>("scan_context", n_chunks, [=] PTX_HD(size_t i) { return vec[i]; }, [=] PTX_HD(size_t i, uint32_t v) { vec[i] = v; },
                                ComposeOp(), CX_IDENTITY);
     // A3: token boundaries, byte-parallel: one bit per text byte and the token / error count of every chunk
-    const size_t n_tiles = ((size_t)n_chunks + LT_CHUNKS - 1) / LT_CHUNKS;
     uint32_t* start_bits = (uint32_t*)bk.alloc(sizeof(uint32_t) * LT_WORDS * (n_tiles + 1));
-    uint32_t* mod_flag = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 1));
-    bk.zero(mod_flag, sizeof(uint32_t) * (n_modules + 1));
+    uint32_t* mod_flag = w.lex_flag = ptx_zalloc<uint32_t>(bk, n_modules + 1);
     uint32_t* word_bits = (uint32_t*)bk.alloc(sizeof(uint32_t) * LT_WORDS * (n_tiles + 1));
-    uint32_t* tile_mod = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_tiles + 1));
-    bk.pf("lex_tile_modules", n_tiles, [=] PTX_HD(size_t t) { tile_mod[t] = ptx_upper_bound_u32(mcb, n_modules, (uint32_t)t * LT_CHUNKS) - 1; });
     PtxLexTileArgs la{info, text, vec, n_chunks, bk.lex_tables(), tile_mod, start_bits, word_bits, cnt, mod_flag, nullptr, nullptr};
     bk.lex_mark("lex_mark", n_tiles, la);
     // modules with a run of soft bytes too long for the look-back of the parallel step: one thread each (rare)
-    bk.pf("lex_serial_modules", n_modules, [=] PTX_HD(size_t m) { lt_lex_module_serial(la, (uint32_t)m); });
+    if (!w.deferred) bk.pf("lex_serial_modules", n_modules, [=] PTX_HD(size_t m) { lt_lex_module_serial(la, (uint32_t)m); });
     // A4: exclusive offsets (cnt[c] = tokens before chunk c; cnt[n_chunks] = total)
-    bk.template scan<PtxPair>("scan_token_counts", n_chunks + 1, [=] PTX_HD(size_t i) { return cnt[i]; }, [=] PTX_HD(size_t i, PtxPair v) { cnt[i] = v; },
+    const uint32_t cap_tokens = w.deferred ? w.cap_tokens : 0xFFFFFFFFu;
+    bk.template scan<PtxPair>("scan_token_counts", n_chunks + 1, [=] PTX_HD(size_t i) { return i ? cnt[i] : PtxPair{0, 0}; },
+                              [=] PTX_HD(size_t i, PtxPair v) {
+                                  cnt[i] = v;
+                                  if (i != n_chunks) return;
+                                  counters->n_tokens = v.a;
+                                  counters->n_lexerrs = v.b;
+                                  if (v.a > cap_tokens) PTX_REDO_SET(counters, PTX_REDO_TOKENS);
+                              },
                               PairAddOp(), PtxPair{0, 0});
-    bk.pf("set_token_total", 1, [=] PTX_HD(size_t) {
-        counters->n_tokens = n_chunks ? cnt[n_chunks].a : 0;
-        counters->n_lexerrs = n_chunks ? cnt[n_chunks].b : 0;
-    });
-    bk.download(&host_counters, counters, sizeof(PtxCounters));
-    const uint32_t n_tokens = host_counters.n_tokens, n_lexerrs = host_counters.n_lexerrs;
-    PtxToken* tokens = w.tokens = (PtxToken*)bk.alloc(sizeof(PtxToken) * (size_t)(n_tokens + 1));
-    uint16_t* kinds = w.kinds = (uint16_t*)bk.alloc(sizeof(uint16_t) * ((size_t)n_tokens + 32));   // the kinds alone, for the passes that read nothing else
-    uint32_t* lexerrs = w.lexerrs = (uint32_t*)bk.alloc(sizeof(uint32_t) * 2 * (size_t)(n_lexerrs + 1));
+    if (!w.deferred) bk.download(&host_counters, counters, sizeof(PtxCounters));
+    w.n_tokens = host_counters.n_tokens;
+    const size_t room = w.deferred ? w.cap_tokens : w.n_tokens;
+    PtxToken* tokens = w.tokens = (PtxToken*)bk.alloc(sizeof(PtxToken) * (room + 1));
+    uint16_t* kinds = w.kinds = (uint16_t*)bk.alloc(sizeof(uint16_t) * (room + 32));   // the kinds alone, for the passes that read nothing else
     // A5: one thread per token: length, kind (identifiers that spell an opcode, modifier or directive word get that
     // kind), literal code; written to the token's final place
     la.tokens = tokens;
     la.kinds = kinds;
     bk.lex_emit("lex_emit", n_tiles, la);
-    // A6: lexer errors are rare: a second walk, only when there are any, and only over the chunks that have one
-    if (n_lexerrs) {
-        bk.pf_text("lex_emit_errors", n_chunks, text, PtxLexErrorsStep{info, text, vec, cnt, lexerrs, mod_flag});
-        // the flagged modules: one thread each, one walk over the module (linear in its length whatever its runs)
-        bk.pf("lex_emit_errors_serial", n_modules, [=] PTX_HD(size_t m) {
-            if (!mod_flag[m]) return;
-            const uint32_t c0 = mcb[m], c1 = mcb[m + 1];
-            if (c0 == c1 || cnt[c1].b == cnt[c0].b) return;
-            const uint32_t ms = (uint32_t)layout[m].text_off, me = ms + (uint32_t)layout[m].text_len;
-            LexErrorSink sink;
-            sink.errors = lexerrs + 2 * (size_t)cnt[c0].b;
-            lx_chunk(PtxGlobalReader{text, me}, text, ms, me, ms, me, CX_CODE, sink);
-        });
-    }
-    uint32_t* mtb = w.mod_tok_begin;
-    bk.pf("module_token_ranges", n_modules + 1, [=] PTX_HD(size_t m) {
-        uint32_t c = mcb[m];   // mod_chunk_begin[n_modules] = n_chunks
-        mtb[m] = n_chunks ? cnt[c].a : 0;
-        mod_lexerr_begin[m] = n_chunks ? cnt[c].b : 0;
-    });
-    PtxModuleResult* results = w.results;
-    bk.pf("module_results_init", n_modules, [=] PTX_HD(size_t m) {
-        PtxModuleResult r;
-        r.tok_begin = mtb[m];
-        r.tok_end = mtb[m + 1];
-        r.lexerr_begin = mod_lexerr_begin[m];
-        r.lexerr_end = mod_lexerr_begin[m + 1];
-        r.unit_begin = r.unit_end = r.word_begin = r.word_end = r.err_begin = r.err_end = 0;
-        r.sequential = r.status = r.n_errors = r.seq_tokens = 0;
-        results[m] = r;
-    });
+    w.lexerrs = nullptr;
+    if (!w.deferred) ptx_lex_errors(bk, w, host_counters.n_lexerrs);
 }
 
 // ------------------------------------------------------------------------------------------------ stage B: structure
@@ -493,54 +569,48 @@ PTX_HD inline bool ptx_is_directive_start(uint16_t k) {
 
 template <class BK>
 inline void ptx_stage_structure(BK& bk, PtxWork& w, PtxCounters& host_counters, uint32_t mode) {
-    const uint32_t n_tokens = host_counters.n_tokens, n_modules = w.n_modules;
-    const uint16_t* kinds = w.kinds;
+    const uint32_t n_modules = w.n_modules;
     const uint32_t* mtb = w.mod_tok_begin;
-    const PtxModuleResult* results = w.results;
-    int32_t* mod_final_scope = w.mod_final_scope = (int32_t*)bk.alloc(sizeof(int32_t) * (n_modules + 1));
-    w.mod_unit_begin = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 2));
+    int32_t* mod_final_scope = w.mod_final_scope = ptx_zalloc<int32_t>(bk, n_modules + 1);
+    uint32_t* mub = w.mod_unit_begin = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 2));
+    w.mod_skip = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 1));
     PtxCounters* counters = w.counters;
-    uint32_t* mod_skip = w.mod_skip = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 1));
-    bk.zero(mod_final_scope, sizeof(int32_t) * (n_modules + 1));
-    bk.pf("reset_skipped", 1, [=] PTX_HD(size_t) { counters->n_skipped = 0; });
-    // B0: a module with a lex error is not parsed unless only its errors
-    // are wanted (lib.rs:392-411 vs 447-449, 487-489)
-    bk.pf("mark_module_skip", n_modules, [=] PTX_HD(size_t m) {
-        bool lexerr = results[m].lexerr_end > results[m].lexerr_begin;
-        mod_skip[m] = (mtb[m] == mtb[m + 1] || (lexerr && mode != 2)) ? 1u : 0u;
-        if (mtb[m] != mtb[m + 1] && lexerr && mode != 2) {
-#ifdef __CUDA_ARCH__
-            atomicAdd(&counters->n_skipped, 1u);
-#else
-            counters->n_skipped++;
-#endif
-        }
-    });
+    // B0: what is known of the modules behind the lexer
+    bk.pf("modules_lexed", n_modules + 1,
+          PtxModulesLexed{w.mod_chunk_begin, w.chunk_cnt, n_modules, w.n_chunks, mode, w.mod_tok_begin, w.mod_skip, w.deferred ? w.lex_flag : nullptr,
+                          w.results, counters});
     // B1: one pass over the token kinds: (scope, paren) depth restarting at every module, the unit starts, their
     // numbering and the unit table (at most one unit per token); nothing per token is kept of it
-    uint32_t* ustart = w.unit_start = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_tokens + 2));
-    uint32_t* udepth = w.unit_depth = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_tokens + 2));
-    uint32_t* mub = w.mod_unit_begin;
-    bk.pf("reset_unit_total", 1, [=] PTX_HD(size_t) { counters->n_units = 0; counters->struct_abort = 0; });
-    bk.structure("structure", PtxStructArgs{kinds, n_tokens, mtb, n_modules, mod_final_scope, ustart, udepth, mub, counters});
-    bk.download(&host_counters, counters, sizeof(PtxCounters));
-    if (host_counters.struct_abort) {
-        bk.fail("the structure pass gave up waiting for an earlier tile");
-        host_counters.n_units = 0;
+    const size_t room = w.deferred ? w.cap_units : w.n_tokens;
+    w.unit_start = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 2));
+    w.unit_depth = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 2));
+    if (PtxStructureTops<BK>::value) {
+        w.unit_dir = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 1));
+        w.unit_top = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 1));
     }
-    const uint32_t n_units = host_counters.n_units;
-    // modules without tokens begin where the next module with tokens begins; mub[n_modules] = n_units
+    PtxStructArgs sa{w.kinds, w.deferred ? w.cap_tokens : w.n_tokens, mtb, n_modules, mod_final_scope, w.unit_start, w.unit_depth, mub, counters};
+    sa.udir = w.unit_dir;
+    sa.top_unit = w.unit_top;
+    sa.cap_units = (uint32_t)room;
+    sa.n_tokens_dev = w.deferred ? &counters->n_tokens : nullptr;
+    bk.structure("structure", sa);
+    if (!w.deferred) {
+        bk.download(&host_counters, counters, sizeof(PtxCounters));
+        if (host_counters.struct_abort) {
+            bk.fail("the structure pass gave up waiting for an earlier tile");
+            host_counters.n_units = 0;
+        }
+        w.n_units = host_counters.n_units;
+    }
+    // modules without tokens begin where the next module with tokens begins; mub[n_modules] = number of units
     bk.pf("module_unit_ranges", n_modules + 1, [=] PTX_HD(size_t m) {
-        if (m < n_modules && mtb[m] < mtb[m + 1]) return;      // written by the scan
+        if (m < n_modules && mtb[m] < mtb[m + 1]) return;      // written by the pass
         size_t k = m;
         while (k < n_modules && mtb[k] == mtb[k + 1]) k++;
-        mub[m] = k < n_modules ? (0x80000000u | (uint32_t)k) : n_units;   // a reference to module k is resolved below
-    });
-    bk.pf("module_unit_ranges_fill", n_modules + 1, [=] PTX_HD(size_t m) {
-        uint32_t v = mub[m];
-        if (v & 0x80000000u) mub[m] = mub[v & 0x7FFFFFFFu];
+        mub[m] = k < n_modules ? mub[k] : counters->n_units;
     });
 }
+
 
 // C5 as a step object: one output word at a time.  unit() is what a word needs of its unit (loaded once per unit by
 // the backend); word() only reads and says what to do with the word, so that a backend can have several words in flight
@@ -552,7 +622,7 @@ struct PtxEmitStep {
     const uint8_t* uflag;
     const uint32_t* utmpl;
     const uint32_t* ustart;
-    const uint32_t* table;
+    const uint32_t* table;       // staged records
     PtxClassStore cs;
     const PtxToken* tokens;
     const uint8_t* text;
@@ -561,14 +631,14 @@ struct PtxEmitStep {
     PTX_HD PtxEmitUnit unit(size_t u) const {
         PtxEmitUnit e;
         e.flag = uflag[u];
-        e.tmpl = e.flag == PTX_UNIT_TEMPLATED ? utmpl[u] : 0u;
+        e.tmpl = e.flag <= PTX_UNIT_TEMPLATED ? utmpl[u] : 0u;      // template, or place of the staged record
         e.start = ustart[u];
         e.first = 0;
         return e;
     }
     PTX_HD int word(const PtxEmitUnit& e, size_t u, uint32_t i, uint32_t& x) const {
         if (e.flag == PTX_UNIT_STAGED) {
-            x = table[u * PTX_TMP_STRIDE + i];
+            x = table[e.tmpl + i];
             return WRITE;
         }
         if (e.flag != PTX_UNIT_TEMPLATED) return NOTHING;
@@ -603,97 +673,75 @@ struct PtxEmitStep {
 };
 
 // ------------------------------------------------------------------------------------------------ stage C: decode
-template <class BK>
-inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
-    const uint32_t n_tokens = host_counters.n_tokens, n_units = host_counters.n_units, n_modules = w.n_modules;
-    const uint8_t* text = w.text;
-    const PtxToken* tokens = w.tokens;
-    const uint16_t* kinds = w.kinds;
-    const PtxModuleLayout* layout = w.layout;
-    const uint32_t* mtb = w.mod_tok_begin;
-    const uint32_t* mub = w.mod_unit_begin;
-    const uint32_t* ustart = w.unit_start;
-    const uint32_t* udepth = w.unit_depth;
-    const int32_t* mod_final_scope = w.mod_final_scope;
-    const uint32_t* mod_skip = w.mod_skip;
-    PtxModuleResult* results = w.results;
-    PtxCounters* counters = w.counters;
-    const uint32_t seq_max_tokens = w.seq_max_tokens;
-    uint32_t* uend = w.unit_end = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_units + 1));
-    uint32_t* udir = w.unit_dir = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_units + 1));
-    PtxPair* usize = w.unit_size = (PtxPair*)bk.alloc(sizeof(PtxPair) * ((size_t)n_units + 2));
-    uint8_t* ustatus = w.unit_status = (uint8_t*)bk.alloc((size_t)n_units + 16);
-    uint32_t* mod_bad = w.mod_bad = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 1));
-    PtxPair* mod_seq = w.mod_seq_size = (PtxPair*)bk.alloc(sizeof(PtxPair) * (n_modules + 1));
-    uint32_t* mod_seq_status = w.mod_seq_status = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 1));
-    // worst case one function per top-level unit; sized after the top-level scan below
-    bk.zero(mod_bad, sizeof(uint32_t) * (n_modules + 1));
-    bk.zero(mod_seq, sizeof(PtxPair) * (n_modules + 1));
-    bk.zero(mod_seq_status, sizeof(uint32_t) * (n_modules + 1));
-
-    // C0: ordinal of the enclosing top-level unit
-    bk.template scan<uint32_t>("scan_toplevel_ordinal", n_units, [=] PTX_HD(size_t u) { return (udepth[u] & 0x7FFFFFFFu) == 0 ? 1u : 0u; },
-                               [=] PTX_HD(size_t u, uint32_t v) { udir[u] = v; }, AddOp(), 0u);
-    // ... and the unit that heads each top-level ordinal (a module's first unit, or a top-level directive's first)
-    uint32_t* top_unit = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_units + 1));
-    bk.pf("list_toplevel_units", n_units, [=] PTX_HD(size_t u) {
-        if ((udepth[u] & 0x7FFFFFFFu) == 0) top_unit[udir[u] - 1] = (uint32_t)u;
-    });
-    // Very long top-level statements (arrays with huge initialisers) are listed for the bulk path
-    PtxBulkInfo* bulk_info = (PtxBulkInfo*)bk.alloc(sizeof(PtxBulkInfo) * PTX_MAX_BULK);
-    bk.pf("reset_bulk", 1, [=] PTX_HD(size_t) { counters->n_bulk = 0; });
-    bk.pf("find_bulk_units", n_units, [=] PTX_HD(size_t u) {
-        uint32_t dp = udepth[u];
-        if (dp != 0) return;       // top level, not the module header
-        uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
-        if (mod_skip[m]) return;
-        uint32_t start = ustart[u];
-        uint32_t end = (u + 1 < mub[m + 1]) ? ustart[u + 1] : mtb[m + 1];
-        if (end - start < PTX_BULK_MIN_TOKENS) return;
-#ifdef __CUDA_ARCH__
-        uint32_t slot = atomicAdd(&counters->n_bulk, 1u);
-#else
-        uint32_t slot = counters->n_bulk++;
-#endif
-        if (slot >= PTX_MAX_BULK) return;
-        PtxBulkInfo bi;
-        bi.first_tok = start;      // for now: the statement's token range
-        bi.close_tok = end;
-        bi.n_elems = bi.n_words = 0;
-        bi.bad = 1;
-        bi.unit = (uint32_t)u;
-        bi.elems = nullptr;
-        bi.dst = nullptr;
-        bulk_info[slot] = bi;
-    });
-    // T0: class key of every unit (see "unit classes and record templates" above)
-    uint16_t* ukey = (uint16_t*)bk.alloc(sizeof(uint16_t) * ((size_t)n_units + 2));
-    uint32_t* order = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_units + 1));
-    uint64_t* ckey_of = (uint64_t*)bk.alloc(sizeof(uint64_t) * ((size_t)n_units + 1));
-    bk.pf("unit_class_key", n_units, [=] PTX_HD(size_t u) {
+// C1 per unit: long top-level statements are listed for the bulk path; every other unit gets its class key (see "unit
+// classes and record templates" above) and its class.  The class table is an open-addressing table on the 64-bit key,
+// shared by the slices of a batch; the thread that inserts a key makes its unit the representative of the class.  Units
+// without a key and new representatives go to the first decode list (a representative with bit 31 set).
+struct PtxUnitClassesStep {
+    const uint8_t* text;
+    const PtxToken* tokens;
+    const uint16_t* kinds;
+    const uint32_t* ustart;
+    const uint32_t* udepth;
+    const uint32_t* mub;
+    const uint32_t* mod_skip;
+    uint32_t n_modules, cap_list;
+    bool deferred;
+    PtxCounters* counters;
+    PtxClassStore cs;
+    PtxBulkInfo* bulk_info;
+    uint32_t* uclass;
+    uint32_t* utmpl;
+    uint32_t* uend;
+    uint32_t* list;
+    PtxPair* uown;
+    uint8_t* uflag;
+    uint8_t* ustatus;
+    PTX_HD void add(uint32_t entry) const {
+        const uint32_t slot = PTX_COUNT_ADD(&counters->n_first, 1);
+        if (slot < cap_list) list[slot] = entry;
+        else redo(PTX_REDO_LIST);
+    }
+    // The slice stops behind this step: classes that it has inserted get no template.  The store says so, and the slices
+    // that were enqueued behind this one stop as well (their second runs start from an empty store).
+    PTX_HD void redo(uint32_t why) const {
+        PTX_REDO_SET(counters, why);
+        cs.state[3] = 1;
+    }
+    PTX_HD void operator()(size_t u) const {
+        if (deferred && *(const volatile uint32_t*)&cs.state[3]) { PTX_REDO_SET(counters, PTX_REDO_STORE); return; }
         // units lie back to back over the whole batch: a unit ends where the next one starts.  The unit's module is looked
         // up only when some module of the slice is not parsed at all (a lexer error outside the errors-only mode)
-        uint32_t start = ustart[u];
-        uint32_t end = u + 1 < n_units ? ustart[u + 1] : n_tokens;
-        uint32_t dp = udepth[u];
-        const bool skipped = counters->n_skipped != 0 && mod_skip[ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1] != 0;
-        ckey_of[u] = skipped ? 0 : ptx_class_key(text, tokens, kinds, start, end, dp & 0x7FFFFFFFu, (dp >> 31) != 0);
-    });
-
-    // T1: class table (open addressing on the 64-bit key), shared by the slices of a batch; the thread that inserts
-    // a key makes its unit the representative of the class
-    const PtxClassStore cs = bk.class_store(w.first_slice);
-    uint32_t* uclass = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_units + 1));
-    uint32_t* utmpl = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_units + 1));
-    uint8_t* uflag = (uint8_t*)bk.alloc((size_t)n_units + 16);
-    bk.pf("reset_flagged", 1, [=] PTX_HD(size_t) {
-        counters->n_flagged = 0;
-        cs.state[2] = cs.state[0] < PTX_MAX_CLASSES ? cs.state[0] : PTX_MAX_CLASSES;
-    });
-    bk.pf("class_insert", n_units, [=] PTX_HD(size_t u) {
+        const uint32_t n_units = counters->n_units;
+        const uint32_t start = ustart[u], end = u + 1 < n_units ? ustart[u + 1] : counters->n_tokens;
+        const uint32_t dp = udepth[u];
         uclass[u] = PTX_ABSENT;
-        unsigned long long key = ckey_of[u];
-        if (!key) return;
+        uflag[u] = PTX_UNIT_UNDECIDED;
+        if (counters->n_skipped && mod_skip[ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1]) {
+            uown[u] = PtxPair{0, 0};
+            uend[u] = 0;
+            ustatus[u] = US_OK;
+            uflag[u] = PTX_UNIT_STAGED;
+            utmpl[u] = 0;
+            return;
+        }
+        if (dp == 0 && end - start >= PTX_BULK_MIN_TOKENS) {       // top level, not the module header
+            const uint32_t slot = PTX_COUNT_ADD(&counters->n_bulk, 1);
+            if (slot < PTX_MAX_BULK) {
+                PtxBulkInfo bi;
+                bi.first_tok = start;      // for now: the statement's token range
+                bi.close_tok = end;
+                bi.n_elems = bi.n_words = 0;
+                bi.bad = 1;
+                bi.unit = (uint32_t)u;
+                bi.elems = nullptr;
+                bi.dst = nullptr;
+                bulk_info[slot] = bi;
+            }
+            if (deferred) redo(PTX_REDO_BULK);
+        }
+        const unsigned long long key = ptx_class_key(text, tokens, kinds, start, end, dp & 0x7FFFFFFFu, (dp >> 31) != 0);
+        if (!key) { add((uint32_t)u); return; }
         uint32_t h = (uint32_t)(key ^ (key >> 29)) & (PTX_CLASS_SLOTS - 1);
         for (int probe = 0; probe < 64; probe++) {
 #ifdef __CUDA_ARCH__
@@ -708,314 +756,128 @@ inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
             if (old == 0) cs.keys[h] = key;
 #endif
             if (old == 0) {
-#ifdef __CUDA_ARCH__
-                uint32_t id = atomicAdd(&cs.state[0], 1u);
-#else
-                uint32_t id = cs.state[0]++;
-#endif
-                if (id < PTX_MAX_CLASSES) {
-                    cs.rep_unit[id] = (uint32_t)u;
-                    cs.slot_tmpl[h] = id;
-                } else {
-                    cs.slot_tmpl[h] = PTX_ABSENT;
-                }
+                const uint32_t id = PTX_COUNT_ADD(&cs.state[0], 1);
                 uclass[u] = h;
+                cs.slot_tmpl[h] = id < PTX_MAX_CLASSES ? id : PTX_ABSENT;
+                if (id < PTX_MAX_CLASSES) {
+                    add((uint32_t)u | 0x80000000u);
+                    PTX_COUNT_ADD(&counters->n_reps, 1);
+                }
                 return;
             }
             if (old == key) { uclass[u] = h; return; }
             h = (h + 1) & (PTX_CLASS_SLOTS - 1);
         }
-    });
-    // T2: decode the representatives of the classes this slice added, with tagged output, and spell out their signature
-    // (thread i takes new class (i / 32) + (i % 32) * (PTX_MAX_CLASSES / 32): the first 8,192 new classes go to lane 0 of
-    // a warp each.  Representatives are statements of different shapes; 32 of them in one warp ran one after the other.)
-    bk.pf("decode_representatives", PTX_MAX_CLASSES, [=] PTX_HD(size_t i) {
-        const size_t k = (i >> 5) + (i & 31u) * (PTX_MAX_CLASSES / 32u);
-        size_t id = (size_t)cs.state[2] + k;
-        if (id >= cs.state[0] || id >= PTX_MAX_CLASSES) return;
-        uint32_t u = cs.rep_unit[id];
-        uint32_t m = ptx_upper_bound_u32(mub, n_modules, u) - 1;
-        uint32_t start = ustart[u];
-        uint32_t end = (u + 1 < mub[m + 1]) ? ustart[u + 1] : mtb[m + 1];
-        PtxSink sink;
-        sink.words = cs.tmpl_words + id * PTX_TMPL_WORDS;
-        sink.tags = cs.tmpl_tags + id * PTX_TMPL_WORDS;
-        sink.words_cap = PTX_TMPL_WORDS;
-        PtxResolver res;
-        res.module = m;
-        PtxDecoder d(text, tokens, mtb[m + 1], layout[m].text_off + layout[m].text_len, sink, res);
-        uint32_t dp = udepth[u];
-        PtxUnitResult r = ptx_decode_unit(d, start, dp & 0x7FFFFFFFu, (dp >> 31) != 0);
-        PtxTemplateInfo ti;
-        ti.n_words = sink.nw;
-        ti.n_tokens = end - start;
-        ti.depth1 = (dp & 0x7FFFFFFFu) == 1 ? 1u : 0u;
-        ti.ok = (r.status == US_OK && sink.ne == 0 && sink.peak <= PTX_TMPL_WORDS && !sink.poison && r.kind != U_FUNC && r.end == end &&
-                 d.max_seen < end) ? 1u : 0u;
-        if (ti.ok) {
-            uint32_t need = ptx_signature_words(tokens, start, ti.n_tokens);
-#ifdef __CUDA_ARCH__
-            uint32_t at = atomicAdd(&cs.state[1], need);
-#else
-            uint32_t at = cs.state[1];
-            cs.state[1] += need;
-#endif
-            if (at + need <= PTX_SIG_POOL_WORDS) {
-                cs.sig_off[id] = at;
-                ptx_signature_write(cs.sig_pool + at, text, tokens, kinds, start, ti.n_tokens, ti.depth1);
-            } else {
-                ti.ok = 0;
-            }
-        }
-        cs.info[id] = ti;
-    });
-    // T3: every unit of a class with a usable template is checked against the class signature and takes its size
-    uint32_t* rest_count = (uint32_t*)bk.alloc(sizeof(uint32_t) * 64);     // striped count of the units left without a template
-    bk.zero(rest_count, sizeof(uint32_t) * 64);
-    bk.pf("apply_templates", n_units, [=] PTX_HD(size_t u) {
-        uflag[u] = PTX_UNIT_UNDECIDED;
-        utmpl[u] = PTX_ABSENT;
-        auto rest = [&]() {      // this unit stays without a template
-#ifdef __CUDA_ARCH__
-            atomicAdd(&rest_count[u & 63], 1u);
-#else
-            rest_count[u & 63]++;
-#endif
-        };
-        uint32_t slot = uclass[u];
-        if (slot == PTX_ABSENT) { rest(); return; }
-        uint32_t id = cs.slot_tmpl[slot];
-        if (id == PTX_ABSENT) { rest(); return; }
-        const PtxTemplateInfo ti = cs.info[id];
-        if (!ti.ok) { rest(); return; }
-        uint32_t start = ustart[u];
-        uint32_t end = u + 1 < n_units ? ustart[u + 1] : n_tokens;
-        uint32_t dp = udepth[u];
-        uint32_t depth1 = (dp & 0x7FFFFFFFu) == 1 ? 1u : 0u;
-        if (end - start != ti.n_tokens || !ptx_signature_matches(cs.sig_pool + cs.sig_off[id], text, tokens, kinds, start, ti.n_tokens, depth1)) { rest(); return; }
-        PtxPair sz;
-        sz.a = ti.n_words;
-        sz.b = 0;
-        usize[u + 1] = sz;
-        if (u == 0) { PtxPair z; z.a = z.b = 0; usize[0] = z; }
-        uend[u] = end;
-        ustatus[u] = US_OK;
-        uflag[u] = PTX_UNIT_TEMPLATED;
-        utmpl[u] = id;
-    });
-
-    bk.pf("reset_func_count", 1, [=] PTX_HD(size_t) {
-        counters->n_funcs = 0;
-        counters->any_sequential = 0;
-        counters->pad = n_units ? udir[n_units - 1] : 0;   // number of top-level units: bound for the function table
-        uint32_t rest = 0;
-        for (int i = 0; i < 64; i++) rest += rest_count[i];
-        counters->n_rest = rest;
-        counters->n_classes = cs.state[0];
-        counters->n_sig_words = cs.state[1];
-    });
-    bk.download(&host_counters, counters, sizeof(PtxCounters));
-    const uint32_t max_funcs = host_counters.pad;
-    bk.pf("reset_mismatch", 1, [=] PTX_HD(size_t) { counters->pad = 0; });
-    // Bulk path: the elements of each listed statement's initialiser are decoded one thread per element into a dense
-    // run; the statement's own decoder later takes the run in one step (PtxDecoder::multi_variable).  A list that is
-    // not plainly "element, element, ... }" followed by ';' stays marked bad and is decoded the ordinary way.
-    const uint32_t n_bulk = host_counters.n_bulk < PTX_MAX_BULK ? host_counters.n_bulk : PTX_MAX_BULK;
-    PtxBulkTable bulk_table;
-    bulk_table.info = bulk_info;
-    bulk_table.n = n_bulk;
-    uint32_t bulk_tokens[PTX_MAX_BULK];     // tokens of each listed statement
-    if (n_bulk) {
-        PtxBulkInfo host_bulk[PTX_MAX_BULK];
-        bk.download(host_bulk, bulk_info, sizeof(PtxBulkInfo) * n_bulk);
-        for (uint32_t j = 0; j < n_bulk; j++) {
-            const uint32_t ts = host_bulk[j].first_tok, te = host_bulk[j].close_tok, nt = te - ts;
-            bulk_tokens[j] = nt;
-            PtxBulkInfo* bi = bulk_info + j;
-            uint32_t* lo_dev = (uint32_t*)bk.alloc(sizeof(uint32_t) * 4);
-            PtxPair* esz = (PtxPair*)bk.alloc(sizeof(PtxPair) * ((size_t)nt + 2));
-            uint32_t* elems = (uint32_t*)bk.alloc(sizeof(uint32_t) * (2 * (size_t)nt + 8));
-            bk.pf("bulk_reset", 1, [=] PTX_HD(size_t) { lo_dev[0] = PTX_ABSENT; lo_dev[1] = 0; });
-            bk.pf("bulk_find_open", nt, [=] PTX_HD(size_t k) {
-                uint32_t i = ts + (uint32_t)k;
-                if (i > ts && PTX_KL_KIND(kinds[i]) == T_LBRACE && PTX_KL_KIND(kinds[i - 1]) == T_EQ) {
-#ifdef __CUDA_ARCH__
-                    atomicMin(&lo_dev[0], i);
-#else
-                    if (i < lo_dev[0]) lo_dev[0] = i;
-#endif
-                }
-            });
-            bk.pf("bulk_measure", nt, [=] PTX_HD(size_t k) {
-                uint32_t i = ts + (uint32_t)k;
-                PtxPair z;
-                z.a = z.b = 0;
-                esz[k] = z;
-                const uint32_t lo = lo_dev[0], hi = te - 2;
-                bool shape_ok = lo != PTX_ABSENT && nt >= 6 && lo + 1 < hi && PTX_KL_KIND(kinds[te - 2]) == T_RBRACE &&
-                                PTX_KL_KIND(kinds[te - 1]) == T_SEMI && PTX_KL_KIND(kinds[hi - 1]) != T_COMMA;
-                if (!shape_ok) { if (k == 0) lo_dev[1] = 1; return; }
-                if (i <= lo || i >= hi) return;
-                uint16_t kd = PTX_KL_KIND(kinds[i]);
-                if (kd == T_LBRACE || kd == T_RBRACE) { lo_dev[1] = 1; return; }
-                if (!(i == lo + 1 || PTX_KL_KIND(kinds[i - 1]) == T_COMMA)) return;
-                // an element starts here: measure it
-                uint32_t mm = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
-                PtxSink sink;
-                PtxResolver res;
-                PtxDecoder d(text, tokens, mtb[mm + 1], layout[mm].text_off + layout[mm].text_len, sink, res);
-                d.pos = i;
-                d.unit_tok0 = i;
-                bool ok = d.reg_or_immediate(true) && sink.ne == 0 && d.pos <= hi;
-                if (ok) {
-                    uint16_t nk = PTX_KL_KIND(kinds[d.pos]);
-                    ok = (d.pos == hi) || nk == T_COMMA;
-                }
-                if (!ok) { lo_dev[1] = 1; return; }
-                z.a = sink.nw;
-                z.b = 1;
-                esz[k] = z;
-            });
-            bk.template scan<PtxPair>("bulk_scan", (size_t)nt, [=] PTX_HD(size_t k) { return esz[k]; }, [=] PTX_HD(size_t k, PtxPair v) {
-                                          PtxPair own = esz[k];
-                                          if (k + 1 == nt) {     // totals, before the entry turns exclusive
-                                              bi->n_words = v.a;
-                                              bi->n_elems = v.b;
-                                          }
-                                          PtxPair ex;
-                                          ex.a = v.a - own.a;
-                                          ex.b = own.b;      // keeps "an element starts here"
-                                          esz[k] = ex;
-                                      },
-                                      PairAddOp(), PtxPair{0, 0});
-            bk.pf("bulk_decode", nt, [=] PTX_HD(size_t k) {
-                if (lo_dev[1] || !esz[k].b) return;
-                uint32_t i = ts + (uint32_t)k;
-                uint32_t mm = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
-                PtxSink sink;
-                sink.words = elems + esz[k].a;
-                PtxResolver res;
-                PtxDecoder d(text, tokens, mtb[mm + 1], layout[mm].text_off + layout[mm].text_len, sink, res);
-                d.pos = i;
-                d.unit_tok0 = i;
-                d.reg_or_immediate(true);
-            });
-            bk.pf("bulk_publish", 1, [=] PTX_HD(size_t) {
-                bi->first_tok = lo_dev[0] + 1;
-                bi->close_tok = te - 2;
-                bi->bad = lo_dev[1];
-                bi->elems = elems;
-                bi->dst = nullptr;
-            });
-        }
+        add((uint32_t)u);
     }
-    PtxFnEntry* fn_entries = w.fn_entries = (PtxFnEntry*)bk.alloc(sizeof(PtxFnEntry) * ((size_t)max_funcs + 1));
+};
 
-    // The units without a template are decoded next.  When they are few (clean input: calls, function headers,
-    // statements whose class was poisoned) they are simply listed; when they are many they are sorted by a "shape key"
-    // (a hash of their token kinds) first: the decoder's control flow depends on token kinds only, so the threads of a
-    // warp then follow the same path.  Results are written at offsets computed in unit order either way, so the order
-    // of processing does not show in the output.  order[0 .. n_rest) = the units to decode.
-    const uint32_t n_rest = host_counters.n_rest;
-    if (n_rest <= 131072) {
-        bk.pf("list_rest_units", n_units, [=] PTX_HD(size_t u) {
-            if (uflag[u] == PTX_UNIT_TEMPLATED) return;
-#ifdef __CUDA_ARCH__
-            uint32_t slot = atomicAdd(&counters->n_listed, 1u);
-#else
-            uint32_t slot = counters->n_listed++;
-#endif
-            order[slot] = (uint32_t)u;
-        });
-    } else {
-        // templated units share the last bucket, so they sort behind all the others
-        bk.pf("unit_shape_key", n_units, [=] PTX_HD(size_t u) {
-            if (uflag[u] == PTX_UNIT_TEMPLATED) { ukey[u] = (uint16_t)(PTX_SORT_BUCKETS - 1); return; }
-            uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
-            uint32_t start = ustart[u];
-            uint32_t end = (u + 1 < mub[m + 1]) ? ustart[u + 1] : mtb[m + 1];
-            if (end > start + 20) end = start + 20;
-            uint32_t h = 2166136261u ^ (udepth[u] >> 31) ^ ((udepth[u] & 0x7FFFFFFFu) ? 2u : 0u);
-            for (uint32_t i = start; i < end; i++) h = (h ^ PTX_KL_KIND(kinds[i])) * 16777619u;
-            h ^= h >> 15;
-            h &= PTX_SORT_BUCKETS - 1;
-            if (h == PTX_SORT_BUCKETS - 1) h = 0;
-            ukey[u] = (uint16_t)h;
-        });
-        bk.sort_by_key("sort_units_by_shape", n_units, ukey, order);
-    }
-
-    // C1: decode every unit once.  The record is built in a small per-thread staging buffer (failed alternatives are
-    // rolled back there) and lands in row u of a table; its final place is known only after the sizes are scanned.
-    // Units that report errors (every `call` reserves one), or whose record outgrows the buffer, are only measured
-    // here and written by the second pass (C6), which also has the function table.
-    uint32_t* table = (uint32_t*)bk.alloc(sizeof(uint32_t) * PTX_TMP_STRIDE * ((size_t)n_units + 1));
-    bk.pf_staged("decode_units", n_rest, table, PTX_TMP_STRIDE, [=] PTX_HD(size_t idx, const PtxScratch& sc) -> PtxStaged {
+// C2: decode the units of a list, one per entry.
+// A unit of its own: the record is built in a small per-thread staging buffer (failed alternatives are rolled back there)
+// and then copied to the pool of staged records; its final place is known only after the sizes are scanned.  Units that
+// report errors (every `call` reserves one), or whose record outgrows the buffer or the pool, are only measured here and
+// written by the second pass (decode_emit_flagged), which also has the function table.
+// A class representative: decoded with tagged output into the class's template, and its signature spelled out.
+struct PtxDecodeListStep {
+    const uint32_t* list;
+    const uint8_t* text;
+    const PtxToken* tokens;
+    const uint16_t* kinds;
+    const PtxModuleLayout* layout;
+    const uint32_t* mtb;
+    const uint32_t* mub;
+    const uint32_t* ustart;
+    const uint32_t* udepth;
+    const uint32_t* udir;
+    const uint32_t* uclass;
+    uint32_t n_modules, cap_staged, cap_funcs;
+    PtxClassStore cs;
+    PtxBulkTable bulk;
+    uint32_t* utmpl;
+    uint32_t* uend;
+    PtxPair* uown;
+    uint8_t* uflag;
+    uint8_t* ustatus;
+    uint32_t* staged;
+    PtxFnEntry* fn_entries;
+    PtxCounters* counters;
+    PTX_HD PtxStaged operator()(size_t idx, const PtxScratch& sc) const {
         PtxStaged ret;
-        size_t u = order[idx];
-        ret.unit = (uint32_t)u;
+        ret.unit = 0;
         ret.n = 0;
-        if (uflag[u] == PTX_UNIT_TEMPLATED) return ret;
-        uint32_t start = ustart[u];
-        uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
+        const uint32_t u = list[idx] & 0x7FFFFFFFu;
+        const bool rep = (list[idx] >> 31) != 0;
+        const uint32_t start = ustart[u];
         // modules without units share their begin with the next one: take the last module that starts at or before u
-        if (u == 0) { PtxPair z; z.a = z.b = 0; usize[0] = z; }
-        if (mod_skip[m]) {
-            PtxPair z;
-            z.a = z.b = 0;
-            usize[u + 1] = z;
-            uend[u] = 0;
-            ustatus[u] = US_OK;
-            uflag[u] = 0;
-            return ret;
-        }
+        const uint32_t m = ptx_upper_bound_u32(mub, n_modules, u) - 1;
+        const uint32_t te = mtb[m + 1];
+        const uint32_t end = u + 1 < mub[m + 1] ? ustart[u + 1] : te;
+        const uint32_t id = rep ? cs.slot_tmpl[uclass[u]] : 0u;
         PtxSink sink;
-        sink.stage = sc.stage;
-        sink.stage_stride = sc.stage_stride;
-        sink.stage_cap = sc.stage_cap < PTX_TMP_STRIDE ? sc.stage_cap : PTX_TMP_STRIDE;
+        if (rep) {
+            sink.words = cs.tmpl_words + (size_t)id * PTX_TMPL_WORDS;
+            sink.tags = cs.tmpl_tags + (size_t)id * PTX_TMPL_WORDS;
+            sink.words_cap = PTX_TMPL_WORDS;
+        } else {
+            sink.stage = sc.stage;
+            sink.stage_stride = sc.stage_stride;
+            sink.stage_cap = sc.stage_cap;
+        }
         PtxResolver res;
         res.module = m;
-        PtxDecoder d(text, tokens, mtb[m + 1], layout[m].text_off + layout[m].text_len, sink, res);
-        d.bulk = bulk_table;
+        PtxDecoder d(text, tokens, te, layout[m].text_off + layout[m].text_len, sink, res);
+        d.bulk = bulk;
         // the unit's first tokens go to the fast window: the decoder looks at every token many times
         {
-            uint32_t avail = mtb[m + 1] - start;
-            uint32_t nwin = avail < sc.win_cap ? avail : sc.win_cap;
+            uint32_t nwin = te - start < sc.win_cap ? te - start : sc.win_cap;
+            if (nwin > end - start + 1u) nwin = end - start + 1u;
             const PtxTokenWord* src = (const PtxTokenWord*)(tokens + start);
-            for (uint32_t k = 0; k < sc.win_cap; k++)
-                if (k < nwin) sc.win[k * sc.win_stride] = src[k];
+            for (uint32_t k = 0; k < nwin; k++) sc.win[k * sc.win_stride] = src[k];
             d.win = sc.win;
             d.win_base = start;
             d.win_n = nwin;
             d.win_stride = sc.win_stride;
         }
-        uint32_t dp = udepth[u];
-        PtxUnitResult r = ptx_decode_unit(d, start, dp & 0x7FFFFFFFu, (dp >> 31) != 0);
+        const uint32_t dp = udepth[u];
+        const PtxUnitResult r = ptx_decode_unit(d, start, dp & 0x7FFFFFFFu, (dp >> 31) != 0);
+        if (rep) {
+            PtxTemplateInfo ti;
+            ti.n_words = sink.nw;
+            ti.n_tokens = end - start;
+            ti.depth1 = (dp & 0x7FFFFFFFu) == 1 ? 1u : 0u;
+            ti.ok = (r.status == US_OK && sink.ne == 0 && sink.peak <= PTX_TMPL_WORDS && !sink.poison && r.kind != U_FUNC && r.end == end &&
+                     d.max_seen < end) ? 1u : 0u;
+            if (ti.ok) {
+                const uint32_t need = ptx_signature_words(tokens, start, ti.n_tokens);
+                const uint32_t at = PTX_COUNT_ADD(&cs.state[1], need);
+                if (at + need <= PTX_SIG_POOL_WORDS) {
+                    cs.sig_off[id] = at;
+                    ptx_signature_write(cs.sig_pool + at, text, tokens, kinds, start, ti.n_tokens, ti.depth1);
+                } else {
+                    ti.ok = 0;
+                }
+            }
+            cs.info[id] = ti;
+            return ret;
+        }
         uend[u] = r.end;
         ustatus[u] = (uint8_t)r.status;
         bool flagged = sink.peak > sink.stage_cap || sink.ne > 0;
-        PtxPair sz;
-        sz.a = flagged ? sink.peak : sink.nw;
-        sz.b = sink.ne;
-        usize[u + 1] = sz;
-        uflag[u] = flagged ? 1 : 0;
-        if (flagged) {
-#ifdef __CUDA_ARCH__
-            atomicAdd(&counters->n_flagged, 1u);
-#else
-            counters->n_flagged++;
-#endif
-        } else {
-            ret.n = sink.nw;
+        if (!flagged && sink.nw) {
+            const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_words, sink.nw);
+            flagged = (uint64_t)at + sink.nw > cap_staged;
+            if (!flagged) {
+                for (uint32_t k = 0; k < sink.nw; k++) staged[at + k] = sc.stage[k * sc.stage_stride];
+                utmpl[u] = at;
+            }
         }
+        uown[u] = PtxPair{flagged ? sink.peak : sink.nw, sink.ne};
+        uflag[u] = flagged ? PTX_UNIT_FLAGGED : PTX_UNIT_STAGED;
+        if (flagged) PTX_COUNT_ADD(&counters->n_flagged, 1);
         if (r.status == US_OK && r.kind == U_FUNC) {
-#ifdef __CUDA_ARCH__
-            uint32_t slot = atomicAdd(&counters->n_funcs, 1u);
-#else
-            uint32_t slot = counters->n_funcs++;
-#endif
+            const uint32_t slot = PTX_COUNT_ADD(&counters->n_funcs, 1);
             PtxFnEntry e;
-            e.unit = (uint32_t)u;
+            e.unit = u;
             e.dir_ord = udir[u];
             e.name_off = tokens[r.name_tok].start;
             e.name_len = ptx_token_len(text, tokens[r.name_tok], layout[m].text_off + layout[m].text_len);
@@ -1023,41 +885,348 @@ inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
             e.n_inputs = r.n_inputs;
             e.module = m;
             e.pad = 0;
-            fn_entries[slot] = e;
+            if (slot < cap_funcs) fn_entries[slot] = e;      // function headers are units of the first list: there is room
         }
         return ret;
-    });
-    // C2: do consecutive units meet, and does every module return to depth 0?  Where they do not, everything from
-    // the top-level directive that holds the first such place to the end of the module is parsed again by one thread
-    // with the reference's recovery rules; the directives in front of it keep their units.  (A module that does not
-    // return to depth 0 went wrong in or behind its last top-level unit: nothing behind an unclosed scope is one.)
-    // mod_bad[m] = 1 + the unit that heads the first bad directive, 0 = none
-    bk.pf("chain_check", n_units, [=] PTX_HD(size_t u) {
+    }
+};
+
+// C3 per unit: a unit of a class with a usable template is checked against the class signature and takes its size; one
+// whose class has none after all goes to the second list
+struct PtxApplyTemplatesStep {
+    const uint8_t* text;
+    const PtxToken* tokens;
+    const uint16_t* kinds;
+    const uint32_t* ustart;
+    const uint32_t* udepth;
+    const uint32_t* uclass;
+    uint32_t cap_list;
+    PtxClassStore cs;
+    uint32_t* list;
+    uint32_t* utmpl;
+    uint32_t* uend;
+    PtxPair* uown;
+    uint8_t* uflag;
+    uint8_t* ustatus;
+    PtxCounters* counters;
+    PTX_HD void operator()(size_t u) const {
+        const uint32_t slot = uclass[u];
+        if (slot == PTX_ABSENT) return;          // in the first list, or not parsed
+        const uint32_t id = cs.slot_tmpl[slot];
+        if (id != PTX_ABSENT) {
+            const PtxTemplateInfo ti = cs.info[id];
+            const uint32_t start = ustart[u];
+            const uint32_t end = u + 1 < counters->n_units ? ustart[u + 1] : counters->n_tokens;
+            const uint32_t depth1 = (udepth[u] & 0x7FFFFFFFu) == 1 ? 1u : 0u;
+            if (ti.ok && end - start == ti.n_tokens &&
+                ptx_signature_matches(cs.sig_pool + cs.sig_off[id], text, tokens, kinds, start, ti.n_tokens, depth1)) {
+                uown[u] = PtxPair{ti.n_words, 0};
+                uend[u] = end;
+                ustatus[u] = US_OK;
+                uflag[u] = PTX_UNIT_TEMPLATED;
+                utmpl[u] = id;
+                return;
+            }
+        }
+        const uint32_t at = PTX_COUNT_ADD(&counters->n_second, 1);
+        if (at < cap_list) list[at] = (uint32_t)u;
+        else PTX_REDO_SET(counters, PTX_REDO_LIST);
+    }
+};
+
+// C4 per unit: do consecutive units meet, and does every module return to depth 0?  Where they do not, everything from
+// the top-level directive that holds the first such place to the end of the module is parsed again by one thread with the
+// reference's recovery rules; the directives in front of it keep their units.  (A module that does not return to depth 0
+// went wrong in or behind its last top-level unit: nothing behind an unclosed scope is one.)
+// mod_bad[m] = ~(the unit that heads the first bad directive), 0 = none
+struct PtxChainCheckStep {
+    const uint32_t* ustart;
+    const uint32_t* udepth;
+    const uint32_t* udir;
+    const uint32_t* uend;
+    const uint8_t* ustatus;
+    const uint32_t* top_unit;
+    const uint32_t* mub;
+    const uint32_t* mtb;
+    const uint32_t* mod_skip;
+    const int32_t* mod_final_scope;
+    uint32_t n_modules;
+    uint32_t* mod_bad;
+    PtxCounters* counters;
+    PTX_HD void operator()(size_t u) const {
         // units lie back to back over the whole batch, and a module's first unit says so in its depth word: the common
         // case (the unit meets the next one, which is in the same module) needs no module look-up
+        const uint32_t n_units = counters->n_units;
         const bool last_of_module = u + 1 == n_units || (udepth[u + 1] >> 31) != 0;
-        const uint32_t next_start = u + 1 < n_units ? ustart[u + 1] : n_tokens;
+        const uint32_t next_start = u + 1 < n_units ? ustart[u + 1] : counters->n_tokens;
         if (!last_of_module && ustatus[u] == US_OK && uend[u] == next_start) return;
-        uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
+        const uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
         if (mod_skip[m]) return;
-        uint32_t next = (u + 1 < mub[m + 1]) ? ustart[u + 1] : mtb[m + 1];
+        const uint32_t next = (u + 1 < mub[m + 1]) ? ustart[u + 1] : mtb[m + 1];
         bool ok = ustatus[u] == US_OK && uend[u] == next;
         if (u + 1 == mub[m + 1]) ok = ok && mod_final_scope[m] == 0;
         if (ok) return;
         const uint32_t head = top_unit[udir[u] - 1];
+        counters->any_sequential = 1;
 #ifdef __CUDA_ARCH__
         atomicMax(&mod_bad[m], 0xFFFFFFFFu - head);       // the smallest head wins
 #else
         if (0xFFFFFFFFu - head > mod_bad[m]) mod_bad[m] = 0xFFFFFFFFu - head;
 #endif
+    }
+};
+
+// A list of more than this many entries is sorted by the shape of its units before it is decoded: the decoder's control
+// flow depends on token kinds only, so the threads of a warp then follow the same path.  Shorter lists are spread over
+// more warps instead (the backend's business).  Results are written at offsets computed in unit order either way.
+#define PTX_SORT_MIN 131072u
+template <class BK>
+inline uint32_t* ptx_sort_list(BK& bk, PtxWork& w, const uint32_t* list, uint32_t n) {
+    uint16_t* key = (uint16_t*)bk.alloc(sizeof(uint16_t) * ((size_t)n + 2));
+    uint32_t* order = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n + 1));
+    uint32_t* sorted = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n + 1));
+    const uint16_t* kinds = w.kinds;
+    const uint32_t* ustart = w.unit_start;
+    const uint32_t* udepth = w.unit_depth;
+    const uint32_t n_units = w.n_units, n_tokens = w.n_tokens;
+    bk.pf("unit_shape_key", n, [=] PTX_HD(size_t x) {
+        const uint32_t u = list[x] & 0x7FFFFFFFu, start = ustart[u];
+        uint32_t end = u + 1 < n_units ? ustart[u + 1] : n_tokens;
+        if (end > start + 20) end = start + 20;
+        uint32_t h = 2166136261u ^ (udepth[u] >> 31) ^ ((udepth[u] & 0x7FFFFFFFu) ? 2u : 0u);
+        for (uint32_t i = start; i < end; i++) h = (h ^ PTX_KL_KIND(kinds[i])) * 16777619u;
+        h ^= h >> 15;
+        key[x] = (uint16_t)(h & (PTX_SORT_BUCKETS - 1));
     });
+    bk.sort_by_key("sort_units_by_shape", n, key, order);
+    bk.pf("gather_sorted_list", n, [=] PTX_HD(size_t x) { sorted[x] = list[order[x]]; });
+    return sorted;
+}
+
+// Bulk path: the elements of each listed statement's initialiser are decoded one thread per element into a dense
+// run; the statement's own decoder later takes the run in one step (PtxDecoder::multi_variable).  A list that is
+// not plainly "element, element, ... }" followed by ';' stays marked bad and is decoded the ordinary way.
+template <class BK>
+inline void ptx_bulk_elements(BK& bk, PtxWork& w, PtxBulkInfo* bulk_info, uint32_t n_bulk) {
+    const uint8_t* text = w.text;
+    const PtxToken* tokens = w.tokens;
+    const uint16_t* kinds = w.kinds;
+    const PtxModuleLayout* layout = w.layout;
+    const uint32_t* mtb = w.mod_tok_begin;
+    const uint32_t n_modules = w.n_modules;
+    PtxBulkInfo host_bulk[PTX_MAX_BULK];
+    bk.download(host_bulk, bulk_info, sizeof(PtxBulkInfo) * n_bulk);
+    for (uint32_t j = 0; j < n_bulk; j++) {
+        const uint32_t ts = host_bulk[j].first_tok, te = host_bulk[j].close_tok, nt = te - ts;
+        w.bulk_tokens[j] = nt;
+        PtxBulkInfo* bi = bulk_info + j;
+        uint32_t* lo_dev = (uint32_t*)bk.alloc(sizeof(uint32_t) * 4);
+        PtxPair* esz = (PtxPair*)bk.alloc(sizeof(PtxPair) * ((size_t)nt + 2));
+        uint32_t* elems = (uint32_t*)bk.alloc(sizeof(uint32_t) * (2 * (size_t)nt + 8));
+        bk.pf("bulk_reset", 1, [=] PTX_HD(size_t) { lo_dev[0] = PTX_ABSENT; lo_dev[1] = 0; });
+        bk.pf("bulk_find_open", nt, [=] PTX_HD(size_t k) {
+            uint32_t i = ts + (uint32_t)k;
+            if (i > ts && PTX_KL_KIND(kinds[i]) == T_LBRACE && PTX_KL_KIND(kinds[i - 1]) == T_EQ) {
+#ifdef __CUDA_ARCH__
+                atomicMin(&lo_dev[0], i);
+#else
+                if (i < lo_dev[0]) lo_dev[0] = i;
+#endif
+            }
+        });
+        bk.pf("bulk_measure", nt, [=] PTX_HD(size_t k) {
+            uint32_t i = ts + (uint32_t)k;
+            PtxPair z;
+            z.a = z.b = 0;
+            esz[k] = z;
+            const uint32_t lo = lo_dev[0], hi = te - 2;
+            bool shape_ok = lo != PTX_ABSENT && nt >= 6 && lo + 1 < hi && PTX_KL_KIND(kinds[te - 2]) == T_RBRACE &&
+                            PTX_KL_KIND(kinds[te - 1]) == T_SEMI && PTX_KL_KIND(kinds[hi - 1]) != T_COMMA;
+            if (!shape_ok) { if (k == 0) lo_dev[1] = 1; return; }
+            if (i <= lo || i >= hi) return;
+            uint16_t kd = PTX_KL_KIND(kinds[i]);
+            if (kd == T_LBRACE || kd == T_RBRACE) { lo_dev[1] = 1; return; }
+            if (!(i == lo + 1 || PTX_KL_KIND(kinds[i - 1]) == T_COMMA)) return;
+            // an element starts here: measure it
+            uint32_t mm = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
+            PtxSink sink;
+            PtxResolver res;
+            PtxDecoder d(text, tokens, mtb[mm + 1], layout[mm].text_off + layout[mm].text_len, sink, res);
+            d.pos = i;
+            d.unit_tok0 = i;
+            bool ok = d.reg_or_immediate(true) && sink.ne == 0 && d.pos <= hi;
+            if (ok) {
+                uint16_t nk = PTX_KL_KIND(kinds[d.pos]);
+                ok = (d.pos == hi) || nk == T_COMMA;
+            }
+            if (!ok) { lo_dev[1] = 1; return; }
+            z.a = sink.nw;
+            z.b = 1;
+            esz[k] = z;
+        });
+        bk.template scan<PtxPair>("bulk_scan", (size_t)nt, [=] PTX_HD(size_t k) { return esz[k]; }, [=] PTX_HD(size_t k, PtxPair v) {
+                                      PtxPair own = esz[k];
+                                      if (k + 1 == nt) {     // totals, before the entry turns exclusive
+                                          bi->n_words = v.a;
+                                          bi->n_elems = v.b;
+                                      }
+                                      PtxPair ex;
+                                      ex.a = v.a - own.a;
+                                      ex.b = own.b;      // keeps "an element starts here"
+                                      esz[k] = ex;
+                                  },
+                                  PairAddOp(), PtxPair{0, 0});
+        bk.pf("bulk_decode", nt, [=] PTX_HD(size_t k) {
+            if (lo_dev[1] || !esz[k].b) return;
+            uint32_t i = ts + (uint32_t)k;
+            uint32_t mm = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
+            PtxSink sink;
+            sink.words = elems + esz[k].a;
+            PtxResolver res;
+            PtxDecoder d(text, tokens, mtb[mm + 1], layout[mm].text_off + layout[mm].text_len, sink, res);
+            d.pos = i;
+            d.unit_tok0 = i;
+            d.reg_or_immediate(true);
+        });
+        bk.pf("bulk_publish", 1, [=] PTX_HD(size_t) {
+            bi->first_tok = lo_dev[0] + 1;
+            bi->close_tok = te - 2;
+            bi->bad = lo_dev[1];
+            bi->elems = elems;
+            bi->dst = nullptr;
+        });
+    }
+}
+
+// Everything up to the size of every unit's records
+template <class BK>
+inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
+    const uint32_t n_modules = w.n_modules;
+    PtxCounters* counters = w.counters;
+    const size_t nu = w.deferred ? w.cap_units : w.n_units;
+    w.unit_end = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
+    w.unit_own = (PtxPair*)bk.alloc(sizeof(PtxPair) * (nu + 1));
+    w.unit_size = (PtxPair*)bk.alloc(sizeof(PtxPair) * (nu + 2));
+    w.unit_status = (uint8_t*)bk.alloc(nu + 16);
+    w.unit_flag = (uint8_t*)bk.alloc(nu + 16);
+    w.unit_tmpl = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
+    uint32_t* uclass = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
+    w.mod_bad = ptx_zalloc<uint32_t>(bk, n_modules + 1);
+    w.mod_seq_size = ptx_zalloc<PtxPair>(bk, n_modules + 1);
+    w.mod_seq_status = ptx_zalloc<uint32_t>(bk, n_modules + 1);
+    if (!PtxStructureTops<BK>::value) {
+        // ordinal of the enclosing top-level unit, and the unit that heads each ordinal (a module's first unit, or a
+        // top-level directive's first)
+        uint32_t* udir = w.unit_dir = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
+        uint32_t* top_unit = w.unit_top = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
+        const uint32_t* udepth = w.unit_depth;
+        bk.template scan<uint32_t>("scan_toplevel_ordinal", nu, [=] PTX_HD(size_t u) { return (udepth[u] & 0x7FFFFFFFu) == 0 ? 1u : 0u; },
+                                   [=] PTX_HD(size_t u, uint32_t v) { udir[u] = v; }, AddOp(), 0u);
+        bk.pf("list_toplevel_units", nu, [=] PTX_HD(size_t u) {
+            if ((udepth[u] & 0x7FFFFFFFu) == 0) top_unit[udir[u] - 1] = (uint32_t)u;
+        });
+    }
+    // ---- classes
+    const uint32_t cap_list = w.deferred ? w.cap_list : (uint32_t)nu;
+    uint32_t* first = w.list = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)cap_list + 1));
+    uint32_t* second = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)cap_list + 1));
+    PtxBulkInfo* bulk_info = (PtxBulkInfo*)bk.alloc(sizeof(PtxBulkInfo) * PTX_MAX_BULK);
+    const PtxClassStore cs = w.cs = bk.class_store(w.first_slice);
+    bk.pf("unit_classes", w.units_n(),
+          PtxUnitClassesStep{w.text, w.tokens, w.kinds, w.unit_start, w.unit_depth, w.mod_unit_begin, w.mod_skip, n_modules, cap_list, w.deferred, counters, cs,
+                             bulk_info, uclass, w.unit_tmpl, w.unit_end, first, w.unit_own, w.unit_flag, w.unit_status});
+    if (!w.deferred) bk.download(&host_counters, counters, sizeof(PtxCounters));
+    // ---- bulk initialisers
+    w.bulk = PtxBulkTable();
+    if (!w.deferred && host_counters.n_bulk) {
+        w.bulk.info = bulk_info;
+        w.bulk.n = host_counters.n_bulk < PTX_MAX_BULK ? host_counters.n_bulk : PTX_MAX_BULK;
+        ptx_bulk_elements(bk, w, bulk_info, w.bulk.n);
+    }
+    // ---- first list: units without a class, and the representatives of the classes this slice added
+    const uint32_t n_first = host_counters.n_first;
+    // the pool of staged records: what does not fit is measured now and written by the second decode pass
+    const size_t pool = w.deferred ? 64 * (size_t)cap_list : 32 * ((size_t)n_first + (nu - n_first < (1u << 20) ? nu - n_first : (1u << 20))) + 4096;
+    const uint32_t cap_staged = pool < 0xFFFF0000u ? (uint32_t)pool : 0xFFFF0000u;
+    const uint32_t cap_funcs = w.deferred ? cap_list : n_first;
+    w.staged = (uint32_t*)bk.alloc(sizeof(uint32_t) * (size_t)cap_staged);
+    w.fn_entries = (PtxFnEntry*)bk.alloc(sizeof(PtxFnEntry) * ((size_t)cap_funcs + 1));
+    if (!w.deferred && n_first > PTX_SORT_MIN) w.list = ptx_sort_list(bk, w, first, n_first);
+    PtxDecodeListStep step{w.list, w.text, w.tokens, w.kinds, w.layout, w.mod_tok_begin, w.mod_unit_begin, w.unit_start, w.unit_depth, w.unit_dir, uclass,
+                           n_modules, cap_staged, cap_funcs, cs, w.bulk, w.unit_tmpl, w.unit_end, w.unit_own, w.unit_flag, w.unit_status, w.staged,
+                           w.fn_entries, counters};
+    bk.pf_staged("decode_first", w.deferred ? PtxCount(cap_list, &counters->n_first) : PtxCount(n_first), w.staged, 0, step);
+    // ---- templates, and the units that have none after all
+    bk.pf("apply_templates", w.units_n(),
+          PtxApplyTemplatesStep{w.text, w.tokens, w.kinds, w.unit_start, w.unit_depth, uclass, cap_list, cs, second, w.unit_tmpl, w.unit_end, w.unit_own,
+                                w.unit_flag, w.unit_status, counters});
+    w.second = second;
+    if (!w.deferred) {
+        bk.download(&host_counters, counters, sizeof(PtxCounters));
+        if (host_counters.n_second > PTX_SORT_MIN) w.second = ptx_sort_list(bk, w, second, host_counters.n_second);
+    }
+    step.list = w.second;
+    bk.pf_staged("decode_second", w.deferred ? PtxCount(cap_list, &counters->n_second) : PtxCount(host_counters.n_second), w.staged, 0, step);
+}
+
+inline PtxChainCheckStep ptx_chain_check(const PtxWork& w) {
+    return PtxChainCheckStep{w.unit_start, w.unit_depth, w.unit_dir, w.unit_end, w.unit_status, w.unit_top, w.mod_unit_begin, w.mod_tok_begin, w.mod_skip,
+                             w.mod_final_scope, w.n_modules, w.mod_bad, w.counters};
+}
+// sizes -> offsets and totals; with `check` the chain check rides along (each unit's size is read once, by one thread)
+template <class BK>
+inline void ptx_scan_sizes(BK& bk, PtxWork& w, bool check) {
+    PtxPair* usize = w.unit_size;
+    const PtxPair* uown = w.unit_own;
+    PtxCounters* counters = w.counters;
+    const PtxClassStore cs = w.cs;
+    const uint32_t cap_words = w.deferred ? w.cap_words : 0xFFFFFFFFu;
+    const bool deferred = w.deferred;
+    auto store = [=] PTX_HD(size_t i, PtxPair v) {
+        usize[i] = v;
+        if (i != counters->n_units) return;
+        counters->n_words = v.a;
+        counters->n_errs = v.b;
+        counters->n_rest = counters->n_first - counters->n_reps + counters->n_second;
+        counters->n_classes = cs.state[0];
+        counters->n_sig_words = cs.state[1];
+        if (v.a > cap_words) PTX_REDO_SET(counters, PTX_REDO_WORDS);
+        if (!deferred && counters->any_sequential) counters->n_flagged += 1;
+    };
+    if (check) {
+        const PtxChainCheckStep chain = ptx_chain_check(w);
+        bk.template scan<PtxPair>("scan_unit_sizes", w.units_n(1), [=] PTX_HD(size_t i) {
+            if (i == 0) return PtxPair{0, 0};
+            chain(i - 1);
+            return uown[i - 1];
+        }, store, PairAddOp(), PtxPair{0, 0});
+    } else {
+        bk.template scan<PtxPair>("scan_unit_sizes", w.units_n(1), [=] PTX_HD(size_t i) { return i ? uown[i - 1] : PtxPair{0, 0}; }, store, PairAddOp(), PtxPair{0, 0});
+    }
+}
+// the modules that the chain check found damaged: their tails through the one-thread parser (sizes)
+template <class BK>
+inline void ptx_sequential_sizes(BK& bk, PtxWork& w) {
+    const uint8_t* text = w.text;
+    const PtxToken* tokens = w.tokens;
+    const PtxModuleLayout* layout = w.layout;
+    const uint32_t* mtb = w.mod_tok_begin;
+    const uint32_t* mub = w.mod_unit_begin;
+    const uint32_t* ustart = w.unit_start;
+    uint32_t* mod_bad = w.mod_bad;
+    PtxPair* mod_seq = w.mod_seq_size;
+    uint32_t* mod_seq_status = w.mod_seq_status;
+    PtxPair* uown = w.unit_own;
+    uint8_t* uflag = w.unit_flag;
+    PtxCounters* counters = w.counters;
+    const uint32_t seq_max_tokens = w.seq_max_tokens, n_modules = w.n_modules;
+    const PtxBulkTable bulk = w.bulk;
+    // mod_bad[m] becomes 1 + the unit that heads the first bad directive
     bk.pf("first_bad_directive", n_modules, [=] PTX_HD(size_t m) {
         if (mod_bad[m]) mod_bad[m] = (0xFFFFFFFFu - mod_bad[m]) + 1u;
     });
-    // C3: the sequential parse, one thread per such module (count)
     bk.pf("sequential_count", n_modules, [=] PTX_HD(size_t m) {
         if (!mod_bad[m]) return;
-        counters->any_sequential = 1;
         const uint32_t head = mod_bad[m] - 1u;
         if (mtb[m + 1] - ustart[head] > seq_max_tokens) {
             mod_seq_status[m] = US_REFUSED;       // sizes stay 0: the module's verdict says so, nothing is parsed
@@ -1066,7 +1235,7 @@ inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
         PtxSink sink;
         PtxResolver res;
         PtxDecoder d(text, tokens, mtb[m + 1], layout[m].text_off + layout[m].text_len, sink, res);
-        d.bulk = bulk_table;
+        d.bulk = bulk;
         int st = ptx_decode_module_sequential(d, ustart[head], 0, head != mub[m]);
         PtxPair sz;
         sz.a = sink.peak;
@@ -1074,59 +1243,73 @@ inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
         mod_seq[m] = sz;
         mod_seq_status[m] = (uint32_t)st;
     });
-    // C4: its sizes replace those of the units it covers
-    bk.pf("merge_sequential_sizes", n_units, [=] PTX_HD(size_t u) {
+    // its sizes replace those of the units it covers
+    bk.pf("merge_sequential_sizes", w.n_units, [=] PTX_HD(size_t u) {
         if (!counters->any_sequential) return;       // no module of this slice needs the sequential parser
         uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
         if (!mod_bad[m] || u < mod_bad[m] - 1u) return;
         PtxPair z;
         z.a = z.b = 0;
         const bool head = u == mod_bad[m] - 1u;
-        usize[u + 1] = head ? mod_seq[m] : z;
-        uflag[u] = head ? 1 : 2;    // the head unit stands for the whole tail in C6; the others write nothing
+        uown[u] = head ? mod_seq[m] : z;
+        uflag[u] = head ? PTX_UNIT_FLAGGED : PTX_UNIT_NOTHING;    // the head stands for the whole tail in the second pass; the others write nothing
     });
-    bk.template scan<PtxPair>("scan_unit_sizes", (size_t)n_units + 1, [=] PTX_HD(size_t i) { return usize[i]; },
-                              [=] PTX_HD(size_t i, PtxPair v) { usize[i] = v; }, PairAddOp(), PtxPair{0, 0});
-    bk.pf("set_output_totals", 1, [=] PTX_HD(size_t) {
-        counters->n_words = n_units ? usize[n_units].a : 0;
-        counters->n_errs = n_units ? usize[n_units].b : 0;
-        if (counters->any_sequential) counters->n_flagged += 1;
-    });
-    bk.download(&host_counters, counters, sizeof(PtxCounters));
-    const uint32_t n_words = host_counters.n_words, n_errs = host_counters.n_errs, n_funcs = host_counters.n_funcs;
-    uint32_t* words = w.words = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n_words + 4));
-    PtxErrRec* errs = w.errs = (PtxErrRec*)bk.alloc(sizeof(PtxErrRec) * ((size_t)n_errs + 1));
-    // C5: records of the units that were staged go to their final place
-    // one thread per output word (the backend maps words to units): staged records come from their table row,
-    // templated ones are instantiated from the class template and the unit's own tokens
-    // Literal values are converted in a second round, one thread per literal with the warps full: the low-word thread
-    // also writes the high word when the template has it next (the two value words of an immediate)
-    bk.emit_records("emit_records", n_units, usize, PtxEmitStep{uflag, utmpl, ustart, table, cs, tokens, text, words});
-    if (host_counters.n_flagged) {
-        // function table for `call`
-        uint32_t mask = 1;
-        while (mask < 2 * n_funcs + 2) mask <<= 1;
-        mask -= 1;
-        uint32_t* slots = w.fn_slots = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)mask + 1));
-        w.fn_mask = mask;
-        bk.pf("fn_table_clear", (size_t)mask + 1, [=] PTX_HD(size_t i) { slots[i] = PTX_ABSENT; });
-        bk.pf("fn_table_insert", n_funcs, [=] PTX_HD(size_t i) {
-            const PtxFnEntry e = fn_entries[i];
-            uint32_t h = ptx_name_hash(text, e.name_off, e.name_len, e.module) & mask;
-            for (;;) {
+}
+template <class BK>
+inline void ptx_emit_records(BK& bk, PtxWork& w) {
+    bk.emit_records("emit_records", w.units_n(), w.unit_size,
+                    PtxEmitStep{w.unit_flag, w.unit_tmpl, w.unit_start, w.staged, w.cs, w.tokens, w.text, w.words});
+}
+// the flagged units are decoded again, writing in place
+template <class BK>
+inline void ptx_emit_flagged(BK& bk, PtxWork& w, const PtxCounters& host_counters) {
+    if (!host_counters.n_flagged) return;
+    const uint8_t* text = w.text;
+    const PtxToken* tokens = w.tokens;
+    const PtxModuleLayout* layout = w.layout;
+    const uint32_t* mtb = w.mod_tok_begin;
+    const uint32_t* mub = w.mod_unit_begin;
+    const uint32_t* ustart = w.unit_start;
+    const uint32_t* udepth = w.unit_depth;
+    const uint32_t* udir = w.unit_dir;
+    const uint32_t* mod_skip = w.mod_skip;
+    const uint32_t* mod_bad = w.mod_bad;
+    const uint32_t* mod_seq_status = w.mod_seq_status;
+    const uint8_t* uflag = w.unit_flag;
+    const PtxPair* usize = w.unit_size;
+    const PtxFnEntry* fn_entries = w.fn_entries;
+    uint32_t* words = w.words;
+    PtxErrRec* errs = w.errs;
+    PtxCounters* counters = w.counters;
+    const PtxBulkTable bulk_table = w.bulk;
+    const uint32_t n_modules = w.n_modules, n_funcs = host_counters.n_funcs;
+    // function table for `call`
+    uint32_t mask = 1;
+    while (mask < 2 * n_funcs + 2) mask <<= 1;
+    mask -= 1;
+    uint32_t* slots = w.fn_slots = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)mask + 1));
+    w.fn_mask = mask;
+    bk.pf("fn_table_clear", (size_t)mask + 1, [=] PTX_HD(size_t i) { slots[i] = PTX_ABSENT; });
+    bk.pf("fn_table_insert", n_funcs, [=] PTX_HD(size_t i) {
+        const PtxFnEntry e = fn_entries[i];
+        uint32_t h = ptx_name_hash(text, e.name_off, e.name_len, e.module) & mask;
+        for (;;) {
 #ifdef __CUDA_ARCH__
-                uint32_t old = atomicCAS(&slots[h], PTX_ABSENT, (uint32_t)i);
+            uint32_t old = atomicCAS(&slots[h], PTX_ABSENT, (uint32_t)i);
 #else
-                uint32_t old = slots[h];
-                if (old == PTX_ABSENT) slots[h] = (uint32_t)i;
+            uint32_t old = slots[h];
+            if (old == PTX_ABSENT) slots[h] = (uint32_t)i;
 #endif
-                if (old == PTX_ABSENT) break;
-                h = (h + 1) & mask;
-            }
-        });
-        // C6: decode the flagged units again, writing in place
-    bk.pf("decode_emit_flagged", n_rest, [=] PTX_HD(size_t idx) {
-        size_t u = order[idx];
+            if (old == PTX_ABSENT) break;
+            h = (h + 1) & mask;
+        }
+    });
+    const uint32_t* list = w.list;
+    const uint32_t* second = w.second;
+    const uint32_t n_first = host_counters.n_first;
+    bk.pf("decode_emit_flagged", (size_t)n_first + host_counters.n_second, [=] PTX_HD(size_t idx) {
+        const size_t u = idx < n_first ? list[idx] & 0x7FFFFFFFu : second[idx - n_first];
+        if (idx < n_first && (list[idx] >> 31)) return;
         if (uflag[u] != 1) return;
         uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
         PtxSink sink;
@@ -1168,45 +1351,126 @@ inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
         if (sink.peak != usize[u + 1].a - usize[u].a || sink.ne != usize[u + 1].b - usize[u].b) counters->pad = (uint32_t)u + 1;
         sink.pad_to(usize[u + 1].a - usize[u].a);
     });
+}
+// the rows of the modules, finished
+template <class BK>
+inline void ptx_module_results(BK& bk, PtxWork& w, uint32_t n_errs) {
+    const uint32_t n_modules = w.n_modules;
+    const uint32_t* mtb = w.mod_tok_begin;
+    const uint32_t* mub = w.mod_unit_begin;
+    const uint32_t* ustart = w.unit_start;
+    const PtxPair* usize = w.unit_size;
+    const PtxErrRec* errs = w.errs;
+    const uint32_t* mod_bad = w.mod_bad;
+    const uint32_t* mod_seq_status = w.mod_seq_status;
+    const PtxModuleResult* results = w.results;
+    PtxModuleResult* out = w.results_out ? w.results_out : w.results;
+    PtxCounters* counters_out = w.counters_out;
+    const PtxCounters* counters = w.counters;
+    const bool deferred = w.deferred;
+    uint32_t* mod_nerr = nullptr;
+    if (n_errs) {
+        // parser errors per module, so that a module's verdict can be read off its result row
+        mod_nerr = ptx_zalloc<uint32_t>(bk, n_modules + 1);
+        bk.pf("count_module_errors", n_errs, [=] PTX_HD(size_t e) {
+            if ((errs[e].w0 & 0xFFFFu) == E_NONE) return;
+            uint32_t lo = 0, hi = n_modules;       // last module whose errors begin at or before e
+            while (hi - lo > 1) {
+                uint32_t mid = (lo + hi) >> 1;
+                if (usize[mub[mid]].b <= (uint32_t)e) lo = mid; else hi = mid;
+            }
+            PTX_COUNT_ADD(&mod_nerr[lo], 1);
+        });
     }
+    PtxCount rows(n_modules);
+    rows.always = true;
+    bk.pf("module_results_final", rows, [=] PTX_HD(size_t m) {
+        if (m == 0 && counters_out) *counters_out = *counters;
+        if (counters->redo) return;
+        PtxModuleResult r = results[m];
+        const bool any = counters->n_units != 0;
+        r.n_errors = mod_nerr ? mod_nerr[m] : 0u;
+        r.unit_begin = mub[m];
+        r.unit_end = mub[m + 1];
+        r.word_begin = any ? usize[mub[m]].a : 0;
+        r.word_end = any ? usize[mub[m + 1]].a : 0;
+        r.err_begin = any ? usize[mub[m]].b : 0;
+        r.err_end = any ? usize[mub[m + 1]].b : 0;
+        const uint32_t bad = deferred ? 0u : mod_bad[m];      // (with deferred counts a slice with a bad module is finished by a second round)
+        r.sequential = bad ? 1u : 0u;
+        r.status = mod_seq_status[m];
+        r.seq_tokens = bad ? mtb[m + 1] - ustart[bad - 1u] : 0u;
+        out[m] = r;
+    });
+}
+
+template <class BK>
+inline void ptx_bulk_copy(BK& bk, PtxWork& w) {
     // the element runs of the bulk path go where the statements' decoders left room for them
-    for (uint32_t j = 0; j < n_bulk; j++) {
-        const PtxBulkInfo* bi = bulk_info + j;
-        bk.pf("bulk_copy", 2 * (size_t)bulk_tokens[j], [=] PTX_HD(size_t k) {
+    for (uint32_t j = 0; j < w.bulk.n; j++) {
+        const PtxBulkInfo* bi = w.bulk.info + j;
+        bk.pf("bulk_copy", 2 * (size_t)w.bulk_tokens[j], [=] PTX_HD(size_t k) {
             if (bi->bad || !bi->dst || k >= bi->n_words) return;
             bi->dst[k] = bi->elems[k];
         });
     }
-    // parser errors per module, so that a module's verdict can be read off its result row
-    uint32_t* mod_nerr = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 1));
-    bk.zero(mod_nerr, sizeof(uint32_t) * (n_modules + 1));
-    bk.pf("count_module_errors", n_errs, [=] PTX_HD(size_t e) {
-        if ((errs[e].w0 & 0xFFFFu) == E_NONE) return;
-        uint32_t lo = 0, hi = n_modules;       // last module whose errors begin at or before e
-        while (hi - lo > 1) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (usize[mub[mid]].b <= (uint32_t)e) lo = mid; else hi = mid;
-        }
-#ifdef __CUDA_ARCH__
-        atomicAdd(&mod_nerr[lo], 1u);
-#else
-        mod_nerr[lo]++;
-#endif
-    });
-    bk.pf("module_results_final", n_modules, [=] PTX_HD(size_t m) {
-        PtxModuleResult r = results[m];
-        r.n_errors = mod_nerr[m];
-        r.unit_begin = mub[m];
-        r.unit_end = mub[m + 1];
-        r.word_begin = n_units ? usize[mub[m]].a : 0;
-        r.word_end = n_units ? usize[mub[m + 1]].a : 0;
-        r.err_begin = n_units ? usize[mub[m]].b : 0;
-        r.err_end = n_units ? usize[mub[m + 1]].b : 0;
-        r.sequential = mod_bad[m] ? 1u : 0u;
-        r.status = mod_seq_status[m];
-        r.seq_tokens = mod_bad[m] ? mtb[m + 1] - ustart[mod_bad[m] - 1u] : 0u;
-        results[m] = r;
-    });
+}
+
+// Sizes known: offsets, records, second decode pass, module rows; the host reads the counts on the way.
+// again = a slice whose first round ran with deferred counts: its units are decoded and checked
+template <class BK>
+inline void ptx_decode_finish(BK& bk, PtxWork& w, PtxCounters& host_counters, bool again) {
+    PtxCounters* counters = w.counters;
+    if (!again) bk.pf("chain_check", w.n_units, ptx_chain_check(w));
+    if (!again || host_counters.any_sequential) {
+        ptx_sequential_sizes(bk, w);
+        ptx_scan_sizes(bk, w, false);
+        bk.download(&host_counters, counters, sizeof(PtxCounters));
+    }
+    if (!again || host_counters.n_words > w.cap_words) {
+        w.words = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)host_counters.n_words + 4));
+        w.cap_words = host_counters.n_words;
+    }
+    w.errs = (PtxErrRec*)bk.alloc(sizeof(PtxErrRec) * ((size_t)host_counters.n_errs + 1));
+    if (!again || host_counters.any_sequential) ptx_emit_records(bk, w);
+    ptx_emit_flagged(bk, w, host_counters);
+    ptx_bulk_copy(bk, w);
+    ptx_module_results(bk, w, host_counters.n_errs);
     bk.download(&host_counters, counters, sizeof(PtxCounters));   // .pad != 0: unit (index + 1) whose two passes disagreed
-    (void)n_tokens;
+}
+
+template <class BK>
+inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
+    ptx_decode_units(bk, w, host_counters);
+    if (!w.deferred) { ptx_decode_finish(bk, w, host_counters, false); return; }
+    // nothing is read back: the caller looks at the counters when everything has run, and calls ptx_stage_again or runs
+    // the slice anew if they ask for it
+    ptx_scan_sizes(bk, w, true);
+    ptx_emit_records(bk, w);
+    ptx_module_results(bk, w, 0);
+}
+// Second round of a slice that ran with deferred counts and has lexer errors, damaged modules or flagged units
+// (host_counters = the counters of the first round)
+inline bool ptx_needs_again(const PtxCounters& c) { return c.n_lexerrs || c.any_sequential || c.n_flagged || c.n_errs; }
+template <class BK>
+inline void ptx_stage_again(BK& bk, PtxWork& w, PtxCounters& host_counters) {
+    w.deferred = false;
+    w.n_tokens = host_counters.n_tokens;
+    w.n_units = host_counters.n_units;
+    ptx_lex_errors(bk, w, host_counters.n_lexerrs);
+    ptx_decode_finish(bk, w, host_counters, true);
+}
+// The decode stage of a slice that stopped itself in or behind it (PTX_REDO_DECODE), with the host reading the counts
+template <class BK>
+inline void ptx_stage_decode_anew(BK& bk, PtxWork& w, PtxCounters& host_counters) {
+    PtxCounters* counters = w.counters;
+    w.deferred = false;
+    w.n_tokens = host_counters.n_tokens;
+    w.n_units = host_counters.n_units;
+    bk.pf("reset_decode_counters", 1, [=] PTX_HD(size_t) {
+        counters->n_bulk = counters->n_first = counters->n_reps = counters->n_second = counters->n_flagged = counters->n_funcs = 0;
+        counters->n_staged_words = counters->any_sequential = counters->redo = 0;
+    });
+    ptx_lex_errors(bk, w, host_counters.n_lexerrs);
+    ptx_stage_decode(bk, w, host_counters);
 }
