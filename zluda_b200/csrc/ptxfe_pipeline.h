@@ -842,10 +842,10 @@ struct PtxDecodeListStep {
         const PtxUnitResult r = ptx_decode_unit(d, start, dp & 0x7FFFFFFFu, (dp >> 31) != 0);
         if (rep) {
             PtxTemplateInfo ti;
-            ti.n_words = sink.nw;
+            ti.n_words = d.out.nw;
             ti.n_tokens = end - start;
             ti.depth1 = (dp & 0x7FFFFFFFu) == 1 ? 1u : 0u;
-            ti.ok = (r.status == US_OK && sink.ne == 0 && sink.peak <= PTX_TMPL_WORDS && !sink.poison && r.kind != U_FUNC && r.end == end &&
+            ti.ok = (r.status == US_OK && d.out.ne == 0 && d.out.high() <= PTX_TMPL_WORDS && !d.out.poison && r.kind != U_FUNC && r.end == end &&
                      d.max_seen < end) ? 1u : 0u;
             if (ti.ok) {
                 const uint32_t need = ptx_signature_words(tokens, start, ti.n_tokens);
@@ -862,16 +862,16 @@ struct PtxDecodeListStep {
         }
         uend[u] = r.end;
         ustatus[u] = (uint8_t)r.status;
-        bool flagged = sink.peak > sink.stage_cap || sink.ne > 0;
-        if (!flagged && sink.nw) {
-            const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_words, sink.nw);
-            flagged = (uint64_t)at + sink.nw > cap_staged;
+        bool flagged = d.out.high() > d.out.stage_cap || d.out.ne > 0;
+        if (!flagged && d.out.nw) {
+            const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_words, d.out.nw);
+            flagged = (uint64_t)at + d.out.nw > cap_staged;
             if (!flagged) {
-                for (uint32_t k = 0; k < sink.nw; k++) staged[at + k] = sc.stage[k * sc.stage_stride];
+                for (uint32_t k = 0; k < d.out.nw; k++) staged[at + k] = sc.stage[k * sc.stage_stride];
                 utmpl[u] = at;
             }
         }
-        uown[u] = PtxPair{flagged ? sink.peak : sink.nw, sink.ne};
+        uown[u] = PtxPair{flagged ? d.out.high() : d.out.nw, d.out.ne};
         uflag[u] = flagged ? PTX_UNIT_FLAGGED : PTX_UNIT_STAGED;
         if (flagged) PTX_COUNT_ADD(&counters->n_flagged, 1);
         if (r.status == US_OK && r.kind == U_FUNC) {
@@ -1054,13 +1054,13 @@ inline void ptx_bulk_elements(BK& bk, PtxWork& w, PtxBulkInfo* bulk_info, uint32
             PtxDecoder d(text, tokens, mtb[mm + 1], layout[mm].text_off + layout[mm].text_len, sink, res);
             d.pos = i;
             d.unit_tok0 = i;
-            bool ok = d.reg_or_immediate(true) && sink.ne == 0 && d.pos <= hi;
+            bool ok = d.reg_or_immediate(true) && d.out.ne == 0 && d.pos <= hi;
             if (ok) {
                 uint16_t nk = PTX_KL_KIND(kinds[d.pos]);
                 ok = (d.pos == hi) || nk == T_COMMA;
             }
             if (!ok) { lo_dev[1] = 1; return; }
-            z.a = sink.nw;
+            z.a = d.out.nw;
             z.b = 1;
             esz[k] = z;
         });
@@ -1238,8 +1238,8 @@ inline void ptx_sequential_sizes(BK& bk, PtxWork& w) {
         d.bulk = bulk;
         int st = ptx_decode_module_sequential(d, ustart[head], 0, head != mub[m]);
         PtxPair sz;
-        sz.a = sink.peak;
-        sz.b = sink.ne;
+        sz.a = d.out.high();
+        sz.b = d.out.ne;
         mod_seq[m] = sz;
         mod_seq_status[m] = (uint32_t)st;
     });
@@ -1332,8 +1332,8 @@ inline void ptx_emit_flagged(BK& bk, PtxWork& w, const PtxCounters& host_counter
             PtxDecoder d(text, tokens, mtb[m + 1], text_end, sink, res);
             d.bulk = bulk_table;
             ptx_decode_module_sequential(d, ustart[u], usize[u].a, u != mub[m]);
-            if (sink.peak != usize[u + 1].a - usize[u].a || sink.ne != usize[u + 1].b - usize[u].b) counters->pad = (uint32_t)u + 1;
-            sink.pad_to(usize[u + 1].a - usize[u].a);
+            if (d.out.high() != usize[u + 1].a - usize[u].a || d.out.ne != usize[u + 1].b - usize[u].b) counters->pad = (uint32_t)u + 1;
+            d.out.pad_to(usize[u + 1].a - usize[u].a);
             return;
         }
         PtxResolver res;
@@ -1348,8 +1348,8 @@ inline void ptx_emit_flagged(BK& bk, PtxWork& w, const PtxCounters& host_counter
         uint32_t dp = udepth[u];
         ptx_decode_unit(d, ustart[u], dp & 0x7FFFFFFFu, (dp >> 31) != 0);
         // both passes must agree on the size of every record (a mismatch would overwrite a neighbour's record)
-        if (sink.peak != usize[u + 1].a - usize[u].a || sink.ne != usize[u + 1].b - usize[u].b) counters->pad = (uint32_t)u + 1;
-        sink.pad_to(usize[u + 1].a - usize[u].a);
+        if (d.out.high() != usize[u + 1].a - usize[u].a || d.out.ne != usize[u + 1].b - usize[u].b) counters->pad = (uint32_t)u + 1;
+        d.out.pad_to(usize[u + 1].a - usize[u].a);
     });
 }
 // the rows of the modules, finished

@@ -770,6 +770,8 @@ def emit(spec, out_dirs):
     pat_rows = []
     slot_rows = []
     alt_rows = []
+    alt_sets = {}       # the alternatives of a slot -> number of the set
+    places = []         # per pattern: modifier -> (slot + 1) << 8 | value of the unordered slot that takes it
     parg_rows = []
     pat_index = {}
     all_pats = []
@@ -777,20 +779,28 @@ def emit(spec, out_dirs):
         for di, d in enumerate(defs[op]):
             pat_index[(op, di)] = len(pat_rows)
             sfirst = len(slot_rows)
-            for s in d.unordered + d.ordered:
+            place, typed_mask, required_mask = {}, 0, 0
+            for si, s in enumerate(d.unordered + d.ordered):
                 afirst = len(alt_rows)
                 enum_vals = enums[s.typ] if s.typ else None
                 for a in s.alts:
                     val = enum_vals.index(variant_capitalized(a)) if enum_vals else 1
                     alt_rows.append((mod_id[a], val))
-                slot_rows.append((1 if s.optional else 0, 1 if s.typ else 0, afirst, len(s.alts)))
+                alts = tuple(alt_rows[afirst:])
+                slot_rows.append((1 if s.optional else 0, 1 if s.typ else 0, afirst, len(s.alts), alt_sets.setdefault(alts, len(alt_sets))))
+                typed_mask |= (1 if s.typ else 0) << si
+                if si < len(d.unordered):
+                    required_mask |= (0 if s.optional else 1) << si
+                    for mod, val in alts:
+                        place.setdefault(mod, (si + 1) << 8 | val)
+            places.append(place)
             afirst = len(parg_rows)
             for a in d.pat.args:
                 flags = (a["optional"] * 1 | a["pre_bracket"] * 2 | a["post_bracket"] * 4 | a["pre_pipe"] * 8 |
                          a["can_be_negated"] * 16 | a["unified"] * 32)
                 parg_rows.append(flags)
             pat_rows.append((opcodes.index(op), len(d.unordered), len(d.ordered), sfirst, afirst, len(d.pat.args),
-                             instr_id[d.pat.variant], d.pat.head()))
+                             instr_id[d.pat.variant], d.pat.head(), typed_mask, required_mask))
             all_pats.append(d)
     chain_rows = []
     op_rows = []
@@ -809,20 +819,36 @@ def emit(spec, out_dirs):
     w("#define PTX_ARG_OPTIONAL 1\n#define PTX_ARG_PRE_BRACKET 2\n#define PTX_ARG_POST_BRACKET 4\n#define PTX_ARG_PRE_PIPE 8\n#define PTX_ARG_NEGATED 16\n#define PTX_ARG_UNIFIED 32")
     w("#define PTX_MAX_SLOTS 12\n#define PTX_MAX_ARGS 8")
     assert max(r[1] + r[2] for r in pat_rows) <= 12 and max(r[5] for r in pat_rows) <= 8
-    w("struct PtxPattern { uint8_t opcode, n_unordered, n_ordered, n_args; uint16_t first_slot, first_arg, instr; };")
-    w("struct PtxSlot { uint8_t optional, typed; uint16_t first_alt; uint16_t n_alt; };")
+    # typed_mask: slots whose absence reads as -1; required_mask: unordered slots that must be there
+    w("struct alignas(16) PtxPattern { uint8_t opcode, n_unordered, n_ordered, n_args; uint16_t first_slot, first_arg, instr, typed_mask, required_mask; };")
+    w("struct alignas(8) PtxSlot { uint8_t optional, typed; uint16_t first_alt; uint16_t n_alt, set; };")
     w("struct PtxAlt { uint8_t mod; int8_t value; };")
     w("struct PtxChain { uint16_t pattern; uint16_t is_default; uint64_t key[PTX_MOD_WORDS]; };")
     w("struct PtxOpcode { uint16_t first_chain, n_chain, special; };   // special: 1 bra, 2 call, 3 vshr")
     w("#define PTX_N_PATTERNS %d" % len(pat_rows))
     w("PTX_TABLE PtxPattern ptx_patterns[PTX_N_PATTERNS] = {")
-    for opi, nu, no, sf, af, na, ins, head in pat_rows:
-        w("    {%d,%d,%d,%d,%d,%d,%d},   // %s" % (opi, nu, no, na, sf, af, ins, head))
+    for opi, nu, no, sf, af, na, ins, head, tm, rm in pat_rows:
+        w("    {%d,%d,%d,%d,%d,%d,%d,%d,%d},   // %s" % (opi, nu, no, na, sf, af, ins, tm, rm, head))
     w("};")
     w("PTX_TABLE PtxSlot ptx_slots[] = {")
-    for o, t, af, na in slot_rows:
-        w("    {%d,%d,%d,%d}," % (o, t, af, na))
-    w("    {0,0,0,0}};")
+    for row in slot_rows:
+        w("    {%d,%d,%d,%d,%d}," % row)
+    w("    {0,0,0,0,0}};")
+    n_mods = max(mod_id.values()) + 1
+    assert all(0 <= val < 127 for val in (v for alts in alt_sets for _, v in alts))
+    w("// value of a modifier in a set of alternatives, -1 = not among them")
+    w("PTX_TABLE int8_t ptx_set_value[][%d] = {" % n_mods)
+    for alts in sorted(alt_sets, key=alt_sets.get):
+        first = {}
+        for mod, val in alts:
+            first.setdefault(mod, val)
+        w("    {" + ",".join(str(first.get(m, -1)) for m in range(n_mods)) + "},")
+    w("};")
+    w("// the unordered slot of a pattern that takes a modifier: (slot + 1) << 8 | value, 0 = none")
+    w("PTX_TABLE uint16_t ptx_mod_place[PTX_N_PATTERNS][%d] = {" % n_mods)
+    for place in places:
+        w("    {" + ",".join(str(place.get(m, 0)) for m in range(n_mods)) + "},")
+    w("};")
     w("PTX_TABLE PtxAlt ptx_alts[] = {")
     for i in range(0, len(alt_rows), 10):
         w("    " + ",".join("{%d,%d}" % r for r in alt_rows[i:i + 10]) + ",")
