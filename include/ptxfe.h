@@ -121,6 +121,8 @@ void ptxfe_batch_free(ptxfe_batch* batch);
 uint32_t ptxfe_batch_size(const ptxfe_batch* batch);
 int ptxfe_module_status(const ptxfe_batch* batch, uint32_t i);
 uint32_t ptxfe_module_error_count(const ptxfe_batch* batch, uint32_t i);
+/* The two for the modules [first, first + n) at once; either array may be NULL. */
+int ptxfe_module_verdicts(const ptxfe_batch* batch, uint32_t first, uint32_t n, int32_t* status, uint32_t* errors);
 void ptxfe_get_stats(const ptxfe_ctx* ctx, ptxfe_stats* out);
 /* When the environment variable PTXFE_PROFILE=1 was set at ptxfe_create: one line "step_name milliseconds" per pipeline
  * step of the last ptxfe_run (CUDA-event time on the context's stream).  Empty otherwise. */

@@ -65,6 +65,7 @@ def lib():
         L.ptxfe_module_status.argtypes = [vp, u32]
         L.ptxfe_module_error_count.argtypes = [vp, u32]
         L.ptxfe_module_error_count.restype = u32
+        L.ptxfe_module_verdicts.argtypes = [vp, u32, u32, ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(u32)]
         L.ptxfe_get_stats.argtypes = [vp, ctypes.POINTER(Stats)]
         L.ptxfe_profile.argtypes = [vp]
         L.ptxfe_profile.restype = ctypes.c_char_p
@@ -108,19 +109,15 @@ def _as_buffers(texts):
     """-> (keepalive list, char* array, length array).  Accepts bytes, str, or (address, length) pairs."""
     if isinstance(texts, Texts):
         return texts.buffers
-    keep, ptrs, lens = [], [], []
-    for t in texts:
-        if isinstance(t, tuple):
-            ptrs.append(ctypes.c_char_p(t[0]))
-            lens.append(t[1])
-            continue
-        if isinstance(t, str):
-            t = t.encode()
-        keep.append(t)
-        ptrs.append(ctypes.cast(ctypes.c_char_p(t), ctypes.c_char_p))
-        lens.append(len(t))
-    n = len(ptrs)
-    return keep, (ctypes.c_char_p * n)(*ptrs), (ctypes.c_uint64 * n)(*lens)
+    texts = list(texts)
+    if not all(type(t) is bytes for t in texts):
+        texts = [t.encode() if isinstance(t, str) else t for t in texts]
+    n = len(texts)
+    if not any(type(t) is tuple for t in texts):      # ctypes takes the addresses of the bytes objects itself
+        return texts, (ctypes.c_char_p * n)(*texts), (ctypes.c_uint64 * n)(*map(len, texts))
+    ptrs = [t[0] if type(t) is tuple else ctypes.cast(ctypes.c_char_p(t), ctypes.c_void_p).value for t in texts]
+    lens = [t[1] if type(t) is tuple else len(t) for t in texts]
+    return texts, (ctypes.c_char_p * n)(*ptrs), (ctypes.c_uint64 * n)(*lens)
 
 
 class Batch:
@@ -128,6 +125,7 @@ class Batch:
 
     def __init__(self, ctx, handle, keep):
         self._ctx, self._h, self._keep = ctx, handle, keep
+        self._rows = None      # (verdict, error count) of every module, fetched by the first question
 
     def __len__(self):
         return lib().ptxfe_batch_size(self._h)
@@ -143,8 +141,16 @@ class Batch:
         except Exception:
             pass
 
+    def _verdicts(self):
+        n = len(self)
+        status, errors = (ctypes.c_int32 * n)(), (ctypes.c_uint32 * n)()
+        lib().ptxfe_module_verdicts(self._h, 0, n, status, errors)
+        self._rows = status[:], errors[:]
+        return self._rows
+
     def status(self, i):
-        return lib().ptxfe_module_status(self._h, i)
+        rows = self._rows or self._verdicts()
+        return rows[0][i] if 0 <= i < len(rows[0]) else lib().ptxfe_module_status(self._h, i)
 
     def materialize(self, threads=None):
         """Build (and drop) the tree of every module on `threads` host threads; returns the number of nodes built."""
@@ -159,7 +165,8 @@ class Batch:
         return lib().ptxfe_multi_part_of(self._h, i)
 
     def error_count(self, i):
-        return lib().ptxfe_module_error_count(self._h, i)
+        rows = self._rows or self._verdicts()
+        return rows[1][i] if 0 <= i < len(rows[1]) else lib().ptxfe_module_error_count(self._h, i)
 
     def _text(self, fn, i):
         p = ctypes.c_void_p()

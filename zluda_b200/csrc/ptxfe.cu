@@ -19,6 +19,7 @@
 #define PTX_TABLE static __device__ const
 #include "../../include/ptxfe.h"
 #include "ptxfe_pipeline.h"
+#include "ptx_gather.h"
 #include "ptx_partition.h"
 #include <thread>
 
@@ -847,6 +848,9 @@ struct ptxfe_ctx {
     std::unordered_map<const void*, unsigned> resident;      // persistent kernels: blocks that the device holds
     char* h_meta = nullptr; size_t h_meta_cap = 0;           // pinned: layouts of all slices, as they go to the device
     char* d_meta = nullptr; size_t d_meta_cap = 0;
+    GatherPool* gather = nullptr;                            // made by the first batch that needs it
+    char* h_ring = nullptr;                                  // pinned: GATHER_PIECES pieces on their way to the device
+    cudaEvent_t ring_ev[GATHER_PIECES] = {nullptr};
     // What deferred counts prepare for, per byte of text: a little more than the batches so far had (the first guess is
     // above what real modules have).  A slice beyond it costs a second run, nothing else.
     double tokens_per_byte = 0.36, units_per_byte = 0.05, words_per_byte = 0.44;
@@ -1154,6 +1158,10 @@ void ptxfe_destroy(ptxfe_ctx* ctx) {
     if (ctx->s_out) cudaStreamDestroy(ctx->s_out);
     if (ctx->d_text) cudaFree(ctx->d_text);
     if (ctx->d_raw) cudaFree(ctx->d_raw);
+    delete ctx->gather;
+    if (ctx->h_ring) cudaFreeHost(ctx->h_ring);
+    for (cudaEvent_t e : ctx->ring_ev)
+        if (e) cudaEventDestroy(e);
     if (ctx->d_meta) cudaFree(ctx->d_meta);
     if (ctx->h_meta) cudaFreeHost(ctx->h_meta);
     if (ctx->d_class_store) cudaFree(ctx->d_class_store);
@@ -1237,6 +1245,68 @@ static void write_meta(ptxfe_ctx* ctx, size_t at, uint32_t m0, uint32_t m1, cons
     mcb[n] = chunks;
 }
 
+// ---- host text -> device
+// How the texts of a slice travel:
+//   RUNS    pinned memory in long stretches, the modules back to back: one copy per stretch, a kernel moves the modules to
+//           their slots
+//   SLOTS   pinned memory, large modules here and there: a copy per module, straight into its slot
+//   GATHER  everything else (pageable memory, many small modules): through the pinned ring, on several threads
+// and, up to PTXFE_SMALL_BYTES in all, by this thread into the metadata buffer, in one copy with it: waking threads or
+// starting a second copy takes longer than copying that much.
+enum UploadWay { UPLOAD_RUNS, UPLOAD_SLOTS, UPLOAD_GATHER };
+#define PTXFE_SMALL_BYTES (384u << 10)
+static bool is_pinned(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
+}
+static UploadWay upload_way(const char* const* texts, const uint64_t* lens, uint32_t m0, uint32_t m1, uint32_t* n_runs) {
+    uint32_t runs = 0;
+    uint64_t bytes = 0;
+    const char* probe = nullptr;
+    for (uint32_t m = m0; m < m1; m++) {
+        bytes += lens[m];
+        if (m == m0 || texts[m] != texts[m - 1] + lens[m - 1]) runs++;
+        if (!probe && lens[m]) probe = texts[m];
+    }
+    *n_runs = runs;
+    // (the last byte as well: a batch whose texts come from several buffers may begin in a pinned one)
+    if (!probe || !is_pinned(probe)) return UPLOAD_GATHER;
+    for (uint32_t m = m1; m-- > m0;)
+        if (lens[m]) {
+            if (!is_pinned(texts[m] + lens[m] - 1)) return UPLOAD_GATHER;
+            break;
+        }
+    if (runs * 2 <= m1 - m0 && bytes / runs >= (64u << 10)) return UPLOAD_RUNS;
+    return bytes / runs >= (128u << 10) ? UPLOAD_SLOTS : UPLOAD_GATHER;
+}
+// The modules [m0, m1) of a slice of `padded` bytes through the ring to `dst`, on `stream`.
+static int gather_text(ptxfe_ctx* ctx, cudaStream_t stream, const char* const* texts, uint32_t m0, uint32_t m1, uint64_t padded, uint8_t* dst) {
+    if (!ctx->h_ring) {
+        CUDA_TRY(cudaMallocHost((void**)&ctx->h_ring, GATHER_PIECE * GATHER_PIECES));
+        for (cudaEvent_t& e : ctx->ring_ev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    if (!ctx->gather) {
+        unsigned cores = std::thread::hardware_concurrency();
+        ctx->gather = new GatherPool(cores > 16 ? 8 : cores > 2 ? cores / 2 : 1);
+    }
+    // what an earlier slice sent from the ring may still be on its way
+    for (cudaEvent_t e : ctx->ring_ev) CUDA_TRY(cudaEventSynchronize(e));
+    cudaError_t err = cudaSuccess;
+    const bool ok = ctx->gather->run(GatherSource{texts + m0, ctx->layout.data() + m0, m1 - m0}, padded, ctx->h_ring,
+        [&](unsigned slot, uint64_t at, uint64_t len) {
+            err = cudaMemcpyAsync(dst + at, ctx->h_ring + slot * GATHER_PIECE, len, cudaMemcpyHostToDevice, stream);
+            if (err == cudaSuccess) err = cudaEventRecord(ctx->ring_ev[slot], stream);
+            return err == cudaSuccess;
+        },
+        [&](unsigned slot) { return cudaEventQuery(ctx->ring_ev[slot]) == cudaSuccess; });
+    if (!ok) {
+        snprintf(ctx->err, sizeof ctx->err, "text copy failed: %s", cudaGetErrorString(err));
+        return PTXFE_ERR_CUDA;
+    }
+    return PTXFE_OK;
+}
+
 int ptxfe_stage(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, uint32_t n) {
     if (!ctx || (n && (!texts || !lens))) return PTXFE_ERR_BAD_ARG;
     CUDA_TRY(cudaSetDevice(ctx->device));
@@ -1253,9 +1323,14 @@ int ptxfe_stage(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, 
     int st = ensure_text(ctx, off);
     if (st != PTXFE_OK) return st;
     CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->stream));
-    for (uint32_t m = 0; m < n; m++)
-        if (lens[m])
-            CUDA_TRY(cudaMemcpyAsync(ctx->d_text + ctx->layout[m].text_off, texts[m], lens[m], cudaMemcpyHostToDevice, ctx->stream));
+    uint32_t runs;
+    if (upload_way(texts, lens, 0, n, &runs) == UPLOAD_GATHER) {
+        if ((st = gather_text(ctx, ctx->stream, texts, 0, n, off, ctx->d_text)) != PTXFE_OK) return st;
+    } else {
+        for (uint32_t m = 0; m < n; m++)
+            if (lens[m])
+                CUDA_TRY(cudaMemcpyAsync(ctx->d_text + ctx->layout[m].text_off, texts[m], lens[m], cudaMemcpyHostToDevice, ctx->stream));
+    }
     if ((st = ensure_meta(ctx, meta_bytes(n))) != PTXFE_OK) return st;
     write_meta(ctx, 0, 0, n, nullptr);
     CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_bytes(n), cudaMemcpyHostToDevice, ctx->stream));
@@ -1606,7 +1681,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     }
     if (slices.empty()) slices.push_back(Slice{0, 0, 0, 0, 0});
     const size_t ns = slices.size();
-    int st = ensure_text(ctx, text_off);
+    int st = text_off <= PTXFE_SMALL_BYTES ? PTXFE_OK : ensure_text(ctx, text_off);
     if (st != PTXFE_OK) return st;
     while (ctx->slice_ev.size() < ns * 5) {
         cudaEvent_t e;
@@ -1614,19 +1689,18 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         ctx->slice_ev.push_back(e);
     }
     // ---- text copies, in slice order, on their own stream; submitted two slices ahead of the kernels.
-    // Modules that follow one another in host memory travel as one copy into a raw buffer and are moved to their
-    // chunk-aligned slots by a kernel; modules scattered over the host are copied straight into their slots.
-    std::vector<RepackModule> repack(n);
+    std::vector<RepackModule> repack;
     std::vector<uint64_t> raw_base(ns, 0);
-    std::vector<char> use_raw(ns, 0);
+    std::vector<UploadWay> way(ns, UPLOAD_GATHER);
+    const bool small = ns == 1 && text_off <= PTXFE_SMALL_BYTES;
     uint64_t raw_total = 0;
     for (size_t k = 0; k < ns; k++) {
         const Slice& sl = slices[k];
-        uint32_t runs = 0;
-        for (uint32_t m = sl.m0; m < sl.m1; m++)
-            if (m == sl.m0 || texts[m] != texts[m - 1] + lens[m - 1]) runs++;
-        if (runs * 2 <= sl.m1 - sl.m0) {
-            use_raw[k] = 1;
+        if (small) break;
+        uint32_t runs;
+        way[k] = upload_way(texts, lens, sl.m0, sl.m1, &runs);
+        if (way[k] == UPLOAD_RUNS) {
+            repack.resize(n);
             raw_base[k] = raw_total;
             raw_total += ((sl.bytes + 15) & ~(uint64_t)15) + 16 * (uint64_t)runs;
             uint64_t at = 0;     // offset of the current run inside the slice's raw region (multiple of 16)
@@ -1650,8 +1724,8 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         meta_at[k] = meta_total;
         meta_total += meta_bytes(slices[k].m1 - slices[k].m0);
     }
-    if ((st = ensure_meta(ctx, meta_total)) != PTXFE_OK) return st;
-    for (size_t k = 0; k < ns; k++) write_meta(ctx, meta_at[k], slices[k].m0, slices[k].m1, use_raw[k] ? repack.data() : nullptr);
+    if ((st = ensure_meta(ctx, meta_total + (small ? text_off + 256 : 0))) != PTXFE_OK) return st;
+    for (size_t k = 0; k < ns; k++) write_meta(ctx, meta_at[k], slices[k].m0, slices[k].m1, way[k] == UPLOAD_RUNS ? repack.data() : nullptr);
     if (raw_total + 64 > ctx->d_raw_cap) {
         if (ctx->d_raw) cudaFree(ctx->d_raw);
         ctx->d_raw = nullptr;
@@ -1664,9 +1738,10 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         const Slice& sl = slices[k];
         if (k == 0) {
             CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->s_in));
-            CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_total, cudaMemcpyHostToDevice, ctx->s_in));
+            if (small) GatherSource{texts, ctx->layout.data(), n}.fill(ctx->h_meta + meta_total, 0, text_off);
+            CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_total + (small ? text_off : 0), cudaMemcpyHostToDevice, ctx->s_in));
         }
-        if (use_raw[k]) {
+        if (way[k] == UPLOAD_RUNS) {
             for (uint32_t m = sl.m0; m < sl.m1;) {
                 uint32_t e = m + 1;
                 uint64_t bytes = lens[m];
@@ -1674,7 +1749,10 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
                 if (bytes) CUDA_TRY(cudaMemcpyAsync(ctx->d_raw + raw_base[k] + repack[m].raw_off, texts[m], bytes, cudaMemcpyHostToDevice, ctx->s_in));
                 m = e;
             }
-        } else {
+        } else if (way[k] == UPLOAD_GATHER && !small) {
+            int st = gather_text(ctx, ctx->s_in, texts, sl.m0, sl.m1, sl.padded, ctx->d_text + sl.text_off);
+            if (st != PTXFE_OK) return st;
+        } else if (!small) {
             for (uint32_t m = sl.m0; m < sl.m1; m++)
                 if (lens[m])
                     CUDA_TRY(cudaMemcpyAsync(ctx->d_text + sl.text_off + ctx->layout[m].text_off, texts[m], lens[m], cudaMemcpyHostToDevice, ctx->s_in));
@@ -1699,8 +1777,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
             return drain(PTXFE_ERR_CUDA);                                                   \
         }                                                                                   \
     } while (0)
-    for (size_t k = 0; k < ns && k < 2; k++)
-        if ((st = submit_text(k)) != PTXFE_OK) return drain(st);
+    if ((st = submit_text(0)) != PTXFE_OK) return drain(st);
     // ---- host result buffers: sized from the text; grown (after the copies in flight have landed) if a slice needs more
     int rc;
     if ((rc = grow_pinned(ctx, &ctx->h_results, &ctx->h_results_cap, sizeof(PtxModuleResult) * (size_t)n + 16, 0)) != PTXFE_OK) return drain(rc);
@@ -1722,11 +1799,11 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         // this arena held the results of slice k-2: they leave the device first
         if (k >= 2) CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->slice_ev[5 * (k - 2) + 4], 0));
         CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->slice_ev[5 * k], 0));
-        r.text = ctx->d_text + sl.text_off;
+        r.text = small ? (uint8_t*)ctx->d_meta + meta_total : ctx->d_text + sl.text_off;
         r.meta = meta_at[k];
         r.n = sl.m1 - sl.m0;
         r.mode = mode;
-        r.raw = use_raw[k] ? ctx->d_raw + raw_base[k] : nullptr;
+        r.raw = way[k] == UPLOAD_RUNS ? ctx->d_raw + raw_base[k] : nullptr;
         r.first = k == 0;
         r.results_out = (PtxModuleResult*)ctx->h_results + sl.m0;
         if (ns == 1 && total <= PTXFE_DIRECT_OUT_BYTES) {
@@ -1738,10 +1815,11 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         return enqueue_slice(ctx, r);
     };
     if ((rc = enqueue(0)) != PTXFE_OK) return drain(rc);
+    if (ns > 1 && (rc = submit_text(1)) != PTXFE_OK) return drain(rc);
     for (size_t k = 0; k < ns; k++) {
         const Slice& sl = slices[k];
-        if (k + 2 < ns && (rc = submit_text(k + 2)) != PTXFE_OK) return drain(rc);
         if (k + 1 < ns && (rc = enqueue(k + 1)) != PTXFE_OK) return drain(rc);
+        if (k + 2 < ns && (rc = submit_text(k + 2)) != PTXFE_OK) return drain(rc);
         if ((rc = finish_slice(ctx, runs[k])) != PTXFE_OK) return drain(rc);
         const PtxCounters& c = ctx->counters;
         const PtxWork& w = ctx->works[k & 1];
@@ -1905,6 +1983,16 @@ uint32_t ptxfe_module_error_count(const ptxfe_batch* b, uint32_t i) {
     if (r.sequential && ((r.status & US_MASK) == US_DIVERGE || (r.status & US_MASK) == US_REFUSED)) return 0;
     // a module without tokens: the implicit Parser error of the reference (the header does not parse)
     return n_lex + r.n_errors + (r.word_end == r.word_begin ? 1u : 0u);
+}
+
+// both for a range of modules
+int ptxfe_module_verdicts(const ptxfe_batch* b, uint32_t first, uint32_t n, int32_t* status, uint32_t* errors) {
+    if (!b || first > b->n || n > b->n - first) return PTXFE_ERR_BAD_ARG;
+    for (uint32_t i = 0; i < n; i++) {
+        if (status) status[i] = ptxfe_module_status(b, first + i);
+        if (errors) errors[i] = ptxfe_module_error_count(b, first + i);
+    }
+    return PTXFE_OK;
 }
 
 int ptxfe_module_records(const ptxfe_batch* b, uint32_t i, const uint32_t** words, uint64_t* n_words, uint64_t* text_base) {
