@@ -14,11 +14,41 @@
 #include <thread>
 #include <vector>
 
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
+
 #include "ptxfe_pipeline.h"
 
 constexpr size_t GATHER_PIECE = (size_t)2 << 20;      // bytes per copy to the device
 constexpr size_t GATHER_BLOCK = (size_t)128 << 10;    // bytes a thread takes at a time
 constexpr unsigned GATHER_PIECES = 8;                 // pieces in the ring
+
+// memcpy past the caches.  What the gathering threads write is read next by the device; out of the cores' caches, where
+// plain stores leave it modified, the device reads at 9 GB/s, out of memory at 50.
+inline void gather_copy(char* dst, const char* src, size_t n) {
+#ifdef __SSE2__
+    const size_t head = (16 - ((uintptr_t)dst & 15)) & 15;
+    if (n >= 64 + head) {
+        memcpy(dst, src, head);
+        dst += head; src += head; n -= head;
+        for (; n >= 64; dst += 64, src += 64, n -= 64) {
+            const __m128i a = _mm_loadu_si128((const __m128i*)src), b = _mm_loadu_si128((const __m128i*)(src + 16));
+            const __m128i c = _mm_loadu_si128((const __m128i*)(src + 32)), d = _mm_loadu_si128((const __m128i*)(src + 48));
+            _mm_stream_si128((__m128i*)dst, a);
+            _mm_stream_si128((__m128i*)(dst + 16), b);
+            _mm_stream_si128((__m128i*)(dst + 32), c);
+            _mm_stream_si128((__m128i*)(dst + 48), d);
+        }
+    }
+#endif
+    memcpy(dst, src, n);
+}
+inline void gather_fence() {
+#ifdef __SSE2__
+    _mm_sfence();
+#endif
+}
 
 // one slice's texts: module m of it starts at layout[m].text_off of the slice
 struct GatherSource {
@@ -35,8 +65,9 @@ struct GatherSource {
         for (uint32_t m = lo; m < n && layout[m].text_off < b; m++) {
             const uint64_t s = layout[m].text_off, e = s + layout[m].text_len;
             const uint64_t from = s > a ? s : a, to = e < b ? e : b;
-            if (from < to) memcpy(dst + (from - a), texts[m] + (from - s), (size_t)(to - from));
+            if (from < to) gather_copy(dst + (from - a), texts[m] + (from - s), (size_t)(to - from));
         }
+        gather_fence();
     }
 };
 
