@@ -161,7 +161,24 @@ struct PtxLexTileArgs {
     uint32_t* mod_flag;         // [n_modules] 1 = a run of soft bytes outgrew the look-back: the module is lexed by one thread
     PtxToken* tokens;           // emit step
     uint16_t* kinds;
+    uint64_t capacity = ~0ull;  // token rows there is room for (OWN = false; the others are dropped)
 };
+// The steps come in two forms.  OWN: text, tokens and kinds are the pipeline's own arrays - whole chunks of text are
+// readable, on a 16-byte boundary, and every token has a row and a kinds entry.  Not OWN (the lexer that allocates nothing):
+// the caller's text may begin at any address, nothing behind its last byte is read, there is no kinds array, and rows
+// beyond the caller's capacity are dropped.
+// four bytes of text at any address; all of them are readable, and with them the aligned words they lie in
+PTX_HD inline uint32_t lt_load4(const uint8_t* p) {
+#ifdef __CUDA_ARCH__
+    const uint32_t sh = ((uint32_t)(uintptr_t)p & 3u) * 8u;
+    const uint32_t* w = (const uint32_t*)((uintptr_t)p & ~(uintptr_t)3);
+    return sh ? __funnelshift_r(w[0], w[1], sh) : w[0];
+#else
+    uint32_t v = 0;
+    for (int i = 0; i < 4; i++) v |= (uint32_t)p[i] << (8 * i);
+    return v;
+#endif
+}
 
 // working memory of one tile (shared memory on the GPU)
 struct PtxLexMarkShared {
@@ -206,6 +223,7 @@ struct alignas(16) LtWord4 {
     uint32_t x, y, z, w;
 };
 // ---- phase 1: chunk geometry, and 32 bytes per thread through the tables; the thread owns one word of each bit map
+template <bool OWN = true>
 PTX_HD inline void lt_mark_simple(PtxLexMarkShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t tid, uint32_t nt) {
     for (uint32_t win = tid; win < LT_WORDS; win += nt) {
         const uint32_t k = win >> 2, c = tile * LT_CHUNKS + k;
@@ -217,11 +235,20 @@ PTX_HD inline void lt_mark_simple(PtxLexMarkShared& sh, const PtxLexTileArgs& a,
         uint32_t ms = 0, me = 0;
         int cx = CX_CODE;
         if (c < a.n_chunks) {
-            const LtWord4* w = (const LtWord4*)(a.text + pos0);
-            lo = w[0];
-            hi = w[1];
             bool first;
-            lt_locate(a, tile, c, &ms, &me, &first);
+            if (OWN) {
+                const LtWord4* w = (const LtWord4*)(a.text + pos0);
+                lo = w[0];
+                hi = w[1];
+                lt_locate(a, tile, c, &ms, &me, &first);
+            } else {
+                lt_locate(a, tile, c, &ms, &me, &first);
+                if ((uint64_t)pos0 + 32u <= me) {       // a shorter window is read byte by byte below
+                    const uint8_t* p = a.text + pos0;
+                    lo = {lt_load4(p), lt_load4(p + 4), lt_load4(p + 8), lt_load4(p + 12)};
+                    hi = {lt_load4(p + 16), lt_load4(p + 20), lt_load4(p + 24), lt_load4(p + 28)};
+                }
+            }
             if (!first) cx = (int)(a.vec[c - 1] & 7u);
         }
         if ((win & 3u) == 0) {
@@ -547,10 +574,20 @@ PTX_HD inline void lt_emit_tables(PtxLexEmitShared& sh, const PtxLexTileArgs& a,
     for (uint32_t i = tid; i < PTX_KW8_SIZE; i += nt) sh.kw[i] = ptx_kw8_table[i];
 }
 #define LT_TEXT_LOADS 8u              // text words a thread of a 256-thread block holds in registers during the init phase
+template <bool OWN = true>
 PTX_HD inline void lt_emit_init(PtxLexEmitShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t tid, uint32_t nt) {
     const uint32_t c0 = tile * LT_CHUNKS;
     const uint32_t n_words = (c0 + LT_CHUNKS <= a.n_chunks ? LT_CHUNKS : a.n_chunks - c0) * (PTX_CHUNK / 4);
     const uint32_t* src = (const uint32_t*)(a.text + (size_t)tile * LT_BYTES);
+    const uint64_t text_end = OWN ? 0 : a.info.layout[0].text_len;       // (one module)
+    auto load = [&](uint32_t i) -> uint32_t {
+        if (OWN) return src[i];
+        const uint64_t at = (uint64_t)tile * LT_BYTES + 4u * i;
+        if (at + 4 <= text_end) return lt_load4(a.text + at);
+        uint32_t v = 0;
+        for (uint32_t b = 0; at + b < text_end; b++) v |= (uint32_t)a.text[at + b] << (8 * b);
+        return v;
+    };
     // The text loads go out first and land in registers: the look-ups below (three dependent loads per chunk) then
     // run under their latency instead of after it.
     const bool held = nt * LT_TEXT_LOADS >= LT_BYTES / 4;
@@ -561,7 +598,7 @@ PTX_HD inline void lt_emit_init(PtxLexEmitShared& sh, const PtxLexTileArgs& a, u
 #endif
         for (uint32_t j = 0; j < LT_TEXT_LOADS; j++) {
             const uint32_t i = tid + j * nt;
-            tx[j] = i < n_words ? src[i] : 0u;
+            tx[j] = i < n_words ? load(i) : 0u;
         }
     }
     for (uint32_t w = tid; w < LT_WORDS + 2; w += nt) {
@@ -589,7 +626,7 @@ PTX_HD inline void lt_emit_init(PtxLexEmitShared& sh, const PtxLexTileArgs& a, u
         }
         for (uint32_t i = LT_BYTES / 4 + tid; i < LT_BYTES / 4 + 12; i += nt) sh.text[i] = 0u;
     } else {
-        for (uint32_t i = tid; i < LT_BYTES / 4 + 12; i += nt) sh.text[i] = i < n_words ? src[i] : 0u;
+        for (uint32_t i = tid; i < LT_BYTES / 4 + 12; i += nt) sh.text[i] = i < n_words ? load(i) : 0u;
     }
 }
 // length of the run of word characters that starts at tile offset o (at most 32; the bits behind the tile are zero)
@@ -605,20 +642,24 @@ PTX_HD inline uint32_t lt_word_run(const PtxLexEmitShared& sh, uint32_t o) {
     return inv ? (uint32_t)__builtin_ctz(inv) : 32u;
 #endif
 }
+template <bool OWN = true>
 PTX_HD inline void lt_put_token(const PtxLexTileArgs& a, uint32_t j, uint32_t start, uint32_t len, uint16_t kind) {
+    if (!OWN && j >= a.capacity) return;
     PtxTokenWord t;
     t.x = start;
     t.y = (len >= 0xFFFFu ? 0xFFFFu : len) | ((uint32_t)kind << 16);
     ((PtxTokenWord*)a.tokens)[j] = t;
-    a.kinds[j] = ptx_kind_entry(a.text, start, len, kind);
+    if (OWN) a.kinds[j] = ptx_kind_entry(a.text, start, len, kind);
 }
 // a token that is no numeric literal: the kinds entry is kind and capped length
+template <bool OWN = true>
 PTX_HD inline void lt_put_plain(const PtxLexTileArgs& a, uint32_t j, uint32_t start, uint32_t len, uint32_t kind) {
+    if (!OWN && j >= a.capacity) return;
     PtxTokenWord t;
     t.x = start;
     t.y = len | (kind << 16);
     ((PtxTokenWord*)a.tokens)[j] = t;
-    a.kinds[j] = (uint16_t)(kind | ((len < 127u ? len : 127u) << 9));
+    if (OWN) a.kinds[j] = (uint16_t)(kind | ((len < 127u ? len : 127u) << 9));
 }
 // the keyword table through the tile's text in shared memory: the token lies inside the tile
 PTX_HD inline uint32_t lt_keyword8(const PtxLexEmitShared& sh, uint32_t off, uint32_t len) {
@@ -653,6 +694,7 @@ PTX_HD inline uint32_t lt_keyword8(const PtxLexEmitShared& sh, uint32_t off, uin
     }
 }
 // the exact rules for one token
+template <bool OWN = true>
 PTX_HD inline void lt_emit_exact(const PtxLexTileArgs& a, uint32_t j, uint32_t pos, uint32_t me) {
     uint32_t len;
     uint16_t k;
@@ -664,7 +706,7 @@ PTX_HD inline void lt_emit_exact(const PtxLexTileArgs& a, uint32_t j, uint32_t p
     } else {
         k = lx_one(a.text, pos, me, &len);
     }
-    lt_put_token(a, j, pos, len, k);
+    lt_put_token<OWN>(a, j, pos, len, k);
 }
 // The tile's text in shared memory as something to index by byte offset
 struct LtTileBytes {
@@ -675,6 +717,7 @@ struct LtTileBytes {
 // Numbers are most of what the exact rules see: the number rules and the literal code straight from the tile in shared
 // memory, unless the number, or what the rules look at behind it (three bytes: an exponent's 'e', sign and first digit;
 // eighteen for the shortest reading of what may be a hexadecimal float), may lie behind the tile (then, as everything else, through lt_emit_exact)
+template <bool OWN = true>
 PTX_HD inline void lt_emit_exact_tile(const PtxLexEmitShared& sh, const PtxLexTileArgs& a, uint32_t tile_base, uint32_t j, uint32_t off, uint32_t me) {
     const bool module_ends_here = me - tile_base <= LT_BYTES;
     const uint32_t end = module_ends_here ? me - tile_base : LT_BYTES;
@@ -705,11 +748,12 @@ PTX_HD inline void lt_emit_exact_tile(const PtxLexEmitShared& sh, const PtxLexTi
             }
         }
         if (len) {
+            if (!OWN && j >= a.capacity) return;
             PtxTokenWord t;
             t.x = tile_base + off;
             t.y = len | (kind << 16);
             ((PtxTokenWord*)a.tokens)[j] = t;
-            a.kinds[j] = (uint16_t)kind;
+            if (OWN) a.kinds[j] = (uint16_t)kind;
             return;
         }
     }
@@ -718,16 +762,17 @@ PTX_HD inline void lt_emit_exact_tile(const PtxLexEmitShared& sh, const PtxLexTi
         uint32_t len;
         const uint16_t k = lx_number(bytes, off, end, &len);
         if (module_ends_here || off + (len > 18u ? len : 18u) + 3u <= end) {
+            if (!OWN && j >= a.capacity) return;
             PtxTokenWord t;
             t.x = tile_base + off;
             t.y = len | ((uint32_t)k << 16);                  // a length inside a tile
             ((PtxTokenWord*)a.tokens)[j] = t;
             uint64_t mag;
-            a.kinds[j] = (uint16_t)(k | (ptx_literal_scan(LtTileBytes{&sh, off}, len, k, &mag) << 9));
+            if (OWN) a.kinds[j] = (uint16_t)(k | (ptx_literal_scan(LtTileBytes{&sh, off}, len, k, &mag) << 9));
             return;
         }
     }
-    lt_emit_exact(a, j, tile_base + off, me);
+    lt_emit_exact<OWN>(a, j, tile_base + off, me);
 }
 PTX_HD inline uint32_t lt_window_rank(const PtxLexEmitShared& sh, uint32_t w) {
     uint32_t rank = sh.chunk_rank[w >> 2];
@@ -807,6 +852,7 @@ PTX_HD inline void lt_emit_list(PtxLexEmitShared& sh, uint32_t pass, uint32_t ti
 // bits, kind by the first byte.  Every token but the numbers, strings and the unusual (second round: exact rules) is
 // written here; words that may spell a keyword are written as plain words and listed for the keyword round, so that
 // no thread looks up a keyword while its neighbours wait.  Every thread of the block makes the same number of turns.
+template <bool OWN = true>
 PTX_HD inline void lt_emit_first(PtxLexEmitShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t pass, uint32_t tid, uint32_t nt) {
     const uint32_t tile_base = tile * LT_BYTES;
     const uint32_t j0 = a.cnt[tile * LT_CHUNKS].a;
@@ -842,23 +888,24 @@ PTX_HD inline void lt_emit_first(PtxLexEmitShared& sh, const PtxLexTileArgs& a, 
         const uint32_t j = j0 + p.base + r;
         if (exact) {
             if (slot_e < LT_EXACT_CAP) sh.exact[slot_e] = (uint16_t)r;
-            else lt_emit_exact_tile(sh, a, tile_base, j, off, sh.chunk_me[off >> 7]);       // no room in the list (a tile of numbers)
+            else lt_emit_exact_tile<OWN>(sh, a, tile_base, j, off, sh.chunk_me[off >> 7]);       // no room in the list (a tile of numbers)
             continue;
         }
-        lt_put_plain(a, j, tile_base + off, len, kind);
+        lt_put_plain<OWN>(a, j, tile_base + off, len, kind);
         if (want_kw) {
             if (slot_k < LT_KW_CAP) sh.kwlist[slot_k] = (uint16_t)r;
             else {
                 const uint32_t k = lt_keyword8(sh, off, len);
-                if (k != T_ERROR) {
+                if (k != T_ERROR && (OWN || j < a.capacity)) {
                     a.tokens[j].kind = (uint16_t)k;
-                    a.kinds[j] = (uint16_t)(k | (len << 9));
+                    if (OWN) a.kinds[j] = (uint16_t)(k | (len << 9));
                 }
             }
         }
     }
 }
 // keyword round: the listed words through the keyword table; a word that spells one gets that kind
+template <bool OWN = true>
 PTX_HD inline void lt_emit_keywords(PtxLexEmitShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t pass, uint32_t tid, uint32_t nt) {
     const uint32_t j0 = a.cnt[tile * LT_CHUNKS].a;
     const LtPass p = lt_emit_pass(sh, pass);
@@ -869,12 +916,14 @@ PTX_HD inline void lt_emit_keywords(PtxLexEmitShared& sh, const PtxLexTileArgs& 
         const uint32_t k = lt_keyword8(sh, off, len);
         if (k != T_ERROR) {
             const uint32_t j = j0 + p.base + r;
+            if (!OWN && j >= a.capacity) continue;
             a.tokens[j].kind = (uint16_t)k;
-            a.kinds[j] = (uint16_t)(k | (len << 9));      // a keyword is at most 20 bytes long
+            if (OWN) a.kinds[j] = (uint16_t)(k | (len << 9));      // a keyword is at most 20 bytes long
         }
     }
 }
 // second round: the exact rules, one thread per token left over
+template <bool OWN = true>
 PTX_HD inline void lt_emit_second(PtxLexEmitShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t pass, uint32_t tid, uint32_t nt) {
     const uint32_t tile_base = tile * LT_BYTES, j0 = a.cnt[tile * LT_CHUNKS].a;
     const LtPass p = lt_emit_pass(sh, pass);
@@ -883,7 +932,7 @@ PTX_HD inline void lt_emit_second(PtxLexEmitShared& sh, const PtxLexTileArgs& a,
     // partly filled turn to the first threads
     for (uint32_t x = nt - 1 - tid; x < n_exact; x += nt) {
         const uint32_t r = sh.exact[x], off = sh.tokoff[r];
-        lt_emit_exact_tile(sh, a, tile_base, j0 + p.base + r, off, sh.chunk_me[off >> 7]);
+        lt_emit_exact_tile<OWN>(sh, a, tile_base, j0 + p.base + r, off, sh.chunk_me[off >> 7]);
     }
 }
 

@@ -5,6 +5,7 @@
 // Device memory comes from a per-context arena of retained cudaMalloc blocks, so a steady stream of batches allocates
 // nothing.  There is no host parsing path: without a device every entry point returns PTXFE_ERR_CUDA.
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -84,8 +85,9 @@ struct PtxTileReader {
 
 #define LEX_TILE_BYTES (LEX_TILE_CHUNKS * LEX_ROW_WORDS * 4u)
 #define LEX_TABLE_BYTES (LS_COUNT * 256u * 2u)
+// text_len: 0 = whole chunks are readable on a 16-byte boundary, else nothing behind that many bytes is (text at any address)
 template <bool TABLES, class F>
-__global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const uint8_t* text, F f) {
+__global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const uint8_t* text, F f, uint32_t text_len = 0) {
     extern __shared__ __align__(16) uint32_t lex_smem[];
     uint32_t* tile = lex_smem;                                       // [LEX_TILE_CHUNKS][LEX_ROW_WORDS]
     uint16_t* fused = (uint16_t*)(lex_smem + LEX_TILE_CHUNKS * LEX_ROW_WORDS);    // [LS_COUNT][256] when TABLES
@@ -96,7 +98,15 @@ __global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const 
         uint32_t idx = threadIdx.x + k * 256;      // 16-byte piece of the tile
         uint32_t row = idx >> 3;
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (c0 + row < n_chunks) v = src[idx];
+        if (text_len) {
+            const uint64_t at = (uint64_t)c0 * PTX_CHUNK + 16u * idx;
+            const uint8_t* p = text + at;
+            if (at + 16 <= text_len) v = make_uint4(lt_load4(p), lt_load4(p + 4), lt_load4(p + 8), lt_load4(p + 12));
+            else
+                for (uint32_t b = 0; at + b < text_len; b++) (&v.x)[b >> 2] |= (uint32_t)p[b] << (8 * (b & 3u));
+        } else if (c0 + row < n_chunks) {
+            v = src[idx];
+        }
         uint32_t* d = tile + row * LEX_ROW_WORDS + (idx & 7u) * 4;
         d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
@@ -111,14 +121,15 @@ __global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const 
 // ---- the two block-cooperative lexer steps (ptx_lex_tile.h): one block per tile, a barrier between the phases
 __global__ void lex_fill_tables_kernel(PtxLexTables* t) { lt_fill_tables(t, threadIdx.x, blockDim.x); }
 // Persistent blocks: the tables are loaded once, then the block takes every gridDim.x-th tile.
-__global__ void __launch_bounds__(256, 8) lex_mark_kernel(PtxLexTileArgs a, uint32_t n_tiles) {
+template <bool OWN>
+__global__ void __launch_bounds__(256, 8) lex_mark_kernel(PtxLexTileArgs a, uint32_t tile0, uint32_t n_tiles) {
     __shared__ PtxLexMarkShared sh;
     const uint32_t tid = threadIdx.x;
     lt_mark_tables(sh, a, tid, 256);
     lt_mark_reset(sh, tid, 256);
-    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    for (uint32_t tile = tile0 + blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         __syncthreads();
-        lt_mark_simple(sh, a, tile, tid, 256);
+        lt_mark_simple<OWN>(sh, a, tile, tid, 256);
         __syncthreads();
         // ask for the text of the block's next tile while the rest of this one is settled
         if (tid < LT_BYTES / 128u && (uint64_t)tile + gridDim.x + 1 < n_tiles)       // a whole tile
@@ -130,15 +141,16 @@ __global__ void __launch_bounds__(256, 8) lex_mark_kernel(PtxLexTileArgs a, uint
         lt_mark_finish(sh, a, tile, tid, 256);
     }
 }
-__global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint32_t n_tiles, const uint32_t* stop) {
+template <bool OWN>
+__global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint32_t tile0, uint32_t n_tiles, const uint32_t* stop) {
     if (stop && *(const volatile uint32_t*)stop) return;
     extern __shared__ __align__(16) unsigned char lex_emit_smem[];
     PtxLexEmitShared& sh = *(PtxLexEmitShared*)lex_emit_smem;
     const uint32_t tid = threadIdx.x;
     lt_emit_tables(sh, a, tid, 256);
-    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    for (uint32_t tile = tile0 + blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         __syncthreads();
-        lt_emit_init(sh, a, tile, tid, 256);
+        lt_emit_init<OWN>(sh, a, tile, tid, 256);
         __syncthreads();
         // ask for the block's next tile (text, start bits, word bits) while this one is worked on
         if ((uint64_t)tile + gridDim.x + 1 < n_tiles) {     // a whole tile: every line asked for lies inside the arrays
@@ -152,10 +164,10 @@ __global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint
             if (pass) __syncthreads();
             lt_emit_list(sh, pass, tid, 256);
             __syncthreads();
-            lt_emit_first(sh, a, tile, pass, tid, 256);
+            lt_emit_first<OWN>(sh, a, tile, pass, tid, 256);
             __syncthreads();
-            lt_emit_keywords(sh, a, tile, pass, tid, 256);
-            lt_emit_second(sh, a, tile, pass, tid, 256);
+            lt_emit_keywords<OWN>(sh, a, tile, pass, tid, 256);
+            lt_emit_second<OWN>(sh, a, tile, pass, tid, 256);
         }
     }
 }
@@ -472,39 +484,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, L
     __syncthreads();
     if (!s_ok) return;
     const T prefix = op(s_before, excl);
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++)
-        if (base + k < n) st(base + k, op(prefix, vals[k]));
-}
-
-template <class T, class Op, class Ld>
-__global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(size_t n, Ld ld, Op op, T identity, T* partial) {
-    __shared__ T warp_tot[SCAN_THREADS / 32];
-    size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
-    T acc = identity;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++)
-        if (base + k < n) acc = op(acc, ld(base + k));
-    T incl, excl;
-    block_scan(acc, op, identity, warp_tot, incl, excl);
-    if (threadIdx.x == SCAN_THREADS - 1) partial[blockIdx.x] = incl;
-}
-
-template <class T, class Op, class Ld, class St>
-__global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(size_t n, Ld ld, St st, Op op, T identity, const T* partial_incl) {
-    __shared__ T warp_tot[SCAN_THREADS / 32];
-    size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
-    T vals[SCAN_ITEMS];
-    T acc = identity;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++) {
-        if (base + k < n) acc = op(acc, ld(base + k));
-        vals[k] = acc;
-    }
-    T incl, excl;
-    block_scan(acc, op, identity, warp_tot, incl, excl);
-    // everything before this thread: the tiles before this block, then the threads before it in the block
-    T prefix = blockIdx.x ? op(partial_incl[blockIdx.x - 1], excl) : excl;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; k++)
         if (base + k < n) st(base + k, op(prefix, vals[k]));
@@ -1041,14 +1020,14 @@ struct CudaBackend {
     void lex_mark(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
         prof_begin(name);
-        lex_mark_kernel<<<resident_blocks((const void*)lex_mark_kernel, 0, n_tiles), 256, 0, ctx->stream>>>(a, (uint32_t)n_tiles);
+        lex_mark_kernel<true><<<resident_blocks((const void*)lex_mark_kernel<true>, 0, n_tiles), 256, 0, ctx->stream>>>(a, 0u, (uint32_t)n_tiles);
         prof_end();
         ctx->launches++;
     }
     void lex_emit(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
         prof_begin(name);
-        lex_emit_kernel<<<resident_blocks((const void*)lex_emit_kernel, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), ctx->stream>>>(a, (uint32_t)n_tiles, stop);
+        lex_emit_kernel<true><<<resident_blocks((const void*)lex_emit_kernel<true>, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), ctx->stream>>>(a, 0u, (uint32_t)n_tiles, stop);
         prof_end();
         ctx->launches++;
     }
@@ -2160,33 +2139,68 @@ int ptxfe_lex_module(ptxfe_ctx* ctx, const char* text, uint64_t len, uint32_t** 
 
 // ------------------------------------------------------------------------------------------------ allocation-free lexer
 // Working memory of ptxfe_lex_device_noalloc: it lives in the library image, one copy per GPU that loads the library,
-// for the life of the process.  Layout (bytes): [0, 512K+4) chunk transition vectors, then the per-chunk
-// token/error counts, then two levels of scan tile totals.
+// for the life of the process.  The text goes through the lexer's tile kernels (their not-OWN form) in segments whose bit
+// maps and counts fit: two bits per byte and 8 bytes per chunk, 4 MiB at a time; the context vectors (4 bytes per chunk)
+// are those of the whole text.  (One thread per chunk, twice, reading bytes from global memory: 387 us for 3 MB against
+// 95 like this.)
 #define PTXFE_NOALLOC_MAX_TEXT (16u << 20)
 #define PTXFE_NOALLOC_MAX_CHUNKS (PTXFE_NOALLOC_MAX_TEXT / PTX_CHUNK)
+#define PTXFE_NOALLOC_SEG_TILES ((4u << 20) / LT_BYTES)
+#define PTXFE_NOALLOC_MAX_SEGS (PTXFE_NOALLOC_MAX_TEXT / (PTXFE_NOALLOC_SEG_TILES * LT_BYTES))
 #define PTXFE_NOALLOC_SCRATCH_BYTES (2u << 20)
 #define PTXFE_NOALLOC_MAX_BACK (64u << 10)
+struct NoallocScratch {
+    // cleared by the first kernel of a call: everything up to `cleared`
+    uint32_t mod_flag[2];          // 1 = a run of soft bytes outgrew the tile kernels' look-back
+    uint32_t serial;               // then: number of chunks of the text, else 0
+    uint32_t refused, aborted, pad[3];
+    uint32_t ctl[2 * (PTXFE_NOALLOC_MAX_SEGS + 2)];
+    ScanDesc<uint32_t> vec_desc[PTXFE_NOALLOC_MAX_CHUNKS / SCAN_TILE + 1];
+    ScanDesc<PtxPair> cnt_desc[PTXFE_NOALLOC_MAX_CHUNKS / SCAN_TILE + 2 * PTXFE_NOALLOC_MAX_SEGS + 2];
+    ScanDesc<PtxPair> serial_desc[PTXFE_NOALLOC_MAX_CHUNKS / SCAN_TILE + 2];
+    uint32_t cleared;
+    PtxPair carry;                 // tokens and errors in front of the segment
+    PtxModuleLayout layout;
+    uint32_t mcb[2];
+    PtxLexTables tables;
+    uint32_t tile_mod[PTXFE_NOALLOC_MAX_TEXT / LT_BYTES + 8];
+    uint32_t vec[PTXFE_NOALLOC_MAX_CHUNKS + 8];
+    union {
+        struct {
+            PtxPair cnt[PTXFE_NOALLOC_SEG_TILES * LT_CHUNKS + 8];
+            uint32_t start[PTXFE_NOALLOC_SEG_TILES * LT_WORDS];
+            uint32_t word[PTXFE_NOALLOC_SEG_TILES * LT_WORDS];
+        } seg;
+        PtxPair cnt[PTXFE_NOALLOC_MAX_CHUNKS + 8];      // the chunk-by-chunk walk: counts of the whole text
+    };
+};
+static_assert(sizeof(NoallocScratch) <= PTXFE_NOALLOC_SCRATCH_BYTES, "fixed working memory");
 static __device__ __align__(256) unsigned char ptxfe_noalloc_scratch[PTXFE_NOALLOC_SCRATCH_BYTES];
 
-// inclusive scan of at most SCAN_TILE * SCAN_TILE elements with caller-provided room for the tile totals
-template <class T, class Ld, class St, class Op>
-static void scan_in_scratch(cudaStream_t stream, size_t n, Ld ld, St st, Op op, T identity, T* partial) {
-    if (n == 0) return;
-    size_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    scan_reduce_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, stream>>>(n, ld, op, identity, partial);
-    if (tiles > 1) {
-        T* partial2 = partial + tiles;   // one tile is enough for the second level
-        scan_reduce_kernel<T><<<1, SCAN_THREADS, 0, stream>>>(tiles, ArrayLoad<T>{partial}, op, identity, partial2);
-        scan_apply_kernel<T><<<1, SCAN_THREADS, 0, stream>>>(tiles, ArrayLoad<T>{partial}, ArrayStore<T>{partial}, op, identity, partial2);
-    }
-    scan_apply_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, stream>>>(n, ld, st, op, identity, partial);
+__global__ void noalloc_init_kernel(NoallocScratch* s, uint32_t len, uint32_t n_chunks) {
+    uint32_t* w = (uint32_t*)s;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (uint32_t)(offsetof(NoallocScratch, cleared) / 4); i += gridDim.x * blockDim.x) w[i] = 0;
+    if (blockIdx.x != 0) return;
+    lt_fill_tables(&s->tables, threadIdx.x, blockDim.x);
+    if (threadIdx.x) return;
+    s->carry = PtxPair{0, 0};
+    s->layout.text_off = 0;
+    s->layout.text_len = len;
+    s->layout.chunk_begin = 0;
+    s->mcb[0] = 0;
+    s->mcb[1] = n_chunks;
 }
 
 extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64_t len, void* d_tokens_v, uint64_t token_capacity,
                              uint32_t* d_counts, void* stream_v) {
-    // Device addresses of the scratch array, looked up once per device.  The array's name is only a host-side handle:
-    // kernels must be given the address that cudaGetSymbolAddress returns while that device is current.
-    static std::atomic<unsigned char*> scratch_addr[64];
+    // Per device: the address of the scratch array (the array's name is only a host-side handle: kernels must be given
+    // the address that cudaGetSymbolAddress returns while that device is current) and the blocks the device holds of
+    // the two tile kernels.
+    struct PerDevice {
+        std::atomic<unsigned char*> scratch{nullptr};
+        unsigned mark_blocks = 0, emit_blocks = 0;
+    };
+    static PerDevice per_device[64];
     if (!d_text_v || !d_tokens_v || !d_counts || device < 0 || device >= 64) return PTXFE_ERR_BAD_ARG;
     if (len > PTXFE_NOALLOC_MAX_TEXT) {
         fprintf(stderr, "ptxfe_lex_device_noalloc: %llu bytes of text exceed the fixed working memory (limit %u bytes)\n",
@@ -2201,76 +2215,108 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
         ~RestoreDevice() { if (dev >= 0) cudaSetDevice(dev); }
     } restore{caller_device != device ? caller_device : -1};
     if (caller_device != device && cudaSetDevice(device) != cudaSuccess) return PTXFE_ERR_CUDA;
-    unsigned char* scratch = scratch_addr[device].load(std::memory_order_acquire);
-    if (!scratch) {
+    PerDevice& pd = per_device[device];
+    unsigned char* base = pd.scratch.load(std::memory_order_acquire);
+    if (!base) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, ptxfe_noalloc_scratch);
+        int sms = 0, mark = 0, emit = 0;
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(lex_emit_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtxLexEmitShared));
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mark, lex_mark_kernel<false>, 256, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&emit, lex_emit_kernel<false>, 256, sizeof(PtxLexEmitShared));
         if (e != cudaSuccess || !p) {
-            fprintf(stderr, "ptxfe_lex_device_noalloc: cudaGetSymbolAddress failed: %s\n", cudaGetErrorString(e));
+            fprintf(stderr, "ptxfe_lex_device_noalloc: set-up failed: %s\n", cudaGetErrorString(e));
             return PTXFE_ERR_CUDA;
         }
-        scratch = (unsigned char*)p;
-        scratch_addr[device].store(scratch, std::memory_order_release);      // every thread that looks it up stores the same address
+        // every thread that looks them up stores the same values, the address last
+        pd.mark_blocks = (unsigned)(sms * (mark > 0 ? mark : 1));
+        pd.emit_blocks = (unsigned)(sms * (emit > 0 ? emit : 1));
+        base = (unsigned char*)p;
+        pd.scratch.store(base, std::memory_order_release);
     }
     cudaStream_t stream = (cudaStream_t)stream_v;
     const uint8_t* text = (const uint8_t*)d_text_v;
     PtxToken* tokens = (PtxToken*)d_tokens_v;
     const uint32_t n_chunks = (uint32_t)((len + PTX_CHUNK - 1) / PTX_CHUNK);
-    unsigned char* base = scratch;
-    uint32_t* vec = (uint32_t*)base;                                                    // n_chunks + 1
-    PtxPair* cnt = (PtxPair*)(base + sizeof(uint32_t) * (PTXFE_NOALLOC_MAX_CHUNKS + 64));   // n_chunks + 2
-    unsigned char* tail = (unsigned char*)(cnt + PTXFE_NOALLOC_MAX_CHUNKS + 64);
-    uint32_t* partial_u32 = (uint32_t*)tail;                                            // <= 64 + 1 tile totals
-    PtxPair* partial_pair = (PtxPair*)(tail + 4096);
-    uint32_t* refused = (uint32_t*)(tail + 8192);                                       // 1 = a run of soft bytes outgrew the look-back
+    NoallocScratch* s = (NoallocScratch*)base;
     if (n_chunks == 0) {
         if (cudaMemsetAsync(d_counts, 0, 2 * sizeof(uint32_t), stream) != cudaSuccess) return PTXFE_ERR_CUDA;
         return PTXFE_OK;
     }
-    const uint64_t me = len;
+    const uint32_t me = (uint32_t)len;
     // every scratch word that is read below is written first by this call, so what an earlier call left behind
     // does not matter
-    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>(LaunchCount{n_chunks, nullptr, nullptr, 0}, [=] __device__(size_t c) {
-        uint64_t cs = (uint64_t)c * PTX_CHUNK;
-        uint64_t ce = cs + PTX_CHUNK < me ? cs + PTX_CHUNK : me;
-        uint32_t v = cx_chunk_vector(PtxGlobalReader{text, (uint32_t)me}, (uint32_t)cs, (uint32_t)ce);
-        vec[c] = c == 0 ? cx_restart(v) : v;
-        if (c == 0) *refused = 0;
-    });
+    noalloc_init_kernel<<<4, 256, 0, stream>>>(s, me, n_chunks);
+    const PtxLexChunkInfo info{&s->layout, s->mcb, 1};
+    lex_tile_kernel<false><<<(n_chunks + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS, 256, LEX_TILE_BYTES, stream>>>(
+        n_chunks, text, PtxLexVectorsStep{info, s->vec, s->tile_mod}, me);
+    scan_kernel<uint32_t><<<(n_chunks + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, stream>>>(
+        LaunchCount{n_chunks, nullptr, nullptr, 0}, ArrayLoad<uint32_t>{s->vec}, ArrayStore<uint32_t>{s->vec}, ComposeOp(), CX_IDENTITY, s->vec_desc, s->ctl,
+        &s->aborted);
+    const uint32_t n_tiles = (n_chunks + LT_CHUNKS - 1) / LT_CHUNKS;
+    ScanDesc<PtxPair>* desc = s->cnt_desc;
+    for (uint32_t seg = 0, t0 = 0; t0 < n_tiles; seg++, t0 += PTXFE_NOALLOC_SEG_TILES) {
+        const uint32_t t1 = t0 + PTXFE_NOALLOC_SEG_TILES < n_tiles ? t0 + PTXFE_NOALLOC_SEG_TILES : n_tiles;
+        const uint32_t c0 = t0 * LT_CHUNKS, c1 = t1 * LT_CHUNKS < n_chunks ? t1 * LT_CHUNKS : n_chunks, items = c1 - c0 + 1;
+        // the arrays hold the segment: their bases are moved so that tiles and chunks keep their numbers
+        PtxPair* cnt = s->seg.cnt - c0;
+        PtxLexTileArgs a{info, text, s->vec, n_chunks, &s->tables, s->tile_mod, s->seg.start - (size_t)t0 * LT_WORDS, s->seg.word - (size_t)t0 * LT_WORDS,
+                         cnt, s->mod_flag, tokens, nullptr, token_capacity};
+        lex_mark_kernel<false><<<t1 - t0 < pd.mark_blocks ? t1 - t0 : pd.mark_blocks, 256, 0, stream>>>(a, t0, t1);
+        const bool last = t1 == n_tiles;
+        scan_kernel<PtxPair><<<(items + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, stream>>>(
+            LaunchCount{items, nullptr, nullptr, 0}, [=] __device__(size_t i) { return i ? cnt[c0 + i] : s->carry; },
+            [=] __device__(size_t i, PtxPair v) {
+                cnt[c0 + i] = v;
+                if (i + 1 != items) return;
+                s->carry = v;
+                if (!last) return;
+                d_counts[0] = v.a;
+                d_counts[1] = v.b;
+                s->serial = s->mod_flag[0] ? n_chunks : 0u;
+            },
+            PairAddOp(), PtxPair{0, 0}, desc, s->ctl + 2 * (seg + 1), &s->aborted);
+        desc += (items + SCAN_TILE - 1) / SCAN_TILE;
+        lex_emit_kernel<false><<<t1 - t0 < pd.emit_blocks ? t1 - t0 : pd.emit_blocks, 256, sizeof(PtxLexEmitShared), stream>>>(a, t0, t1, nullptr);
+    }
+    // A run of soft bytes longer than the tile kernels look back (2 KiB): the text again, chunk by chunk, from the context
+    // vectors; the steps below have nothing to do otherwise.
+    const LaunchCount chunks{n_chunks, &s->serial, nullptr, 0};
+    const uint32_t* vec = s->vec;
+    PtxPair* cnt = s->cnt;
     // The byte walk of a chunk that begins inside a run of soft bytes starts over at the head of that run: bounded
     // here, so that a module made of one enormous run cannot keep the kernels busy for hours
     auto run_too_long = [=] __device__(uint32_t cs) -> bool {
-        if (cs == 0 || cs >= (uint32_t)me || !lx_soft(text[cs - 1]) || !lx_soft(text[cs])) return false;
+        if (cs == 0 || cs >= me || !lx_soft(text[cs - 1]) || !lx_soft(text[cs])) return false;
         uint32_t q = cs - 1;
         while (q > 0 && cs - q <= PTXFE_NOALLOC_MAX_BACK && lx_soft(text[q - 1])) q--;
         return cs - q > PTXFE_NOALLOC_MAX_BACK;
     };
-    scan_in_scratch<uint32_t>(stream, n_chunks, ArrayLoad<uint32_t>{vec}, ArrayStore<uint32_t>{vec}, ComposeOp(), CX_IDENTITY, partial_u32);
-    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>(LaunchCount{n_chunks, nullptr, nullptr, 0}, [=] __device__(size_t c) {
-        uint64_t cs = (uint64_t)c * PTX_CHUNK;
+    const unsigned walk_blocks = (n_chunks + 255) / 256;
+    pf_kernel<<<walk_blocks, 256, 0, stream>>>(chunks, [=] __device__(size_t c) {
+        const uint32_t cs = (uint32_t)c * PTX_CHUNK;
         int state = c == 0 ? CX_CODE : (int)(vec[c - 1] & 7u);
         LexCountSink sink;
-        if (state == CX_CODE && run_too_long((uint32_t)cs)) *refused = 1;
-        else lx_chunk(PtxGlobalReader{text, (uint32_t)me}, text, 0u, (uint32_t)me, (uint32_t)cs, (uint32_t)cs + PTX_CHUNK, state, sink);
-        PtxPair p;
-        p.a = sink.n_tokens;
-        p.b = sink.n_errors;
-        cnt[c + 1] = p;
-        if (c == 0) { PtxPair z; z.a = z.b = 0; cnt[0] = z; }
+        if (state == CX_CODE && run_too_long(cs)) s->refused = 1;
+        else lx_chunk(PtxGlobalReader{text, me}, text, 0u, me, cs, cs + PTX_CHUNK, state, sink);
+        cnt[c + 1] = PtxPair{sink.n_tokens, sink.n_errors};
     });
-    scan_in_scratch<PtxPair>(stream, (size_t)n_chunks + 1, ArrayLoad<PtxPair>{cnt}, ArrayStore<PtxPair>{cnt}, PairAddOp(), PtxPair{0, 0}, partial_pair);
-    pf_kernel<<<(n_chunks + 255) / 256, 256, 0, stream>>>(LaunchCount{n_chunks, nullptr, nullptr, 0}, [=] __device__(size_t c) {
-        uint64_t cs = (uint64_t)c * PTX_CHUNK;
+    scan_kernel<PtxPair><<<(n_chunks + 1 + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, stream>>>(
+        LaunchCount{(size_t)n_chunks + 1, &s->serial, nullptr, 1}, [=] __device__(size_t i) { return i ? cnt[i] : PtxPair{0, 0}; }, ArrayStore<PtxPair>{cnt},
+        PairAddOp(), PtxPair{0, 0}, s->serial_desc, s->ctl + 2 * (PTXFE_NOALLOC_MAX_SEGS + 1), &s->aborted);
+    pf_kernel<<<walk_blocks, 256, 0, stream>>>(chunks, [=] __device__(size_t c) {
+        const uint32_t cs = (uint32_t)c * PTX_CHUNK;
         int state = c == 0 ? CX_CODE : (int)(vec[c - 1] & 7u);
         LexCapSink sink;
         sink.tokens = tokens;
         sink.text = text;
         sink.next = cnt[c].a;
         sink.capacity = token_capacity;
-        if (!*refused) lx_chunk(PtxGlobalReader{text, (uint32_t)me}, text, 0u, (uint32_t)me, (uint32_t)cs, (uint32_t)cs + PTX_CHUNK, state, sink);
+        if (!s->refused) lx_chunk(PtxGlobalReader{text, me}, text, 0u, me, cs, cs + PTX_CHUNK, state, sink);
         if (c == 0) {
-            d_counts[0] = *refused ? 0xFFFFFFFFu : cnt[n_chunks].a;
-            d_counts[1] = *refused ? 0xFFFFFFFFu : cnt[n_chunks].b;
+            d_counts[0] = s->refused ? 0xFFFFFFFFu : cnt[n_chunks].a;
+            d_counts[1] = s->refused ? 0xFFFFFFFFu : cnt[n_chunks].b;
         }
     });
     cudaError_t e = cudaGetLastError();
