@@ -49,8 +49,10 @@ struct PtxSeg3 {
 };
 
 #define PTX_SORT_BUCKETS 4096u
-#define PTX_BULK_MIN_TOKENS 8192u   // statements at least this long get the bulk initialiser path
-#define PTX_MAX_BULK 32u            // per batch slice; further ones are decoded by one thread each
+// Top-level statements at least this long get the bulk initialiser path.  One thread takes about 5 us per element of an
+// array, the bulk path 100 us for any number of arrays (most of it for the host to learn that there are some): they meet
+// at some 20 elements; 48 elements leave short lists to the ordinary path.
+#define PTX_BULK_MIN_TOKENS 96u
 
 // fast per-thread memory the backend lends to a staged decoder: room for `stage_cap` record words (word k at
 // stage[k * stage_stride]) and for `win_cap` tokens (token k at win[k * win_stride])
@@ -252,7 +254,8 @@ struct PtxCounters {
     uint32_t n_reps;            // ... of which representatives
     uint32_t n_staged_words;    // words of the staged records so far
     uint32_t redo;              // PTX_REDO_*: something that the counts-stay-on-the-device flow does not cover
-    uint32_t spare[11];
+    uint32_t n_bulk_tokens;     // tokens of those statements
+    uint32_t spare[10];
 };
 // why a slice that was enqueued whole is run again with the host reading the counts on the way
 enum { PTX_REDO_TOKENS = 1, PTX_REDO_SERIAL_LEX = 2, PTX_REDO_UNITS = 4, PTX_REDO_BULK = 8, PTX_REDO_LIST = 16, PTX_REDO_WORDS = 64, PTX_REDO_STORE = 128,
@@ -355,7 +358,9 @@ struct PtxWork {
     uint32_t* second = nullptr;            // [n_second] units that a class promised a template and that have none
     PtxClassStore cs;
     PtxBulkTable bulk;
-    uint32_t bulk_tokens[PTX_MAX_BULK];
+    uint32_t n_bulk_tokens = 0;
+    uint32_t* bulk_base = nullptr;         // [bulk.n + 1] tokens of the listed statements in front of each
+    uint32_t* bulk_words = nullptr;        // [n_bulk_tokens] words of the elements up to and including each token
 };
 
 struct ComposeOp {
@@ -727,14 +732,13 @@ struct PtxUnitClassesStep {
         }
         if (dp == 0 && end - start >= PTX_BULK_MIN_TOKENS) {       // top level, not the module header
             const uint32_t slot = PTX_COUNT_ADD(&counters->n_bulk, 1);
-            if (slot < PTX_MAX_BULK) {
+            PTX_COUNT_ADD(&counters->n_bulk_tokens, end - start);
+            if (!deferred) {             // (there are at most n_tokens / PTX_BULK_MIN_TOKENS: room for all)
                 PtxBulkInfo bi;
-                bi.first_tok = start;      // for now: the statement's token range
-                bi.close_tok = end;
-                bi.n_elems = bi.n_words = 0;
-                bi.bad = 1;
-                bi.unit = (uint32_t)u;
-                bi.elems = nullptr;
+                bi.tok_begin = start;
+                bi.first_tok = PTX_ABSENT;
+                bi.close_tok = end;      // for now: the end of the statement
+                bi.n_elems = bi.n_words = bi.bad = bi.words_before = bi.pad = 0;
                 bi.dst = nullptr;
                 bulk_info[slot] = bi;
             }
@@ -862,7 +866,7 @@ struct PtxDecodeListStep {
         }
         uend[u] = r.end;
         ustatus[u] = (uint8_t)r.status;
-        bool flagged = d.out.high() > d.out.stage_cap || d.out.ne > 0;
+        bool flagged = d.out.high() > d.out.stage_cap || d.out.ne > 0 || d.bulk_used;
         if (!flagged && d.out.nw) {
             const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_words, d.out.nw);
             flagged = (uint64_t)at + d.out.nw > cap_staged;
@@ -1003,99 +1007,155 @@ inline uint32_t* ptx_sort_list(BK& bk, PtxWork& w, const uint32_t* list, uint32_
     return sorted;
 }
 
-// Bulk path: the elements of each listed statement's initialiser are decoded one thread per element into a dense
-// run; the statement's own decoder later takes the run in one step (PtxDecoder::multi_variable).  A list that is
-// not plainly "element, element, ... }" followed by ';' stays marked bad and is decoded the ordinary way.
+// Bulk path.  The work items of its steps are the tokens of all listed statements, one after the other: item k belongs to
+// the last statement whose base is at or below k.
+struct PtxBulkItems {
+    PtxBulkInfo* info;
+    const uint32_t* base;
+    const uint16_t* kinds;
+    uint32_t n;
+    PTX_HD uint32_t statement(uint32_t k) const { return ptx_upper_bound_u32(base, n, k) - 1; }
+    PTX_HD uint32_t kind(uint32_t i) const { return PTX_KL_KIND(kinds[i]); }
+    // does an element of statement b start at token i?
+    PTX_HD bool starts(const PtxBulkInfo& b, uint32_t i) const {
+        return i >= b.first_tok && i < b.close_tok && (i == b.first_tok || kind(i - 1) == T_COMMA);
+    }
+    // a number that converts without error, alone between commas: three words, whatever its digits
+    PTX_HD bool plain(const PtxBulkInfo& b, uint32_t i) const {
+        const uint32_t kl = kinds[i];
+        return ptx_is_numeric_kind(PTX_KL_KIND(kl)) && !(PTX_KL_LEN(kl) & (PTX_LC_ERR | PTX_LC_LONG)) && (i + 1 == b.close_tok || kind(i + 1) == T_COMMA);
+    }
+};
+// The elements of the listed statements' initialisers are measured, one thread per token.  A list that is not plainly
+// "element, element, ... }" followed by ';' is marked bad and decoded the ordinary way.
+// (Array by array, eleven launches each and every element decoded twice into a buffer of its own: 2.6 ms for 16 arrays
+// in 41 MB of text, 0.4 ms with ptx_bulk_write like this.)
 template <class BK>
-inline void ptx_bulk_elements(BK& bk, PtxWork& w, PtxBulkInfo* bulk_info, uint32_t n_bulk) {
+inline void ptx_bulk_measure(BK& bk, PtxWork& w, PtxBulkInfo* info, const PtxCounters& host_counters) {
     const uint8_t* text = w.text;
     const PtxToken* tokens = w.tokens;
-    const uint16_t* kinds = w.kinds;
     const PtxModuleLayout* layout = w.layout;
     const uint32_t* mtb = w.mod_tok_begin;
-    const uint32_t n_modules = w.n_modules;
-    PtxBulkInfo host_bulk[PTX_MAX_BULK];
-    bk.download(host_bulk, bulk_info, sizeof(PtxBulkInfo) * n_bulk);
-    for (uint32_t j = 0; j < n_bulk; j++) {
-        const uint32_t ts = host_bulk[j].first_tok, te = host_bulk[j].close_tok, nt = te - ts;
-        w.bulk_tokens[j] = nt;
-        PtxBulkInfo* bi = bulk_info + j;
-        uint32_t* lo_dev = (uint32_t*)bk.alloc(sizeof(uint32_t) * 4);
-        PtxPair* esz = (PtxPair*)bk.alloc(sizeof(PtxPair) * ((size_t)nt + 2));
-        uint32_t* elems = (uint32_t*)bk.alloc(sizeof(uint32_t) * (2 * (size_t)nt + 8));
-        bk.pf("bulk_reset", 1, [=] PTX_HD(size_t) { lo_dev[0] = PTX_ABSENT; lo_dev[1] = 0; });
-        bk.pf("bulk_find_open", nt, [=] PTX_HD(size_t k) {
-            uint32_t i = ts + (uint32_t)k;
-            if (i > ts && PTX_KL_KIND(kinds[i]) == T_LBRACE && PTX_KL_KIND(kinds[i - 1]) == T_EQ) {
+    const uint32_t n_modules = w.n_modules, n = host_counters.n_bulk, nt = host_counters.n_bulk_tokens;
+    uint32_t* base = w.bulk_base = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)n + 2));
+    uint32_t* words = w.bulk_words = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)nt + 1));
+    w.n_bulk_tokens = nt;
+    bk.template scan<uint32_t>("bulk_bases", (size_t)n + 1, [=] PTX_HD(size_t j) { return j ? info[j - 1].close_tok - info[j - 1].tok_begin : 0u; },
+                               [=] PTX_HD(size_t j, uint32_t v) { base[j] = v; }, AddOp(), 0u);
+    const PtxBulkItems it{info, base, w.kinds, n};
+    bk.pf("bulk_find_open", nt, [=] PTX_HD(size_t k) {
+        const uint32_t j = it.statement((uint32_t)k), i = info[j].tok_begin + ((uint32_t)k - base[j]);
+        if (k > base[j] && it.kind(i) == T_LBRACE && it.kind(i - 1) == T_EQ) {
 #ifdef __CUDA_ARCH__
-                atomicMin(&lo_dev[0], i);
+            atomicMin(&info[j].first_tok, i + 1);
 #else
-                if (i < lo_dev[0]) lo_dev[0] = i;
+            if (i + 1 < info[j].first_tok) info[j].first_tok = i + 1;
 #endif
-            }
-        });
-        bk.pf("bulk_measure", nt, [=] PTX_HD(size_t k) {
-            uint32_t i = ts + (uint32_t)k;
-            PtxPair z;
-            z.a = z.b = 0;
-            esz[k] = z;
-            const uint32_t lo = lo_dev[0], hi = te - 2;
-            bool shape_ok = lo != PTX_ABSENT && nt >= 6 && lo + 1 < hi && PTX_KL_KIND(kinds[te - 2]) == T_RBRACE &&
-                            PTX_KL_KIND(kinds[te - 1]) == T_SEMI && PTX_KL_KIND(kinds[hi - 1]) != T_COMMA;
-            if (!shape_ok) { if (k == 0) lo_dev[1] = 1; return; }
-            if (i <= lo || i >= hi) return;
-            uint16_t kd = PTX_KL_KIND(kinds[i]);
-            if (kd == T_LBRACE || kd == T_RBRACE) { lo_dev[1] = 1; return; }
-            if (!(i == lo + 1 || PTX_KL_KIND(kinds[i - 1]) == T_COMMA)) return;
-            // an element starts here: measure it
-            uint32_t mm = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
-            PtxSink sink;
-            PtxResolver res;
-            PtxDecoder d(text, tokens, mtb[mm + 1], layout[mm].text_off + layout[mm].text_len, sink, res);
-            d.pos = i;
-            d.unit_tok0 = i;
-            bool ok = d.reg_or_immediate(true) && d.out.ne == 0 && d.pos <= hi;
-            if (ok) {
-                uint16_t nk = PTX_KL_KIND(kinds[d.pos]);
-                ok = (d.pos == hi) || nk == T_COMMA;
-            }
-            if (!ok) { lo_dev[1] = 1; return; }
-            z.a = d.out.nw;
-            z.b = 1;
-            esz[k] = z;
-        });
-        bk.template scan<PtxPair>("bulk_scan", (size_t)nt, [=] PTX_HD(size_t k) { return esz[k]; }, [=] PTX_HD(size_t k, PtxPair v) {
-                                      PtxPair own = esz[k];
-                                      if (k + 1 == nt) {     // totals, before the entry turns exclusive
-                                          bi->n_words = v.a;
-                                          bi->n_elems = v.b;
-                                      }
-                                      PtxPair ex;
-                                      ex.a = v.a - own.a;
-                                      ex.b = own.b;      // keeps "an element starts here"
-                                      esz[k] = ex;
-                                  },
-                                  PairAddOp(), PtxPair{0, 0});
-        bk.pf("bulk_decode", nt, [=] PTX_HD(size_t k) {
-            if (lo_dev[1] || !esz[k].b) return;
-            uint32_t i = ts + (uint32_t)k;
-            uint32_t mm = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
-            PtxSink sink;
-            sink.words = elems + esz[k].a;
-            PtxResolver res;
-            PtxDecoder d(text, tokens, mtb[mm + 1], layout[mm].text_off + layout[mm].text_len, sink, res);
-            d.pos = i;
-            d.unit_tok0 = i;
-            d.reg_or_immediate(true);
-        });
-        bk.pf("bulk_publish", 1, [=] PTX_HD(size_t) {
-            bi->first_tok = lo_dev[0] + 1;
-            bi->close_tok = te - 2;
-            bi->bad = lo_dev[1];
-            bi->elems = elems;
-            bi->dst = nullptr;
-        });
-    }
+        }
+    });
+    // the statement's shape, and its place in the table that the decoders look in
+    uint32_t mask = 1;
+    while (mask < 2 * n) mask <<= 1;
+    mask -= 1;
+    uint32_t* slots = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)mask + 1));
+    bk.pf("bulk_table_clear", (size_t)mask + 1, [=] PTX_HD(size_t h) { slots[h] = PTX_ABSENT; });
+    bk.pf("bulk_shapes", n, [=] PTX_HD(size_t j) {
+        PtxBulkInfo b = info[j];
+        const uint32_t te = b.close_tok;
+        b.close_tok = te - 2;
+        if (b.first_tok == PTX_ABSENT || b.first_tok >= b.close_tok || it.kind(te - 2) != T_RBRACE || it.kind(te - 1) != T_SEMI || it.kind(te - 3) == T_COMMA)
+            b.bad = 1;
+        info[j] = b;
+        if (b.bad) return;
+        for (uint32_t h = PtxBulkTable::hash(b.first_tok) & mask;; h = (h + 1) & mask) {
+#ifdef __CUDA_ARCH__
+            const uint32_t old = atomicCAS(&slots[h], PTX_ABSENT, (uint32_t)j);
+#else
+            const uint32_t old = slots[h];
+            if (old == PTX_ABSENT) slots[h] = (uint32_t)j;
+#endif
+            if (old == PTX_ABSENT) break;
+        }
+    });
+    // words and elements, counted along all the statements
+    bk.template scan<PtxPair>("bulk_measure", (size_t)nt, [=] PTX_HD(size_t k) {
+        PtxPair z{0, 0};
+        const uint32_t j = it.statement((uint32_t)k), i = info[j].tok_begin + ((uint32_t)k - base[j]);
+        const PtxBulkInfo& b = info[j];
+        if (b.bad || i < b.first_tok || i >= b.close_tok) return z;
+        const uint32_t kd = it.kind(i);
+        if (kd == T_LBRACE || kd == T_RBRACE) { info[j].bad = 1; return z; }
+        if (!it.starts(b, i)) return z;
+        if (it.plain(b, i)) return PtxPair{3, 1};
+        const uint32_t m = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
+        PtxSink sink;
+        PtxResolver res;
+        PtxDecoder d(text, tokens, mtb[m + 1], layout[m].text_off + layout[m].text_len, sink, res);
+        d.pos = i;
+        d.unit_tok0 = i;
+        bool ok = d.reg_or_immediate(true) && d.out.ne == 0 && d.pos <= b.close_tok;
+        if (ok) ok = d.pos == b.close_tok || it.kind(d.pos) == T_COMMA;
+        if (!ok) { info[j].bad = 1; return z; }
+        return PtxPair{d.out.nw, 1};
+    }, [=] PTX_HD(size_t k, PtxPair v) {
+        words[k] = v.a;
+        const uint32_t j = it.statement((uint32_t)k);
+        if (k + 1 != base[j + 1]) return;
+        info[j].n_words = v.a;         // up to the end of this statement: made its own below
+        info[j].n_elems = v.b;
+    }, PairAddOp(), PtxPair{0, 0});
+    uint32_t* ends = (uint32_t*)bk.alloc(sizeof(uint32_t) * 2 * ((size_t)n + 1));
+    bk.pf("bulk_ends", n, [=] PTX_HD(size_t j) {
+        ends[2 * j] = info[j].n_words;
+        ends[2 * j + 1] = info[j].n_elems;
+    });
+    bk.pf("bulk_totals", n, [=] PTX_HD(size_t j) {
+        info[j].words_before = j ? ends[2 * j - 2] : 0u;
+        info[j].n_words = ends[2 * j] - info[j].words_before;
+        info[j].n_elems = ends[2 * j + 1] - (j ? ends[2 * j - 1] : 0u);
+    });
+    w.bulk.info = info;
+    w.bulk.n = n;
+    w.bulk.mask = mask;
+    w.bulk.slots = slots;
+}
+// The elements go where the statements' decoders left room for them, one thread per token
+template <class BK>
+inline void ptx_bulk_write(BK& bk, PtxWork& w) {
+    if (!w.bulk.n) return;
+    const uint8_t* text = w.text;
+    const PtxToken* tokens = w.tokens;
+    const PtxModuleLayout* layout = w.layout;
+    const uint32_t* mtb = w.mod_tok_begin;
+    const uint32_t* base = w.bulk_base;
+    const uint32_t* words = w.bulk_words;
+    const PtxBulkInfo* info = w.bulk.info;
+    const uint32_t n_modules = w.n_modules;
+    const PtxBulkItems it{w.bulk.info, base, w.kinds, w.bulk.n};
+    bk.pf("bulk_write", w.n_bulk_tokens, [=] PTX_HD(size_t k) {
+        const uint32_t j = it.statement((uint32_t)k), i = info[j].tok_begin + ((uint32_t)k - base[j]);
+        const PtxBulkInfo& b = info[j];
+        if (b.bad || !b.dst || !it.starts(b, i)) return;
+        uint32_t* dst = b.dst + (words[k - 1] - b.words_before);      // (the token in front of an element is the statement's own)
+        if (it.plain(b, i)) {
+            const PtxToken t = tokens[i];
+            const uint32_t code = PTX_KL_LEN(it.kinds[i]);
+            const uint64_t v = ptx_literal_value(text, t.start, t.len, t.kind);
+            const uint32_t kind = t.kind == T_F32HEX ? 2u : t.kind == T_F64HEX || t.kind == T_F64 ? 3u : code & (PTX_LC_UNS | PTX_LC_GT_I63) ? 0u : 1u;
+            dst[0] = 1u + kind;
+            dst[1] = (uint32_t)v;
+            dst[2] = (uint32_t)(v >> 32);
+            return;
+        }
+        const uint32_t m = ptx_upper_bound_u32(mtb, n_modules, i) - 1;
+        PtxSink sink;
+        sink.words = dst;
+        PtxResolver res;
+        PtxDecoder d(text, tokens, mtb[m + 1], layout[m].text_off + layout[m].text_len, sink, res);
+        d.pos = i;
+        d.unit_tok0 = i;
+        d.reg_or_immediate(true);
+    });
 }
 
 // Everything up to the size of every unit's records
@@ -1130,7 +1190,7 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     const uint32_t cap_list = w.deferred ? w.cap_list : (uint32_t)nu;
     uint32_t* first = w.list = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)cap_list + 1));
     uint32_t* second = (uint32_t*)bk.alloc(sizeof(uint32_t) * ((size_t)cap_list + 1));
-    PtxBulkInfo* bulk_info = (PtxBulkInfo*)bk.alloc(sizeof(PtxBulkInfo) * PTX_MAX_BULK);
+    PtxBulkInfo* bulk_info = w.deferred ? nullptr : (PtxBulkInfo*)bk.alloc(sizeof(PtxBulkInfo) * ((size_t)w.n_tokens / PTX_BULK_MIN_TOKENS + 1));
     const PtxClassStore cs = w.cs = bk.class_store(w.first_slice);
     bk.pf("unit_classes", w.units_n(),
           PtxUnitClassesStep{w.text, w.tokens, w.kinds, w.unit_start, w.unit_depth, w.mod_unit_begin, w.mod_skip, n_modules, cap_list, w.deferred, counters, cs,
@@ -1138,11 +1198,7 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     if (!w.deferred) bk.download(&host_counters, counters, sizeof(PtxCounters));
     // ---- bulk initialisers
     w.bulk = PtxBulkTable();
-    if (!w.deferred && host_counters.n_bulk) {
-        w.bulk.info = bulk_info;
-        w.bulk.n = host_counters.n_bulk < PTX_MAX_BULK ? host_counters.n_bulk : PTX_MAX_BULK;
-        ptx_bulk_elements(bk, w, bulk_info, w.bulk.n);
-    }
+    if (!w.deferred && host_counters.n_bulk) ptx_bulk_measure(bk, w, bulk_info, host_counters);
     // ---- first list: units without a class, and the representatives of the classes this slice added
     const uint32_t n_first = host_counters.n_first;
     // the pool of staged records: what does not fit is measured now and written by the second decode pass
@@ -1404,18 +1460,6 @@ inline void ptx_module_results(BK& bk, PtxWork& w, uint32_t n_errs) {
     });
 }
 
-template <class BK>
-inline void ptx_bulk_copy(BK& bk, PtxWork& w) {
-    // the element runs of the bulk path go where the statements' decoders left room for them
-    for (uint32_t j = 0; j < w.bulk.n; j++) {
-        const PtxBulkInfo* bi = w.bulk.info + j;
-        bk.pf("bulk_copy", 2 * (size_t)w.bulk_tokens[j], [=] PTX_HD(size_t k) {
-            if (bi->bad || !bi->dst || k >= bi->n_words) return;
-            bi->dst[k] = bi->elems[k];
-        });
-    }
-}
-
 // Sizes known: offsets, records, second decode pass, module rows; the host reads the counts on the way.
 // again = a slice whose first round ran with deferred counts: its units are decoded and checked
 template <class BK>
@@ -1434,7 +1478,7 @@ inline void ptx_decode_finish(BK& bk, PtxWork& w, PtxCounters& host_counters, bo
     w.errs = (PtxErrRec*)bk.alloc(sizeof(PtxErrRec) * ((size_t)host_counters.n_errs + 1));
     if (!again || host_counters.any_sequential) ptx_emit_records(bk, w);
     ptx_emit_flagged(bk, w, host_counters);
-    ptx_bulk_copy(bk, w);
+    ptx_bulk_write(bk, w);
     ptx_module_results(bk, w, host_counters.n_errs);
     bk.download(&host_counters, counters, sizeof(PtxCounters));   // .pad != 0: unit (index + 1) whose two passes disagreed
 }
@@ -1468,7 +1512,7 @@ inline void ptx_stage_decode_anew(BK& bk, PtxWork& w, PtxCounters& host_counters
     w.n_tokens = host_counters.n_tokens;
     w.n_units = host_counters.n_units;
     bk.pf("reset_decode_counters", 1, [=] PTX_HD(size_t) {
-        counters->n_bulk = counters->n_first = counters->n_reps = counters->n_second = counters->n_flagged = counters->n_funcs = 0;
+        counters->n_bulk = counters->n_bulk_tokens = counters->n_first = counters->n_reps = counters->n_second = counters->n_flagged = counters->n_funcs = 0;
         counters->n_staged_words = counters->any_sequential = counters->redo = 0;
     });
     ptx_lex_errors(bk, w, host_counters.n_lexerrs);
