@@ -50,20 +50,21 @@ inline void gather_fence() {
 #endif
 }
 
-// one slice's texts: module m of it starts at layout[m].text_off of the slice
+// one slice's texts: module m of it starts at layout[m].text_off - base of the slice
 struct GatherSource {
     const char* const* texts;
     const PtxModuleLayout* layout;
     uint32_t n;
+    uint64_t base;
     // bytes [a, b) of the slice to dst (what lies between two modules is left as it is)
     void fill(char* dst, uint64_t a, uint64_t b) const {
         uint32_t lo = 0, hi = n;              // last module that starts at or before a
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) / 2;
-            if (layout[mid].text_off <= a) lo = mid; else hi = mid;
+            if (layout[mid].text_off - base <= a) lo = mid; else hi = mid;
         }
-        for (uint32_t m = lo; m < n && layout[m].text_off < b; m++) {
-            const uint64_t s = layout[m].text_off, e = s + layout[m].text_len;
+        for (uint32_t m = lo; m < n && layout[m].text_off - base < b; m++) {
+            const uint64_t s = layout[m].text_off - base, e = s + layout[m].text_len;
             const uint64_t from = s > a ? s : a, to = e < b ? e : b;
             if (from < to) gather_copy(dst + (from - a), texts[m] + (from - s), (size_t)(to - from));
         }
@@ -160,7 +161,7 @@ private:
     std::condition_variable wake_;
     bool quit_ = false;
     uint64_t generation_ = 0, bytes_ = 0;
-    GatherSource src_{nullptr, nullptr, 0};
+    GatherSource src_{nullptr, nullptr, 0, 0};
     char* ring_ = nullptr;
     std::atomic<uint64_t> next_{0}, allowed_{0};
     std::atomic<uint32_t> done_[GATHER_PIECES];

@@ -292,10 +292,10 @@ struct LexCountSink {
 // writes lexer errors only (second pass, run only when the first found some)
 struct LexErrorSink {
     uint32_t* errors;      // pairs (start, len), already offset to this chunk's first error
-    uint32_t n_errors = 0;
+    uint32_t n_errors = 0, bias = 0;
     PTX_HD void token(uint32_t, uint32_t, uint16_t) {}
     PTX_HD void error(uint32_t start, uint32_t len) {
-        errors[2 * n_errors] = start;
+        errors[2 * n_errors] = start + bias;
         errors[2 * n_errors + 1] = len;
         n_errors++;
     }

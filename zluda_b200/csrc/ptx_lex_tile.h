@@ -198,7 +198,7 @@ struct PtxLexMarkShared {
 PTX_HD inline void lt_locate(const PtxLexTileArgs& a, uint32_t tile, uint32_t c, uint32_t* ms, uint32_t* me, bool* first) {
     uint32_t m = a.tile_mod[tile];
     while (m + 1 < a.info.n_modules && a.info.mcb[m + 1] <= c) m++;
-    *ms = (uint32_t)a.info.layout[m].text_off;
+    *ms = a.info.begin(m);
     *me = *ms + (uint32_t)a.info.layout[m].text_len;
     *first = c == a.info.mcb[m];
 }
@@ -523,7 +523,7 @@ struct LexModuleSink {
 PTX_HD inline void lt_lex_module_serial(const PtxLexTileArgs& a, uint32_t m) {
     if (!a.mod_flag[m]) return;
     const uint32_t c0 = a.info.mcb[m], c1 = a.info.mcb[m + 1];
-    const uint32_t ms = (uint32_t)a.info.layout[m].text_off, me = ms + (uint32_t)a.info.layout[m].text_len;
+    const uint32_t ms = a.info.begin(m), me = ms + (uint32_t)a.info.layout[m].text_len;
     for (uint32_t c = c0; c < c1; c++) {
         for (uint32_t w = 0; w < 4; w++) a.start_bits[(size_t)c * 4 + w] = 0;
         PtxPair z;
@@ -646,7 +646,7 @@ template <bool OWN = true>
 PTX_HD inline void lt_put_token(const PtxLexTileArgs& a, uint32_t j, uint32_t start, uint32_t len, uint16_t kind) {
     if (!OWN && j >= a.capacity) return;
     PtxTokenWord t;
-    t.x = start;
+    t.x = start + a.info.bias;
     t.y = (len >= 0xFFFFu ? 0xFFFFu : len) | ((uint32_t)kind << 16);
     ((PtxTokenWord*)a.tokens)[j] = t;
     if (OWN) a.kinds[j] = ptx_kind_entry(a.text, start, len, kind);
@@ -656,7 +656,7 @@ template <bool OWN = true>
 PTX_HD inline void lt_put_plain(const PtxLexTileArgs& a, uint32_t j, uint32_t start, uint32_t len, uint32_t kind) {
     if (!OWN && j >= a.capacity) return;
     PtxTokenWord t;
-    t.x = start;
+    t.x = start + a.info.bias;
     t.y = len | (kind << 16);
     ((PtxTokenWord*)a.tokens)[j] = t;
     if (OWN) a.kinds[j] = (uint16_t)(kind | ((len < 127u ? len : 127u) << 9));
@@ -750,7 +750,7 @@ PTX_HD inline void lt_emit_exact_tile(const PtxLexEmitShared& sh, const PtxLexTi
         if (len) {
             if (!OWN && j >= a.capacity) return;
             PtxTokenWord t;
-            t.x = tile_base + off;
+            t.x = tile_base + off + a.info.bias;
             t.y = len | (kind << 16);
             ((PtxTokenWord*)a.tokens)[j] = t;
             if (OWN) a.kinds[j] = (uint16_t)kind;
@@ -764,7 +764,7 @@ PTX_HD inline void lt_emit_exact_tile(const PtxLexEmitShared& sh, const PtxLexTi
         if (module_ends_here || off + (len > 18u ? len : 18u) + 3u <= end) {
             if (!OWN && j >= a.capacity) return;
             PtxTokenWord t;
-            t.x = tile_base + off;
+            t.x = tile_base + off + a.info.bias;
             t.y = len | ((uint32_t)k << 16);                  // a length inside a tile
             ((PtxTokenWord*)a.tokens)[j] = t;
             uint64_t mag;

@@ -177,6 +177,13 @@ __global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint
 // A short list uses few lanes of every warp (down to one): units of different shapes in one warp run one after the other,
 // and what a lone unit waits for is instruction fetches and dependent loads, which other warps of the SM share.  Fewer
 // slots also means longer records and token windows per slot (a function header of eight parameters has 70 words).
+// reads one word of every 128-byte line, spread over the block's threads
+__device__ inline void touch_lines(const void* table, size_t bytes) {
+    for (uint32_t at = threadIdx.x * 128u; at < bytes; at += blockDim.x * 128u) {
+        uint32_t x;
+        asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(x) : "l"((const char*)table + at));
+    }
+}
 #define STAGE_SLOTS 257u
 #define STAGE_CAP 40u
 #define WIN_CAP 12u
@@ -187,14 +194,34 @@ __global__ void __launch_bounds__(256) staged_kernel(LaunchCount count, F f) {
     PtxTokenWord* win = (PtxTokenWord*)staged_smem;
     uint32_t* stage = (uint32_t*)(staged_smem + WIN_CAP * STAGE_SLOTS * 8u);
     const uint32_t n = (uint32_t)count.get();
+    if (n == 0) return;
+    // The decoders go through the grammar's tables one dependent load after the other, each of which would find the SM's
+    // cache cold and wait for L2 (a mov with two registers: 40,000 cycles).  All lanes ask for the tables at once.
+    touch_lines(ptx_opcodes, sizeof ptx_opcodes);
+    touch_lines(ptx_chains, sizeof ptx_chains);
+    touch_lines(ptx_patterns, sizeof ptx_patterns);
+    touch_lines(ptx_pattern_args, sizeof ptx_pattern_args);
+    touch_lines(ptx_slots, sizeof ptx_slots);
+    touch_lines(ptx_mod_place, sizeof ptx_mod_place);
+    touch_lines(ptx_set_value, sizeof ptx_set_value);
     const uint32_t warps = gridDim.x * 8u, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t lanes = (n + warps - 1u) / warps;                       // active lanes per warp
     if (lanes > 32u) lanes = 32u;
-    if (lanes == 0 || lane >= lanes) return;
-    const uint32_t stride = 8u * lanes + 1u, slot = warp * lanes + lane;
-    const PtxScratch scratch{stage + slot, stride, STAGE_CAP * STAGE_SLOTS / stride, win + slot, stride, WIN_CAP * STAGE_SLOTS / stride};
+    const uint32_t stride = 8u * lanes + 1u, win_cap = WIN_CAP * STAGE_SLOTS / stride;
+    const uint32_t slot = warp * lanes + lane;
+    const PtxScratch scratch{stage + slot, stride, STAGE_CAP * STAGE_SLOTS / stride, win + slot, stride, win_cap, true};
     // neighbouring entries go to one warp when the lanes are full (they may have the same shape), to different SMs else
-    for (uint32_t i = (blockIdx.x * 8u + warp) * lanes + lane; i < n; i += warps * lanes) f((size_t)i, scratch);
+    for (uint32_t i0 = (blockIdx.x * 8u + warp) * lanes; i0 < n; i0 += warps * lanes) {
+        const uint32_t here = n - i0 < lanes ? n - i0 : lanes;
+        __syncwarp();
+        for (uint32_t k = 0; k < here; k++) {       // the whole warp fills the window of each entry
+            uint32_t start;
+            const uint32_t nw = f.window(i0 + k, win_cap, &start);
+            for (uint32_t t = lane; t < nw; t += 32u) win[warp * lanes + k + t * stride] = ((const PtxTokenWord*)(f.tokens + start))[t];
+        }
+        __syncwarp();
+        if (lane < here) f((size_t)(i0 + lane), scratch);
+    }
 }
 
 constexpr int SCAN_THREADS = 256;
@@ -800,15 +827,20 @@ struct ptxfe_batch {
     const uint32_t* lexerrs;
 };
 
+// slices that are on the device at a time
+#define PTXFE_ARENAS 3
+
 struct ptxfe_ctx {
     int device = 0;
-    cudaStream_t stream = nullptr;        // kernels (and everything of the stage / run / fetch calls)
+    cudaStream_t stream = nullptr;        // = streams[0]: everything of the stage / run / fetch calls
+    // Kernels, one stream per arena: a slice is a chain of short steps, several of which leave most of the device idle (the
+    // decoders of a few units, look-backs); the slices next to it fill it.
+    cudaStream_t streams[PTXFE_ARENAS] = {nullptr};
     cudaStream_t s_in = nullptr;          // host -> device copies of the pipelined parse
     cudaStream_t s_out = nullptr;         // device -> host copies of the pipelined parse
     cudaEvent_t ev[8] = {nullptr};
     std::vector<cudaEvent_t> slice_ev;    // 5 per slice: text arrived, kernels begin / end, results begin / end
-    std::vector<ArenaBlock> arenas[2];    // device working memory; the pipelined parse alternates between the two
-    int cur = 0;
+    std::vector<ArenaBlock> arenas[PTXFE_ARENAS];      // device working memory; the pipelined parse goes round them
     char err[512] = {0};
     bool failed = false;
     uint64_t launches = 0;
@@ -818,11 +850,11 @@ struct ptxfe_ctx {
     uint64_t text_bytes = 0, padded_bytes = 0;
     uint8_t* d_text = nullptr;
     size_t d_text_cap = 0;
-    void* d_class_store = nullptr;        // PtxClassStore arrays (one allocation, made at the first parse)
+    void* d_class_store[PTXFE_ARENAS] = {nullptr};     // PtxClassStore arrays (one allocation, made at the first parse)
     PtxLexTables* d_lex_tables = nullptr; // constant tables of the lexer steps (filled at the first parse)
     uint8_t* d_raw = nullptr;             // host-contiguous runs land here before they are repacked into d_text
     size_t d_raw_cap = 0;
-    PtxWork works[2];                     // one per arena
+    PtxWork works[PTXFE_ARENAS];
     PtxCounters counters;                 // of the slice that finished last
     std::unordered_map<const void*, unsigned> resident;      // persistent kernels: blocks that the device holds
     char* h_meta = nullptr; size_t h_meta_cap = 0;           // pinned: layouts of all slices, as they go to the device
@@ -855,6 +887,9 @@ struct ptxfe_ctx {
 struct CudaBackend {
     static constexpr bool kStructureTops = true;
     ptxfe_ctx* ctx;
+    const int arena;
+    const cudaStream_t stream;
+    CudaBackend(ptxfe_ctx* c, int a) : ctx(c), arena(a), stream(c->streams[a]) {}
     const uint32_t* stop = nullptr;        // deferred counts: the word that stops the slice (PtxCounters::redo)
     uint32_t* aborted = nullptr;           // where a look-back that gave up says so
     char* zero_base = nullptr;             // a region cleared ahead of the first step, handed out by zalloc
@@ -873,7 +908,7 @@ struct CudaBackend {
     }
     void* alloc(size_t bytes) {
         bytes = (bytes + 255) & ~(size_t)255;
-        for (ArenaBlock& b : ctx->arenas[ctx->cur])
+        for (ArenaBlock& b : ctx->arenas[arena])
             if (b.size - b.used >= bytes) {
                 void* p = b.base + b.used;
                 b.used += bytes;
@@ -891,22 +926,22 @@ struct CudaBackend {
         }
         nb.size = sz;
         nb.used = bytes;
-        ctx->arenas[ctx->cur].push_back(nb);
+        ctx->arenas[arena].push_back(nb);
         return nb.base;
     }
     void reset() {
-        for (ArenaBlock& b : ctx->arenas[ctx->cur]) b.used = 0;
+        for (ArenaBlock& b : ctx->arenas[arena]) b.used = 0;
     }
     void zero(void* p, size_t bytes) {
         if (ctx->failed || !p) return;
-        cudaMemsetAsync(p, 0, bytes, ctx->stream);
+        cudaMemsetAsync(p, 0, bytes, stream);
     }
     void download(void* host, const void* dev, size_t bytes) {
         if (ctx->failed) { memset(host, 0, bytes); return; }
         // a kernel writes the few words into mapped host memory: a copy-engine transfer would queue behind the
         // result copies of the previous slice, which run on another stream at the same time
-        copy_words_kernel<<<1, 32, 0, ctx->stream>>>((uint32_t*)ctx->d_counters_mapped, (const uint32_t*)dev, (uint32_t)(bytes / 4));
-        cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        copy_words_kernel<<<1, 32, 0, stream>>>((uint32_t*)ctx->d_counters_mapped, (const uint32_t*)dev, (uint32_t)(bytes / 4));
+        cudaError_t e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) {
             snprintf(ctx->err, sizeof ctx->err, "kernel or copy failed: %s", cudaGetErrorString(e));
             ctx->failed = true;
@@ -926,11 +961,11 @@ struct CudaBackend {
             }
         }
         ctx->prof_names.push_back(name);
-        cudaEventRecord(ctx->prof_events[ctx->prof_used++], ctx->stream);
+        cudaEventRecord(ctx->prof_events[ctx->prof_used++], stream);
     }
     void prof_end() {
         if (!ctx->profile) return;
-        cudaEventRecord(ctx->prof_events[ctx->prof_used++], ctx->stream);
+        cudaEventRecord(ctx->prof_events[ctx->prof_used++], stream);
     }
     template <class F> void pf(const char* name, PtxCount n, F f) {
         if (ctx->failed || n.cap == 0) return;
@@ -939,25 +974,25 @@ struct CudaBackend {
         size_t blocks = (n.cap + 255) / 256;
         if (n.dev && blocks > 148 * 64) blocks = 148 * 64;
         prof_begin(name);
-        pf_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(count_of(n), f);
+        pf_kernel<<<(unsigned)blocks, 256, 0, stream>>>(count_of(n), f);
         prof_end();
         ctx->launches++;
     }
     PtxClassStore class_store(bool reset) {
         PtxClassStore cs;
-        if (!ctx->d_class_store) {
-            if (cudaMalloc(&ctx->d_class_store, PtxClassStore::bytes()) != cudaSuccess) {
+        if (!ctx->d_class_store[arena]) {
+            if (cudaMalloc(&ctx->d_class_store[arena], PtxClassStore::bytes()) != cudaSuccess) {
                 if (!ctx->failed) snprintf(ctx->err, sizeof ctx->err, "cudaMalloc of the class store (%zu bytes) failed", PtxClassStore::bytes());
                 ctx->failed = true;
                 cudaGetLastError();
-                ctx->d_class_store = nullptr;
+                ctx->d_class_store[arena] = nullptr;
             }
             reset = true;
         }
-        cs.carve(ctx->d_class_store);
-        if (reset && ctx->d_class_store) {
-            cudaMemsetAsync(cs.keys, 0, sizeof(unsigned long long) * PTX_CLASS_SLOTS, ctx->stream);
-            cudaMemsetAsync(cs.state, 0, 16, ctx->stream);
+        cs.carve(ctx->d_class_store[arena]);
+        if (reset && ctx->d_class_store[arena]) {
+            cudaMemsetAsync(cs.keys, 0, sizeof(unsigned long long) * PTX_CLASS_SLOTS, stream);
+            cudaMemsetAsync(cs.state, 0, 16, stream);
         }
         return cs;
     }
@@ -965,14 +1000,14 @@ struct CudaBackend {
         if (ctx->failed || n.cap == 0) return;
         prof_begin(name);
         // as many blocks as the device holds, or one list entry per warp
-        staged_kernel<<<resident_blocks((const void*)staged_kernel<F>, STAGED_SMEM_BYTES, (n.cap + 7) / 8), 256, STAGED_SMEM_BYTES, ctx->stream>>>(count_of(n), f);
+        staged_kernel<<<resident_blocks((const void*)staged_kernel<F>, STAGED_SMEM_BYTES, (n.cap + 7) / 8), 256, STAGED_SMEM_BYTES, stream>>>(count_of(n), f);
         prof_end();
         ctx->launches++;
     }
     void emit_records(const char* name, PtxCount n, const PtxPair* off, const PtxEmitStep& e) {
         if (ctx->failed || n.cap == 0) return;
         prof_begin(name);
-        emit_records_kernel<<<(unsigned)((n.cap + 255) / 256), 256, 0, ctx->stream>>>(count_of(n), off, e);
+        emit_records_kernel<<<(unsigned)((n.cap + 255) / 256), 256, 0, stream>>>(count_of(n), off, e);
         prof_end();
         ctx->launches++;
     }
@@ -982,11 +1017,11 @@ struct CudaBackend {
         unsigned blocks = (unsigned)((n + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS);
         prof_begin(name);
         if constexpr (std::is_same<F, PtxLexVectorsStep>::value) {
-            lex_tile_kernel<false><<<blocks, 256, LEX_TILE_BYTES, ctx->stream>>>((uint32_t)n, text, f);
+            lex_tile_kernel<false><<<blocks, 256, LEX_TILE_BYTES, stream>>>((uint32_t)n, text, f);
         } else {
             // tile + table need more shared memory than a kernel gets by default
             cudaFuncSetAttribute(lex_tile_kernel<true, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(LEX_TILE_BYTES + LEX_TABLE_BYTES));
-            lex_tile_kernel<true><<<blocks, 256, LEX_TILE_BYTES + LEX_TABLE_BYTES, ctx->stream>>>((uint32_t)n, text, f);
+            lex_tile_kernel<true><<<blocks, 256, LEX_TILE_BYTES + LEX_TABLE_BYTES, stream>>>((uint32_t)n, text, f);
         }
         prof_end();
         ctx->launches++;
@@ -1000,7 +1035,7 @@ struct CudaBackend {
                 ctx->d_lex_tables = nullptr;
                 return nullptr;
             }
-            lex_fill_tables_kernel<<<1, 256, 0, ctx->stream>>>(ctx->d_lex_tables);
+            lex_fill_tables_kernel<<<1, 256, 0, stream>>>(ctx->d_lex_tables);
         }
         return ctx->d_lex_tables;
     }
@@ -1020,14 +1055,14 @@ struct CudaBackend {
     void lex_mark(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
         prof_begin(name);
-        lex_mark_kernel<true><<<resident_blocks((const void*)lex_mark_kernel<true>, 0, n_tiles), 256, 0, ctx->stream>>>(a, 0u, (uint32_t)n_tiles);
+        lex_mark_kernel<true><<<resident_blocks((const void*)lex_mark_kernel<true>, 0, n_tiles), 256, 0, stream>>>(a, 0u, (uint32_t)n_tiles);
         prof_end();
         ctx->launches++;
     }
     void lex_emit(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
         prof_begin(name);
-        lex_emit_kernel<true><<<resident_blocks((const void*)lex_emit_kernel<true>, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), ctx->stream>>>(a, 0u, (uint32_t)n_tiles, stop);
+        lex_emit_kernel<true><<<resident_blocks((const void*)lex_emit_kernel<true>, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), stream>>>(a, 0u, (uint32_t)n_tiles, stop);
         prof_end();
         ctx->launches++;
     }
@@ -1042,8 +1077,8 @@ struct CudaBackend {
         if (!desc) return;
         uint32_t* ctl = (uint32_t*)(desc + n_tiles);      // [0] next tile, [1] abort
         prof_begin(name);
-        structure_mark_kernel<<<(a.n_modules + 255) / 256, 256, 0, ctx->stream>>>(a, desc, stop);
-        structure_kernel<<<resident_blocks((const void*)structure_kernel, 0, n_tiles), SX_THREADS, 0, ctx->stream>>>(a, desc, ctl, stop);
+        structure_mark_kernel<<<(a.n_modules + 255) / 256, 256, 0, stream>>>(a, desc, stop);
+        structure_kernel<<<resident_blocks((const void*)structure_kernel, 0, n_tiles), SX_THREADS, 0, stream>>>(a, desc, ctl, stop);
         prof_end();
         ctx->launches += 2;
     }
@@ -1054,15 +1089,15 @@ struct CudaBackend {
         uint32_t* begin = hist + PTX_SORT_BUCKETS;
         uint32_t* cursor = begin + PTX_SORT_BUCKETS;
         prof_begin(name);
-        cudaMemsetAsync(hist, 0, sizeof(uint32_t) * PTX_SORT_BUCKETS * 3, ctx->stream);
+        cudaMemsetAsync(hist, 0, sizeof(uint32_t) * PTX_SORT_BUCKETS * 3, stream);
         size_t blocks = (n + SORT_TILE - 1) / SORT_TILE;
-        sort_hist_kernel<<<(unsigned)blocks, SORT_THREADS, 0, ctx->stream>>>(n, key, hist);
+        sort_hist_kernel<<<(unsigned)blocks, SORT_THREADS, 0, stream>>>(n, key, hist);
         // exclusive scan of the 4096 counts: begin[b] = sum of hist[0..b)
         ArrayLoad<uint32_t> ld{hist};
         ArrayStore<uint32_t> st{begin};
         scan_impl<uint32_t>((size_t)PTX_SORT_BUCKETS, ld, st, AddOp(), 0u);   // inclusive into begin[]
-        pf_kernel<<<(PTX_SORT_BUCKETS + 255) / 256, 256, 0, ctx->stream>>>(LaunchCount{PTX_SORT_BUCKETS, nullptr, nullptr, 0}, SubtractOwn{begin, hist});
-        sort_scatter_kernel<<<(unsigned)blocks, SORT_THREADS, 0, ctx->stream>>>(n, key, begin, cursor, order);
+        pf_kernel<<<(PTX_SORT_BUCKETS + 255) / 256, 256, 0, stream>>>(LaunchCount{PTX_SORT_BUCKETS, nullptr, nullptr, 0}, SubtractOwn{begin, hist});
+        sort_scatter_kernel<<<(unsigned)blocks, SORT_THREADS, 0, stream>>>(n, key, begin, cursor, order);
         prof_end();
         ctx->launches += 3;
     }
@@ -1077,7 +1112,7 @@ struct CudaBackend {
         ScanDesc<T>* desc = (ScanDesc<T>*)zalloc(sizeof(ScanDesc<T>) * tiles + 16);
         if (!desc) return;
         uint32_t* ctl = (uint32_t*)(desc + tiles);         // [0] next tile, [1] abort
-        scan_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(count_of(n), ld, st, op, identity, desc, ctl, aborted);
+        scan_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, stream>>>(count_of(n), ld, st, op, identity, desc, ctl, aborted);
         ctx->launches++;
     }
 };
@@ -1110,7 +1145,8 @@ int ptxfe_create(int device, ptxfe_ctx** out) {
         return PTXFE_ERR_CUDA;
     }
     cudaError_t e = cudaSetDevice(device);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
+    for (int i = 0; i < PTXFE_ARENAS && e == cudaSuccess; i++) e = cudaStreamCreateWithFlags(&ctx->streams[i], cudaStreamNonBlocking);
+    ctx->stream = ctx->streams[0];
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->s_in, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->s_out, cudaStreamNonBlocking);
     for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&ctx->ev[i]);
@@ -1128,8 +1164,9 @@ int ptxfe_create(int device, ptxfe_ctx** out) {
 void ptxfe_destroy(ptxfe_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
-    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (int a = 0; a < 2; a++)
+    for (cudaStream_t q : ctx->streams)
+        if (q) cudaStreamSynchronize(q);
+    for (int a = 0; a < PTXFE_ARENAS; a++)
         for (ArenaBlock& b : ctx->arenas[a]) cudaFree(b.base);
     for (cudaEvent_t e : ctx->slice_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->prof_events) cudaEventDestroy(e);
@@ -1143,7 +1180,8 @@ void ptxfe_destroy(ptxfe_ctx* ctx) {
         if (e) cudaEventDestroy(e);
     if (ctx->d_meta) cudaFree(ctx->d_meta);
     if (ctx->h_meta) cudaFreeHost(ctx->h_meta);
-    if (ctx->d_class_store) cudaFree(ctx->d_class_store);
+    for (void* p : ctx->d_class_store)
+        if (p) cudaFree(p);
     if (ctx->d_lex_tables) cudaFree(ctx->d_lex_tables);
     if (ctx->h_words) cudaFreeHost(ctx->h_words);
     if (ctx->h_errs) cudaFreeHost(ctx->h_errs);
@@ -1152,7 +1190,8 @@ void ptxfe_destroy(ptxfe_ctx* ctx) {
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
     for (int i = 0; i < 8; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
-    if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    for (cudaStream_t q : ctx->streams)
+        if (q) cudaStreamDestroy(q);
     if (ctx->live) ctx->live->ctx = nullptr;
     delete ctx;
 }
@@ -1260,7 +1299,7 @@ static UploadWay upload_way(const char* const* texts, const uint64_t* lens, uint
     return bytes / runs >= (128u << 10) ? UPLOAD_SLOTS : UPLOAD_GATHER;
 }
 // The modules [m0, m1) of a slice of `padded` bytes through the ring to `dst`, on `stream`.
-static int gather_text(ptxfe_ctx* ctx, cudaStream_t stream, const char* const* texts, uint32_t m0, uint32_t m1, uint64_t padded, uint8_t* dst) {
+static int gather_text(ptxfe_ctx* ctx, cudaStream_t stream, const char* const* texts, uint32_t m0, uint32_t m1, uint64_t base, uint64_t padded, uint8_t* dst) {
     if (!ctx->h_ring) {
         CUDA_TRY(cudaMallocHost((void**)&ctx->h_ring, GATHER_PIECE * GATHER_PIECES));
         for (cudaEvent_t& e : ctx->ring_ev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1272,7 +1311,7 @@ static int gather_text(ptxfe_ctx* ctx, cudaStream_t stream, const char* const* t
     // what an earlier slice sent from the ring may still be on its way
     for (cudaEvent_t e : ctx->ring_ev) CUDA_TRY(cudaEventSynchronize(e));
     cudaError_t err = cudaSuccess;
-    const bool ok = ctx->gather->run(GatherSource{texts + m0, ctx->layout.data() + m0, m1 - m0}, padded, ctx->h_ring,
+    const bool ok = ctx->gather->run(GatherSource{texts + m0, ctx->layout.data() + m0, m1 - m0, base}, padded, ctx->h_ring,
         [&](unsigned slot, uint64_t at, uint64_t len) {
             err = cudaMemcpyAsync(dst + at, ctx->h_ring + slot * GATHER_PIECE, len, cudaMemcpyHostToDevice, stream);
             if (err == cudaSuccess) err = cudaEventRecord(ctx->ring_ev[slot], stream);
@@ -1304,7 +1343,7 @@ int ptxfe_stage(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, 
     CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->stream));
     uint32_t runs;
     if (upload_way(texts, lens, 0, n, &runs) == UPLOAD_GATHER) {
-        if ((st = gather_text(ctx, ctx->stream, texts, 0, n, off, ctx->d_text)) != PTXFE_OK) return st;
+        if ((st = gather_text(ctx, ctx->stream, texts, 0, n, 0, off, ctx->d_text)) != PTXFE_OK) return st;
     } else {
         for (uint32_t m = 0; m < n; m++)
             if (lens[m])
@@ -1328,6 +1367,7 @@ struct SliceRun {
     uint8_t* text = nullptr;              // the slice's text on the device
     size_t meta = 0;                      // where its layouts lie in the metadata buffer
     uint32_t n = 0, mode = 0;
+    uint32_t bias = 0;                    // its offset in the frame that text offsets are relative to
     const uint8_t* raw = nullptr;         // text that came as one run of host memory: the first kernel moves it to its slots
     bool first = true;                    // empties the class store
     int arena = 0;
@@ -1360,12 +1400,13 @@ static int begin_slice(CudaBackend& bk, SliceRun& sl, bool deferred) {
     ptxfe_ctx* ctx = bk.ctx;
     bk.reset();
     const uint32_t n = sl.n;
-    PtxWork& w = ctx->works[ctx->cur];
+    PtxWork& w = ctx->works[sl.arena];
     w = PtxWork();
     w.deferred = deferred;
     w.first_slice = sl.first;
     if (const char* e = getenv("PTXFE_SEQ_MAX_TOKENS")) w.seq_max_tokens = (uint32_t)strtoul(e, nullptr, 10);
-    w.text = sl.text;
+    w.text = sl.text - sl.bias;
+    w.bias = sl.bias;
     w.n_modules = n;
     const size_t mcb_at = sl.meta + (sizeof(PtxModuleLayout) + sizeof(RepackModule)) * (size_t)n;
     w.n_chunks = ((const uint32_t*)(ctx->h_meta + mcb_at))[n];
@@ -1380,41 +1421,40 @@ static int begin_slice(CudaBackend& bk, SliceRun& sl, bool deferred) {
     bk.zero_used = 0;
     w.results = (PtxModuleResult*)bk.alloc(sizeof(PtxModuleResult) * ((size_t)n + 1));
     if (ctx->failed) return PTXFE_ERR_OOM;
-    CUDA_TRY(cudaMemsetAsync(bk.zero_base, 0, zero, ctx->stream));
+    CUDA_TRY(cudaMemsetAsync(bk.zero_base, 0, zero, bk.stream));
     w.counters = (PtxCounters*)bk.zalloc(sizeof(PtxCounters));
     bk.stop = deferred ? &w.counters->redo : nullptr;
     bk.aborted = &w.counters->struct_abort;
     w.results_out = sl.results_out;
-    w.counters_out = deferred ? (PtxCounters*)((char*)ctx->d_counters_mapped + ((char*)PTXFE_COUNTERS_SLOT(ctx, ctx->cur) - (char*)ctx->h_counters)) : nullptr;
+    w.counters_out = deferred ? (PtxCounters*)((char*)ctx->d_counters_mapped + ((char*)PTXFE_COUNTERS_SLOT(ctx, sl.arena) - (char*)ctx->h_counters)) : nullptr;
     return PTXFE_OK;
 }
 static int run_steps(CudaBackend& bk, SliceRun& sl) {
     ptxfe_ctx* ctx = bk.ctx;
-    PtxWork& w = ctx->works[ctx->cur];
+    PtxWork& w = ctx->works[sl.arena];
     if (sl.raw && w.n_chunks) {
         const uint32_t pieces = w.n_chunks * (PTX_CHUNK / 16);
-        repack_text_kernel<<<(pieces + 255) / 256, 256, 0, ctx->stream>>>(pieces, sl.n, (const RepackModule*)(ctx->d_meta + sl.meta + sizeof(PtxModuleLayout) * (size_t)sl.n),
+        repack_text_kernel<<<(pieces + 255) / 256, 256, 0, bk.stream>>>(pieces, sl.n, (const RepackModule*)(ctx->d_meta + sl.meta + sizeof(PtxModuleLayout) * (size_t)sl.n),
                                                                        w.mod_chunk_begin, sl.raw, sl.text);
         ctx->launches++;
     }
     memset(&ctx->counters, 0, sizeof ctx->counters);
     ptx_stage_lex(bk, w, ctx->counters);
-    if (sl.ev_lex) CUDA_TRY(cudaEventRecord(sl.ev_lex, ctx->stream));
+    if (sl.ev_lex) CUDA_TRY(cudaEventRecord(sl.ev_lex, bk.stream));
     if (!ctx->failed) ptx_stage_structure(bk, w, ctx->counters, sl.mode);
-    if (sl.ev_structure) CUDA_TRY(cudaEventRecord(sl.ev_structure, ctx->stream));
+    if (sl.ev_structure) CUDA_TRY(cudaEventRecord(sl.ev_structure, bk.stream));
     if (!ctx->failed) ptx_stage_decode(bk, w, ctx->counters);
-    CUDA_TRY(cudaEventRecord(sl.ev_end, ctx->stream));
+    CUDA_TRY(cudaEventRecord(sl.ev_end, bk.stream));
     return PTXFE_OK;
 }
 // the slice with the host reading the counts on the way; returns when its kernels have finished
 static int run_exact(ptxfe_ctx* ctx, SliceRun& sl) {
-    ctx->cur = sl.arena;
     sl.deferred = false;
-    CudaBackend bk{ctx};
+    CudaBackend bk(ctx, sl.arena);
     int st = begin_slice(bk, sl, false);
     if (st == PTXFE_OK) st = run_steps(bk, sl);
     if (st != PTXFE_OK) return st;
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    cudaError_t e = cudaStreamSynchronize(bk.stream);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
         snprintf(ctx->err, sizeof ctx->err, "pipeline failed: %s", cudaGetErrorString(e));
@@ -1425,15 +1465,14 @@ static int run_exact(ptxfe_ctx* ctx, SliceRun& sl) {
 }
 // Puts the whole slice into the stream without waiting for any of it (deferred counts); finish_slice waits.
 static int enqueue_slice(ptxfe_ctx* ctx, SliceRun& sl) {
-    sl.arena = ctx->cur;
-    CUDA_TRY(cudaEventRecord(sl.ev_begin, ctx->stream));
+    CUDA_TRY(cudaEventRecord(sl.ev_begin, ctx->streams[sl.arena]));
     const uint32_t n_chunks = ((const uint32_t*)(ctx->h_meta + sl.meta + (sizeof(PtxModuleLayout) + sizeof(RepackModule)) * (size_t)sl.n))[sl.n];
     if (n_chunks == 0) return run_exact(ctx, sl);
     sl.deferred = true;
-    CudaBackend bk{ctx};
+    CudaBackend bk(ctx, sl.arena);
     int st = begin_slice(bk, sl, true);
     if (st != PTXFE_OK) return st;
-    PtxWork& w = ctx->works[ctx->cur];
+    PtxWork& w = ctx->works[sl.arena];
     if (sl.words_out) {
         w.words = sl.words_out;
         if (w.cap_words > sl.words_out_cap) w.cap_words = sl.words_out_cap;
@@ -1462,25 +1501,23 @@ static int finish_slice(ptxfe_ctx* ctx, SliceRun& sl) {
         }
         if (ctx->counters.redo && !(ctx->counters.redo & ~PTX_REDO_DECODE)) {
             // tokens and units stand: the decode stage alone, with the host reading its counts
-            ctx->cur = sl.arena;
-            CudaBackend bk{ctx};
+                    CudaBackend bk(ctx, sl.arena);
             bk.aborted = &w.counters->struct_abort;
             w.first_slice = true;
             ptx_stage_decode_anew(bk, w, ctx->counters);
-            CUDA_TRY(cudaEventRecord(sl.ev_end, ctx->stream));
-            CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            CUDA_TRY(cudaEventRecord(sl.ev_end, bk.stream));
+            CUDA_TRY(cudaStreamSynchronize(bk.stream));
             if (ctx->failed) return strstr(ctx->err, "cudaMalloc") ? PTXFE_ERR_OOM : PTXFE_ERR_CUDA;
         } else if (ctx->counters.redo) {
             sl.first = true;
             int st = run_exact(ctx, sl);
             if (st != PTXFE_OK) return st;
         } else if (ptx_needs_again(ctx->counters)) {
-            ctx->cur = sl.arena;
-            CudaBackend bk{ctx};
+                    CudaBackend bk(ctx, sl.arena);
             bk.aborted = &w.counters->struct_abort;
             ptx_stage_again(bk, w, ctx->counters);
-            CUDA_TRY(cudaEventRecord(sl.ev_end, ctx->stream));
-            CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            CUDA_TRY(cudaEventRecord(sl.ev_end, bk.stream));
+            CUDA_TRY(cudaStreamSynchronize(bk.stream));
             if (ctx->failed) return strstr(ctx->err, "cudaMalloc") ? PTXFE_ERR_OOM : PTXFE_ERR_CUDA;
         }
     }
@@ -1515,7 +1552,6 @@ int ptxfe_run(ptxfe_ctx* ctx, uint32_t mode) {
     ctx->prof_used = 0;
     ctx->prof_names.clear();
     ctx->mode = mode;
-    ctx->cur = 0;
     SliceRun sl;
     sl.text = ctx->d_text;
     sl.n = (uint32_t)ctx->layout.size();
@@ -1613,6 +1649,20 @@ int ptxfe_fetch(ptxfe_ctx* ctx, ptxfe_batch** out) {
 // One call, host text in, host records out.  The batch is cut into slices of whole modules; the text of slice k+1
 // travels to the device and the records of slice k-1 travel back while the kernels of slice k run (three streams,
 // two working arenas).  Text offsets inside the records are relative to the slice, as ptxfe_module_records reports.
+// How much text the next slice takes, `done` bytes into a batch of `total`.  Slices grow from 8 MiB and shrink to it again:
+// the first text copy and the last result copy overlap with nothing.  Below 16 MiB in all a batch is one slice, as a slice
+// is a chain of some fifteen short steps (0.25 ms) whatever its size; above 128 MiB a slice gains nothing.  Measured on
+// 64 MiB in 250 modules: 3.12 ms as two slices of 32 MiB, 3.46 from 4 MiB on, 2.82 from 8, 2.96 from 16; on 1 GiB: 32.9 ms
+// in slices of 16 MiB at most, 30.6 at 32, 29.3 at 64, 29.1 at 128.
+#define PTXFE_SLICE_LEAST ((uint64_t)8 << 20)
+static uint64_t slice_target(uint64_t total, uint64_t done) {
+    if (total < 2 * PTXFE_SLICE_LEAST) return ~0ull;
+    const uint64_t most = (uint64_t)128 << 20, left = total - done;
+    uint64_t t = done < left / 2 ? done : left / 2;
+    if (t > most) t = most;
+    return t < PTXFE_SLICE_LEAST ? PTXFE_SLICE_LEAST : t;
+}
+
 int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, uint32_t n, uint32_t mode, ptxfe_batch** out) {
     if (!out) return PTXFE_ERR_BAD_ARG;
     *out = nullptr;
@@ -1633,32 +1683,49 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     uint64_t grand_total = 0;
     for (uint32_t m = 0; m < n; m++) grand_total += lens[m];
     uint64_t edge = (uint64_t)32 << 20, div = 8;
+    bool forced = false;
     if (const char* e = getenv("PTXFE_SLICE_DIV")) { uint64_t v = strtoull(e, nullptr, 10); if (v) div = v; }
     uint64_t middle = grand_total / div;
     if (middle < ((uint64_t)64 << 20)) middle = (uint64_t)64 << 20;
     if (middle > ((uint64_t)512 << 20)) middle = (uint64_t)512 << 20;
     if (const char* e = getenv("PTXFE_SLICE_BYTES")) {
         uint64_t v = strtoull(e, nullptr, 10);
-        if (v) edge = middle = v;
+        if (v) { edge = middle = v; forced = true; }
     }
-    struct Slice { uint32_t m0, m1; uint64_t text_off, padded, bytes; };
+    // A frame is what the text offsets in the records are relative to.  A slice, what is copied and run at a time, is a
+    // part of one frame: `bias` is its offset there.
+    struct Slice { uint32_t m0, m1; uint64_t text_off, padded, bytes, bias; };
     std::vector<Slice> slices;
     uint64_t total = 0, text_off = 0;
+    bool first_frame = true;
     for (uint32_t m = 0; m < n;) {
         uint64_t left = grand_total - total;
-        uint64_t target = slices.empty() ? edge : middle;
-        if (!slices.empty() && left > edge && left <= middle + edge) target = left - edge;   // leave a small last slice
+        uint64_t target = first_frame ? edge : middle;
+        if (!first_frame && left > edge && left <= middle + edge) target = left - edge;   // leave a small last slice
         uint32_t m1 = m;
         uint64_t bytes = 0;
         while (m1 < n && (m1 == m || bytes + lens[m1] <= target)) bytes += lens[m1++];
         uint64_t padded = layout_slice(ctx, lens, m, m1);
         if (padded >= 0xFFFFFF00ull) return PTXFE_ERR_TOO_LARGE;
-        slices.push_back(Slice{m, m1, text_off, padded, bytes});
+        first_frame = false;
+        const uint64_t frame_end = total + bytes;
+        for (uint32_t a = m; a < m1;) {
+            const uint64_t want = forced ? ~0ull : slice_target(grand_total, total);
+            uint32_t e = a;
+            uint64_t part = 0;
+            while (e < m1 && (e == a || part + lens[e] <= want)) part += lens[e++];
+            if (total + part + PTXFE_SLICE_LEAST / 2 > frame_end)      // no crumbs at the end of a frame
+                while (e < m1) part += lens[e++];
+            const uint64_t bias = ctx->layout[a].text_off, end = e < m1 ? ctx->layout[e].text_off : padded;
+            for (uint32_t j = a; j < e; j++) ctx->layout[j].chunk_begin = (uint32_t)((ctx->layout[j].text_off - bias) / PTX_CHUNK);
+            slices.push_back(Slice{a, e, text_off + bias, end - bias, part, bias});
+            total += part;
+            a = e;
+        }
         text_off += padded;
-        total += bytes;
         m = m1;
     }
-    if (slices.empty()) slices.push_back(Slice{0, 0, 0, 0, 0});
+    if (slices.empty()) slices.push_back(Slice{0, 0, 0, 0, 0, 0});
     const size_t ns = slices.size();
     int st = text_off <= PTXFE_SMALL_BYTES ? PTXFE_OK : ensure_text(ctx, text_off);
     if (st != PTXFE_OK) return st;
@@ -1717,7 +1784,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         const Slice& sl = slices[k];
         if (k == 0) {
             CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->s_in));
-            if (small) GatherSource{texts, ctx->layout.data(), n}.fill(ctx->h_meta + meta_total, 0, text_off);
+            if (small) GatherSource{texts, ctx->layout.data(), n, 0}.fill(ctx->h_meta + meta_total, 0, text_off);
             CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_total + (small ? text_off : 0), cudaMemcpyHostToDevice, ctx->s_in));
         }
         if (way[k] == UPLOAD_RUNS) {
@@ -1729,12 +1796,12 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
                 m = e;
             }
         } else if (way[k] == UPLOAD_GATHER && !small) {
-            int st = gather_text(ctx, ctx->s_in, texts, sl.m0, sl.m1, sl.padded, ctx->d_text + sl.text_off);
+            int st = gather_text(ctx, ctx->s_in, texts, sl.m0, sl.m1, sl.bias, sl.padded, ctx->d_text + sl.text_off);
             if (st != PTXFE_OK) return st;
         } else if (!small) {
             for (uint32_t m = sl.m0; m < sl.m1; m++)
                 if (lens[m])
-                    CUDA_TRY(cudaMemcpyAsync(ctx->d_text + sl.text_off + ctx->layout[m].text_off, texts[m], lens[m], cudaMemcpyHostToDevice, ctx->s_in));
+                    CUDA_TRY(cudaMemcpyAsync(ctx->d_text + sl.text_off + (ctx->layout[m].text_off - sl.bias), texts[m], lens[m], cudaMemcpyHostToDevice, ctx->s_in));
         }
         CUDA_TRY(cudaEventRecord(ctx->slice_ev[5 * k], ctx->s_in));
         if (k + 1 == ns) CUDA_TRY(cudaEventRecord(ctx->ev[1], ctx->s_in));
@@ -1745,7 +1812,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     auto drain = [&](int code) -> int {
         cudaStreamSynchronize(ctx->s_in);
         cudaStreamSynchronize(ctx->s_out);
-        cudaStreamSynchronize(ctx->stream);
+        for (cudaStream_t q : ctx->streams) cudaStreamSynchronize(q);
         return code;
     };
 #define DRAIN_TRY(call)                                                                     \
@@ -1774,16 +1841,18 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     auto enqueue = [&](size_t k) -> int {
         const Slice& sl = slices[k];
         SliceRun& r = runs[k];
-        ctx->cur = (int)(k & 1);
-        // this arena held the results of slice k-2: they leave the device first
-        if (k >= 2) CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->slice_ev[5 * (k - 2) + 4], 0));
-        CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->slice_ev[5 * k], 0));
+        r.arena = (int)(k % PTXFE_ARENAS);
+        const cudaStream_t q = ctx->streams[r.arena];
+        // this arena held the results of an earlier slice: they leave the device first
+        if (k >= PTXFE_ARENAS) CUDA_TRY(cudaStreamWaitEvent(q, ctx->slice_ev[5 * (k - PTXFE_ARENAS) + 4], 0));
+        CUDA_TRY(cudaStreamWaitEvent(q, ctx->slice_ev[5 * k], 0));
+        r.bias = (uint32_t)sl.bias;
         r.text = small ? (uint8_t*)ctx->d_meta + meta_total : ctx->d_text + sl.text_off;
         r.meta = meta_at[k];
         r.n = sl.m1 - sl.m0;
         r.mode = mode;
         r.raw = way[k] == UPLOAD_RUNS ? ctx->d_raw + raw_base[k] : nullptr;
-        r.first = k == 0;
+        r.first = k < PTXFE_ARENAS;
         r.results_out = (PtxModuleResult*)ctx->h_results + sl.m0;
         if (ns == 1 && total <= PTXFE_DIRECT_OUT_BYTES) {
             r.words_out = (uint32_t*)ctx->h_words;
@@ -1793,15 +1862,25 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         r.ev_end = ctx->slice_ev[5 * k + 2];
         return enqueue_slice(ctx, r);
     };
-    if ((rc = enqueue(0)) != PTXFE_OK) return drain(rc);
-    if (ns > 1 && (rc = submit_text(1)) != PTXFE_OK) return drain(rc);
+    // The text goes ahead of the kernels: two slices further where the device fetches it itself, as late as possible where
+    // this thread has to gather it.
+    size_t sent = 1;
+    auto send_up_to = [&](size_t last) -> int {
+        for (; sent < ns && (sent <= last || (sent <= last + 2 && way[sent] != UPLOAD_GATHER)); sent++) {
+            int st = submit_text(sent);
+            if (st != PTXFE_OK) return st;
+        }
+        return PTXFE_OK;
+    };
+    for (size_t k = 0; k + 1 < PTXFE_ARENAS && k < ns; k++)
+        if ((rc = send_up_to(k)) != PTXFE_OK || (rc = enqueue(k)) != PTXFE_OK) return drain(rc);
     for (size_t k = 0; k < ns; k++) {
         const Slice& sl = slices[k];
-        if (k + 1 < ns && (rc = enqueue(k + 1)) != PTXFE_OK) return drain(rc);
-        if (k + 2 < ns && (rc = submit_text(k + 2)) != PTXFE_OK) return drain(rc);
+        const size_t ahead = k + PTXFE_ARENAS - 1;
+        if (ahead < ns && ((rc = send_up_to(ahead)) != PTXFE_OK || (rc = enqueue(ahead)) != PTXFE_OK)) return drain(rc);
         if ((rc = finish_slice(ctx, runs[k])) != PTXFE_OK) return drain(rc);
         const PtxCounters& c = ctx->counters;
-        const PtxWork& w = ctx->works[k & 1];
+        const PtxWork& w = ctx->works[k % PTXFE_ARENAS];
         size_t nw = c.n_words, ne = c.n_errs, nl = c.n_lexerrs;
         const bool words_there = w.words == (uint32_t*)ctx->h_words;        // the kernels wrote them to the host themselves
         if ((words_done + nw) * sizeof(uint32_t) + 16 > ctx->h_words_cap || (errs_done + ne) * sizeof(PtxErrRec) + 16 > ctx->h_errs_cap ||
@@ -1830,8 +1909,8 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         s.n_errors += ne;
         s.n_lex_errors += nl;
         s.n_untemplated += c.n_rest;
-        s.n_classes = c.n_classes;
-        s.n_signature_words = c.n_sig_words;
+        if (c.n_classes > s.n_classes) s.n_classes = c.n_classes;      // of the fullest store
+        if (c.n_sig_words > s.n_signature_words) s.n_signature_words = c.n_sig_words;
     }
     DRAIN_TRY(cudaStreamSynchronize(ctx->s_out));
     DRAIN_TRY(cudaStreamSynchronize(ctx->s_in));
@@ -2105,11 +2184,10 @@ int ptxfe_lex_module(ptxfe_ctx* ctx, const char* text, uint64_t len, uint32_t** 
     int st = ptxfe_stage(ctx, texts, lens, 1);
     if (st != PTXFE_OK) return st;
     ctx->failed = false;
-    ctx->cur = 0;
     SliceRun sl;
     sl.text = ctx->d_text;
     sl.n = 1;
-    CudaBackend bk{ctx};
+    CudaBackend bk(ctx, 0);
     PtxWork& w = ctx->works[0];
     if ((st = begin_slice(bk, sl, false)) != PTXFE_OK) return st;
     memset(&ctx->counters, 0, sizeof ctx->counters);

@@ -7,7 +7,7 @@
 //        -> [brace / paren classification | segmented scan] -> [unit starts | scan | compact]
 //        -> [decode units: count] -> [chain check per module] -> [scan sizes] -> [function table] -> [decode units: emit]
 #pragma once
-#include "ptx_units.h"
+#include "ptx_fast.h"
 
 struct PtxModuleLayout {
     uint64_t text_off;    // byte offset in the batch text buffer (multiple of PTX_CHUNK)
@@ -61,6 +61,7 @@ struct PtxScratch {
     uint32_t stage_stride, stage_cap;
     PtxTokenWord* win;
     uint32_t win_stride, win_cap;
+    bool filled = false;         // the backend has put the unit's first tokens there (as many as PtxDecodeListStep::window says)
 };
 
 // ---- unit classes and record templates
@@ -105,6 +106,8 @@ PTX_HD inline uint64_t ptx_class_key(const uint8_t* text, const PtxToken* tokens
     for (uint32_t i = start; i < end; i++) {
         const uint32_t kl = kinds[i];
         const uint16_t kind = PTX_KL_KIND(kl);
+        // a `call` and a counted name (%r<8>) put into their records what no tag can express: no class, decoded at once
+        if (kind == T_OP_CALL || kind == T_LT) return 0;
         h1 = (h1 ^ kind) * 16777619u;
         h2 = (h2 + kind) * 0x9E3779B1u;
         h2 ^= h2 >> 15;
@@ -306,7 +309,8 @@ PTX_HD inline uint32_t ptx_upper_bound_u32(const uint32_t* a, uint32_t n, uint32
 
 // Device-resident working set of one batch.  Pointers are owned by the backend's arena.
 struct PtxWork {
-    const uint8_t* text = nullptr;
+    const uint8_t* text = nullptr;         // what text offsets are relative to
+    uint32_t bias = 0;                     // offset of the slice's first chunk (a multiple of PTX_CHUNK)
     uint32_t n_modules = 0, n_chunks = 0;
     PtxModuleLayout* layout = nullptr;     // [n_modules]
     uint32_t* mod_chunk_begin = nullptr;   // [n_modules + 1]
@@ -400,9 +404,13 @@ struct PtxLexChunkInfo {
     const PtxModuleLayout* layout;
     const uint32_t* mcb;
     uint32_t n_modules;
+    // Text offsets outside the lexer may count from further in front than the slice's first chunk (a batch is cut finer
+    // than the frames that its records' offsets are relative to): inside the lexer everything counts from that chunk.
+    uint32_t bias = 0;
+    PTX_HD uint32_t begin(uint32_t m) const { return (uint32_t)layout[m].text_off - bias; }
     PTX_HD void locate(size_t c, uint32_t& ms, uint32_t& me, bool& first) const {
         uint32_t m = ptx_upper_bound_u32(mcb, n_modules, (uint32_t)c) - 1;
-        ms = (uint32_t)layout[m].text_off;
+        ms = begin(m);
         me = ms + (uint32_t)layout[m].text_len;
         first = c == mcb[m];
     }
@@ -415,7 +423,7 @@ struct PtxLexVectorsStep {
     template <class R> PTX_HD void operator()(size_t c, const R& rd) const {
         uint32_t cs = (uint32_t)c * PTX_CHUNK;
         const uint32_t m = ptx_upper_bound_u32(info.mcb, info.n_modules, (uint32_t)c) - 1;
-        const uint32_t ms = (uint32_t)info.layout[m].text_off, me = ms + (uint32_t)info.layout[m].text_len;
+        const uint32_t ms = info.begin(m), me = ms + (uint32_t)info.layout[m].text_len;
         const bool first = c == info.mcb[m];
         if (c % LT_CHUNKS == 0) tile_mod[c / LT_CHUNKS] = m;
         uint32_t ce = cs + PTX_CHUNK < me ? cs + PTX_CHUNK : me;
@@ -441,6 +449,7 @@ struct PtxLexErrorsStep {
         int state = first ? CX_CODE : (int)(vec[c - 1] & 7u);
         LexErrorSink sink;
         sink.errors = lexerrs + 2 * (size_t)cnt[c].b;
+        sink.bias = info.bias;
         lx_chunk(rd, text, ms, me, cs, cs + PTX_CHUNK, state, sink);
     }
 };
@@ -488,27 +497,29 @@ template <class BK>
 inline void ptx_lex_errors(BK& bk, PtxWork& w, uint32_t n_lexerrs) {
     uint32_t* lexerrs = w.lexerrs = (uint32_t*)bk.alloc(sizeof(uint32_t) * 2 * (size_t)(n_lexerrs + 1));
     if (!n_lexerrs) return;
-    const uint8_t* text = w.text;
+    const uint8_t* text = w.text + w.bias;
     const PtxModuleLayout* layout = w.layout;
     const uint32_t* mcb = w.mod_chunk_begin;
     const PtxPair* cnt = w.chunk_cnt;
     const uint32_t* mod_flag = w.lex_flag;
-    bk.pf_text("lex_emit_errors", w.n_chunks, text, PtxLexErrorsStep{PtxLexChunkInfo{layout, mcb, w.n_modules}, text, w.chunk_vec, cnt, lexerrs, mod_flag});
+    const PtxLexChunkInfo info{layout, mcb, w.n_modules, w.bias};
+    bk.pf_text("lex_emit_errors", w.n_chunks, text, PtxLexErrorsStep{info, text, w.chunk_vec, cnt, lexerrs, mod_flag});
     // the flagged modules: one thread each, one walk over the module (linear in its length whatever its runs)
     bk.pf("lex_emit_errors_serial", w.n_modules, [=] PTX_HD(size_t m) {
         if (!mod_flag[m]) return;
         const uint32_t c0 = mcb[m], c1 = mcb[m + 1];
         if (c0 == c1 || cnt[c1].b == cnt[c0].b) return;
-        const uint32_t ms = (uint32_t)layout[m].text_off, me = ms + (uint32_t)layout[m].text_len;
+        const uint32_t ms = info.begin((uint32_t)m), me = ms + (uint32_t)layout[m].text_len;
         LexErrorSink sink;
         sink.errors = lexerrs + 2 * (size_t)cnt[c0].b;
+        sink.bias = info.bias;
         lx_chunk(PtxGlobalReader{text, me}, text, ms, me, ms, me, CX_CODE, sink);
     });
 }
 
 template <class BK>
 inline void ptx_stage_lex(BK& bk, PtxWork& w, PtxCounters& host_counters) {
-    const uint8_t* text = w.text;
+    const uint8_t* text = w.text + w.bias;
     const PtxModuleLayout* layout = w.layout;
     const uint32_t* mcb = w.mod_chunk_begin;
     const uint32_t n_modules = w.n_modules, n_chunks = w.n_chunks;
@@ -516,7 +527,7 @@ inline void ptx_stage_lex(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     PtxPair* cnt = w.chunk_cnt = (PtxPair*)bk.alloc(sizeof(PtxPair) * (n_chunks + 2));
     w.mod_tok_begin = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 2));
     PtxCounters* counters = w.counters;
-    const PtxLexChunkInfo info{layout, mcb, n_modules};
+    const PtxLexChunkInfo info{layout, mcb, n_modules, w.bias};
 
     // A1: transition vector of every chunk, module of every tile
     const size_t n_tiles = ((size_t)n_chunks + LT_CHUNKS - 1) / LT_CHUNKS;
@@ -805,6 +816,15 @@ struct PtxDecodeListStep {
     uint32_t* staged;
     PtxFnEntry* fn_entries;
     PtxCounters* counters;
+    // the tokens that go to the fast window: the unit's own and the one behind, from `start` on
+    PTX_HD uint32_t window(size_t idx, uint32_t win_cap, uint32_t* start) const {
+        const uint32_t u = list[idx] & 0x7FFFFFFFu;
+        *start = ustart[u];
+        const uint32_t n_tokens = counters->n_tokens;
+        const uint32_t end = u + 1 < counters->n_units ? ustart[u + 1] + 1u : n_tokens;
+        const uint32_t n = (end < n_tokens ? end : n_tokens) - *start;
+        return n < win_cap ? n : win_cap;
+    }
     PTX_HD PtxStaged operator()(size_t idx, const PtxScratch& sc) const {
         PtxStaged ret;
         ret.unit = 0;
@@ -817,40 +837,60 @@ struct PtxDecodeListStep {
         const uint32_t te = mtb[m + 1];
         const uint32_t end = u + 1 < mub[m + 1] ? ustart[u + 1] : te;
         const uint32_t id = rep ? cs.slot_tmpl[uclass[u]] : 0u;
-        PtxSink sink;
-        if (rep) {
-            sink.words = cs.tmpl_words + (size_t)id * PTX_TMPL_WORDS;
-            sink.tags = cs.tmpl_tags + (size_t)id * PTX_TMPL_WORDS;
-            sink.words_cap = PTX_TMPL_WORDS;
+        // the unit's first tokens go to the fast window: the decoder looks at every token many times.  (A token of the next
+        // module may be among them: the decoder does not look at tokens behind its module's last.)
+        uint32_t from;
+        const uint32_t nwin = window(idx, sc.win_cap, &from);
+        if (!sc.filled)
+            for (uint32_t k = 0; k < nwin; k++) sc.win[k * sc.win_stride] = ((const PtxTokenWord*)(tokens + start))[k];
+        const uint32_t dp = udepth[u], depth = dp & 0x7FFFFFFFu;
+        uint32_t* const out_words = rep ? cs.tmpl_words + (size_t)id * PTX_TMPL_WORDS : sc.stage;
+        uint16_t* const out_tags = rep ? cs.tmpl_tags + (size_t)id * PTX_TMPL_WORDS : nullptr;
+        const uint32_t out_stride = rep ? 1u : sc.stage_stride, out_cap = rep ? PTX_TMPL_WORDS : sc.stage_cap;
+        PtxUnitResult r;
+        uint32_t nw, ne = 0, high;
+        bool as_is = true, bulk_used = false;      // as_is: the record depends on nothing that a tag cannot express
+        PtxFast fast{text, (const PtxTokenWord*)(tokens + start), sc.win, nwin, sc.win_stride, end - start, out_words, out_tags, out_stride, out_cap};
+        if (!(dp >> 31) && (depth ? fast.instruction() : fast.kernel_header())) {
+            r.end = end;
+            r.status = US_OK;
+            r.kind = depth ? U_INSTR : U_FUNC;
+            r.name_tok = start + fast.name_tok;
+            r.n_rets = 0;
+            r.n_inputs = fast.n_inputs;
+            nw = high = fast.nw;
         } else {
-            sink.stage = sc.stage;
-            sink.stage_stride = sc.stage_stride;
-            sink.stage_cap = sc.stage_cap;
-        }
-        PtxResolver res;
-        res.module = m;
-        PtxDecoder d(text, tokens, te, layout[m].text_off + layout[m].text_len, sink, res);
-        d.bulk = bulk;
-        // the unit's first tokens go to the fast window: the decoder looks at every token many times
-        {
-            uint32_t nwin = te - start < sc.win_cap ? te - start : sc.win_cap;
-            if (nwin > end - start + 1u) nwin = end - start + 1u;
-            const PtxTokenWord* src = (const PtxTokenWord*)(tokens + start);
-            for (uint32_t k = 0; k < nwin; k++) sc.win[k * sc.win_stride] = src[k];
+            PtxSink sink;
+            if (rep) {
+                sink.words = out_words;
+                sink.tags = out_tags;
+                sink.words_cap = out_cap;
+            } else {
+                sink.stage = out_words;
+                sink.stage_stride = out_stride;
+                sink.stage_cap = out_cap;
+            }
+            PtxResolver res;
+            res.module = m;
+            PtxDecoder d(text, tokens, te, layout[m].text_off + layout[m].text_len, sink, res);
+            d.bulk = bulk;
             d.win = sc.win;
             d.win_base = start;
             d.win_n = nwin;
             d.win_stride = sc.win_stride;
+            r = ptx_decode_unit(d, start, depth, (dp >> 31) != 0);
+            nw = d.out.nw;
+            ne = d.out.ne;
+            high = d.out.high();
+            as_is = !d.out.poison && d.max_seen < end;
+            bulk_used = d.bulk_used;
         }
-        const uint32_t dp = udepth[u];
-        const PtxUnitResult r = ptx_decode_unit(d, start, dp & 0x7FFFFFFFu, (dp >> 31) != 0);
         if (rep) {
             PtxTemplateInfo ti;
-            ti.n_words = d.out.nw;
+            ti.n_words = nw;
             ti.n_tokens = end - start;
-            ti.depth1 = (dp & 0x7FFFFFFFu) == 1 ? 1u : 0u;
-            ti.ok = (r.status == US_OK && d.out.ne == 0 && d.out.high() <= PTX_TMPL_WORDS && !d.out.poison && r.kind != U_FUNC && r.end == end &&
-                     d.max_seen < end) ? 1u : 0u;
+            ti.depth1 = depth == 1 ? 1u : 0u;
+            ti.ok = (r.status == US_OK && ne == 0 && high <= PTX_TMPL_WORDS && as_is && r.kind != U_FUNC && r.end == end) ? 1u : 0u;
             if (ti.ok) {
                 const uint32_t need = ptx_signature_words(tokens, start, ti.n_tokens);
                 const uint32_t at = PTX_COUNT_ADD(&cs.state[1], need);
@@ -866,16 +906,16 @@ struct PtxDecodeListStep {
         }
         uend[u] = r.end;
         ustatus[u] = (uint8_t)r.status;
-        bool flagged = d.out.high() > d.out.stage_cap || d.out.ne > 0 || d.bulk_used;
-        if (!flagged && d.out.nw) {
-            const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_words, d.out.nw);
-            flagged = (uint64_t)at + d.out.nw > cap_staged;
+        bool flagged = high > out_cap || ne > 0 || bulk_used;
+        if (!flagged && nw) {
+            const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_words, nw);
+            flagged = (uint64_t)at + nw > cap_staged;
             if (!flagged) {
-                for (uint32_t k = 0; k < d.out.nw; k++) staged[at + k] = sc.stage[k * sc.stage_stride];
+                for (uint32_t k = 0; k < nw; k++) staged[at + k] = sc.stage[k * sc.stage_stride];
                 utmpl[u] = at;
             }
         }
-        uown[u] = PtxPair{flagged ? d.out.high() : d.out.nw, d.out.ne};
+        uown[u] = PtxPair{flagged ? high : nw, ne};
         uflag[u] = flagged ? PTX_UNIT_FLAGGED : PTX_UNIT_STAGED;
         if (flagged) PTX_COUNT_ADD(&counters->n_flagged, 1);
         if (r.status == US_OK && r.kind == U_FUNC) {
