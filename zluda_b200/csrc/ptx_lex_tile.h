@@ -17,9 +17,9 @@
 //         of "soft" bytes around it (word characters and % . : + -) is lexed from its first byte, a token start;
 //     T3  "::": .shared::cta and its like are single tokens, and what follows them starts a new one; same treatment;
 //     T2  a sigil (_ $ %) that starts a word and is followed by no word character: a lexer error, not a token.
-//   Chunks that contain a comment or string character (/ * ") or start inside a comment or string take the proven
-//   byte-serial walk (lx_chunk), one thread per chunk.  Every writer of the second round sets bits to the true lexing,
-//   so where two of them meet they agree.
+//   Chunks that contain a comment or string character (/ * ") or start inside a comment or string are gone over once
+//   more with the bytes of comments and strings read as blanks (lt_mark_window).  Every writer of the second round sets
+//   bits to the true lexing, so where two of them meet they agree.
 // Step 2, lex_emit: the set bits are first listed (one thread per 32-byte window writes the tile offsets of its tokens
 //   to their ranks in shared memory); then one thread per TOKEN finds the token's length and kind - punctuation and
 //   sigil-led words at once, words that may spell a keyword through the 8-byte keyword table, numbers through the
@@ -33,6 +33,7 @@
 #define LT_PIECES (LT_BYTES / 16u)
 #define LT_WORDS (LT_BYTES / 32u)
 #define LT_TRIG_CAP 1536u          // triggers per tile; a tile with more is lexed chunk by chunk by the serial walk
+#define LT_TRIG_WINDOWS 0x80000000u
 #define LT_BACK_CAP 2048u          // longest look-back over a run of soft bytes; beyond it the module is lexed by one thread
 #define LT_TOK_CAP 3072u           // tokens the emit step lists at a time; a tile with more goes in passes of LT_TOK_CAP / PTX_CHUNK chunks
 #define LT_EXACT_CAP 2048u         // tokens of a pass the emit step leaves to its second round (more are settled on the spot)
@@ -286,7 +287,7 @@ PTX_HD inline void lt_mark_simple(PtxLexMarkShared& sh, const PtxLexTileArgs& a,
                     any |= e;
                     if (e & (LP_ERR | LP_T1 | LP_T2 | LP_T3)) {
                         em |= ((e >> 1) & 1u) << i;
-                        if (e & (LP_T1 | LP_T2 | LP_T3)) {
+                        if ((e & (LP_T1 | LP_T2 | LP_T3)) && cx == CX_CODE) {
                             uint32_t slot = LT_ATOMIC_ADD(&sh.n_trig, 1u);
                             if (slot < LT_TRIG_CAP) sh.trig[slot] = (win * 32u + i) | ((e & (LP_T1 | LP_T2 | LP_T3)) << 16);
                         }
@@ -301,7 +302,7 @@ PTX_HD inline void lt_mark_simple(PtxLexMarkShared& sh, const PtxLexTileArgs& a,
                     em |= ((e >> 1) & 1u) << i;
                     wm |= ((e >> 2) & 1u) << i;
                     any |= e;
-                    if (e & (LP_T1 | LP_T2 | LP_T3)) {
+                    if ((e & (LP_T1 | LP_T2 | LP_T3)) && cx == CX_CODE) {
                         uint32_t slot = LT_ATOMIC_ADD(&sh.n_trig, 1u);
                         if (slot < LT_TRIG_CAP) sh.trig[slot] = (win * 32u + i) | ((e & (LP_T1 | LP_T2 | LP_T3)) << 16);
                     }
@@ -313,7 +314,7 @@ PTX_HD inline void lt_mark_simple(PtxLexMarkShared& sh, const PtxLexTileArgs& a,
             // the module (where nothing follows)
             if ((win == LT_WORDS - 1 && n == 32 && pos0 + 32 < me) || pos0 + n == me) {
                 const uint32_t e = sh.step[(st << 4) | (pos0 + n == me ? (uint32_t)TC_WS : (uint32_t)sh.cls[a.text[pos0 + 32]])];
-                if (e & (LP_T1 | LP_T2 | LP_T3)) {
+                if ((e & (LP_T1 | LP_T2 | LP_T3)) && cx == CX_CODE) {
                     uint32_t slot = LT_ATOMIC_ADD(&sh.n_trig, 1u);
                     if (slot < LT_TRIG_CAP) sh.trig[slot] = (win * 32u + n) | ((e & (LP_T1 | LP_T2 | LP_T3)) << 16);
                 }
@@ -385,35 +386,123 @@ struct LexMarkSink {
     }
 };
 
-// ---- phase 2a: chunks with comment or string characters, one thread per chunk
-PTX_HD inline void lt_mark_special(PtxLexMarkShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t tid, uint32_t nt) {
-    const bool overflow = sh.n_trig > LT_TRIG_CAP;      // too many triggers to list: every chunk takes the serial walk
-    for (uint32_t k = tid; k < LT_CHUNKS; k += nt) {
-        const uint32_t c = tile * LT_CHUNKS + k;
-        if (c >= a.n_chunks) continue;
-        if (overflow) sh.chunk_special[k] = 1;
-        if (!sh.chunk_special[k]) continue;
-        const uint32_t ms = sh.chunk_ms[k], me = sh.chunk_me[k], cs = c * PTX_CHUNK, tile_base = tile * LT_BYTES;
-        for (uint32_t w = 0; w < 4; w++) sh.start[k * 4 + w] = sh.err[k * 4 + w] = 0;
-        if (cs >= me) continue;
-        // the walk looks back over one run of soft bytes; a run longer than the cap goes to the one-thread path
-        uint32_t run_start = cs;
-        if (sh.chunk_cx[k] == CX_CODE && cs > ms && lx_soft(a.text[cs - 1]) && lx_soft(a.text[cs])) {
-            uint32_t q = cs - 1;
-            while (q > ms && cs - q <= LT_BACK_CAP && lx_soft(a.text[q - 1])) q--;
-            if (cs - q > LT_BACK_CAP) { a.mod_flag[ptx_upper_bound_u32(a.info.mcb, a.info.n_modules, c) - 1] = 1; continue; }
-            run_start = q;
+// ---- phase 2a: chunks with comment or string characters
+// One thread per 32-byte window again: it steps the comment / string automaton from the chunk's entry context (scanned over
+// the whole text) to its window, four bytes at a time, and takes its window through the token automaton with the bytes of
+// comments and strings read as blanks; a string's token starts at its opening quote.  A stray '/' or '*' is an error.
+// What is left to the byte-serial walk of a whole chunk by one thread: modules whose last string or block comment does not
+// end (what it hides is one error), and (in the next phase) tiles with more triggers than the list holds.
+// (With the serial walk for every such chunk, 64 of a block's 256 threads lexed byte by byte while the others waited: 783 us
+// of 33 MB with comments on every other line, 297 like this.)
+enum { LT_SERIAL = 1, LT_WINDOWS = 2 };       // chunk_special
+PTX_HD inline uint32_t lt_text4(const uint8_t* text, uint32_t pos, uint32_t me) {      // bytes at and behind me read as 0
+    if (pos + 4u <= me) return lt_load4(text + pos);
+    uint32_t v = 0;
+    for (uint32_t b = 0; pos + b < me; b++) v |= (uint32_t)text[pos + b] << (8 * b);
+    return v;
+}
+// context at `to`, from the context at `from` (both inside one chunk and module)
+PTX_HD inline int lt_context(const uint8_t* text, int cx, uint32_t from, uint32_t to, uint32_t me) {
+    for (uint32_t p = from; p < to; p += 4) {
+        const uint32_t w = lt_text4(text, p, me);
+        if (cx_word_has(w, '/') || cx_word_has(w, '*') || cx_word_has(w, '"')) {
+            for (uint32_t b = 0; b < 4; b++) cx = cx_step(cx, (w >> (8 * b)) & 0xFFu);
+        } else if (cx == CX_SLASH) {
+            cx = CX_CODE;
+        } else if (cx == CX_STAR) {
+            cx = CX_BLOCK;
+        } else if (cx == CX_LINE && (cx_word_has(w, '\n') || cx_word_has(w, '\r'))) {
+            cx = CX_CODE;
         }
-        LexMarkSink sink;
-        sink.sh = &sh;
-        sink.tile_base = tile_base;
-        lx_chunk(PtxGlobalReader{a.text, me}, a.text, ms, me, cs, cs + PTX_CHUNK, (int)sh.chunk_cx[k], sink);
-        sh.chunk_errs[k] = sink.n_errors;
-        // the bytes behind the last token that belong to the same run of soft bytes, in the chunks that follow
-        if (sink.last_end >= cs + PTX_CHUNK) lt_chain(sh, a.text, tile_base, sink.last_end, me);
-        // a run of soft bytes that reaches into the chunk from the chunk in front is code: its triggers may lie in this
-        // chunk, where nobody else answers them, and can change a token start in front of the chunk
-        if (run_start < cs) lt_chain(sh, a.text, tile_base, run_start, me);
+    }
+    return cx;
+}
+PTX_HD inline void lt_mark_window(PtxLexMarkShared& sh, const PtxLexTileArgs& a, uint32_t win, uint32_t c, uint32_t ms, uint32_t me, int cx) {
+    const uint32_t pos0 = c * PTX_CHUNK + (win & 3u) * 32u;
+    uint32_t sm = 0, em = 0, wm = 0;
+    if (pos0 < me) {
+        cx = lt_context(a.text, cx, c * PTX_CHUNK, pos0, me);
+        uint32_t st = TS_OTHER;
+        if (cx == CX_CODE && pos0 > ms && !lt_state_before(sh.cls, a.text, pos0, ms, &st)) {
+            a.mod_flag[ptx_upper_bound_u32(a.info.mcb, a.info.n_modules, c) - 1] = 1;
+            st = TS_WORD;
+        }
+        const uint32_t n = me - pos0 < 32u ? me - pos0 : 32u;
+        const uint8_t* rows = (const uint8_t*)sh.step2;
+        uint32_t row = st * 1024u, wd = 0;
+        auto trigger = [&](uint32_t e, uint32_t at) {
+            if (e & (LP_T1 | LP_T2 | LP_T3)) {
+                const uint32_t slot = LT_ATOMIC_ADD(&sh.n_trig, 1u);
+                if (slot < LT_TRIG_CAP) sh.trig[slot] = at | ((e & (LP_T1 | LP_T2 | LP_T3)) << 16) | LT_TRIG_WINDOWS;
+            }
+        };
+        for (uint32_t i = 0; i < n; i++) {
+            if ((i & 3u) == 0) wd = lt_text4(a.text, pos0 + i, me);
+            const uint32_t ch = (wd >> (8u * (i & 3u))) & 0xFFu;
+            uint32_t code = ' ';
+            const int was = cx;
+            cx = cx_step(cx, ch);
+            if (was == CX_CODE || was == CX_SLASH) {
+                // the slash in front was no comment; one in the window before is that window's to report
+                if (was == CX_SLASH && cx != CX_LINE && cx != CX_BLOCK && i) em |= 1u << (i - 1u);
+                if (cx == CX_STR) sm |= 1u << i;
+                else if (cx == CX_CODE && ch == '*') em |= 1u << i;
+                else if (cx == CX_CODE) code = ch;
+            }
+            const uint32_t e = *(const uint32_t*)(rows + row + code * 4u);
+            sm |= (e & 1u) << i;
+            em |= ((e >> 1) & 1u) << i;
+            wm |= ((e >> 2) & 1u) << i;
+            trigger(e, win * 32u + i);
+            row = e >> 8;
+        }
+        const uint32_t next = pos0 + n < me ? a.text[pos0 + n] : (uint32_t)' ';
+        if (cx == CX_SLASH && next != '/' && next != '*') em |= 1u << (n - 1u);
+        if ((win == LT_WORDS - 1 && n == 32 && pos0 + 32 < me) || pos0 + n == me)
+            trigger(sh.step[(row >> 10 << 4) | (pos0 + n == me ? (uint32_t)TC_WS : (uint32_t)sh.cls[next])], win * 32u + n);
+    }
+    sh.start[win] = sm;
+    sh.err[win] = em;
+    sh.word[win] = wm;
+}
+// the byte-serial walk of chunk k, by one thread
+PTX_HD inline void lt_mark_serial(PtxLexMarkShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t k) {
+    const uint32_t c = tile * LT_CHUNKS + k, ms = sh.chunk_ms[k], me = sh.chunk_me[k], cs = c * PTX_CHUNK, tile_base = tile * LT_BYTES;
+    sh.chunk_special[k] = LT_SERIAL;
+    for (uint32_t w = 0; w < 4; w++) sh.start[k * 4 + w] = sh.err[k * 4 + w] = 0;
+    if (cs >= me) return;
+    // the walk looks back over one run of soft bytes; a run longer than the cap goes to the one-thread path
+    uint32_t run_start = cs;
+    if (sh.chunk_cx[k] == CX_CODE && cs > ms && lx_soft(a.text[cs - 1]) && lx_soft(a.text[cs])) {
+        uint32_t q = cs - 1;
+        while (q > ms && cs - q <= LT_BACK_CAP && lx_soft(a.text[q - 1])) q--;
+        if (cs - q > LT_BACK_CAP) { a.mod_flag[ptx_upper_bound_u32(a.info.mcb, a.info.n_modules, c) - 1] = 1; return; }
+        run_start = q;
+    }
+    LexMarkSink sink;
+    sink.sh = &sh;
+    sink.tile_base = tile_base;
+    lx_chunk(PtxGlobalReader{a.text, me}, a.text, ms, me, cs, cs + PTX_CHUNK, (int)sh.chunk_cx[k], sink);
+    sh.chunk_errs[k] = sink.n_errors;
+    // the bytes behind the last token that belong to the same run of soft bytes, in the chunks that follow
+    if (sink.last_end >= cs + PTX_CHUNK) lt_chain(sh, a.text, tile_base, sink.last_end, me);
+    // a run of soft bytes that reaches into the chunk from the chunk in front is code: its triggers may lie in this
+    // chunk, where nobody else answers them, and can change a token start in front of the chunk
+    if (run_start < cs) lt_chain(sh, a.text, tile_base, run_start, me);
+}
+PTX_HD inline void lt_mark_special(PtxLexMarkShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t tid, uint32_t nt) {
+    for (uint32_t win = tid; win < LT_WORDS; win += nt) {
+        const uint32_t k = win >> 2, c = tile * LT_CHUNKS + k;
+        if (c >= a.n_chunks || !sh.chunk_special[k]) continue;
+        uint32_t m = a.tile_mod[tile];
+        while (m + 1 < a.info.n_modules && a.info.mcb[m + 1] <= c) m++;
+        const int last = (int)(a.vec[a.info.mcb[m + 1] - 1] & 7u);      // the context behind the module's last chunk
+        if (last != CX_STR && last != CX_BLOCK && last != CX_STAR) {
+            sh.chunk_special[k] = LT_WINDOWS;
+            lt_mark_window(sh, a, win, c, sh.chunk_ms[k], sh.chunk_me[k], (int)sh.chunk_cx[k]);
+        } else if ((win & 3u) == 0) {
+            lt_mark_serial(sh, a, tile, k);
+        }
     }
 }
 
@@ -441,13 +530,19 @@ PTX_HD inline bool lt_trigger_benign(const PtxLexMarkShared& sh, const uint8_t* 
 // ---- phase 2b: one thread per trigger, and one for the run of soft bytes that enters the tile
 PTX_HD inline void lt_mark_triggers(PtxLexMarkShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t tid, uint32_t nt) {
     const uint32_t tile_base = tile * LT_BYTES;
-    const uint32_t n_trig = sh.n_trig > LT_TRIG_CAP ? 0u : sh.n_trig;
+    if (sh.n_trig > LT_TRIG_CAP) {      // too many triggers to list: every chunk takes the serial walk
+        for (uint32_t k = tid; k < LT_CHUNKS; k += nt)
+            if (tile * LT_CHUNKS + k < a.n_chunks && sh.chunk_special[k] != LT_SERIAL) lt_mark_serial(sh, a, tile, k);
+        return;
+    }
+    const uint32_t n_trig = sh.n_trig;
     // the block's last thread: a run of soft bytes that begins in front of the tile may hold a number or a "::" literal;
     // it is lexed from its start (the triggers go to the first threads: on the device another warp, at the same time)
     if (tid == nt - 1) {
         const uint32_t c = tile * LT_CHUNKS;
         const uint32_t ms = sh.chunk_ms[0], me = sh.chunk_me[0];
-        if (c < a.n_chunks && !sh.chunk_special[0] && tile_base < me && tile_base > ms && lt_soft_class(sh.cls[a.text[tile_base]]) &&
+        const uint32_t sp = sh.chunk_special[0];
+        if (c < a.n_chunks && (!sp || (sp == LT_WINDOWS && sh.chunk_cx[0] == CX_CODE)) && tile_base < me && tile_base > ms && lt_soft_class(sh.cls[a.text[tile_base]]) &&
             lt_soft_class(sh.cls[a.text[tile_base - 1]])) {
             uint32_t q = tile_base - 1;
             while (q > ms && tile_base - q <= LT_BACK_CAP && lt_soft_class(sh.cls[a.text[q - 1]])) q--;
@@ -457,12 +552,14 @@ PTX_HD inline void lt_mark_triggers(PtxLexMarkShared& sh, const PtxLexTileArgs& 
         }
     }
     for (uint32_t t = tid; t < n_trig; t += nt) {
-        const uint32_t off = sh.trig[t] & 0xFFFFu, kind = sh.trig[t] >> 16;
+        const uint32_t off = sh.trig[t] & 0xFFFFu, kind = (sh.trig[t] >> 16) & 0xFFu;
         const uint32_t pos = tile_base + off;
         // T1 sits on its digit; T2 and T3 sit one byte behind the sigil / the first colon they are about
         const uint32_t at = ((kind & LP_T1) && off < LT_BYTES) ? off : (off ? off - 1 : 0u);
         const uint32_t k = at >> 7;
-        if (sh.chunk_special[k]) continue;        // lexed by the serial walk
+        // a trigger of the first phase counts in a chunk that nobody has been over since, one of the second (lt_mark_window)
+        // in a chunk that it was over
+        if (sh.chunk_special[k] != (sh.trig[t] & LT_TRIG_WINDOWS ? LT_WINDOWS : 0u)) continue;
         const uint32_t ms = sh.chunk_ms[k], me = sh.chunk_me[k];
         if (kind == LP_T1 && off < LT_BYTES && lt_trigger_benign(sh, a.text, pos, ms, me)) continue;
         if (kind & (LP_T1 | LP_T3)) {
@@ -481,7 +578,7 @@ PTX_HD inline void lt_mark_triggers(PtxLexMarkShared& sh, const PtxLexTileArgs& 
 PTX_HD inline void lt_mark_finish(PtxLexMarkShared& sh, const PtxLexTileArgs& a, uint32_t tile, uint32_t tid, uint32_t nt) {
     for (uint32_t k = tid; k < LT_CHUNKS; k += nt) {
         const uint32_t c = tile * LT_CHUNKS + k;
-        const bool special = sh.chunk_special[k];
+        const uint32_t special = sh.chunk_special[k];
         const uint32_t serial_errs = sh.chunk_errs[k];
         sh.chunk_special[k] = 0;         // for the next tile (lt_mark_reset)
         sh.chunk_errs[k] = 0;
@@ -498,7 +595,7 @@ PTX_HD inline void lt_mark_finish(PtxLexMarkShared& sh, const PtxLexTileArgs& a,
         }
         PtxPair p;
         p.a = ntok;
-        p.b = special ? serial_errs : nerr;
+        p.b = special == LT_SERIAL ? serial_errs : nerr;
         a.cnt[c + 1] = p;
         if (c == 0) { PtxPair z; z.a = z.b = 0; a.cnt[0] = z; }
     }
