@@ -593,7 +593,7 @@ struct Printer {
             break;
         }
     }
-    void instruction(const Instruction& x) {
+    void predicate(const Instruction& x) {
         o.put("Instruction(");
         if (x.has_pred) {
             o.put(x.pred_not ? "Some(PredAt { not: true, label: " : "Some(PredAt { not: false, label: ");
@@ -602,7 +602,17 @@ struct Printer {
         } else {
             o.put("None, ");
         }
+    }
+    void instruction(const Instruction& x) {
+        predicate(x);
         const PtxInstr& in = ptx_instrs[x.variant];
+        if (x.variant != I_Bra && x.variant != I_Call) {
+            name_and_data(in, x.data.data());
+            for (int i = 0; i < in.n_args; i++) argument(in, i, x.args[i]);
+            if (in.n_args) o.put(" }");
+            o.put(in.data_type < 0 && in.n_args == 0 ? ")\n" : " })\n");
+            return;
+        }
         o.put(in.name);
         if (x.variant == I_Bra) {
             o.put(" { arguments: BraArgs { src: ");
@@ -624,31 +634,48 @@ struct Printer {
             o.put("], is_external: false } })\n");
             return;
         }
-        if (in.data_type < 0 && in.n_args == 0) { o.put(")\n"); return; }
+    }
+    // an instruction up to its first argument
+    void name_and_data(const PtxInstr& in, const uint32_t* data) {
+        o.put(in.name);
+        if (in.data_type < 0 && in.n_args == 0) return;
         o.put(" { ");
         if (in.data_type >= 0) {
             o.put("data: ");
             if (ptx_types[in.data_type].kind == 2 && ptx_types[in.data_type].b == 0) o.put("()");
-            else {
-                const uint32_t* w = x.data.data();
-                schema(in.data_type, w);
-            }
+            else schema(in.data_type, data);
             if (in.n_args) o.put(", ");
         }
         if (in.n_args) {
-            o.put("arguments: "); o.put(in.name); o.put("Args { ");
-            for (int i = 0; i < in.n_args; i++) {
-                if (i) o.put(", ");
-                const PtxArg& a = ptx_args[in.first_arg + i];
-                o.put(a.name);
-                o.put(": ");
-                if (x.args[i].absent) o.put(a.optional ? "None" : "<missing>");
-                else if (a.optional) { o.put("Some("); operand(x.args[i]); o.put(")"); }
-                else operand(x.args[i]);
-            }
-            o.put(" }");
+            o.put("arguments: ");
+            o.put(in.name);
+            o.put("Args { ");
         }
-        o.put(" })\n");
+    }
+    void argument(const PtxInstr& in, int i, const Operand& op) {
+        // ", name: " of every argument, made once
+        struct Label { uint32_t n; char text[28]; };
+        static const std::vector<Label> labels = [] {
+            std::vector<Label> v(sizeof ptx_args / sizeof ptx_args[0]);
+            for (size_t k = 0; k < v.size(); k++) v[k].n = (uint32_t)snprintf(v[k].text, sizeof v[k].text, ", %s: ", ptx_args[k].name ? ptx_args[k].name : "");
+            return v;
+        }();
+        const PtxArg& a = ptx_args[in.first_arg + i];
+        const Label& l = labels[in.first_arg + i];
+        const uint32_t skip = i ? 0 : 2;
+        if (op.kind == OPK_REG && !op.absent && !a.optional) {      // most operands: a plain name
+            char* p = o.room(l.n - skip + 5);
+            memcpy(p, l.text + skip, l.n - skip);
+            memcpy(p + (l.n - skip), "Reg(", 4);
+            o.n--;
+            str(op.name);
+            *o.room(1) = ')';
+            return;
+        }
+        o.putn(l.text + skip, l.n - skip);
+        if (op.absent) o.put(a.optional ? "None" : "<missing>");
+        else if (a.optional) { o.put("Some("); operand(op); o.put(")"); }
+        else operand(op);
     }
     void variable_statement(const MultiVariable& v) {
         if (v.parameterized) {
@@ -682,8 +709,74 @@ struct Printer {
         }
     }
     void label(const Str& s) { o.put("Label("); str(s); o.put(")\n"); }
-    // the statements of a body straight from its records: each is built like a node of the tree, printed, and its memory
-    // goes to the next one
+    // What stands between the predicate and the first argument of an instruction depends on its variant and its packed data
+    // words alone, and a module has few of those: the texts made so far, by variant.  (It is half of the dump and most of
+    // the steps that printing takes.)
+    struct HeadText {
+        uint32_t n_words;           // data words
+        uint32_t words[8];
+        std::string text;
+        int next;
+    };
+    std::vector<HeadText> heads;
+    std::vector<int> head_of;       // by variant: the last text made, -1 = none
+    // prints it for the data words at w; returns where the operands begin
+    const uint32_t* head(uint16_t variant, const Builder& b, const uint32_t* w, const uint32_t* end) {
+        if (head_of.empty()) head_of.assign(sizeof ptx_instrs / sizeof ptx_instrs[0], -1);
+        for (int i = head_of[variant]; i >= 0; i = heads[i].next) {
+            const HeadText& h = heads[i];
+            if (h.n_words <= (uint32_t)(end - w) && memcmp(h.words, w, 4 * h.n_words) == 0) { o.putn(h.text.data(), h.text.size()); return w + h.n_words; }
+        }
+        const PtxInstr& in = ptx_instrs[variant];
+        std::vector<uint32_t> data;
+        const uint32_t* behind = w;
+        if (in.data_type >= 0 && !(ptx_types[in.data_type].kind == 2 && ptx_types[in.data_type].b == 0)) {
+            ptxdump::PackedCursor cur;
+            cur.w = w;
+            b.data_values(in.data_type, cur, &data);
+            behind = cur.w;
+        }
+        const size_t from = o.n;
+        name_and_data(in, data.data());
+        HeadText h;
+        h.n_words = (uint32_t)(behind - w);
+        if (h.n_words <= sizeof h.words / 4) {
+            memcpy(h.words, w, 4 * h.n_words);
+            h.text.assign(o.b + from, o.n - from);
+            h.next = head_of[variant];
+            head_of[variant] = (int)heads.size();
+            heads.push_back(std::move(h));
+        }
+        return behind;
+    }
+    // an instruction straight from its record
+    void instruction_record(const Builder& b, const uint32_t* rec, Instruction* scratch) {
+        const uint32_t w0 = rec[0];
+        const uint32_t w1 = (w0 & 0xFF) == U_INSTR ? (((w0 >> 29) & 3u) | (((w0 >> 22) & 0x7Fu) << 16)) : rec[ptxdump::rec_len(w0)];
+        const uint16_t variant = (uint16_t)(w1 >> 16);
+        if (variant == I_Bra || variant == I_Call) {
+            b.instruction(rec, scratch);
+            instruction(*scratch);
+            return;
+        }
+        const uint32_t* w = rec + 1;
+        scratch->has_pred = (w1 & 1) != 0;
+        scratch->pred_not = (w1 & 2) != 0;
+        if (scratch->has_pred) { scratch->pred = b.str(w[0], w[1]); w += 2; }
+        predicate(*scratch);
+        w = head(variant, b, w, rec + 1 + ptxdump::rec_len(w0));
+        const PtxInstr& in = ptx_instrs[variant];
+        for (int i = 0; i < in.n_args; i++) {
+            if (*w == PTX_ABSENT) { op.absent = true; w++; }
+            else w = b.operand(w, &op);
+            argument(in, i, op);
+        }
+        if (in.n_args) o.put(" }");
+        o.put(in.data_type < 0 && in.n_args == 0 ? ")\n" : " })\n");
+    }
+    Operand op;
+    // the statements of a body straight from its records: variables, branches and calls are built like nodes of the tree and
+    // printed, and their memory goes to the next one; of the other instructions only the operands are
     void stream(const Builder& b, const uint32_t* q, const uint32_t* end) {
         Instruction ins;
         MultiVariable var;
@@ -693,7 +786,7 @@ struct Printer {
             case U_LABEL: o.indent(depth); label(b.str(q[1], q[2])); break;
             case U_VAR: b.multi_variable(q + 1, &var); o.indent(depth); variable_statement(var); break;
             case U_INSTR:
-            case U_INSTR_LONG: b.instruction(q, &ins); o.indent(depth); instruction(ins); break;
+            case U_INSTR_LONG: o.indent(depth); instruction_record(b, q, &ins); break;
             case U_BLOCK_OPEN: o.indent(depth++); o.put("Block([\n"); break;
             case U_BLOCK_CLOSE:
                 if (depth > 1) { o.indent(--depth); o.put("])\n"); }

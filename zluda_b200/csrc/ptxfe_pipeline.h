@@ -272,6 +272,20 @@ enum { PTX_REDO_TOKENS = 1, PTX_REDO_SERIAL_LEX = 2, PTX_REDO_UNITS = 4, PTX_RED
 #define PTX_COUNT_ADD(p, v) ((*(p) += (uint32_t)(v)) - (uint32_t)(v))
 #endif
 
+// A slot in a list for every caller: the lanes of a warp that call together take theirs with one atomic (a hundred thousand
+// on one address, one by one, were half of the step that lists the calls of a module)
+PTX_HD inline uint32_t ptx_list_slot(uint32_t* count) {
+#ifdef __CUDA_ARCH__
+    const unsigned mask = __activemask();
+    const int lead = __ffs(mask) - 1, lane = (int)(threadIdx.x & 31u);
+    uint32_t base = 0;
+    if (lane == lead) base = atomicAdd(count, (uint32_t)__popc(mask));
+    return __shfl_sync(mask, base, lead) + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+#else
+    return (*count)++;
+#endif
+}
+
 // A number of work items: the host's count, or (dev != nullptr) an upper bound on the host and the count on the device
 struct PtxCount {
     size_t cap;
@@ -714,7 +728,7 @@ struct PtxUnitClassesStep {
     uint8_t* uflag;
     uint8_t* ustatus;
     PTX_HD void add(uint32_t entry) const {
-        const uint32_t slot = PTX_COUNT_ADD(&counters->n_first, 1);
+        const uint32_t slot = ptx_list_slot(&counters->n_first);
         if (slot < cap_list) list[slot] = entry;
         else redo(PTX_REDO_LIST);
     }
@@ -917,7 +931,7 @@ struct PtxDecodeListStep {
         }
         uown[u] = PtxPair{flagged ? high : nw, ne};
         uflag[u] = flagged ? PTX_UNIT_FLAGGED : PTX_UNIT_STAGED;
-        if (flagged) PTX_COUNT_ADD(&counters->n_flagged, 1);
+        if (flagged) ptx_list_slot(&counters->n_flagged);
         if (r.status == US_OK && r.kind == U_FUNC) {
             const uint32_t slot = PTX_COUNT_ADD(&counters->n_funcs, 1);
             PtxFnEntry e;
@@ -972,7 +986,7 @@ struct PtxApplyTemplatesStep {
                 return;
             }
         }
-        const uint32_t at = PTX_COUNT_ADD(&counters->n_second, 1);
+        const uint32_t at = ptx_list_slot(&counters->n_second);
         if (at < cap_list) list[at] = (uint32_t)u;
         else PTX_REDO_SET(counters, PTX_REDO_LIST);
     }
