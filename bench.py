@@ -40,7 +40,7 @@ UNIT = "GB/s"
 
 # (dram__bytes_read.sum + dram__bytes_write.sum) / text bytes, from the ncu captures summarised under profiles/
 NCU_DRAM_BYTES_PER_TEXT_BYTE = {      # from the ncu captures summarised under profiles/ (512 MiB instance of the workload)
-    "lex_emit": 4.20, "lex_mark": 1.32, "structure": 0.74, "lex_context_vectors": 1.03, "emit_records": 4.48,
+    "lex_emit": 4.20, "lex_mark": 1.32, "structure": 0.74, "lex_context": 1.03, "emit_records": 4.48,
 }
 
 
@@ -327,10 +327,9 @@ def main():
     T, W, N = stats["n_tokens"], stats["n_result_words"], nbytes
     U = stats["n_units"]
     algo = {   # algorithmic bytes per launch: text read once, tokens / records read or written once
-        "lex_context_vectors": N, "lex_mark": N + N // 4, "lex_emit": N + N // 4 + 10 * T,
+        "lex_context": N, "lex_mark": N + N // 4, "lex_emit": N + N // 4 + 10 * T,
         "structure": 2 * T + 8 * U,
-        "unit_shape_key": 2 * T + 10 * U, "apply_templates": 2 * T + 16 * U, "class_insert": 12 * U,
-        "emit_records": 4 * W + 9 * U, "decode_units": N + 8 * T + 4 * W, "decode_emit_flagged": 5 * U,
+        "unit_classes": 2 * T + 12 * U, "apply_templates": 2 * T + 16 * U, "emit_records": 4 * W + 9 * U, "decode_emit_flagged": 5 * U,
     }
     top = max(prof, key=prof.get) if prof else None
     roof = None
@@ -344,10 +343,8 @@ def main():
         roof = {"kernel": top, "bound": "hbm", "achieved": ach, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": ach / peak if ach else None, "traffic": tpb * N if tpb else None, "ms_per_launch": ms, "algorithmic_bytes": ab,
                 "lexer_segmenter": None}
-        lex_ms = sum(prof.get(k, 0.0) for k in ("lex_context_vectors", "scan_context", "lex_tile_modules", "lex_mark", "lex_serial_modules",
-                                                  "scan_token_counts", "set_token_total", "lex_emit", "module_token_ranges",
-                                                  "module_results_init", "mark_module_skip", "structure", "reset_unit_total",
-                                                  "module_unit_ranges", "module_unit_ranges_fill")) / a.steps
+        lex_ms = sum(prof.get(k, 0.0) for k in ("lex_context", "scan_context", "lex_mark", "lex_serial_modules", "scan_token_counts", "lex_emit",
+                                                  "modules_lexed", "structure", "module_unit_ranges")) / a.steps
         # whole front end: text read once, records written once (N + O) over the kernel time of a step
         a_fe = N + 4 * W
         fe_ms = kernel_ms / a.steps

@@ -297,8 +297,8 @@ PTX_HD inline uint32_t sx_walk(const PtxStructArgs& a, const SxThread& t, int32_
     }
     return starts;
 }
-PTX_HD inline uint32_t sx_decide(const PtxStructArgs& a, const SxThread& t, int32_t depth) {
-    if (!t.fast) return sx_walk(a, t, depth, false, 0);
+PTX_HD inline uint32_t sx_decide(const PtxStructArgs& a, const SxThread& t, int32_t depth, uint32_t* n_tops = nullptr) {
+    if (!t.fast) return sx_walk(a, t, depth, false, 0, 0, n_tops);
     const uint32_t plus = t.braces & SX_LOW, minus = (t.braces >> 4) & SX_LOW;
     const uint32_t in_scope = (t.marks & SX_LOW) | plus | minus | sx_up(plus | minus) | (t.brace_before & 1u);
     if (depth - (int32_t)sx_popc(minus) > 0) return in_scope;                              // inside a scope all the way
@@ -332,13 +332,10 @@ PTX_HD inline uint32_t sx_decide(const PtxStructArgs& a, const SxThread& t, int3
     return starts;
 }
 
-// how many of the starts are top-level units (for backends that number those in the same pass)
-PTX_HD inline uint32_t sx_count_tops(const PtxStructArgs& a, const SxThread& t, int32_t depth, uint32_t starts) {
+// how many of the starts are top-level units (for backends that number those in the same pass); the threads of the
+// token-by-token case have counted theirs in sx_decide
+PTX_HD inline uint32_t sx_count_tops(const SxThread& t, int32_t depth, uint32_t starts) {
     uint32_t tops = 0;
-    if (!t.fast) {
-        sx_walk(a, t, depth, false, 0, 0, &tops);
-        return tops;
-    }
     const uint32_t plus = t.braces & SX_LOW, minus = (t.braces >> 4) & SX_LOW;
     if (!starts || depth - (int32_t)sx_popc(minus) > 0) return 0;                          // inside a scope all the way
     if (depth == 0 && !plus) return sx_popc(starts);                                       // top level all the way

@@ -85,13 +85,9 @@ struct PtxTileReader {
 
 #define LEX_TILE_BYTES (LEX_TILE_CHUNKS * LEX_ROW_WORDS * 4u)
 #define LEX_TABLE_BYTES (LS_COUNT * 256u * 2u)
+// A tile of text: LEX_TILE_CHUNKS chunks from chunk c0 on, to rows of LEX_ROW_WORDS words.
 // text_len: 0 = whole chunks are readable on a 16-byte boundary, else nothing behind that many bytes is (text at any address)
-template <bool TABLES, class F>
-__global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const uint8_t* text, F f, uint32_t text_len = 0) {
-    extern __shared__ __align__(16) uint32_t lex_smem[];
-    uint32_t* tile = lex_smem;                                       // [LEX_TILE_CHUNKS][LEX_ROW_WORDS]
-    uint16_t* fused = (uint16_t*)(lex_smem + LEX_TILE_CHUNKS * LEX_ROW_WORDS);    // [LS_COUNT][256] when TABLES
-    const uint32_t c0 = blockIdx.x * LEX_TILE_CHUNKS;
+__device__ inline void lex_stage_tile(uint32_t* tile, uint32_t c0, uint32_t n_chunks, const uint8_t* text, uint32_t text_len) {
     const uint4* src = (const uint4*)text + (size_t)c0 * (PTX_CHUNK / 16);
 #pragma unroll
     for (uint32_t k = 0; k < 8; k++) {
@@ -110,9 +106,15 @@ __global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const 
         uint32_t* d = tile + row * LEX_ROW_WORDS + (idx & 7u) * 4;
         d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
-    if (TABLES) {
-        for (uint32_t i = threadIdx.x; i < LS_COUNT * 256; i += 256) fused[i] = ptx_lex_fused[i];
-    }
+}
+template <class F>
+__global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const uint8_t* text, F f) {
+    extern __shared__ __align__(16) uint32_t lex_smem[];
+    uint32_t* tile = lex_smem;                                       // [LEX_TILE_CHUNKS][LEX_ROW_WORDS]
+    uint16_t* fused = (uint16_t*)(lex_smem + LEX_TILE_CHUNKS * LEX_ROW_WORDS);    // [LS_COUNT][256]
+    const uint32_t c0 = blockIdx.x * LEX_TILE_CHUNKS;
+    lex_stage_tile(tile, c0, n_chunks, text, 0);
+    for (uint32_t i = threadIdx.x; i < LS_COUNT * 256; i += 256) fused[i] = ptx_lex_fused[i];
     __syncthreads();
     uint32_t c = c0 + threadIdx.x;
     if (c < n_chunks) f((size_t)c, PtxTileReader{tile, fused, text, c0 * PTX_CHUNK});
@@ -293,13 +295,14 @@ __global__ void __launch_bounds__(256, 6) emit_records_kernel(LaunchCount count,
     __shared__ uint32_t n_later;
     const uint32_t u0 = blockIdx.x * 256;
     const uint32_t nu = n_units - u0 < 256u ? n_units - u0 : 256u;
-    uint32_t mine = 0;
+    uint32_t mine = 0, all = 0;
     if (threadIdx.x < nu) {
         const uint32_t begin = off[u0 + threadIdx.x].a, end = off[u0 + threadIdx.x + 1].a;
         PtxEmitUnit eu = e.unit(u0 + threadIdx.x);
         eu.first = begin;
         su[threadIdx.x] = eu;
-        if (eu.flag == PTX_UNIT_STAGED || eu.flag == PTX_UNIT_TEMPLATED) mine = end - begin;
+        all = end - begin;
+        if (eu.flag == PTX_UNIT_STAGED || eu.flag == PTX_UNIT_TEMPLATED) mine = all;
     }
     if (threadIdx.x == 0) n_later = 0;
     {
@@ -308,8 +311,9 @@ __global__ void __launch_bounds__(256, 6) emit_records_kernel(LaunchCount count,
         so[threadIdx.x] = excl;
         if (threadIdx.x == 255) so[256] = incl;
     }
-    __syncthreads();
-    const uint32_t total = so[nu];
+    // the common case: every word of the block's units is this kernel's, so they are one stretch of the record stream
+    const bool one_stretch = __syncthreads_and(mine == all);
+    const uint32_t total = so[nu], first = su[0].first;
     // Every warp takes a contiguous eighth of the block's words, 32 at a time.  The unit of a word: `ua` is the unit of
     // the window's first word; the lanes read the next 32 unit offsets, those inside the window mark their place in a
     // 32-bit mask, and a lane's unit is ua + the number of marks at or below it.  (Units without words put two marks on
@@ -363,7 +367,7 @@ __global__ void __launch_bounds__(256, 6) emit_records_kernel(LaunchCount count,
         for (int q = 0; q < EMIT_ILP; q++) {
             const uint32_t j = jb + q * 32 + lane;
             if (what[q] == PtxEmitStep::WRITE) {
-                e.words[su[unit[q]].first + (j - so[unit[q]])] = x[q];
+                e.words[one_stretch ? first + j : su[unit[q]].first + (j - so[unit[q]])] = x[q];
             } else if (what[q] == PtxEmitStep::SECOND_ROUND) {
                 const uint32_t slot = atomicAdd(&n_later, 1u);
                 const uint32_t i = j - so[unit[q]];
@@ -446,6 +450,43 @@ template <class T> struct ScanDesc {
         return same ? state : 0ull;
     }
 };
+// Warp 0 of a block, with the aggregate of the block's tile: what the tiles in front of it amount to goes to *s_before.
+template <class T, class Op>
+__device__ inline void look_back(ScanDesc<T>* desc, uint32_t tile, T agg, Op op, T identity, uint32_t* ctl, T* s_before, uint32_t* s_ok, uint32_t* aborted) {
+    const uint32_t lane = threadIdx.x;
+    T before = identity;
+    bool ok = true;
+    if (tile == 0) {
+        if (lane == 0) desc[0].publish(SXD_PREFIX, agg);
+    } else {
+        if (lane == 0) desc[tile].publish(SXD_AGG, agg);
+        for (int64_t back = (int64_t)tile - 1; ok; back -= 32) {
+            const int64_t mine = back - (int64_t)lane;
+            T v = identity;
+            unsigned long long state = SXD_PREFIX;         // in front of tile 0: nothing, and known
+            for (uint32_t spin = 0; mine >= 0; spin++) {
+                state = desc[mine].look(v);
+                if (state) break;
+                if ((spin & 63u) == 63u && *(volatile uint32_t*)&ctl[1]) break;
+                if (spin >= SX_WAIT_LIMIT) { atomicExch(&ctl[1], 1u); break; }
+                __nanosleep(20);
+            }
+            if (!__all_sync(0xFFFFFFFFu, state != 0)) { ok = false; break; }
+            const unsigned ends = __ballot_sync(0xFFFFFFFFu, state == SXD_PREFIX);
+            const uint32_t last = ends ? (uint32_t)(__ffs(ends) - 1) : 31u;
+            if (lane > last) v = identity;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {             // ordered: lane 0 ends up with op(v[last], ..., v[1], v[0])
+                T y = shfl_down_words(v, d);
+                if (lane + d < 32) v = op(y, v);
+            }
+            before = op(shfl_words(v, 0), before);
+            if (ends) break;
+        }
+        if (ok && lane == 0) desc[tile].publish(SXD_PREFIX, op(before, agg));
+    }
+    if (lane == 0) { *s_before = before; if (!ok) { *s_ok = 0; *aborted = 1; } }
+}
 template <class T, class Op, class Ld, class St>
 __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, Ld ld, St st, Op op, T identity, ScanDesc<T>* desc, uint32_t* ctl, uint32_t* aborted) {
     __shared__ T warp_tot[SCAN_THREADS / 32];
@@ -472,41 +513,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, L
     if (threadIdx.x == SCAN_THREADS - 1) s_before = incl;
     __syncthreads();
     if (threadIdx.x < 32) {
-        const uint32_t lane = threadIdx.x;
         const T agg = s_before;
         __syncwarp();
-        T before = identity;
-        bool ok = true;
-        if (tile == 0) {
-            if (lane == 0) desc[0].publish(SXD_PREFIX, agg);
-        } else {
-            if (lane == 0) desc[tile].publish(SXD_AGG, agg);
-            for (int64_t back = (int64_t)tile - 1; ok; back -= 32) {
-                const int64_t mine = back - (int64_t)lane;
-                T v = identity;
-                unsigned long long state = SXD_PREFIX;         // in front of tile 0: nothing, and known
-                for (uint32_t spin = 0; mine >= 0; spin++) {
-                    state = desc[mine].look(v);
-                    if (state) break;
-                    if ((spin & 63u) == 63u && *(volatile uint32_t*)&ctl[1]) break;
-                    if (spin >= SX_WAIT_LIMIT) { atomicExch(&ctl[1], 1u); break; }
-                    __nanosleep(20);
-                }
-                if (!__all_sync(0xFFFFFFFFu, state != 0)) { ok = false; break; }
-                const unsigned ends = __ballot_sync(0xFFFFFFFFu, state == SXD_PREFIX);
-                const uint32_t last = ends ? (uint32_t)(__ffs(ends) - 1) : 31u;
-                if (lane > last) v = identity;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {             // ordered: lane 0 ends up with op(v[last], ..., v[1], v[0])
-                    T y = shfl_down_words(v, d);
-                    if (lane + d < 32) v = op(y, v);
-                }
-                before = op(shfl_words(v, 0), before);
-                if (ends) break;
-            }
-            if (ok && lane == 0) desc[tile].publish(SXD_PREFIX, op(before, agg));
-        }
-        if (lane == 0) { s_before = before; if (!ok) { s_ok = 0; *aborted = 1; } }
+        look_back(desc, tile, agg, op, identity, ctl, &s_before, &s_ok, aborted);
     }
     __syncthreads();
     if (!s_ok) return;
@@ -514,6 +523,43 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, L
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; k++)
         if (base + k < n) st(base + k, op(prefix, vals[k]));
+}
+
+// ---- context vectors and their scan in one step: a block stages a tile of text, every thread makes the transition vector of
+// its chunk, and the tile's place in the whole is found by looking back.  (One launch less than vectors first and a scan
+// behind it, 5 us in a small slice.  Where the tiles are more than the device takes at once, blocks that wait for the tiles
+// in front of them hold back the ones behind: 148 us for 130 MB against 95 + 21, so then it is two steps, SCAN = false.)
+template <bool SCAN>
+__global__ void __launch_bounds__(256) lex_context_kernel(uint32_t n_chunks, const uint8_t* text, PtxLexVectorsStep f, uint32_t text_len, ScanDesc<uint32_t>* desc,
+                                                          uint32_t* ctl, uint32_t* aborted) {
+    extern __shared__ __align__(16) uint32_t lex_smem[];
+    __shared__ uint32_t warp_tot[8], s_tile, s_before, s_ok;
+    if (SCAN) {
+        if (threadIdx.x == 0) {
+            s_tile = atomicAdd(&ctl[0], 1u);
+            s_ok = 1;
+        }
+        __syncthreads();
+    }
+    const uint32_t tile = SCAN ? s_tile : blockIdx.x, c0 = tile * LEX_TILE_CHUNKS, c = c0 + threadIdx.x;
+    lex_stage_tile(lex_smem, c0, n_chunks, text, text_len);
+    __syncthreads();
+    const uint32_t v = c < n_chunks ? f.vector((size_t)c, PtxTileReader{lex_smem, nullptr, text, c0 * PTX_CHUNK}) : (uint32_t)CX_IDENTITY;
+    if (!SCAN) {
+        if (c < n_chunks) f.vec[c] = v;
+        return;
+    }
+    uint32_t incl, excl;
+    block_scan(v, ComposeOp(), (uint32_t)CX_IDENTITY, warp_tot, incl, excl);
+    if (threadIdx.x == 255) s_before = incl;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t agg = s_before;
+        __syncwarp();
+        look_back(desc, tile, agg, ComposeOp(), (uint32_t)CX_IDENTITY, ctl, &s_before, &s_ok, aborted);
+    }
+    __syncthreads();
+    if (s_ok && c < n_chunks) f.vec[c] = cx_compose(s_before, incl);
 }
 
 // ---- stage B in one pass (ptx_struct_tile.h).  Tiles are handed out in order by an atomic counter, so a tile only
@@ -526,14 +572,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, L
 // host reads struct_abort with the counters.
 struct StructDesc {
     unsigned long long depth0, depth1, count;
-    uint32_t has_first, pad;      // has_first: set ahead of the pass (sx_mark_tiles)
+    uint32_t has_first, pad;      // has_first: set ahead of the pass (PtxModulesLexed)
 };
-__global__ void structure_mark_kernel(PtxStructArgs a, StructDesc* desc, const uint32_t* stop) {
-    if (stop && *(const volatile uint32_t*)stop) return;
-    if (a.n_tokens_dev) a.n_tokens = *a.n_tokens_dev;
-    uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < a.n_modules) sx_mark_tiles(a, m, &desc[0].has_first, (uint32_t)(sizeof(StructDesc) / 4));
-}
 constexpr int SX_DEPTH_PER_LANE = 1, SX_COUNT_PER_LANE = 1;     // tiles a lane of the look-back reads per trip to memory
 
 __device__ inline void sx_publish_depth(StructDesc* d, unsigned long long state, PtxSeg3 v) {
@@ -659,10 +699,12 @@ __global__ void __launch_bounds__(SX_THREADS) structure_kernel(PtxStructArgs a, 
             return;
         }
         const int32_t before = sx_depth(op(s_before, excl));
-        const uint32_t starts = sx_decide(a, t, before);
+        uint32_t tops = 0;
+        const uint32_t starts = sx_decide(a, t, before, &tops);
+        if (t.fast) tops = sx_count_tops(t, before, starts);
         // units in the low half, top-level units in the high half (at most 4,096 of each)
         uint32_t cincl, cexcl;
-        block_scan((uint32_t)__popc(starts) | (sx_count_tops(a, t, before, starts) << 16), AddOp(), 0u, warp_count, cincl, cexcl);
+        block_scan((uint32_t)__popc(starts) | (tops << 16), AddOp(), 0u, warp_count, cincl, cexcl);
         if (threadIdx.x == SX_THREADS - 1) s_units_before = cincl;
         __syncthreads();
         if (threadIdx.x < 32) {
@@ -885,7 +927,7 @@ struct ptxfe_ctx {
 };
 
 struct CudaBackend {
-    static constexpr bool kStructureTops = true;
+    static constexpr bool kFusedSteps = true;
     ptxfe_ctx* ctx;
     const int arena;
     const cudaStream_t stream;
@@ -1012,17 +1054,26 @@ struct CudaBackend {
         ctx->launches++;
     }
     // per-chunk lexer steps; text holds n whole chunks and is 16-byte aligned (it is an arena block)
+    void lex_context(const char* name, size_t n, const uint8_t* text, const PtxLexVectorsStep& f) {
+        if (ctx->failed || n == 0) return;
+        const unsigned blocks = (unsigned)((n + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS);
+        const bool one_wave = blocks <= 148;
+        ScanDesc<uint32_t>* desc = one_wave ? (ScanDesc<uint32_t>*)zalloc(sizeof(ScanDesc<uint32_t>) * blocks + 16) : nullptr;
+        if (one_wave && !desc) return;
+        prof_begin(name);
+        if (one_wave) lex_context_kernel<true><<<blocks, 256, LEX_TILE_BYTES, stream>>>((uint32_t)n, text, f, 0u, desc, (uint32_t*)(desc + blocks), aborted);
+        else lex_context_kernel<false><<<blocks, 256, LEX_TILE_BYTES, stream>>>((uint32_t)n, text, f, 0u, nullptr, nullptr, nullptr);
+        prof_end();
+        ctx->launches++;
+        if (!one_wave) scan<uint32_t>("scan_context", n, ArrayLoad<uint32_t>{f.vec}, ArrayStore<uint32_t>{f.vec}, ComposeOp(), (uint32_t)CX_IDENTITY);
+    }
     template <class F> void pf_text(const char* name, size_t n, const uint8_t* text, F f) {
         if (ctx->failed || n == 0) return;
         unsigned blocks = (unsigned)((n + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS);
         prof_begin(name);
-        if constexpr (std::is_same<F, PtxLexVectorsStep>::value) {
-            lex_tile_kernel<false><<<blocks, 256, LEX_TILE_BYTES, stream>>>((uint32_t)n, text, f);
-        } else {
-            // tile + table need more shared memory than a kernel gets by default
-            cudaFuncSetAttribute(lex_tile_kernel<true, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(LEX_TILE_BYTES + LEX_TABLE_BYTES));
-            lex_tile_kernel<true><<<blocks, 256, LEX_TILE_BYTES + LEX_TABLE_BYTES, stream>>>((uint32_t)n, text, f);
-        }
+        // tile + table need more shared memory than a kernel gets by default
+        cudaFuncSetAttribute(lex_tile_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(LEX_TILE_BYTES + LEX_TABLE_BYTES));
+        lex_tile_kernel<<<blocks, 256, LEX_TILE_BYTES + LEX_TABLE_BYTES, stream>>>((uint32_t)n, text, f);
         prof_end();
         ctx->launches++;
     }
@@ -1070,17 +1121,22 @@ struct CudaBackend {
         if (!ctx->failed) snprintf(ctx->err, sizeof ctx->err, "%s", why);
         ctx->failed = true;
     }
+    StructDesc* struct_desc = nullptr;
+    uint32_t* structure_marks(uint32_t cap_tokens, uint32_t* stride) {
+        struct_desc = (StructDesc*)zalloc(sizeof(StructDesc) * (((size_t)cap_tokens + SX_TILE - 1) / SX_TILE) + 256);
+        *stride = (uint32_t)(sizeof(StructDesc) / 4);
+        return struct_desc ? &struct_desc[0].has_first : nullptr;
+    }
     void structure(const char* name, const PtxStructArgs& a) {
         if (ctx->failed || a.n_tokens == 0) return;
         const size_t n_tiles = ((size_t)a.n_tokens + SX_TILE - 1) / SX_TILE;
-        StructDesc* desc = (StructDesc*)zalloc(sizeof(StructDesc) * n_tiles + 256);
+        StructDesc* const desc = struct_desc;
         if (!desc) return;
         uint32_t* ctl = (uint32_t*)(desc + n_tiles);      // [0] next tile, [1] abort
         prof_begin(name);
-        structure_mark_kernel<<<(a.n_modules + 255) / 256, 256, 0, stream>>>(a, desc, stop);
         structure_kernel<<<resident_blocks((const void*)structure_kernel, 0, n_tiles), SX_THREADS, 0, stream>>>(a, desc, ctl, stop);
         prof_end();
-        ctx->launches += 2;
+        ctx->launches++;
     }
     void sort_by_key(const char* name, size_t n, const uint16_t* key, uint32_t* order) {
         if (ctx->failed || n == 0) return;
@@ -1381,6 +1437,9 @@ struct SliceRun {
 #define PTXFE_DIRECT_OUT_BYTES (1u << 20)
 #define PTXFE_COUNTERS_SLOT(ctx, arena) ((PtxCounters*)((char*)(ctx)->h_counters + 2048 + 512 * (arena)))
 
+// Up to this much text every unit is decoded on its own (PtxWork::direct): there are then no more units than the device holds
+// warps that decode one each (some 3,500).
+#define PTXFE_DIRECT_BYTES (96u << 10)
 // capacities of a slice that runs with deferred counts: `bytes` of padded text
 static void deferred_caps(const ptxfe_ctx* ctx, uint64_t bytes, PtxWork& w) {
     auto cap = [&](double per_byte, uint64_t least, uint64_t most) -> uint32_t {
@@ -1393,6 +1452,7 @@ static void deferred_caps(const ptxfe_ctx* ctx, uint64_t bytes, PtxWork& w) {
     w.cap_units = cap(ctx->units_per_byte, 4096, w.cap_tokens);
     w.cap_words = cap(ctx->words_per_byte, 16384, 0xFFFFFF00ull);
     w.cap_list = w.cap_units < PTX_SORT_MIN ? w.cap_units : PTX_SORT_MIN;
+    w.direct = bytes <= PTXFE_DIRECT_BYTES;
 }
 
 // working memory and parameters of a slice, in the current arena
@@ -1414,7 +1474,7 @@ static int begin_slice(CudaBackend& bk, SliceRun& sl, bool deferred) {
     w.mod_chunk_begin = (uint32_t*)(ctx->d_meta + mcb_at);
     if (deferred) deferred_caps(ctx, (uint64_t)w.n_chunks * PTX_CHUNK, w);
     // everything that the steps want cleared, in one go: per-module words, look-back descriptors, the counters
-    const size_t zero = 8192 + 48 * ((size_t)n + 2) + 24 * ((size_t)w.n_chunks / SCAN_TILE + 2) + 16 * ((size_t)w.cap_units / SCAN_TILE + 2) +
+    const size_t zero = 8192 + 48 * ((size_t)n + 2) + 16 * ((size_t)w.n_chunks / SCAN_TILE + 2) + 8 * ((size_t)w.n_chunks / LEX_TILE_CHUNKS + 2) + 16 * ((size_t)w.cap_units / SCAN_TILE + 2) +
                         sizeof(StructDesc) * ((size_t)w.cap_tokens / SX_TILE + 2);
     bk.zero_base = (char*)bk.alloc(zero);
     bk.zero_size = bk.zero_base ? zero : 0;
@@ -2233,7 +2293,7 @@ struct NoallocScratch {
     uint32_t serial;               // then: number of chunks of the text, else 0
     uint32_t refused, aborted, pad[3];
     uint32_t ctl[2 * (PTXFE_NOALLOC_MAX_SEGS + 2)];
-    ScanDesc<uint32_t> vec_desc[PTXFE_NOALLOC_MAX_CHUNKS / SCAN_TILE + 1];
+    ScanDesc<uint32_t> vec_desc[PTXFE_NOALLOC_MAX_CHUNKS / LEX_TILE_CHUNKS + 1];
     ScanDesc<PtxPair> cnt_desc[PTXFE_NOALLOC_MAX_CHUNKS / SCAN_TILE + 2 * PTXFE_NOALLOC_MAX_SEGS + 2];
     ScanDesc<PtxPair> serial_desc[PTXFE_NOALLOC_MAX_CHUNKS / SCAN_TILE + 2];
     uint32_t cleared;
@@ -2327,11 +2387,8 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
     // does not matter
     noalloc_init_kernel<<<4, 256, 0, stream>>>(s, me, n_chunks);
     const PtxLexChunkInfo info{&s->layout, s->mcb, 1};
-    lex_tile_kernel<false><<<(n_chunks + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS, 256, LEX_TILE_BYTES, stream>>>(
-        n_chunks, text, PtxLexVectorsStep{info, s->vec, s->tile_mod}, me);
-    scan_kernel<uint32_t><<<(n_chunks + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, stream>>>(
-        LaunchCount{n_chunks, nullptr, nullptr, 0}, ArrayLoad<uint32_t>{s->vec}, ArrayStore<uint32_t>{s->vec}, ComposeOp(), CX_IDENTITY, s->vec_desc, s->ctl,
-        &s->aborted);
+    lex_context_kernel<true><<<(n_chunks + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS, 256, LEX_TILE_BYTES, stream>>>(
+        n_chunks, text, PtxLexVectorsStep{info, s->vec, s->tile_mod}, me, s->vec_desc, s->ctl, &s->aborted);
     const uint32_t n_tiles = (n_chunks + LT_CHUNKS - 1) / LT_CHUNKS;
     ScanDesc<PtxPair>* desc = s->cnt_desc;
     for (uint32_t seg = 0, t0 = 0; t0 < n_tiles; seg++, t0 += PTXFE_NOALLOC_SEG_TILES) {

@@ -306,9 +306,10 @@ inline void* ptx_zalloc_impl(BK& bk, size_t bytes, long) {
 }
 template <class T, class BK>
 inline T* ptx_zalloc(BK& bk, size_t n) { return (T*)ptx_zalloc_impl(bk, sizeof(T) * n, 0); }
-// a backend whose structure pass numbers the top-level units on the way says so with kStructureTops
-template <class BK, class = void> struct PtxStructureTops { static constexpr bool value = false; };
-template <class BK> struct PtxStructureTops<BK, decltype((void)BK::kStructureTops)> { static constexpr bool value = BK::kStructureTops; };
+// A backend that says kFusedSteps scans the context vectors in the step that makes them (lex_context), has the modules mark
+// their tiles for the structure pass in modules_lexed (structure_marks), and numbers the top-level units in that pass.
+template <class BK, class = void> struct PtxFusedSteps { static constexpr bool value = false; };
+template <class BK> struct PtxFusedSteps<BK, decltype((void)BK::kFusedSteps)> { static constexpr bool value = BK::kFusedSteps; };
 
 PTX_HD inline uint32_t ptx_upper_bound_u32(const uint32_t* a, uint32_t n, uint32_t x) {
     // number of entries <= x
@@ -361,6 +362,9 @@ struct PtxWork {
     // capacities below, steps take their counts from `counters`, and a slice that does not fit, or that needs a step
     // that only the host can size (PTX_REDO_*), stops itself and is run again with deferred = false.
     bool deferred = false;
+    // Little text (deferred counts only): every unit is decoded on its own.  Keys, classes and templates are four steps more
+    // whose work is shared by few units.
+    bool direct = false;
     uint32_t cap_tokens = 0, cap_units = 0, cap_words = 0, cap_list = 0;
     PtxCount tokens_n() const { return deferred ? PtxCount(cap_tokens, &counters->n_tokens) : PtxCount(n_tokens); }
     PtxCount units_n(uint32_t plus = 0) const { return deferred ? PtxCount((size_t)cap_units + plus, &counters->n_units, plus) : PtxCount((size_t)n_units + plus); }
@@ -434,7 +438,8 @@ struct PtxLexVectorsStep {
     PtxLexChunkInfo info;
     uint32_t* vec;
     uint32_t* tile_mod;      // module of every tile's first chunk, for the steps that work on tiles
-    template <class R> PTX_HD void operator()(size_t c, const R& rd) const {
+    template <class R> PTX_HD void operator()(size_t c, const R& rd) const { vec[c] = vector(c, rd); }
+    template <class R> PTX_HD uint32_t vector(size_t c, const R& rd) const {
         uint32_t cs = (uint32_t)c * PTX_CHUNK;
         const uint32_t m = ptx_upper_bound_u32(info.mcb, info.n_modules, (uint32_t)c) - 1;
         const uint32_t ms = info.begin(m), me = ms + (uint32_t)info.layout[m].text_len;
@@ -442,7 +447,7 @@ struct PtxLexVectorsStep {
         if (c % LT_CHUNKS == 0) tile_mod[c / LT_CHUNKS] = m;
         uint32_t ce = cs + PTX_CHUNK < me ? cs + PTX_CHUNK : me;
         uint32_t v = cx_chunk_vector(rd, cs, ce);
-        vec[c] = first ? cx_restart(v) : v;
+        return first ? cx_restart(v) : v;
     }
 };
 struct PtxLexErrorsStep {
@@ -468,6 +473,21 @@ struct PtxLexErrorsStep {
     }
 };
 
+// ---- what the structure pass goes by
+PTX_HD inline bool ptx_opens_operand(uint16_t prev) {
+    // a '{' after one of these starts a vector operand or an initialiser, not a scope
+    return prev == T_COMMA || prev == T_EQ || prev == T_LPAREN || (prev >= T_OP_FIRST && prev < T_COUNT);
+}
+PTX_HD inline bool ptx_is_directive_start(uint16_t k) {
+    return k == T_DOT_EXTERN || k == T_DOT_VISIBLE || k == T_MOD_weak || k == T_DOT_FUNC || k == T_DOT_ENTRY ||
+           k == T_MOD_global || k == T_MOD_const || k == T_MOD_shared || k == T_DOT_FILE || k == T_DOT_SECTION;
+}
+
+// Scope delta of a token: +1 for a '{' that opens a scope, -1 for a '}' that closes one, 0 otherwise (also for the
+// braces of vector operands, initialisers and .section bodies, told apart by two tokens of left context): sx_brace.
+#include "ptx_struct_tile.h"
+
+
 // rows that depend on the lexer alone: token and error ranges, whether the module is parsed at all
 struct PtxModulesLexed {
     const uint32_t* mcb;
@@ -478,6 +498,8 @@ struct PtxModulesLexed {
     const uint32_t* mod_flag;     // deferred counts: a module that asks for the one-thread lexer stops the slice
     PtxModuleResult* results;
     PtxCounters* counters;
+    uint32_t* marks = nullptr;    // the tiles of the structure pass in which a module begins (sx_mark_tiles)
+    uint32_t marks_stride = 0, cap_tokens = 0;
     PTX_HD void operator()(size_t m) const {
         const PtxPair none{0, 0};
         const PtxPair b = n_chunks ? cnt[mcb[m]] : none;
@@ -503,6 +525,12 @@ struct PtxModulesLexed {
 #endif
         }
         if (mod_flag && mod_flag[m]) PTX_REDO_SET(counters, PTX_REDO_SERIAL_LEX);
+        if (marks) {
+            PtxStructArgs a{};
+            a.mtb = mtb;
+            a.n_tokens = counters->n_tokens;
+            if (a.n_tokens <= cap_tokens) sx_mark_tiles(a, (uint32_t)m, marks, marks_stride);
+        }
     }
 };
 
@@ -546,10 +574,14 @@ inline void ptx_stage_lex(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     // A1: transition vector of every chunk, module of every tile
     const size_t n_tiles = ((size_t)n_chunks + LT_CHUNKS - 1) / LT_CHUNKS;
     uint32_t* tile_mod = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_tiles + 1));
-    bk.pf_text("lex_context_vectors", n_chunks, text, PtxLexVectorsStep{info, vec, tile_mod});
     // A2: inclusive scan with composition; chunk c starts in state (prefix[c-1])[CODE]
-    bk.template scan<uint32_t>("scan_context", n_chunks, [=] PTX_HD(size_t i) { return vec[i]; }, [=] PTX_HD(size_t i, uint32_t v) { vec[i] = v; },
-                               ComposeOp(), CX_IDENTITY);
+    if constexpr (PtxFusedSteps<BK>::value) {
+        bk.lex_context("lex_context", n_chunks, text, PtxLexVectorsStep{info, vec, tile_mod});
+    } else {
+        bk.pf_text("lex_context_vectors", n_chunks, text, PtxLexVectorsStep{info, vec, tile_mod});
+        bk.template scan<uint32_t>("scan_context", n_chunks, [=] PTX_HD(size_t i) { return vec[i]; }, [=] PTX_HD(size_t i, uint32_t v) { vec[i] = v; },
+                                   ComposeOp(), CX_IDENTITY);
+    }
     // A3: token boundaries, byte-parallel: one bit per text byte and the token / error count of every chunk
     uint32_t* start_bits = (uint32_t*)bk.alloc(sizeof(uint32_t) * LT_WORDS * (n_tiles + 1));
     uint32_t* mod_flag = w.lex_flag = ptx_zalloc<uint32_t>(bk, n_modules + 1);
@@ -584,19 +616,6 @@ inline void ptx_stage_lex(BK& bk, PtxWork& w, PtxCounters& host_counters) {
 }
 
 // ------------------------------------------------------------------------------------------------ stage B: structure
-PTX_HD inline bool ptx_opens_operand(uint16_t prev) {
-    // a '{' after one of these starts a vector operand or an initialiser, not a scope
-    return prev == T_COMMA || prev == T_EQ || prev == T_LPAREN || (prev >= T_OP_FIRST && prev < T_COUNT);
-}
-PTX_HD inline bool ptx_is_directive_start(uint16_t k) {
-    return k == T_DOT_EXTERN || k == T_DOT_VISIBLE || k == T_MOD_weak || k == T_DOT_FUNC || k == T_DOT_ENTRY ||
-           k == T_MOD_global || k == T_MOD_const || k == T_MOD_shared || k == T_DOT_FILE || k == T_DOT_SECTION;
-}
-
-// Scope delta of a token: +1 for a '{' that opens a scope, -1 for a '}' that closes one, 0 otherwise (also for the
-// braces of vector operands, initialisers and .section bodies, told apart by two tokens of left context): sx_brace.
-#include "ptx_struct_tile.h"
-
 template <class BK>
 inline void ptx_stage_structure(BK& bk, PtxWork& w, PtxCounters& host_counters, uint32_t mode) {
     const uint32_t n_modules = w.n_modules;
@@ -606,15 +625,18 @@ inline void ptx_stage_structure(BK& bk, PtxWork& w, PtxCounters& host_counters, 
     w.mod_skip = (uint32_t*)bk.alloc(sizeof(uint32_t) * (n_modules + 1));
     PtxCounters* counters = w.counters;
     // B0: what is known of the modules behind the lexer
-    bk.pf("modules_lexed", n_modules + 1,
-          PtxModulesLexed{w.mod_chunk_begin, w.chunk_cnt, n_modules, w.n_chunks, mode, w.mod_tok_begin, w.mod_skip, w.deferred ? w.lex_flag : nullptr,
-                          w.results, counters});
+    PtxModulesLexed lexed{w.mod_chunk_begin, w.chunk_cnt, n_modules, w.n_chunks, mode, w.mod_tok_begin, w.mod_skip, w.deferred ? w.lex_flag : nullptr, w.results, counters};
+    if constexpr (PtxFusedSteps<BK>::value) {
+        lexed.cap_tokens = w.deferred ? w.cap_tokens : w.n_tokens;
+        lexed.marks = bk.structure_marks(lexed.cap_tokens, &lexed.marks_stride);
+    }
+    bk.pf("modules_lexed", n_modules + 1, lexed);
     // B1: one pass over the token kinds: (scope, paren) depth restarting at every module, the unit starts, their
     // numbering and the unit table (at most one unit per token); nothing per token is kept of it
     const size_t room = w.deferred ? w.cap_units : w.n_tokens;
     w.unit_start = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 2));
     w.unit_depth = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 2));
-    if (PtxStructureTops<BK>::value) {
+    if (PtxFusedSteps<BK>::value) {
         w.unit_dir = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 1));
         w.unit_top = (uint32_t*)bk.alloc(sizeof(uint32_t) * (room + 1));
     }
@@ -808,13 +830,14 @@ struct PtxUnitClassesStep {
 // written by the second pass (decode_emit_flagged), which also has the function table.
 // A class representative: decoded with tagged output into the class's template, and its signature spelled out.
 struct PtxDecodeListStep {
-    const uint32_t* list;
+    const uint32_t* list;         // nullptr: all units (PtxWork::direct)
     const uint8_t* text;
     const PtxToken* tokens;
     const uint16_t* kinds;
     const PtxModuleLayout* layout;
     const uint32_t* mtb;
     const uint32_t* mub;
+    const uint32_t* mod_skip;
     const uint32_t* ustart;
     const uint32_t* udepth;
     const uint32_t* udir;
@@ -832,7 +855,7 @@ struct PtxDecodeListStep {
     PtxCounters* counters;
     // the tokens that go to the fast window: the unit's own and the one behind, from `start` on
     PTX_HD uint32_t window(size_t idx, uint32_t win_cap, uint32_t* start) const {
-        const uint32_t u = list[idx] & 0x7FFFFFFFu;
+        const uint32_t u = list ? list[idx] & 0x7FFFFFFFu : (uint32_t)idx;
         *start = ustart[u];
         const uint32_t n_tokens = counters->n_tokens;
         const uint32_t end = u + 1 < counters->n_units ? ustart[u + 1] + 1u : n_tokens;
@@ -843,13 +866,30 @@ struct PtxDecodeListStep {
         PtxStaged ret;
         ret.unit = 0;
         ret.n = 0;
-        const uint32_t u = list[idx] & 0x7FFFFFFFu;
-        const bool rep = (list[idx] >> 31) != 0;
+        const uint32_t entry = list ? list[idx] : (uint32_t)idx, u = entry & 0x7FFFFFFFu;
+        const bool rep = (entry >> 31) != 0;
         const uint32_t start = ustart[u];
         // modules without units share their begin with the next one: take the last module that starts at or before u
         const uint32_t m = ptx_upper_bound_u32(mub, n_modules, u) - 1;
         const uint32_t te = mtb[m + 1];
         const uint32_t end = u + 1 < mub[m + 1] ? ustart[u + 1] : te;
+        if (!list) {
+            // what the class step does on the way elsewhere
+            if (counters->n_skipped && mod_skip[m]) {
+                uown[u] = PtxPair{0, 0};
+                uend[u] = 0;
+                ustatus[u] = US_OK;
+                uflag[u] = PTX_UNIT_STAGED;
+                utmpl[u] = 0;
+                return ret;
+            }
+            if (udepth[u] == 0 && end - start >= PTX_BULK_MIN_TOKENS) {
+                PTX_COUNT_ADD(&counters->n_bulk, 1);
+                PTX_COUNT_ADD(&counters->n_bulk_tokens, end - start);
+                PTX_REDO_SET(counters, PTX_REDO_BULK);
+                return ret;
+            }
+        }
         const uint32_t id = rep ? cs.slot_tmpl[uclass[u]] : 0u;
         // the unit's first tokens go to the fast window: the decoder looks at every token many times.  (A token of the next
         // module may be among them: the decoder does not look at tokens behind its module's last.)
@@ -1228,7 +1268,7 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     w.mod_bad = ptx_zalloc<uint32_t>(bk, n_modules + 1);
     w.mod_seq_size = ptx_zalloc<PtxPair>(bk, n_modules + 1);
     w.mod_seq_status = ptx_zalloc<uint32_t>(bk, n_modules + 1);
-    if (!PtxStructureTops<BK>::value) {
+    if (!PtxFusedSteps<BK>::value) {
         // ordinal of the enclosing top-level unit, and the unit that heads each ordinal (a module's first unit, or a
         // top-level directive's first)
         uint32_t* udir = w.unit_dir = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
@@ -1239,6 +1279,17 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
         bk.pf("list_toplevel_units", nu, [=] PTX_HD(size_t u) {
             if ((udepth[u] & 0x7FFFFFFFu) == 0) top_unit[udir[u] - 1] = (uint32_t)u;
         });
+    }
+    if (w.direct) {
+        const uint32_t cap_staged = 64 * w.cap_units;
+        w.staged = (uint32_t*)bk.alloc(sizeof(uint32_t) * (size_t)cap_staged);
+        w.fn_entries = (PtxFnEntry*)bk.alloc(sizeof(PtxFnEntry) * ((size_t)w.cap_units + 1));
+        w.list = w.second = nullptr;
+        bk.pf_staged("decode_units", w.units_n(), w.staged, 0,
+                     PtxDecodeListStep{nullptr, w.text, w.tokens, w.kinds, w.layout, w.mod_tok_begin, w.mod_unit_begin, w.mod_skip, w.unit_start, w.unit_depth,
+                                       w.unit_dir, nullptr, n_modules, cap_staged, w.cap_units, PtxClassStore(), PtxBulkTable(), w.unit_tmpl, w.unit_end, w.unit_own,
+                                       w.unit_flag, w.unit_status, w.staged, w.fn_entries, counters});
+        return;
     }
     // ---- classes
     const uint32_t cap_list = w.deferred ? w.cap_list : (uint32_t)nu;
@@ -1262,8 +1313,8 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     w.staged = (uint32_t*)bk.alloc(sizeof(uint32_t) * (size_t)cap_staged);
     w.fn_entries = (PtxFnEntry*)bk.alloc(sizeof(PtxFnEntry) * ((size_t)cap_funcs + 1));
     if (!w.deferred && n_first > PTX_SORT_MIN) w.list = ptx_sort_list(bk, w, first, n_first);
-    PtxDecodeListStep step{w.list, w.text, w.tokens, w.kinds, w.layout, w.mod_tok_begin, w.mod_unit_begin, w.unit_start, w.unit_depth, w.unit_dir, uclass,
-                           n_modules, cap_staged, cap_funcs, cs, w.bulk, w.unit_tmpl, w.unit_end, w.unit_own, w.unit_flag, w.unit_status, w.staged,
+    PtxDecodeListStep step{w.list, w.text, w.tokens, w.kinds, w.layout, w.mod_tok_begin, w.mod_unit_begin, w.mod_skip, w.unit_start, w.unit_depth, w.unit_dir,
+                           uclass, n_modules, cap_staged, cap_funcs, cs, w.bulk, w.unit_tmpl, w.unit_end, w.unit_own, w.unit_flag, w.unit_status, w.staged,
                            w.fn_entries, counters};
     bk.pf_staged("decode_first", w.deferred ? PtxCount(cap_list, &counters->n_first) : PtxCount(n_first), w.staged, 0, step);
     // ---- templates, and the units that have none after all
@@ -1291,15 +1342,16 @@ inline void ptx_scan_sizes(BK& bk, PtxWork& w, bool check) {
     PtxCounters* counters = w.counters;
     const PtxClassStore cs = w.cs;
     const uint32_t cap_words = w.deferred ? w.cap_words : 0xFFFFFFFFu;
-    const bool deferred = w.deferred;
+    const bool deferred = w.deferred, direct = w.direct;
     auto store = [=] PTX_HD(size_t i, PtxPair v) {
         usize[i] = v;
         if (i != counters->n_units) return;
         counters->n_words = v.a;
         counters->n_errs = v.b;
+        if (direct) counters->n_first = counters->n_units;
         counters->n_rest = counters->n_first - counters->n_reps + counters->n_second;
-        counters->n_classes = cs.state[0];
-        counters->n_sig_words = cs.state[1];
+        counters->n_classes = direct ? 0u : cs.state[0];
+        counters->n_sig_words = direct ? 0u : cs.state[1];
         if (v.a > cap_words) PTX_REDO_SET(counters, PTX_REDO_WORDS);
         if (!deferred && counters->any_sequential) counters->n_flagged += 1;
     };
@@ -1418,8 +1470,8 @@ inline void ptx_emit_flagged(BK& bk, PtxWork& w, const PtxCounters& host_counter
     const uint32_t* second = w.second;
     const uint32_t n_first = host_counters.n_first;
     bk.pf("decode_emit_flagged", (size_t)n_first + host_counters.n_second, [=] PTX_HD(size_t idx) {
-        const size_t u = idx < n_first ? list[idx] & 0x7FFFFFFFu : second[idx - n_first];
-        if (idx < n_first && (list[idx] >> 31)) return;
+        const size_t u = !list ? idx : idx < n_first ? list[idx] & 0x7FFFFFFFu : second[idx - n_first];
+        if (list && idx < n_first && (list[idx] >> 31)) return;
         if (uflag[u] != 1) return;
         uint32_t m = ptx_upper_bound_u32(mub, n_modules, (uint32_t)u) - 1;
         PtxSink sink;
@@ -1562,7 +1614,7 @@ inline void ptx_stage_again(BK& bk, PtxWork& w, PtxCounters& host_counters) {
 template <class BK>
 inline void ptx_stage_decode_anew(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     PtxCounters* counters = w.counters;
-    w.deferred = false;
+    w.deferred = w.direct = false;
     w.n_tokens = host_counters.n_tokens;
     w.n_units = host_counters.n_units;
     bk.pf("reset_decode_counters", 1, [=] PTX_HD(size_t) {
