@@ -16,9 +16,9 @@ struct PtxFast {
     const PtxTokenWord* win;         // the same in fast memory: win_n of them, win_stride apart
     uint32_t win_n, win_stride;
     uint32_t n;                      // tokens of the unit
-    // where the record goes: word k to words[k * stride], its tag to tags[k] (nullptr: none)
+    // where the record goes: word k to words[k * stride], its tag to tags[k * stride] (nullptr: none)
     uint32_t* words;
-    uint16_t* tags;
+    uint32_t* tags;
     uint32_t stride, cap;
     uint32_t nw = 0;
     bool ok = true;
@@ -30,7 +30,7 @@ struct PtxFast {
     PTX_HD void w(uint32_t x, uint32_t tag = 0) {
         if (nw < cap) {
             words[nw * stride] = x;
-            if (tags) tags[nw] = (uint16_t)tag;
+            if (tags) tags[nw * stride] = tag;
         }
         nw++;
     }

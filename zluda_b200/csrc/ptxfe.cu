@@ -276,113 +276,101 @@ __device__ inline void block_scan(T v, Op op, T identity, T* warp_tot, T& incl, 
     excl = op(wp, prev);
 }
 
-// ---- record emission (PtxEmitStep): a block takes 256 consecutive units, loads what a word needs of its unit into
-// shared memory once, and then goes over their words with EMIT_ILP words per thread at a time: all their reads are
-// issued before the first of them is written, so that several chains of dependent loads (unit -> template -> token)
-// are in flight per thread.  The literals are collected and converted in a second round with the warps full.
-// The words counted are those of staged and templated units only (at most PTX_TMP_STRIDE each): a unit that the second
-// decode pass writes can have millions of words - an array with its initialiser - and one block that stepped over them
-// word by word took 16.3 of 19.5 ms of a 41 MB module of constant tables (0.1 ms without them).
-#define SEG_DEFER_CAP 2048u
+// ---- record emission (PtxEmitStep): a block takes 256 consecutive units and goes over their words, one lane per word and
+// EMIT_ILP words per thread at a time: all their reads are issued before the first of them is written, so that several
+// chains of dependent loads (unit -> template -> token) are in flight per thread.  Literal values are collected and
+// converted in a second round with the warps full.
+// Which unit a word belongs to: the first words of the units are bits of a map, EMIT_PASS words of it at a time, with the
+// number of bits in front of each of its 32-bit windows; a word's unit is that number plus the bits at or below it.  (With
+// a search along the offsets by ballot and reduction it was 217 warp instructions per 32 words and 390 us for 34 million
+// words.)  The words counted are those of staged and templated units only: a unit that the second decode pass writes can have
+// millions of words - an array with its initialiser - and one block that stepped over them took 16.3 of 19.5 ms of a
+// 41 MB module of constant tables.
 #define EMIT_ILP 4
+#define EMIT_PASS 8192u
 __global__ void __launch_bounds__(256, 6) emit_records_kernel(LaunchCount count, const PtxPair* off, PtxEmitStep e) {
     const uint32_t n_units = (uint32_t)count.get();
     if (blockIdx.x * 256u >= n_units) return;
-    __shared__ uint32_t so[257];              // words of the units in front of unit k that this kernel writes
-    __shared__ PtxEmitUnit su[256];
+    __shared__ uint4 su[256];                         // the units that have words here: PtxEmitUnit
+    __shared__ uint32_t so[256];                      // the words in front of each
     __shared__ uint32_t warp_tot[8];
-    __shared__ uint32_t later[SEG_DEFER_CAP];
-    __shared__ uint32_t n_later;
-    const uint32_t u0 = blockIdx.x * 256;
+    __shared__ uint32_t bits[EMIT_PASS / 32], before[EMIT_PASS / 32];
+    __shared__ uint32_t later[EMIT_PASS / 2];         // literals of the pass (each has a word in front of it that is none)
+    __shared__ uint32_t n_later, s_total;
+    const uint32_t u0 = blockIdx.x * 256, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t nu = n_units - u0 < 256u ? n_units - u0 : 256u;
     uint32_t mine = 0, all = 0;
+    PtxEmitUnit eu{0, 0, 0, 0};
     if (threadIdx.x < nu) {
         const uint32_t begin = off[u0 + threadIdx.x].a, end = off[u0 + threadIdx.x + 1].a;
-        PtxEmitUnit eu = e.unit(u0 + threadIdx.x);
+        eu = e.unit(u0 + threadIdx.x);
         eu.first = begin;
-        su[threadIdx.x] = eu;
         all = end - begin;
         if (eu.flag == PTX_UNIT_STAGED || eu.flag == PTX_UNIT_TEMPLATED) mine = all;
     }
-    if (threadIdx.x == 0) n_later = 0;
-    {
-        uint32_t incl, excl;
-        block_scan(mine, AddOp(), 0u, warp_tot, incl, excl);
-        so[threadIdx.x] = excl;
-        if (threadIdx.x == 255) so[256] = incl;
+    // words in the low 20 bits (a staged record has at most STAGE_CAP * STAGE_SLOTS / 9), units with words above them
+    uint32_t incl, excl;
+    block_scan(mine | (mine ? 1u << 20 : 0u), AddOp(), 0u, warp_tot, incl, excl);
+    const uint32_t my_so = excl & 0xFFFFFu;
+    if (mine) {
+        su[excl >> 20] = make_uint4(eu.tmpl, eu.start, eu.flag, eu.first);
+        so[excl >> 20] = my_so;
     }
+    if (threadIdx.x == 255) s_total = incl & 0xFFFFFu;
     // the common case: every word of the block's units is this kernel's, so they are one stretch of the record stream
     const bool one_stretch = __syncthreads_and(mine == all);
-    const uint32_t total = so[nu], first = su[0].first;
-    // Every warp takes a contiguous eighth of the block's words, 32 at a time.  The unit of a word: `ua` is the unit of
-    // the window's first word; the lanes read the next 32 unit offsets, those inside the window mark their place in a
-    // 32-bit mask, and a lane's unit is ua + the number of marks at or below it.  (Units without words put two marks on
-    // one place: such a window searches, as does the first of a warp.)
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t per_warp = ((total + 255u) / 256u) * 32u;
-    const uint32_t wbeg = warp * per_warp, wend = wbeg + per_warp < total ? wbeg + per_warp : total;
-    uint32_t ua = 0;
-    if (wbeg < wend) {
-        const uint32_t o = wbeg;
-        uint32_t lo = 0, hi = nu;              // last k with so[k] <= o
-        while (hi - lo > 1) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (so[mid] <= o) lo = mid; else hi = mid;
-        }
-        ua = lo;
-    }
-    for (uint32_t jb = wbeg; jb < wend; jb += 32 * EMIT_ILP) {
-        uint32_t x[EMIT_ILP], unit[EMIT_ILP];
-        int what[EMIT_ILP];
+    const uint32_t total = s_total;
+    if (total == 0) return;
+    const uint32_t first = su[0].w;
+    uint32_t begun = 0;                               // units that begin in front of the pass
+    for (uint32_t p0 = 0; p0 < total; p0 += EMIT_PASS) {
+        bits[threadIdx.x] = 0;
+        if (threadIdx.x == 0) n_later = 0;
+        __syncthreads();
+        const uint32_t at = my_so - p0;
+        if (mine && my_so >= p0 && at < EMIT_PASS) atomicOr(&bits[at >> 5], 1u << (at & 31u));
+        __syncthreads();
+        uint32_t bi, be;
+        block_scan((uint32_t)__popc(bits[threadIdx.x]), AddOp(), 0u, warp_tot, bi, be);
+        before[threadIdx.x] = begun + be;
+        if (threadIdx.x == 255) s_total = begun + bi;
+        __syncthreads();
+        begun = s_total;
+        const uint32_t n_here = total - p0 < EMIT_PASS ? total - p0 : EMIT_PASS, windows = (n_here + 31u) >> 5;
+        for (uint32_t w0 = warp * EMIT_ILP; w0 < windows; w0 += 8 * EMIT_ILP) {
+            uint32_t x[EMIT_ILP], to[EMIT_ILP], tag[EMIT_ILP];
+            int what[EMIT_ILP];
 #pragma unroll
-        for (int q = 0; q < EMIT_ILP; q++) {
-            const uint32_t j0 = jb + q * 32, j = j0 + lane;       // j0 is the same for the whole warp
-            what[q] = PtxEmitStep::NOTHING;
-            unit[q] = 0;
-            if (j0 >= wend) continue;
-            const uint32_t o0 = j0, o = o0 + lane;
-            while (ua + 1 < nu && so[ua + 1] <= o0) ua++;        // the unit of the window's first word (a step or none)
-            const uint32_t k = ua + 1 + lane;
-            const uint32_t rel = k <= nu ? so[k] - o0 : 0xFFFFFFFFu;
-            const bool inside = rel < 32u;
-            const uint32_t n_in = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, inside));
-            const uint32_t marks = __reduce_or_sync(0xFFFFFFFFu, inside ? 1u << rel : 0u);
-            uint32_t lo;
-            if ((uint32_t)__popc(marks) == n_in) {
-                lo = ua + (uint32_t)__popc(marks & (0xFFFFFFFFu >> (31u - lane)));
-            } else {
-                uint32_t hi = nu;
-                lo = ua;
-                while (hi - lo > 1) {
-                    uint32_t mid = (lo + hi) >> 1;
-                    if (so[mid] <= o) lo = mid; else hi = mid;
+            for (int q = 0; q < EMIT_ILP; q++) {
+                const uint32_t w = w0 + q, j = p0 + w * 32u + lane;
+                what[q] = PtxEmitStep::NOTHING;
+                if (j >= total || w >= windows) continue;
+                const uint32_t r = before[w] + (uint32_t)__popc(bits[w] & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+                const uint4 v = su[r];
+                const uint32_t i = j - so[r];
+                tag[q] = i | (r << 24);
+                to[q] = one_stretch ? first + j : v.w + i;
+                what[q] = e.word(PtxEmitUnit{v.x, v.y, v.z, v.w}, 0, i, x[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < EMIT_ILP; q++) {
+                if (what[q] == PtxEmitStep::WRITE) {
+                    e.words[to[q]] = x[q];
+                } else if (what[q] == PtxEmitStep::SECOND_ROUND) {
+                    later[atomicAdd(&n_later, 1u)] = tag[q];
                 }
             }
-            ua = ua + n_in < nu - 1u ? ua + n_in : nu - 1u;     // the marks are all in front of the next window
-            if (j >= wend) continue;
-            unit[q] = lo;
-            what[q] = e.word(su[lo], (size_t)(u0 + lo), o - so[lo], x[q]);
         }
-#pragma unroll
-        for (int q = 0; q < EMIT_ILP; q++) {
-            const uint32_t j = jb + q * 32 + lane;
-            if (what[q] == PtxEmitStep::WRITE) {
-                e.words[one_stretch ? first + j : su[unit[q]].first + (j - so[unit[q]])] = x[q];
-            } else if (what[q] == PtxEmitStep::SECOND_ROUND) {
-                const uint32_t slot = atomicAdd(&n_later, 1u);
-                const uint32_t i = j - so[unit[q]];
-                if (slot < SEG_DEFER_CAP) later[slot] = i | (unit[q] << 24);
-                else e.literal(su[unit[q]], i, su[unit[q]].first + i);
-            }
+        __syncthreads();
+        for (uint32_t x = threadIdx.x; x < n_later; x += 256) {
+            const uint32_t i = later[x] & 0xFFFFFFu;
+            const uint4 v = su[later[x] >> 24];
+            e.literal(PtxEmitUnit{v.x, v.y, v.z, v.w}, i, v.w + i);
         }
-    }
-    __syncthreads();
-    const uint32_t nl = n_later < SEG_DEFER_CAP ? n_later : SEG_DEFER_CAP;
-    for (uint32_t x = threadIdx.x; x < nl; x += 256) {
-        const uint32_t i = later[x] & 0xFFFFFFu, lo = later[x] >> 24;
-        e.literal(su[lo], i, su[lo].first + i);
+        __syncthreads();
     }
 }
+
 __global__ void copy_words_kernel(uint32_t* dst, const uint32_t* src, uint32_t n) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
     __threadfence_system();

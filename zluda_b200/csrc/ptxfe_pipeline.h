@@ -97,6 +97,21 @@ PTX_HD inline uint32_t ptx_text_word(const uint8_t* text, uint32_t off, uint32_t
     if (rem < 4) v &= (1u << (8u * rem)) - 1u;
     return v;
 }
+// Sixteen bytes of text at any offset, held in registers and indexed like text: five independent loads where a loop over the
+// digits of a literal would wait for one byte after the other.  (Reads up to 19 bytes past off: see ptx_text_word.)
+struct PtxBytes16 {
+    uint64_t lo, hi;
+    PTX_HD PtxBytes16(const uint8_t* text, uint32_t off) {
+        const uint8_t* a = text + off;
+        const uint32_t mis = (uint32_t)((uintptr_t)a & 3u), sh = 8u * mis;
+        const uint32_t* w = (const uint32_t*)(a - mis);
+        const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+        const uint64_t a0 = w0 | ((uint64_t)w1 << 32), a1 = w2 | ((uint64_t)w3 << 32);
+        lo = sh ? (a0 >> sh) | (a1 << (64u - sh)) : a0;
+        hi = sh ? (a1 >> sh) | ((uint64_t)w4 << (64u - sh)) : a1;
+    }
+    PTX_HD unsigned operator[](uint32_t i) const { return (unsigned)((i < 8u ? lo >> (8u * i) : hi >> (8u * (i - 8u))) & 0xFFu); }
+};
 PTX_HD inline bool ptx_text_matters(uint16_t k) { return k == T_DOTIDENT || k == T_STRING; }
 // 64-bit class key of the tokens [start, end); 0 = this unit gets no template
 PTX_HD inline uint64_t ptx_class_key(const uint8_t* text, const PtxToken* tokens, const uint16_t* kinds, uint32_t start, uint32_t end, uint32_t depth,
@@ -146,19 +161,20 @@ PTX_HD inline uint64_t ptx_class_key(const uint8_t* text, const PtxToken* tokens
 //                ceil(len / 4) words of text]
 #define PTX_CLASS_SLOTS (1u << 20)          // hash slots (power of two)
 #define PTX_SIG_POOL_WORDS (16u << 20)      // 64 MiB of signatures
+struct alignas(8) PtxTmplWord {
+    uint32_t x, tag;            // one load for the emission
+};
 struct PtxClassStore {
     unsigned long long* keys;   // [PTX_CLASS_SLOTS] 0 = empty
     uint32_t* slot_tmpl;        // [PTX_CLASS_SLOTS] template id of the slot's class, PTX_ABSENT = none
-    uint32_t* tmpl_words;       // [PTX_MAX_CLASSES][PTX_TMPL_WORDS]
-    uint16_t* tmpl_tags;        // [PTX_MAX_CLASSES][PTX_TMPL_WORDS]
+    PtxTmplWord* tmpl;          // [PTX_MAX_CLASSES][PTX_TMPL_WORDS]
     PtxTemplateInfo* info;      // [PTX_MAX_CLASSES]
     uint32_t* sig_off;          // [PTX_MAX_CLASSES] word offset of the signature in sig_pool
     uint32_t* sig_pool;         // [PTX_SIG_POOL_WORDS]
     uint32_t* rep_unit;         // [PTX_MAX_CLASSES] representative unit (valid for the classes added by the current slice)
     uint32_t* state;            // [0] classes so far, [1] signature words used, [3] classes were inserted and never decoded
     static size_t bytes() {
-        return sizeof(unsigned long long) * PTX_CLASS_SLOTS + 4ull * PTX_CLASS_SLOTS + 4ull * PTX_TMPL_WORDS * PTX_MAX_CLASSES +
-               2ull * PTX_TMPL_WORDS * PTX_MAX_CLASSES + sizeof(PtxTemplateInfo) * PTX_MAX_CLASSES + 4ull * PTX_MAX_CLASSES +
+        return sizeof(unsigned long long) * PTX_CLASS_SLOTS + 4ull * PTX_CLASS_SLOTS + sizeof(PtxTmplWord) * PTX_TMPL_WORDS * PTX_MAX_CLASSES + sizeof(PtxTemplateInfo) * PTX_MAX_CLASSES + 4ull * PTX_MAX_CLASSES +
                4ull * PTX_SIG_POOL_WORDS + 4ull * PTX_MAX_CLASSES + 256;
     }
     // carve the arrays out of one allocation of bytes() bytes (256-byte aligned)
@@ -166,8 +182,7 @@ struct PtxClassStore {
         char* p = (char*)base;
         keys = (unsigned long long*)p; p += sizeof(unsigned long long) * PTX_CLASS_SLOTS;
         slot_tmpl = (uint32_t*)p; p += 4ull * PTX_CLASS_SLOTS;
-        tmpl_words = (uint32_t*)p; p += 4ull * PTX_TMPL_WORDS * PTX_MAX_CLASSES;
-        tmpl_tags = (uint16_t*)p; p += 2ull * PTX_TMPL_WORDS * PTX_MAX_CLASSES;
+        tmpl = (PtxTmplWord*)p; p += sizeof(PtxTmplWord) * PTX_TMPL_WORDS * PTX_MAX_CLASSES;
         info = (PtxTemplateInfo*)p; p += sizeof(PtxTemplateInfo) * PTX_MAX_CLASSES;
         sig_off = (uint32_t*)p; p += 4ull * PTX_MAX_CLASSES;
         sig_pool = (uint32_t*)p; p += 4ull * PTX_SIG_POOL_WORDS;
@@ -668,7 +683,9 @@ inline void ptx_stage_structure(BK& bk, PtxWork& w, PtxCounters& host_counters, 
 // the backend); word() only reads and says what to do with the word, so that a backend can have several words in flight
 // per thread; literal() is the second round (one literal per call, written in place).
 struct PtxEmitUnit {
-    uint32_t tmpl, start, flag, first;      // first: its first word in the record stream (filled in by the backend)
+    uint32_t tmpl;          // first word of the template, or of the staged record
+    uint32_t start, flag;
+    uint32_t first;         // its first word in the record stream (filled in by the backend)
 };
 struct PtxEmitStep {
     const uint8_t* uflag;
@@ -683,44 +700,42 @@ struct PtxEmitStep {
     PTX_HD PtxEmitUnit unit(size_t u) const {
         PtxEmitUnit e;
         e.flag = uflag[u];
-        e.tmpl = e.flag <= PTX_UNIT_TEMPLATED ? utmpl[u] : 0u;      // template, or place of the staged record
+        e.tmpl = e.flag == PTX_UNIT_TEMPLATED ? utmpl[u] * PTX_TMPL_WORDS : e.flag == PTX_UNIT_STAGED ? utmpl[u] : 0u;
         e.start = ustart[u];
         e.first = 0;
         return e;
     }
-    PTX_HD int word(const PtxEmitUnit& e, size_t u, uint32_t i, uint32_t& x) const {
-        if (e.flag == PTX_UNIT_STAGED) {
+    PTX_HD int word(const PtxEmitUnit& e, size_t, uint32_t i, uint32_t& x) const {
+        if (e.flag != PTX_UNIT_TEMPLATED) {
+            if (e.flag != PTX_UNIT_STAGED) return NOTHING;
             x = table[e.tmpl + i];
             return WRITE;
         }
-        if (e.flag != PTX_UNIT_TEMPLATED) return NOTHING;
-        const size_t at = (size_t)e.tmpl * PTX_TMPL_WORDS + i;
-        x = cs.tmpl_words[at];
-        const uint32_t g = cs.tmpl_tags[at];
-        if (g) {
-            const uint32_t type = g >> 8;
-            if (type >= PTX_TAG_VAL_LO) {
-                if (!(type & 1u)) return SECOND_ROUND;      // low word
-                // high word: written by the low-word thread in front of it, unless it stands alone
-                if (i > 0 && cs.tmpl_tags[at - 1] == (uint16_t)(g - 0x100u)) return NOTHING;
-                return SECOND_ROUND;
-            }
-            const PtxToken t = tokens[e.start + (g & 0xFFu)];
-            x = type == PTX_TAG_START ? t.start : type == PTX_TAG_LEN ? (uint32_t)t.len : ((x & 0xFFu) | ((uint32_t)t.len << 8));
+        const PtxTmplWord t = cs.tmpl[e.tmpl + i];
+        x = t.x;
+        if (!t.tag) return WRITE;
+        const uint32_t type = t.tag >> 8;
+        if (type >= PTX_TAG_VAL_LO) {
+            // a high word is written with the low word in front of it, unless it stands alone
+            return (type & 1u) && i > 0 && cs.tmpl[e.tmpl + i - 1].tag == t.tag - 0x100u ? NOTHING : SECOND_ROUND;
         }
+        const PtxTokenWord k = ((const PtxTokenWord*)tokens)[e.start + (t.tag & 0xFFu)];
+        const uint32_t len = k.y & 0xFFFFu;
+        x = type == PTX_TAG_START ? k.x : type == PTX_TAG_LEN ? len : ((x & 0xFFu) | (len << 8));
         return WRITE;
     }
     // Literal values, one thread per literal with the warps full: the low-word thread also writes the high word when
     // the template has it next (the two value words of an immediate)
     PTX_HD void literal(const PtxEmitUnit& e, uint32_t i, uint32_t j) const {
-        const size_t at = (size_t)e.tmpl * PTX_TMPL_WORDS + i;
-        const uint32_t g = cs.tmpl_tags[at], type = g >> 8;
+        const uint32_t g = cs.tmpl[e.tmpl + i].tag, type = g >> 8;
         const PtxToken t = tokens[e.start + (g & 0xFFu)];
-        uint64_t v = ptx_literal_value(text, t.start, t.len, t.kind);
+        uint64_t v;
+        if (t.kind != T_F64 && t.len <= 16) ptx_literal_scan(PtxBytes16(text, t.start), t.len, t.kind, &v);
+        else v = ptx_literal_value(text, t.start, t.len, t.kind);
         if (type >= PTX_TAG_NEG_LO) v = 0 - v;
         if (type & 1u) { words[j] = (uint32_t)(v >> 32); return; }
         words[j] = (uint32_t)v;
-        if (i + 1 < cs.info[e.tmpl].n_words && cs.tmpl_tags[at + 1] == (uint16_t)(g + 0x100u)) words[j + 1] = (uint32_t)(v >> 32);
+        if (i + 1 < PTX_TMPL_WORDS && i + 1 < cs.info[e.tmpl / PTX_TMPL_WORDS].n_words && cs.tmpl[e.tmpl + i + 1].tag == g + 0x100u) words[j + 1] = (uint32_t)(v >> 32);
     }
 };
 
@@ -898,9 +913,10 @@ struct PtxDecodeListStep {
         if (!sc.filled)
             for (uint32_t k = 0; k < nwin; k++) sc.win[k * sc.win_stride] = ((const PtxTokenWord*)(tokens + start))[k];
         const uint32_t dp = udepth[u], depth = dp & 0x7FFFFFFFu;
-        uint32_t* const out_words = rep ? cs.tmpl_words + (size_t)id * PTX_TMPL_WORDS : sc.stage;
-        uint16_t* const out_tags = rep ? cs.tmpl_tags + (size_t)id * PTX_TMPL_WORDS : nullptr;
-        const uint32_t out_stride = rep ? 1u : sc.stage_stride, out_cap = rep ? PTX_TMPL_WORDS : sc.stage_cap;
+        PtxTmplWord* const tmpl = cs.tmpl + (size_t)id * PTX_TMPL_WORDS;
+        uint32_t* const out_words = rep ? &tmpl->x : sc.stage;
+        uint32_t* const out_tags = rep ? &tmpl->tag : nullptr;
+        const uint32_t out_stride = rep ? (uint32_t)(sizeof(PtxTmplWord) / 4) : sc.stage_stride, out_cap = rep ? PTX_TMPL_WORDS : sc.stage_cap;
         PtxUnitResult r;
         uint32_t nw, ne = 0, high;
         bool as_is = true, bulk_used = false;      // as_is: the record depends on nothing that a tag cannot express
@@ -918,6 +934,7 @@ struct PtxDecodeListStep {
             if (rep) {
                 sink.words = out_words;
                 sink.tags = out_tags;
+                sink.words_stride = out_stride;
                 sink.words_cap = out_cap;
             } else {
                 sink.stage = out_words;
