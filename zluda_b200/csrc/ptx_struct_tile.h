@@ -292,7 +292,10 @@ PTX_HD inline uint32_t sx_walk(const PtxStructArgs& a, const SxThread& t, int32_
         bc_prev = bc;
         if (j + 1 == a.n_tokens) {
             a.mod_final_scope[ptx_upper_bound_u32(a.mtb, a.n_modules, j) - 1] = sd;
-            if (write) a.counters->n_units = u;
+            if (write) {
+                a.counters->n_units = u;
+                a.mub[a.n_modules] = u;
+            }
         }
     }
     return starts;

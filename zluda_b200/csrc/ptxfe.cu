@@ -371,6 +371,14 @@ __global__ void __launch_bounds__(256, 6) emit_records_kernel(LaunchCount count,
     }
 }
 
+// The beginning of a small batch in one launch: layouts and text from pinned host memory to their place, and the region that
+// the steps want cleared.  (A copy on the engine and a memset: 9 us, this: 4.)
+__global__ void __launch_bounds__(256) begin_kernel(uint4* dst, const uint4* src, uint32_t n, uint4* zero, uint32_t n_zero) {
+    const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (uint32_t i = at; i < n; i += step) dst[i] = src[i];
+    for (uint32_t i = at; i < n_zero; i += step) zero[i] = make_uint4(0, 0, 0, 0);
+}
+#define PTXFE_KERNEL_UPLOAD (128u << 10)
 __global__ void copy_words_kernel(uint32_t* dst, const uint32_t* src, uint32_t n) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
     __threadfence_system();
@@ -1412,6 +1420,7 @@ struct SliceRun {
     size_t meta = 0;                      // where its layouts lie in the metadata buffer
     uint32_t n = 0, mode = 0;
     uint32_t bias = 0;                    // its offset in the frame that text offsets are relative to
+    size_t up_bytes = 0;                  // a small batch: layouts and text, still to be brought from h_meta to d_meta
     const uint8_t* raw = nullptr;         // text that came as one run of host memory: the first kernel moves it to its slots
     bool first = true;                    // empties the class store
     int arena = 0;
@@ -1462,14 +1471,22 @@ static int begin_slice(CudaBackend& bk, SliceRun& sl, bool deferred) {
     w.mod_chunk_begin = (uint32_t*)(ctx->d_meta + mcb_at);
     if (deferred) deferred_caps(ctx, (uint64_t)w.n_chunks * PTX_CHUNK, w);
     // everything that the steps want cleared, in one go: per-module words, look-back descriptors, the counters
-    const size_t zero = 8192 + 48 * ((size_t)n + 2) + 16 * ((size_t)w.n_chunks / SCAN_TILE + 2) + 8 * ((size_t)w.n_chunks / LEX_TILE_CHUNKS + 2) + 16 * ((size_t)w.cap_units / SCAN_TILE + 2) +
+    size_t zero = 8192 + 48 * ((size_t)n + 2) + 16 * ((size_t)w.n_chunks / SCAN_TILE + 2) + 8 * ((size_t)w.n_chunks / LEX_TILE_CHUNKS + 2) + 16 * ((size_t)w.cap_units / SCAN_TILE + 2) +
                         sizeof(StructDesc) * ((size_t)w.cap_tokens / SX_TILE + 2);
+    zero &= ~(size_t)15;
     bk.zero_base = (char*)bk.alloc(zero);
     bk.zero_size = bk.zero_base ? zero : 0;
     bk.zero_used = 0;
     w.results = (PtxModuleResult*)bk.alloc(sizeof(PtxModuleResult) * ((size_t)n + 1));
     if (ctx->failed) return PTXFE_ERR_OOM;
-    CUDA_TRY(cudaMemsetAsync(bk.zero_base, 0, zero, bk.stream));
+    if (sl.up_bytes && sl.up_bytes <= PTXFE_KERNEL_UPLOAD) {
+        begin_kernel<<<32, 256, 0, bk.stream>>>((uint4*)ctx->d_meta, (const uint4*)ctx->h_meta, (uint32_t)((sl.up_bytes + 15) / 16), (uint4*)bk.zero_base, (uint32_t)(zero / 16));
+        ctx->launches++;
+    } else {
+        if (sl.up_bytes) CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, sl.up_bytes, cudaMemcpyHostToDevice, bk.stream));
+        CUDA_TRY(cudaMemsetAsync(bk.zero_base, 0, zero, bk.stream));
+    }
+    sl.up_bytes = 0;
     w.counters = (PtxCounters*)bk.zalloc(sizeof(PtxCounters));
     bk.stop = deferred ? &w.counters->redo : nullptr;
     bk.aborted = &w.counters->struct_abort;
@@ -1830,10 +1847,13 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     }
     auto submit_text = [&](size_t k) -> int {
         const Slice& sl = slices[k];
+        if (small) {       // goes up with the slice, on its stream
+            GatherSource{texts, ctx->layout.data(), n, 0}.fill(ctx->h_meta + meta_total, 0, text_off);
+            return PTXFE_OK;
+        }
         if (k == 0) {
             CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->s_in));
-            if (small) GatherSource{texts, ctx->layout.data(), n, 0}.fill(ctx->h_meta + meta_total, 0, text_off);
-            CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_total + (small ? text_off : 0), cudaMemcpyHostToDevice, ctx->s_in));
+            CUDA_TRY(cudaMemcpyAsync(ctx->d_meta, ctx->h_meta, meta_total, cudaMemcpyHostToDevice, ctx->s_in));
         }
         if (way[k] == UPLOAD_RUNS) {
             for (uint32_t m = sl.m0; m < sl.m1;) {
@@ -1843,10 +1863,10 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
                 if (bytes) CUDA_TRY(cudaMemcpyAsync(ctx->d_raw + raw_base[k] + repack[m].raw_off, texts[m], bytes, cudaMemcpyHostToDevice, ctx->s_in));
                 m = e;
             }
-        } else if (way[k] == UPLOAD_GATHER && !small) {
+        } else if (way[k] == UPLOAD_GATHER) {
             int st = gather_text(ctx, ctx->s_in, texts, sl.m0, sl.m1, sl.bias, sl.padded, ctx->d_text + sl.text_off);
             if (st != PTXFE_OK) return st;
-        } else if (!small) {
+        } else {
             for (uint32_t m = sl.m0; m < sl.m1; m++)
                 if (lens[m])
                     CUDA_TRY(cudaMemcpyAsync(ctx->d_text + sl.text_off + (ctx->layout[m].text_off - sl.bias), texts[m], lens[m], cudaMemcpyHostToDevice, ctx->s_in));
@@ -1886,6 +1906,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     // The kernels of slice k + 1 go into the stream before the host waits for those of slice k: the device does not idle
     // while the host looks at the counts and sends the results of slice k on their way.
     std::vector<SliceRun> runs(ns);
+    bool sent_back = false;
     auto enqueue = [&](size_t k) -> int {
         const Slice& sl = slices[k];
         SliceRun& r = runs[k];
@@ -1893,7 +1914,8 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         const cudaStream_t q = ctx->streams[r.arena];
         // this arena held the results of an earlier slice: they leave the device first
         if (k >= PTXFE_ARENAS) CUDA_TRY(cudaStreamWaitEvent(q, ctx->slice_ev[5 * (k - PTXFE_ARENAS) + 4], 0));
-        CUDA_TRY(cudaStreamWaitEvent(q, ctx->slice_ev[5 * k], 0));
+        if (small) r.up_bytes = meta_total + text_off;
+        else CUDA_TRY(cudaStreamWaitEvent(q, ctx->slice_ev[5 * k], 0));
         r.bias = (uint32_t)sl.bias;
         r.text = small ? (uint8_t*)ctx->d_meta + meta_total : ctx->d_text + sl.text_off;
         r.meta = meta_at[k];
@@ -1943,11 +1965,13 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
             if ((rc = grow_pinned(ctx, &ctx->h_lexerrs, &ctx->h_lexerrs_cap, (size_t)((lexerrs_done + nl) * scale) * 8 + 4096, lexerrs_done * 8)) != PTXFE_OK) return drain(rc);
         }
         // the kernels of this slice have finished
-        DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 3], ctx->s_out));
+        const bool nothing_to_send = small && words_there && !ne && !nl;
+        sent_back = sent_back || !nothing_to_send;
+        if (!nothing_to_send) DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 3], ctx->s_out));
         if (nw && !words_there) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_words + words_done, w.words, nw * 4, cudaMemcpyDeviceToHost, ctx->s_out));
         if (ne) DRAIN_TRY(cudaMemcpyAsync((PtxErrRec*)ctx->h_errs + errs_done, w.errs, ne * sizeof(PtxErrRec), cudaMemcpyDeviceToHost, ctx->s_out));
         if (nl) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_lexerrs + 2 * lexerrs_done, w.lexerrs, nl * 8, cudaMemcpyDeviceToHost, ctx->s_out));
-        DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 4], ctx->s_out));
+        if (!nothing_to_send) DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 4], ctx->s_out));
         if (words_done + nw > 0xFFFFFFFFull) return drain(PTXFE_ERR_TOO_LARGE);   // module results index words with 32 bits
         base_w[k] = words_done; base_e[k] = errs_done; base_l[k] = lexerrs_done;
         words_done += nw; errs_done += ne; lexerrs_done += nl;
@@ -1960,8 +1984,8 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         if (c.n_classes > s.n_classes) s.n_classes = c.n_classes;      // of the fullest store
         if (c.n_sig_words > s.n_signature_words) s.n_signature_words = c.n_sig_words;
     }
-    DRAIN_TRY(cudaStreamSynchronize(ctx->s_out));
-    DRAIN_TRY(cudaStreamSynchronize(ctx->s_in));
+    if (sent_back) DRAIN_TRY(cudaStreamSynchronize(ctx->s_out));
+    if (!small) DRAIN_TRY(cudaStreamSynchronize(ctx->s_in));
 #undef DRAIN_TRY
     // ---- module results index the batch-wide host arrays
     PtxModuleResult* res = (PtxModuleResult*)ctx->h_results;
@@ -1975,17 +1999,19 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
             seq_tokens += res[m].seq_tokens;
         }
     // ---- statistics: busy time of each of the three streams
-    cudaEventElapsedTime(&s.h2d_ms, ctx->ev[0], ctx->ev[1]);
+    s.h2d_ms = 0;
+    if (!small) cudaEventElapsedTime(&s.h2d_ms, ctx->ev[0], ctx->ev[1]);      // (of a small batch: part of kernel_ms)
     s.kernel_ms = s.d2h_ms = 0;
     s.lex_ms = s.structure_ms = s.decode_ms = 0;
     for (size_t k = 0; k < ns; k++) {
         float ms = 0;
         cudaEventElapsedTime(&ms, ctx->slice_ev[5 * k + 1], ctx->slice_ev[5 * k + 2]);
         s.kernel_ms += ms;
+        if (!sent_back) continue;
         cudaEventElapsedTime(&ms, ctx->slice_ev[5 * k + 3], ctx->slice_ev[5 * k + 4]);
         s.d2h_ms += ms;
     }
-    if (getenv("PTXFE_TRACE")) {
+    if (!small && getenv("PTXFE_TRACE")) {
         // device-side timeline of the three streams, milliseconds since the first text copy was submitted
         for (size_t k = 0; k < ns; k++) {
             float t[5];

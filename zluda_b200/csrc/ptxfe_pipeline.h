@@ -515,6 +515,7 @@ struct PtxModulesLexed {
     PtxCounters* counters;
     uint32_t* marks = nullptr;    // the tiles of the structure pass in which a module begins (sx_mark_tiles)
     uint32_t marks_stride = 0, cap_tokens = 0;
+    uint32_t* mub = nullptr;      // of a single module: zeros if it has no tokens, the structure pass writes them else
     PTX_HD void operator()(size_t m) const {
         const PtxPair none{0, 0};
         const PtxPair b = n_chunks ? cnt[mcb[m]] : none;
@@ -540,6 +541,7 @@ struct PtxModulesLexed {
 #endif
         }
         if (mod_flag && mod_flag[m]) PTX_REDO_SET(counters, PTX_REDO_SERIAL_LEX);
+        if (mub && b.a == e.a) mub[0] = mub[1] = 0;
         if (marks) {
             PtxStructArgs a{};
             a.mtb = mtb;
@@ -644,6 +646,7 @@ inline void ptx_stage_structure(BK& bk, PtxWork& w, PtxCounters& host_counters, 
     if constexpr (PtxFusedSteps<BK>::value) {
         lexed.cap_tokens = w.deferred ? w.cap_tokens : w.n_tokens;
         lexed.marks = bk.structure_marks(lexed.cap_tokens, &lexed.marks_stride);
+        lexed.mub = n_modules == 1 ? mub : nullptr;
     }
     bk.pf("modules_lexed", n_modules + 1, lexed);
     // B1: one pass over the token kinds: (scope, paren) depth restarting at every module, the unit starts, their
@@ -669,7 +672,9 @@ inline void ptx_stage_structure(BK& bk, PtxWork& w, PtxCounters& host_counters, 
         }
         w.n_units = host_counters.n_units;
     }
-    // modules without tokens begin where the next module with tokens begins; mub[n_modules] = number of units
+    // modules without tokens begin where the next module with tokens begins; mub[n_modules] = number of units (of a single
+    // module everything is there)
+    if (PtxFusedSteps<BK>::value && n_modules == 1) return;
     bk.pf("module_unit_ranges", n_modules + 1, [=] PTX_HD(size_t m) {
         if (m < n_modules && mtb[m] < mtb[m + 1]) return;      // written by the pass
         size_t k = m;
