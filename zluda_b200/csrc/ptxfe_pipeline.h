@@ -273,8 +273,20 @@ struct PtxCounters {
     uint32_t n_staged_words;    // words of the staged records so far
     uint32_t redo;              // PTX_REDO_*: something that the counts-stay-on-the-device flow does not cover
     uint32_t n_bulk_tokens;     // tokens of those statements
-    uint32_t spare[10];
+    uint32_t n_staged_errs;     // errors of staged units so far
+    uint32_t spare[9];
 };
+// an error of a unit whose record is staged: number k of the unit's
+struct PtxStagedErr {
+    PtxErrRec rec;
+    uint32_t unit, k;
+};
+// Errors are listed beside the staged records and put to their places with the module rows.  A slice that decoded its units
+// with errors a second time waited for the counts in between: a 100 KB module with errors took 245 us, and takes 200.  The
+// lines: a unit is a statement, and one that the grammar does not know has one error; the four stay in the thread's
+// registers and stack.  What the first pass must leave to the second all the same are calls (their errors depend on the
+// headers of other units).
+#define PTX_UNIT_ERRS 4u          // a unit with more than these is left to the second decode pass
 // why a slice that was enqueued whole is run again with the host reading the counts on the way
 enum { PTX_REDO_TOKENS = 1, PTX_REDO_SERIAL_LEX = 2, PTX_REDO_UNITS = 4, PTX_REDO_BULK = 8, PTX_REDO_LIST = 16, PTX_REDO_WORDS = 64, PTX_REDO_STORE = 128,
        PTX_REDO_DECODE = PTX_REDO_BULK | PTX_REDO_LIST | PTX_REDO_WORDS | PTX_REDO_STORE };    // these leave tokens and units as they are
@@ -391,6 +403,8 @@ struct PtxWork {
     uint8_t* unit_flag = nullptr;          // [n_units] PTX_UNIT_*
     uint32_t* unit_tmpl = nullptr;         // [n_units] template, or place of the staged record
     uint32_t* staged = nullptr;            // staged records
+    PtxStagedErr* staged_errs = nullptr;
+    uint32_t cap_errs = 0;                 // room in errs (deferred counts) and in staged_errs
     uint32_t* list = nullptr;              // [n_first] units decoded first (bit 31: as a class representative)
     uint32_t* second = nullptr;            // [n_second] units that a class promised a template and that have none
     PtxClassStore cs;
@@ -862,7 +876,7 @@ struct PtxDecodeListStep {
     const uint32_t* udepth;
     const uint32_t* udir;
     const uint32_t* uclass;
-    uint32_t n_modules, cap_staged, cap_funcs;
+    uint32_t n_modules, cap_staged, cap_funcs, cap_errs;
     PtxClassStore cs;
     PtxBulkTable bulk;
     uint32_t* utmpl;
@@ -871,6 +885,7 @@ struct PtxDecodeListStep {
     uint8_t* uflag;
     uint8_t* ustatus;
     uint32_t* staged;
+    PtxStagedErr* staged_errs;
     PtxFnEntry* fn_entries;
     PtxCounters* counters;
     // the tokens that go to the fast window: the unit's own and the one behind, from `start` on
@@ -924,6 +939,7 @@ struct PtxDecodeListStep {
         const uint32_t out_stride = rep ? (uint32_t)(sizeof(PtxTmplWord) / 4) : sc.stage_stride, out_cap = rep ? PTX_TMPL_WORDS : sc.stage_cap;
         PtxUnitResult r;
         uint32_t nw, ne = 0, high;
+        PtxErrRec errs[PTX_UNIT_ERRS];
         bool as_is = true, bulk_used = false;      // as_is: the record depends on nothing that a tag cannot express
         PtxFast fast{text, (const PtxTokenWord*)(tokens + start), sc.win, nwin, sc.win_stride, end - start, out_words, out_tags, out_stride, out_cap};
         if (!(dp >> 31) && (depth ? fast.instruction() : fast.kernel_header())) {
@@ -945,6 +961,8 @@ struct PtxDecodeListStep {
                 sink.stage = out_words;
                 sink.stage_stride = out_stride;
                 sink.stage_cap = out_cap;
+                sink.errs = errs;
+                sink.errs_cap = PTX_UNIT_ERRS;
             }
             PtxResolver res;
             res.module = m;
@@ -982,7 +1000,16 @@ struct PtxDecodeListStep {
         }
         uend[u] = r.end;
         ustatus[u] = (uint8_t)r.status;
-        bool flagged = high > out_cap || ne > 0 || bulk_used;
+        bool flagged = high > out_cap || ne > PTX_UNIT_ERRS || bulk_used;
+        for (uint32_t k = 0; k < ne && !flagged; k++) flagged = (errs[k].w0 & 0xFFFFu) == E_NONE;      // a call: to be resolved
+        if (ne && !flagged) {
+            const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_errs, ne);
+            flagged = (uint64_t)at + ne > cap_errs;
+            for (uint32_t k = 0; k < ne && at + k < cap_errs; k++) staged_errs[at + k] = PtxStagedErr{errs[k], u, k};      // (of a flagged unit: passed over later)
+            // a record with errors keeps the room of the alternatives that were rolled back, as one skip record
+            if (nw < high) sc.stage[nw * sc.stage_stride] = 13u /* U_PAD */ | ((high - nw - 1) << 8);
+            nw = high;
+        }
         if (!flagged && nw) {
             const uint32_t at = PTX_COUNT_ADD(&counters->n_staged_words, nw);
             flagged = (uint64_t)at + nw > cap_staged;
@@ -1288,6 +1315,9 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     w.unit_tmpl = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
     uint32_t* uclass = (uint32_t*)bk.alloc(sizeof(uint32_t) * (nu + 1));
     w.mod_bad = ptx_zalloc<uint32_t>(bk, n_modules + 1);
+    w.cap_errs = (uint32_t)(nu < PTX_SORT_MIN ? nu + 64 : PTX_SORT_MIN);
+    w.staged_errs = (PtxStagedErr*)bk.alloc(sizeof(PtxStagedErr) * (size_t)w.cap_errs);
+    if (w.deferred) w.errs = (PtxErrRec*)bk.alloc(sizeof(PtxErrRec) * (size_t)w.cap_errs);
     w.mod_seq_size = ptx_zalloc<PtxPair>(bk, n_modules + 1);
     w.mod_seq_status = ptx_zalloc<uint32_t>(bk, n_modules + 1);
     if (!PtxFusedSteps<BK>::value) {
@@ -1309,8 +1339,8 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
         w.list = w.second = nullptr;
         bk.pf_staged("decode_units", w.units_n(), w.staged, 0,
                      PtxDecodeListStep{nullptr, w.text, w.tokens, w.kinds, w.layout, w.mod_tok_begin, w.mod_unit_begin, w.mod_skip, w.unit_start, w.unit_depth,
-                                       w.unit_dir, nullptr, n_modules, cap_staged, w.cap_units, PtxClassStore(), PtxBulkTable(), w.unit_tmpl, w.unit_end, w.unit_own,
-                                       w.unit_flag, w.unit_status, w.staged, w.fn_entries, counters});
+                                       w.unit_dir, nullptr, n_modules, cap_staged, w.cap_units, w.cap_errs, PtxClassStore(), PtxBulkTable(), w.unit_tmpl, w.unit_end, w.unit_own,
+                                       w.unit_flag, w.unit_status, w.staged, w.staged_errs, w.fn_entries, counters});
         return;
     }
     // ---- classes
@@ -1336,8 +1366,8 @@ inline void ptx_decode_units(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     w.fn_entries = (PtxFnEntry*)bk.alloc(sizeof(PtxFnEntry) * ((size_t)cap_funcs + 1));
     if (!w.deferred && n_first > PTX_SORT_MIN) w.list = ptx_sort_list(bk, w, first, n_first);
     PtxDecodeListStep step{w.list, w.text, w.tokens, w.kinds, w.layout, w.mod_tok_begin, w.mod_unit_begin, w.mod_skip, w.unit_start, w.unit_depth, w.unit_dir,
-                           uclass, n_modules, cap_staged, cap_funcs, cs, w.bulk, w.unit_tmpl, w.unit_end, w.unit_own, w.unit_flag, w.unit_status, w.staged,
-                           w.fn_entries, counters};
+                           uclass, n_modules, cap_staged, cap_funcs, w.cap_errs, cs, w.bulk, w.unit_tmpl, w.unit_end, w.unit_own, w.unit_flag, w.unit_status, w.staged,
+                           w.staged_errs, w.fn_entries, counters};
     bk.pf_staged("decode_first", w.deferred ? PtxCount(cap_list, &counters->n_first) : PtxCount(n_first), w.staged, 0, step);
     // ---- templates, and the units that have none after all
     bk.pf("apply_templates", w.units_n(),
@@ -1363,7 +1393,7 @@ inline void ptx_scan_sizes(BK& bk, PtxWork& w, bool check) {
     const PtxPair* uown = w.unit_own;
     PtxCounters* counters = w.counters;
     const PtxClassStore cs = w.cs;
-    const uint32_t cap_words = w.deferred ? w.cap_words : 0xFFFFFFFFu;
+    const uint32_t cap_words = w.deferred ? w.cap_words : 0xFFFFFFFFu, cap_errs = w.cap_errs;
     const bool deferred = w.deferred, direct = w.direct;
     auto store = [=] PTX_HD(size_t i, PtxPair v) {
         usize[i] = v;
@@ -1375,6 +1405,7 @@ inline void ptx_scan_sizes(BK& bk, PtxWork& w, bool check) {
         counters->n_classes = direct ? 0u : cs.state[0];
         counters->n_sig_words = direct ? 0u : cs.state[1];
         if (v.a > cap_words) PTX_REDO_SET(counters, PTX_REDO_WORDS);
+        if (deferred && v.b > cap_errs) counters->n_flagged += 1;      // a second round, with room for them
         if (!deferred && counters->any_sequential) counters->n_flagged += 1;
     };
     if (check) {
@@ -1538,7 +1569,7 @@ inline void ptx_emit_flagged(BK& bk, PtxWork& w, const PtxCounters& host_counter
 }
 // the rows of the modules, finished
 template <class BK>
-inline void ptx_module_results(BK& bk, PtxWork& w, uint32_t n_errs) {
+inline void ptx_module_results(BK& bk, PtxWork& w, uint32_t n_errs, uint32_t n_staged_errs) {
     const uint32_t n_modules = w.n_modules;
     const uint32_t* mtb = w.mod_tok_begin;
     const uint32_t* mub = w.mod_unit_begin;
@@ -1552,6 +1583,19 @@ inline void ptx_module_results(BK& bk, PtxWork& w, uint32_t n_errs) {
     PtxCounters* counters_out = w.counters_out;
     const PtxCounters* counters = w.counters;
     const bool deferred = w.deferred;
+    const PtxStagedErr* staged_errs = w.staged_errs;
+    const uint8_t* uflag = w.unit_flag;
+    PtxErrRec* errs_out = w.errs;
+    const uint32_t cap_errs = w.cap_errs;
+    // the errors of staged units go to their places (a unit that the sequential parser took over has none); with deferred
+    // counts by the threads behind the modules' own
+    auto place = [=] PTX_HD(size_t e) {
+        const PtxStagedErr x = staged_errs[e];
+        if (uflag[x.unit] == PTX_UNIT_STAGED) errs_out[usize[x.unit].b + x.k] = x.rec;
+    };
+    constexpr size_t n_place = 1024;
+    if (n_staged_errs > cap_errs) n_staged_errs = cap_errs;
+    if (!deferred && n_staged_errs) bk.pf("place_errors", n_staged_errs, place);
     uint32_t* mod_nerr = nullptr;
     if (n_errs) {
         // parser errors per module, so that a module's verdict can be read off its result row
@@ -1566,20 +1610,27 @@ inline void ptx_module_results(BK& bk, PtxWork& w, uint32_t n_errs) {
             PTX_COUNT_ADD(&mod_nerr[lo], 1);
         });
     }
-    PtxCount rows(n_modules);
+    PtxCount rows(n_modules + (deferred ? n_place : 0));
     rows.always = true;
     bk.pf("module_results_final", rows, [=] PTX_HD(size_t m) {
         if (m == 0 && counters_out) *counters_out = *counters;
         if (counters->redo) return;
+        if (m >= n_modules) {
+            uint32_t n = counters->n_errs <= cap_errs ? counters->n_staged_errs : 0u;      // (else there is a second round)
+            if (n > cap_errs) n = cap_errs;
+            for (size_t e = m - n_modules; e < n; e += n_place) place(e);
+            return;
+        }
         PtxModuleResult r = results[m];
         const bool any = counters->n_units != 0;
-        r.n_errors = mod_nerr ? mod_nerr[m] : 0u;
         r.unit_begin = mub[m];
         r.unit_end = mub[m + 1];
         r.word_begin = any ? usize[mub[m]].a : 0;
         r.word_end = any ? usize[mub[m + 1]].a : 0;
         r.err_begin = any ? usize[mub[m]].b : 0;
         r.err_end = any ? usize[mub[m + 1]].b : 0;
+        // (with deferred counts there are no slots that a call reserved: a slice with calls has a second round)
+        r.n_errors = mod_nerr ? mod_nerr[m] : r.err_end - r.err_begin;
         const uint32_t bad = deferred ? 0u : mod_bad[m];      // (with deferred counts a slice with a bad module is finished by a second round)
         r.sequential = bad ? 1u : 0u;
         r.status = mod_seq_status[m];
@@ -1607,7 +1658,7 @@ inline void ptx_decode_finish(BK& bk, PtxWork& w, PtxCounters& host_counters, bo
     if (!again || host_counters.any_sequential) ptx_emit_records(bk, w);
     ptx_emit_flagged(bk, w, host_counters);
     ptx_bulk_write(bk, w);
-    ptx_module_results(bk, w, host_counters.n_errs);
+    ptx_module_results(bk, w, host_counters.n_errs, host_counters.n_staged_errs);
     bk.download(&host_counters, counters, sizeof(PtxCounters));   // .pad != 0: unit (index + 1) whose two passes disagreed
 }
 
@@ -1619,11 +1670,11 @@ inline void ptx_stage_decode(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     // the slice anew if they ask for it
     ptx_scan_sizes(bk, w, true);
     ptx_emit_records(bk, w);
-    ptx_module_results(bk, w, 0);
+    ptx_module_results(bk, w, 0, 0);
 }
 // Second round of a slice that ran with deferred counts and has lexer errors, damaged modules or flagged units
 // (host_counters = the counters of the first round)
-inline bool ptx_needs_again(const PtxCounters& c) { return c.n_lexerrs || c.any_sequential || c.n_flagged || c.n_errs; }
+inline bool ptx_needs_again(const PtxCounters& c) { return c.n_lexerrs || c.any_sequential || c.n_flagged; }
 template <class BK>
 inline void ptx_stage_again(BK& bk, PtxWork& w, PtxCounters& host_counters) {
     w.deferred = false;
@@ -1641,7 +1692,7 @@ inline void ptx_stage_decode_anew(BK& bk, PtxWork& w, PtxCounters& host_counters
     w.n_units = host_counters.n_units;
     bk.pf("reset_decode_counters", 1, [=] PTX_HD(size_t) {
         counters->n_bulk = counters->n_bulk_tokens = counters->n_first = counters->n_reps = counters->n_second = counters->n_flagged = counters->n_funcs = 0;
-        counters->n_staged_words = counters->any_sequential = counters->redo = 0;
+        counters->n_staged_words = counters->n_staged_errs = counters->any_sequential = counters->redo = 0;
     });
     ptx_lex_errors(bk, w, host_counters.n_lexerrs);
     ptx_stage_decode(bk, w, host_counters);
