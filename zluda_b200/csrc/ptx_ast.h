@@ -12,6 +12,11 @@
 // 1228-1232).  ptx_ast_print writes the same canonical text as the record reader in ptx_dump.h; the tests hold the two
 // against each other and against the oracle.
 #pragma once
+#include <atomic>
+#include <memory>
+#include <system_error>
+#include <thread>
+
 #include "ptx_dump.h"
 
 namespace ptxast {
@@ -715,20 +720,30 @@ struct Printer {
     struct HeadText {
         uint32_t n_words;           // data words
         uint32_t words[8];
-        std::string text;
+        size_t at, n_text;          // where it stands in what is printed so far
         int next;
     };
     std::vector<HeadText> heads;
     std::vector<int> head_of;       // by variant: the last text made, -1 = none
+    std::vector<uint32_t> data;
+    void prepare() {
+        head_of.assign(sizeof ptx_instrs / sizeof ptx_instrs[0], -1);
+        heads.reserve(256);
+        data.reserve(64);
+    }
     // prints it for the data words at w; returns where the operands begin
     const uint32_t* head(uint16_t variant, const Builder& b, const uint32_t* w, const uint32_t* end) {
-        if (head_of.empty()) head_of.assign(sizeof ptx_instrs / sizeof ptx_instrs[0], -1);
+        if (head_of.empty()) prepare();
         for (int i = head_of[variant]; i >= 0; i = heads[i].next) {
             const HeadText& h = heads[i];
-            if (h.n_words <= (uint32_t)(end - w) && memcmp(h.words, w, 4 * h.n_words) == 0) { o.putn(h.text.data(), h.text.size()); return w + h.n_words; }
+            if (h.n_words <= (uint32_t)(end - w) && memcmp(h.words, w, 4 * h.n_words) == 0) {
+                char* p = o.room(h.n_text);      // (may move the buffer)
+                memcpy(p, o.b + h.at, h.n_text);
+                return w + h.n_words;
+            }
         }
         const PtxInstr& in = ptx_instrs[variant];
-        std::vector<uint32_t> data;
+        data.clear();
         const uint32_t* behind = w;
         if (in.data_type >= 0 && !(ptx_types[in.data_type].kind == 2 && ptx_types[in.data_type].b == 0)) {
             ptxdump::PackedCursor cur;
@@ -742,7 +757,8 @@ struct Printer {
         h.n_words = (uint32_t)(behind - w);
         if (h.n_words <= sizeof h.words / 4) {
             memcpy(h.words, w, 4 * h.n_words);
-            h.text.assign(o.b + from, o.n - from);
+            h.at = from;
+            h.n_text = o.n - from;
             h.next = head_of[variant];
             head_of[variant] = (int)heads.size();
             heads.push_back(std::move(h));
@@ -777,10 +793,10 @@ struct Printer {
     Operand op;
     // the statements of a body straight from its records: variables, branches and calls are built like nodes of the tree and
     // printed, and their memory goes to the next one; of the other instructions only the operands are
-    void stream(const Builder& b, const uint32_t* q, const uint32_t* end) {
+    // Begins at the nesting `depth` and returns the one it ends at.
+    int stream(const Builder& b, const uint32_t* q, const uint32_t* end, int depth) {
         Instruction ins;
         MultiVariable var;
-        int depth = 1;
         for (; q < end; q += 1 + ptxdump::rec_len(q[0])) {
             switch (q[0] & 0xFF) {
             case U_LABEL: o.indent(depth); label(b.str(q[1], q[2])); break;
@@ -794,9 +810,157 @@ struct Printer {
             default: break;
             }
         }
-        while (depth > 1) { o.indent(--depth); o.put("])\n"); }
+        return depth;
+    }
+    // a directive up to the first statement of its body
+    void directive(const Directive& d) {
+        if (!d.is_method) {
+            o.putf("Variable(LinkingDirective(%u), ", d.linking);
+            variable(d.var);
+            o.put(")\n");
+            return;
+        }
+        const Function& f = d.func;
+        o.putf("Method(LinkingDirective(%u), Function { func_directive: MethodDeclaration { return_arguments: [", d.linking);
+        for (size_t i = 0; i < f.rets.size(); i++) { if (i) o.put(", "); variable(f.rets[i]); }
+        o.put(f.is_kernel ? "], name: Kernel(" : "], name: Func(");
+        str(f.name);
+        o.put("), input_arguments: [");
+        for (size_t i = 0; i < f.inputs.size(); i++) { if (i) o.put(", "); variable(f.inputs[i]); }
+        o.put("], shared_mem: None }, tuning: [");
+        for (size_t i = 0; i < f.tuning.size(); i++) {
+            if (i) o.put(", ");
+            const Tuning& t = f.tuning[i];
+            switch (t.kind) {
+            case 0: o.putf("MaxNReg(%u)", t.v[0]); break;
+            case 1: o.putf("MaxNtid(%u, %u, %u)", t.v[0], t.v[1], t.v[2]); break;
+            case 2: o.putf("ReqNtid(%u, %u, %u)", t.v[0], t.v[1], t.v[2]); break;
+            case 3: o.putf("MinNCtaPerSm(%u)", t.v[0]); break;
+            default: o.put("NoReturn"); break;
+            }
+        }
+        o.put(f.has_body ? "], body: Some([\n" : "], body: None })\n");
     }
 };
+
+// A directive, or a run of records of its body: whoever prints the body's first record prints what is in front of it, whoever
+// prints the last one what is behind it.
+struct Piece {
+    const Directive* d;
+    const uint32_t* q;
+    const uint32_t* end;
+    int depth;      // nesting at q
+};
+inline void print_pieces(Printer& p, const ptxdump::Reader& r, const std::vector<Piece>& pieces) {
+    ptxdump::Out& o = p.o;
+    Module scratch;      // the builder counts the nodes that it makes
+    for (const Piece& x : pieces) {
+        const Function& f = x.d->func;
+        if (x.q == f.body_rec) p.directive(*x.d);
+        if (!x.d->is_method || !f.has_body) continue;
+        int depth = x.depth;
+        if (f.body_rec) depth = p.stream(Builder{r, scratch}, x.q, x.end, depth);
+        else p.statements(f.body, 1);
+        if (x.end != f.body_end) continue;
+        while (depth > 1) { o.indent(--depth); o.put("])\n"); }
+        o.put("]) })\n");
+    }
+}
+// Record words that are worth a thread of their own: they print in some 110 us, a thread costs 15 to 30.
+constexpr size_t PRINT_PART_WORDS = 8192;
+constexpr size_t PRINT_WORD_ROOM = 24;      // characters (a word of code prints as 18 to 20)
+// All directives, on several threads where the bodies' records are many: the records are cut into parts of equal size, between
+// two statements and with the nesting noted, and every part is printed into its share of the buffer.  (The bound is the steps per
+// statement on one core; a 131 KB module with 34,000 words: 540 us, in four parts 255; in eight no less.)
+inline void print_directives(ptxdump::Out& o, const ptxdump::Reader& r, const std::vector<Directive>& dirs) {
+    size_t total = 0;
+    for (const Directive& d : dirs) total += (size_t)(d.func.body_end - d.func.body_rec);
+    size_t n_parts = total / PRINT_PART_WORDS;
+    if (n_parts > 8) n_parts = 8;
+    if (n_parts > 1 && n_parts > std::thread::hardware_concurrency()) n_parts = std::thread::hardware_concurrency();
+    std::vector<std::vector<Piece>> parts(1);
+    std::vector<size_t> begins(1, 0);      // words in front of each part
+    size_t at = 0;
+    for (const Directive& d : dirs) {
+        Piece x{&d, d.func.body_rec, d.func.body_end, 1};
+        if (n_parts > 1) {
+            int depth = 1;
+            for (const uint32_t* q = x.q; q < x.end; q += 1 + ptxdump::rec_len(q[0])) {
+                if (parts.size() < n_parts && at >= total / n_parts * parts.size()) {
+                    if (q != x.q) {
+                        parts.back().push_back(Piece{&d, x.q, q, x.depth});
+                        x.q = q;
+                        x.depth = depth;
+                    }
+                    parts.emplace_back();
+                    begins.push_back(at);
+                }
+                at += 1 + ptxdump::rec_len(q[0]);
+                const uint32_t kind = q[0] & 0xFF;
+                if (kind == U_BLOCK_OPEN) depth++;
+                else if (kind == U_BLOCK_CLOSE && depth > 1) depth--;
+            }
+        }
+        parts.back().push_back(x);
+    }
+    // (parts on lines of their own: two threads that count characters in one line take three times as long)
+    struct alignas(128) Part {
+        ptxdump::Out out;
+        Printer printer{out};
+    };
+    struct Others {
+        std::unique_ptr<Part[]> part;
+        std::vector<std::thread> threads;
+        std::atomic<bool> failed{false};
+        void join() { for (std::thread& t : threads) t.join(); threads.clear(); }
+        ~Others() { join(); }
+    } others;
+    const size_t n = parts.size();
+    if (n == 1) {
+        Printer p{o};
+        print_pieces(p, r, parts[0]);
+        return;
+    }
+    // Everybody prints into the one buffer, with room for a part's text as a record word prints at most on the whole; the parts
+    // are moved together in the end.  A part that needs more gets a buffer of its own.
+    begins.push_back(total);
+    const size_t from = o.n;
+    o.reserve(total * PRINT_WORD_ROOM + n * 4096);
+    others.part.reset(new Part[n]);
+    others.threads.reserve(n);
+    for (size_t k = 0; k < n; k++) {
+        others.part[k].out.borrow(o.b + from + begins[k] * PRINT_WORD_ROOM + k * 4096, (begins[k + 1] - begins[k]) * PRINT_WORD_ROOM + 4096);
+        others.part[k].printer.prepare();
+    }
+    auto part = [&](size_t k) {
+        try { print_pieces(others.part[k].printer, r, parts[k]); }
+        catch (...) { others.failed = true; }
+    };
+    size_t started = 1;
+    try {
+        for (; started < n; started++) others.threads.emplace_back(part, started);
+    } catch (const std::system_error&) {}      // no thread to be had: its part is printed here
+    part(0);
+    for (size_t k = started; k < n; k++) part(k);
+    others.join();
+    if (others.failed) throw std::bad_alloc();
+    size_t text = from;
+    bool own = false;
+    for (size_t k = 0; k < n; k++) {
+        text += others.part[k].out.n;
+        own = own || !others.part[k].out.borrowed;
+    }
+    if (own) {      // (a buffer for the whole: the move below wants every part where it was begun)
+        ptxdump::Out whole;
+        whole.reserve(text + 1024);
+        whole.putn(o.b, from);
+        for (size_t k = 0; k < n; k++) whole.putn(others.part[k].out.b, others.part[k].out.n);
+        o.swap(whole);
+        return;
+    }
+    for (size_t k = 0, at = from; k < n; at += others.part[k].out.n, k++) memmove(o.b + at, others.part[k].out.b, others.part[k].out.n);
+    o.n = text;
+}
 
 // the ordered list of a module's errors, one per line; returns how many there are
 inline size_t print_errors(const PtxBatchView& v, const ptxdump::Reader& r, ptxdump::Out* o, const Module& m) {
@@ -817,7 +981,6 @@ inline size_t print_errors(const PtxBatchView& v, const ptxdump::Reader& r, ptxd
 }
 
 inline void print_to(ptxdump::Out& o, const PtxBatchView& v, uint32_t mi, Module& m) {
-    Printer p{o};
     ptxdump::Reader r(v, mi);
     static const char* const verdicts[] = {"Ok", "Err", "Module", "Empty", "Errors", "ReferencePanics", "ReferenceDiverges", "SequentialPathRefused"};
     o.putf("mode: %s\nstatus: %s\n", v.mode == 0 ? "checked" : v.mode == 1 ? "unchecked" : "errors", verdicts[m.verdict]);
@@ -826,38 +989,7 @@ inline void print_to(ptxdump::Out& o, const PtxBatchView& v, uint32_t mi, Module
         uint64_t kept = m.directives.size();
         o.putf("Module { ptx_version: (%u, %u), sm_version: %u, address_size: %u, invalid_directives: %llu, directives: %llu }\n", m.major, m.minor,
                m.sm, m.address_size, (unsigned long long)m.invalid_directives, (unsigned long long)kept);
-        for (const Directive& d : m.directives) {
-            if (!d.is_method) {
-                o.putf("Variable(LinkingDirective(%u), ", d.linking);
-                p.variable(d.var);
-                o.put(")\n");
-                continue;
-            }
-            const Function& f = d.func;
-            o.putf("Method(LinkingDirective(%u), Function { func_directive: MethodDeclaration { return_arguments: [", d.linking);
-            for (size_t i = 0; i < f.rets.size(); i++) { if (i) o.put(", "); p.variable(f.rets[i]); }
-            o.put(f.is_kernel ? "], name: Kernel(" : "], name: Func(");
-            p.str(f.name);
-            o.put("), input_arguments: [");
-            for (size_t i = 0; i < f.inputs.size(); i++) { if (i) o.put(", "); p.variable(f.inputs[i]); }
-            o.put("], shared_mem: None }, tuning: [");
-            for (size_t i = 0; i < f.tuning.size(); i++) {
-                if (i) o.put(", ");
-                const Tuning& t = f.tuning[i];
-                switch (t.kind) {
-                case 0: o.putf("MaxNReg(%u)", t.v[0]); break;
-                case 1: o.putf("MaxNtid(%u, %u, %u)", t.v[0], t.v[1], t.v[2]); break;
-                case 2: o.putf("ReqNtid(%u, %u, %u)", t.v[0], t.v[1], t.v[2]); break;
-                case 3: o.putf("MinNCtaPerSm(%u)", t.v[0]); break;
-                default: o.put("NoReturn"); break;
-                }
-            }
-            if (!f.has_body) { o.put("], body: None })\n"); continue; }
-            o.put("], body: Some([\n");
-            if (f.body_rec) p.stream(Builder{r, m}, f.body_rec, f.body_end);
-            else p.statements(f.body, 1);
-            o.put("]) })\n");
-        }
+        print_directives(o, r, m.directives);
     } else if (v.mode == 1) {
         o.put("Module { ptx_version: (1, 0), sm_version: 0, address_size: 64, invalid_directives: 18446744073709551615, directives: 0 }\n");
     }

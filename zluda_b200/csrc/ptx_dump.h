@@ -13,6 +13,7 @@
 
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "ptxfe_pipeline.h"
@@ -33,7 +34,7 @@ struct Out {
     Out() = default;
     Out(const Out&) = delete;
     Out& operator=(const Out&) = delete;
-    ~Out() { free(b); }
+    ~Out() { if (!borrowed) free(b); }
     void fold() {
         for (size_t i = 0; i < n; i++) h = (h ^ (unsigned char)b[i]) * 1099511628211ull;
         n = 0;
@@ -43,8 +44,10 @@ struct Out {
         if (n + k <= cap) return;
         size_t want = cap * 2 > n + k ? cap * 2 : n + k;
         if (want < 4096) want = 4096;
-        char* nb = (char*)realloc(b, want);
+        char* nb = (char*)realloc(borrowed ? nullptr : b, want);
         if (!nb) throw std::bad_alloc();
+        if (borrowed) memcpy(nb, b, n);
+        borrowed = false;
         b = nb;
         cap = want;
     }
@@ -113,6 +116,18 @@ struct Out {
         *room(1) = '"';
     }
     void indent(int d) { memset(room((size_t)d * 2), ' ', (size_t)d * 2); }
+    // a part of another one's buffer, until it is full
+    bool borrowed = false;
+    void borrow(char* p, size_t k) {
+        b = p;
+        cap = k;
+        borrowed = true;
+    }
+    void swap(Out& x) {
+        std::swap(b, x.b);
+        std::swap(n, x.n);
+        std::swap(cap, x.cap);
+    }
     std::string take() const { return std::string(b ? b : "", n); }
     char* release(size_t* len) {      // NUL-terminated, malloc'ed; the caller frees it
         *room(1) = 0;
