@@ -18,6 +18,11 @@ import os
 
 import numpy as np
 
+try:
+    from . import _texts
+except ImportError:      # not built yet
+    _texts = None
+
 CHECKED, UNCHECKED, ERRORS_ONLY = 0, 1, 2
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -89,14 +94,6 @@ def lib():
     return _lib
 
 
-def _bytes_offset():
-    """Where the bytes of a bytes object lie in it (the header's size), or None where a look does not confirm it."""
-    at, probe = bytes.__basicsize__ - 1, b"0123456789abcdef"
-    return at if ctypes.string_at(id(probe) + at, len(probe)) == probe else None
-
-
-_BYTES_AT = _bytes_offset()
-
 # bytes at an address -> str without a bytes object in between
 _decode_utf8 = ctypes.pythonapi.PyUnicode_DecodeUTF8
 _decode_utf8.restype = ctypes.py_object
@@ -118,18 +115,17 @@ def _as_buffers(texts):
     if isinstance(texts, Texts):
         return texts.buffers
     texts = list(texts)
-    kinds = set(map(type, texts))
-    if str in kinds:
-        texts = [t.encode() if isinstance(t, str) else t for t in texts]
-        kinds.discard(str)
-        kinds.add(bytes)
     n = len(texts)
-    if kinds <= {bytes} and _BYTES_AT is not None:      # ctypes takes 0.4 us to fetch the address of each
-        ptrs = np.fromiter(map(id, texts), np.uint64, n) + np.uint64(_BYTES_AT)
-        return texts, ptrs, np.fromiter(map(len, texts), np.uint64, n)
-    ptrs = [t[0] if isinstance(t, tuple) else ctypes.cast(ctypes.c_char_p(t), ctypes.c_void_p).value for t in texts]
-    lens = [t[1] if isinstance(t, tuple) else len(t) for t in texts]
-    return texts, np.array(ptrs, np.uint64), np.array(lens, np.uint64)
+    ptrs, lens = np.empty(n, np.uint64), np.empty(n, np.uint64)
+    if _texts is None:
+        raise PtxfeError("zluda_b200/_texts.so is missing: build it with `python -m zluda_b200.build`")
+    first = _texts.addresses(texts, ptrs.ctypes.data, lens.ctypes.data)
+    for i in range(first, n):      # what is not a bytes object
+        t = texts[i]
+        if isinstance(t, str):
+            t = texts[i] = t.encode()
+        ptrs[i], lens[i] = t if isinstance(t, tuple) else (ctypes.cast(ctypes.c_char_p(t), ctypes.c_void_p).value, len(t))
+    return texts, ptrs, lens
 
 
 class Batch:
@@ -137,7 +133,7 @@ class Batch:
 
     def __init__(self, ctx, handle, keep):
         self._ctx, self._h, self._keep = ctx, handle, keep
-        self._rows = None      # (verdict, error count) of every module, fetched by the first question
+        self._status = self._errors = ()      # verdict and error count of every module, fetched by the first question
 
     def __len__(self):
         return lib().ptxfe_batch_size(self._h)
@@ -157,12 +153,18 @@ class Batch:
         n = len(self)
         status, errors = (ctypes.c_int32 * n)(), (ctypes.c_uint32 * n)()
         lib().ptxfe_module_verdicts(self._h, 0, n, status, errors)
-        self._rows = status[:], errors[:]
-        return self._rows
+        self._status, self._errors = status[:], errors[:]
 
     def status(self, i):
-        rows = self._rows or self._verdicts()
-        return rows[0][i] if 0 <= i < len(rows[0]) else lib().ptxfe_module_status(self._h, i)
+        try:
+            if i >= 0:
+                return self._status[i]
+        except IndexError:
+            if not self._status:
+                self._verdicts()
+                if i < len(self._status):
+                    return self._status[i]
+        return lib().ptxfe_module_status(self._h, i)
 
     def materialize(self, threads=None):
         """Build (and drop) the tree of every module on `threads` host threads; returns the number of nodes built."""
@@ -177,8 +179,15 @@ class Batch:
         return lib().ptxfe_multi_part_of(self._h, i)
 
     def error_count(self, i):
-        rows = self._rows or self._verdicts()
-        return rows[1][i] if 0 <= i < len(rows[1]) else lib().ptxfe_module_error_count(self._h, i)
+        try:
+            if i >= 0:
+                return self._errors[i]
+        except IndexError:
+            if not self._errors:
+                self._verdicts()
+                if i < len(self._errors):
+                    return self._errors[i]
+        return lib().ptxfe_module_error_count(self._h, i)
 
     def _text(self, fn, i):
         p = ctypes.c_void_p()

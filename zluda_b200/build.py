@@ -8,12 +8,14 @@ backend, are built by tests/build_helpers.py.)
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libptxfe.so")
 CORPUS_LIB = os.path.join(PKG, "libptxcorpus.so")
+TEXTS_LIB = os.path.join(PKG, "_texts.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--extended-lambda",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -62,9 +64,17 @@ def build_corpus_generator(force=False):
         _run(["gcc", "-O2", "-fPIC", "-shared", "-o", CORPUS_LIB, src, "-lm"])
 
 
+def build_texts(force=False):
+    """The extension module that reads addresses and lengths off a list of bytes objects."""
+    src = os.path.join(CSRC, "py_texts.c")
+    if force or _newer(TEXTS_LIB, [src]):
+        _run(["gcc", "-O2", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], "-o", TEXTS_LIB, src])
+
+
 def build(force=False):
     generate()
     log = build_library(force)
+    build_texts(force)
     build_corpus_generator(force)
     return log
 
