@@ -54,8 +54,36 @@ struct LaunchCount {
         return n < cap ? n : cap;
     }
 };
+// First statement of every step's kernel.  The steps of a small batch are launched ahead of the end of the step before
+// (launch_step): the next kernel may come as soon as all blocks of this one are there, and waits here until the one before has
+// finished and its writes are visible.  A small batch is a chain of a dozen steps of a few microseconds, and this takes more
+// than one of them out of each gap: 2 KB 172 -> 158 us with printing, the error list of 40 KB 192 -> 174, the lexer without
+// allocation on 3 MB 107 -> 97.  The line: 4.6 MB in one slice come out equal, and of 40 MB and more the waiting blocks take
+// room from the steps that run (3110 -> 3180 us, 4390 -> 4500).
+#define PTXFE_AHEAD_BYTES ((uint64_t)1 << 20)
+__device__ __forceinline__ void step_begins() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+template <class... P, class... A>
+static inline void launch_step(bool ahead, void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = ahead ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
 template <class F>
 __global__ void __launch_bounds__(256) pf_kernel(LaunchCount count, F f) {
+    step_begins();
     const size_t n = count.get();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) f(i);
 }
@@ -109,6 +137,7 @@ __device__ inline void lex_stage_tile(uint32_t* tile, uint32_t c0, uint32_t n_ch
 }
 template <class F>
 __global__ void __launch_bounds__(256) lex_tile_kernel(uint32_t n_chunks, const uint8_t* text, F f) {
+    step_begins();
     extern __shared__ __align__(16) uint32_t lex_smem[];
     uint32_t* tile = lex_smem;                                       // [LEX_TILE_CHUNKS][LEX_ROW_WORDS]
     uint16_t* fused = (uint16_t*)(lex_smem + LEX_TILE_CHUNKS * LEX_ROW_WORDS);    // [LS_COUNT][256]
@@ -125,6 +154,7 @@ __global__ void lex_fill_tables_kernel(PtxLexTables* t) { lt_fill_tables(t, thre
 // Persistent blocks: the tables are loaded once, then the block takes every gridDim.x-th tile.
 template <bool OWN>
 __global__ void __launch_bounds__(256, 8) lex_mark_kernel(PtxLexTileArgs a, uint32_t tile0, uint32_t n_tiles) {
+    step_begins();
     __shared__ PtxLexMarkShared sh;
     const uint32_t tid = threadIdx.x;
     lt_mark_tables(sh, a, tid, 256);
@@ -145,6 +175,7 @@ __global__ void __launch_bounds__(256, 8) lex_mark_kernel(PtxLexTileArgs a, uint
 }
 template <bool OWN>
 __global__ void __launch_bounds__(256, 5) lex_emit_kernel(PtxLexTileArgs a, uint32_t tile0, uint32_t n_tiles, const uint32_t* stop) {
+    step_begins();
     if (stop && *(const volatile uint32_t*)stop) return;
     extern __shared__ __align__(16) unsigned char lex_emit_smem[];
     PtxLexEmitShared& sh = *(PtxLexEmitShared*)lex_emit_smem;
@@ -192,6 +223,7 @@ __device__ inline void touch_lines(const void* table, size_t bytes) {
 #define STAGED_SMEM_BYTES (STAGE_CAP * STAGE_SLOTS * 4u + WIN_CAP * STAGE_SLOTS * 8u)
 template <class F>
 __global__ void __launch_bounds__(256) staged_kernel(LaunchCount count, F f) {
+    step_begins();
     extern __shared__ __align__(16) unsigned char staged_smem[];
     PtxTokenWord* win = (PtxTokenWord*)staged_smem;
     uint32_t* stage = (uint32_t*)(staged_smem + WIN_CAP * STAGE_SLOTS * 8u);
@@ -289,6 +321,7 @@ __device__ inline void block_scan(T v, Op op, T identity, T* warp_tot, T& incl, 
 #define EMIT_ILP 4
 #define EMIT_PASS 8192u
 __global__ void __launch_bounds__(256, 6) emit_records_kernel(LaunchCount count, const PtxPair* off, PtxEmitStep e) {
+    step_begins();
     const uint32_t n_units = (uint32_t)count.get();
     if (blockIdx.x * 256u >= n_units) return;
     __shared__ uint4 su[256];                         // the units that have words here: PtxEmitUnit
@@ -485,6 +518,7 @@ __device__ inline void look_back(ScanDesc<T>* desc, uint32_t tile, T agg, Op op,
 }
 template <class T, class Op, class Ld, class St>
 __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, Ld ld, St st, Op op, T identity, ScanDesc<T>* desc, uint32_t* ctl, uint32_t* aborted) {
+    step_begins();
     __shared__ T warp_tot[SCAN_THREADS / 32];
     __shared__ T s_before;
     __shared__ uint32_t s_tile, s_ok;
@@ -528,6 +562,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(LaunchCount count, L
 template <bool SCAN>
 __global__ void __launch_bounds__(256) lex_context_kernel(uint32_t n_chunks, const uint8_t* text, PtxLexVectorsStep f, uint32_t text_len, ScanDesc<uint32_t>* desc,
                                                           uint32_t* ctl, uint32_t* aborted) {
+    step_begins();
     extern __shared__ __align__(16) uint32_t lex_smem[];
     __shared__ uint32_t warp_tot[8], s_tile, s_before, s_ok;
     if (SCAN) {
@@ -604,6 +639,7 @@ __device__ inline bool sx_read_count(const StructDesc* d, uint32_t* ctl, unsigne
 }
 
 __global__ void __launch_bounds__(SX_THREADS) structure_kernel(PtxStructArgs a, StructDesc* desc, uint32_t* ctl, const uint32_t* stop) {
+    step_begins();
     if (stop && *(const volatile uint32_t*)stop) return;
     if (a.n_tokens_dev) a.n_tokens = *a.n_tokens_dev;
     const uint32_t n_tiles = (uint32_t)(((uint64_t)a.n_tokens + SX_TILE - 1) / SX_TILE);
@@ -923,12 +959,21 @@ struct ptxfe_ctx {
     std::string prof_text;
 };
 
+template <class F>
+static void launch_pf(bool ahead, unsigned blocks, cudaStream_t stream, LaunchCount count, F f) {
+    launch_step(ahead, pf_kernel<F>, blocks, 256, 0, stream, count, f);
+}
+template <class T, class Ld, class St, class Op>
+static void launch_scan(bool ahead, unsigned tiles, cudaStream_t stream, LaunchCount count, Ld ld, St st, Op op, T identity, ScanDesc<T>* desc, uint32_t* ctl, uint32_t* aborted) {
+    launch_step(ahead, scan_kernel<T, Op, Ld, St>, tiles, SCAN_THREADS, 0, stream, count, ld, st, op, identity, desc, ctl, aborted);
+}
 struct CudaBackend {
     static constexpr bool kFusedSteps = true;
     ptxfe_ctx* ctx;
     const int arena;
     const cudaStream_t stream;
     CudaBackend(ptxfe_ctx* c, int a) : ctx(c), arena(a), stream(c->streams[a]) {}
+    bool ahead = false;                    // steps are launched ahead of the end of the one before (step_begins)
     const uint32_t* stop = nullptr;        // deferred counts: the word that stops the slice (PtxCounters::redo)
     uint32_t* aborted = nullptr;           // where a look-back that gave up says so
     char* zero_base = nullptr;             // a region cleared ahead of the first step, handed out by zalloc
@@ -1013,7 +1058,7 @@ struct CudaBackend {
         size_t blocks = (n.cap + 255) / 256;
         if (n.dev && blocks > 148 * 64) blocks = 148 * 64;
         prof_begin(name);
-        pf_kernel<<<(unsigned)blocks, 256, 0, stream>>>(count_of(n), f);
+        launch_pf(ahead, (unsigned)blocks, stream, count_of(n), f);
         prof_end();
         ctx->launches++;
     }
@@ -1039,14 +1084,14 @@ struct CudaBackend {
         if (ctx->failed || n.cap == 0) return;
         prof_begin(name);
         // as many blocks as the device holds, or one list entry per warp
-        staged_kernel<<<resident_blocks((const void*)staged_kernel<F>, STAGED_SMEM_BYTES, (n.cap + 7) / 8), 256, STAGED_SMEM_BYTES, stream>>>(count_of(n), f);
+        launch_step(ahead, staged_kernel<F>, resident_blocks((const void*)staged_kernel<F>, STAGED_SMEM_BYTES, (n.cap + 7) / 8), 256, STAGED_SMEM_BYTES, stream, count_of(n), f);
         prof_end();
         ctx->launches++;
     }
     void emit_records(const char* name, PtxCount n, const PtxPair* off, const PtxEmitStep& e) {
         if (ctx->failed || n.cap == 0) return;
         prof_begin(name);
-        emit_records_kernel<<<(unsigned)((n.cap + 255) / 256), 256, 0, stream>>>(count_of(n), off, e);
+        launch_step(ahead, emit_records_kernel, (unsigned)((n.cap + 255) / 256), 256, 0, stream, count_of(n), off, e);
         prof_end();
         ctx->launches++;
     }
@@ -1058,8 +1103,8 @@ struct CudaBackend {
         ScanDesc<uint32_t>* desc = one_wave ? (ScanDesc<uint32_t>*)zalloc(sizeof(ScanDesc<uint32_t>) * blocks + 16) : nullptr;
         if (one_wave && !desc) return;
         prof_begin(name);
-        if (one_wave) lex_context_kernel<true><<<blocks, 256, LEX_TILE_BYTES, stream>>>((uint32_t)n, text, f, 0u, desc, (uint32_t*)(desc + blocks), aborted);
-        else lex_context_kernel<false><<<blocks, 256, LEX_TILE_BYTES, stream>>>((uint32_t)n, text, f, 0u, nullptr, nullptr, nullptr);
+        if (one_wave) launch_step(ahead, lex_context_kernel<true>, blocks, 256, LEX_TILE_BYTES, stream, (uint32_t)n, text, f, 0u, desc, (uint32_t*)(desc + blocks), aborted);
+        else launch_step(ahead, lex_context_kernel<false>, blocks, 256, LEX_TILE_BYTES, stream, (uint32_t)n, text, f, 0u, nullptr, nullptr, nullptr);
         prof_end();
         ctx->launches++;
         if (!one_wave) scan<uint32_t>("scan_context", n, ArrayLoad<uint32_t>{f.vec}, ArrayStore<uint32_t>{f.vec}, ComposeOp(), (uint32_t)CX_IDENTITY);
@@ -1070,7 +1115,7 @@ struct CudaBackend {
         prof_begin(name);
         // tile + table need more shared memory than a kernel gets by default
         cudaFuncSetAttribute(lex_tile_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(LEX_TILE_BYTES + LEX_TABLE_BYTES));
-        lex_tile_kernel<<<blocks, 256, LEX_TILE_BYTES + LEX_TABLE_BYTES, stream>>>((uint32_t)n, text, f);
+        launch_step(ahead, lex_tile_kernel<F>, blocks, 256, LEX_TILE_BYTES + LEX_TABLE_BYTES, stream, (uint32_t)n, text, f);
         prof_end();
         ctx->launches++;
     }
@@ -1103,14 +1148,14 @@ struct CudaBackend {
     void lex_mark(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
         prof_begin(name);
-        lex_mark_kernel<true><<<resident_blocks((const void*)lex_mark_kernel<true>, 0, n_tiles), 256, 0, stream>>>(a, 0u, (uint32_t)n_tiles);
+        launch_step(ahead, lex_mark_kernel<true>, resident_blocks((const void*)lex_mark_kernel<true>, 0, n_tiles), 256, 0, stream, a, 0u, (uint32_t)n_tiles);
         prof_end();
         ctx->launches++;
     }
     void lex_emit(const char* name, size_t n_tiles, const PtxLexTileArgs& a) {
         if (ctx->failed || n_tiles == 0) return;
         prof_begin(name);
-        lex_emit_kernel<true><<<resident_blocks((const void*)lex_emit_kernel<true>, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), stream>>>(a, 0u, (uint32_t)n_tiles, stop);
+        launch_step(ahead, lex_emit_kernel<true>, resident_blocks((const void*)lex_emit_kernel<true>, sizeof(PtxLexEmitShared), n_tiles), 256, sizeof(PtxLexEmitShared), stream, a, 0u, (uint32_t)n_tiles, stop);
         prof_end();
         ctx->launches++;
     }
@@ -1131,7 +1176,7 @@ struct CudaBackend {
         if (!desc) return;
         uint32_t* ctl = (uint32_t*)(desc + n_tiles);      // [0] next tile, [1] abort
         prof_begin(name);
-        structure_kernel<<<resident_blocks((const void*)structure_kernel, 0, n_tiles), SX_THREADS, 0, stream>>>(a, desc, ctl, stop);
+        launch_step(ahead, structure_kernel, resident_blocks((const void*)structure_kernel, 0, n_tiles), SX_THREADS, 0, stream, a, desc, ctl, stop);
         prof_end();
         ctx->launches++;
     }
@@ -1165,7 +1210,7 @@ struct CudaBackend {
         ScanDesc<T>* desc = (ScanDesc<T>*)zalloc(sizeof(ScanDesc<T>) * tiles + 16);
         if (!desc) return;
         uint32_t* ctl = (uint32_t*)(desc + tiles);         // [0] next tile, [1] abort
-        scan_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, stream>>>(count_of(n), ld, st, op, identity, desc, ctl, aborted);
+        launch_scan<T>(ahead, (unsigned)tiles, stream, count_of(n), ld, st, op, identity, desc, ctl, aborted);
         ctx->launches++;
     }
 };
@@ -1421,6 +1466,7 @@ struct SliceRun {
     size_t meta = 0;                      // where its layouts lie in the metadata buffer
     uint32_t n = 0, mode = 0;
     uint32_t bias = 0;                    // its offset in the frame that text offsets are relative to
+    bool ahead = false;                   // the only slice of its batch: steps launched ahead
     size_t up_bytes = 0;                  // a small batch: layouts and text, still to be brought from h_meta to d_meta
     const uint8_t* raw = nullptr;         // text that came as one run of host memory: the first kernel moves it to its slots
     bool first = true;                    // empties the class store
@@ -1517,6 +1563,7 @@ static int run_steps(CudaBackend& bk, SliceRun& sl) {
 static int run_exact(ptxfe_ctx* ctx, SliceRun& sl) {
     sl.deferred = false;
     CudaBackend bk(ctx, sl.arena);
+    bk.ahead = sl.ahead;
     int st = begin_slice(bk, sl, false);
     if (st == PTXFE_OK) st = run_steps(bk, sl);
     if (st != PTXFE_OK) return st;
@@ -1536,6 +1583,7 @@ static int enqueue_slice(ptxfe_ctx* ctx, SliceRun& sl) {
     if (n_chunks == 0) return run_exact(ctx, sl);
     sl.deferred = true;
     CudaBackend bk(ctx, sl.arena);
+    bk.ahead = sl.ahead;
     int st = begin_slice(bk, sl, true);
     if (st != PTXFE_OK) return st;
     PtxWork& w = ctx->works[sl.arena];
@@ -1568,6 +1616,7 @@ static int finish_slice(ptxfe_ctx* ctx, SliceRun& sl) {
         if (ctx->counters.redo && !(ctx->counters.redo & ~PTX_REDO_DECODE)) {
             // tokens and units stand: the decode stage alone, with the host reading its counts
                     CudaBackend bk(ctx, sl.arena);
+                    bk.ahead = sl.ahead;
             bk.aborted = &w.counters->struct_abort;
             w.first_slice = true;
             ptx_stage_decode_anew(bk, w, ctx->counters);
@@ -1580,6 +1629,7 @@ static int finish_slice(ptxfe_ctx* ctx, SliceRun& sl) {
             if (st != PTXFE_OK) return st;
         } else if (ptx_needs_again(ctx->counters)) {
                     CudaBackend bk(ctx, sl.arena);
+                    bk.ahead = sl.ahead;
             bk.aborted = &w.counters->struct_abort;
             ptx_stage_again(bk, w, ctx->counters);
             CUDA_TRY(cudaEventRecord(sl.ev_end, bk.stream));
@@ -1623,6 +1673,7 @@ int ptxfe_run(ptxfe_ctx* ctx, uint32_t mode) {
     sl.n = (uint32_t)ctx->layout.size();
     sl.meta = 0;
     sl.mode = mode;
+    sl.ahead = ctx->text_bytes <= PTXFE_AHEAD_BYTES;
     sl.ev_begin = ctx->ev[2]; sl.ev_lex = ctx->ev[3]; sl.ev_structure = ctx->ev[4]; sl.ev_end = ctx->ev[5];
     int st = enqueue_slice(ctx, sl);
     if (st == PTXFE_OK) st = finish_slice(ctx, sl);
@@ -1924,6 +1975,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         r.mode = mode;
         r.raw = way[k] == UPLOAD_RUNS ? ctx->d_raw + raw_base[k] : nullptr;
         r.first = k < PTXFE_ARENAS;
+        r.ahead = ns == 1 && total <= PTXFE_AHEAD_BYTES;
         r.results_out = (PtxModuleResult*)ctx->h_results + sl.m0;
         if (ns == 1 && total <= PTXFE_DIRECT_OUT_BYTES) {
             r.words_out = (uint32_t*)ctx->h_words;
@@ -2402,7 +2454,7 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
     // does not matter
     noalloc_init_kernel<<<4, 256, 0, stream>>>(s, me, n_chunks);
     const PtxLexChunkInfo info{&s->layout, s->mcb, 1};
-    lex_context_kernel<true><<<(n_chunks + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS, 256, LEX_TILE_BYTES, stream>>>(
+    launch_step(true, lex_context_kernel<true>, (n_chunks + LEX_TILE_CHUNKS - 1) / LEX_TILE_CHUNKS, 256, LEX_TILE_BYTES, stream,
         n_chunks, text, PtxLexVectorsStep{info, s->vec, s->tile_mod}, me, s->vec_desc, s->ctl, &s->aborted);
     const uint32_t n_tiles = (n_chunks + LT_CHUNKS - 1) / LT_CHUNKS;
     ScanDesc<PtxPair>* desc = s->cnt_desc;
@@ -2413,9 +2465,9 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
         PtxPair* cnt = s->seg.cnt - c0;
         PtxLexTileArgs a{info, text, s->vec, n_chunks, &s->tables, s->tile_mod, s->seg.start - (size_t)t0 * LT_WORDS, s->seg.word - (size_t)t0 * LT_WORDS,
                          cnt, s->mod_flag, tokens, nullptr, token_capacity};
-        lex_mark_kernel<false><<<t1 - t0 < pd.mark_blocks ? t1 - t0 : pd.mark_blocks, 256, 0, stream>>>(a, t0, t1);
+        launch_step(true, lex_mark_kernel<false>, t1 - t0 < pd.mark_blocks ? t1 - t0 : pd.mark_blocks, 256, 0, stream, a, t0, t1);
         const bool last = t1 == n_tiles;
-        scan_kernel<PtxPair><<<(items + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, stream>>>(
+        launch_scan<PtxPair>(true, (items + SCAN_TILE - 1) / SCAN_TILE, stream,
             LaunchCount{items, nullptr, nullptr, 0}, [=] __device__(size_t i) { return i ? cnt[c0 + i] : s->carry; },
             [=] __device__(size_t i, PtxPair v) {
                 cnt[c0 + i] = v;
@@ -2428,7 +2480,7 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
             },
             PairAddOp(), PtxPair{0, 0}, desc, s->ctl + 2 * (seg + 1), &s->aborted);
         desc += (items + SCAN_TILE - 1) / SCAN_TILE;
-        lex_emit_kernel<false><<<t1 - t0 < pd.emit_blocks ? t1 - t0 : pd.emit_blocks, 256, sizeof(PtxLexEmitShared), stream>>>(a, t0, t1, nullptr);
+        launch_step(true, lex_emit_kernel<false>, t1 - t0 < pd.emit_blocks ? t1 - t0 : pd.emit_blocks, 256, sizeof(PtxLexEmitShared), stream, a, t0, t1, nullptr);
     }
     // A run of soft bytes longer than the tile kernels look back (2 KiB): the text again, chunk by chunk, from the context
     // vectors; the steps below have nothing to do otherwise.
@@ -2444,7 +2496,7 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
         return cs - q > PTXFE_NOALLOC_MAX_BACK;
     };
     const unsigned walk_blocks = (n_chunks + 255) / 256;
-    pf_kernel<<<walk_blocks, 256, 0, stream>>>(chunks, [=] __device__(size_t c) {
+    launch_pf(true, walk_blocks, stream, chunks, [=] __device__(size_t c) {
         const uint32_t cs = (uint32_t)c * PTX_CHUNK;
         int state = c == 0 ? CX_CODE : (int)(vec[c - 1] & 7u);
         LexCountSink sink;
@@ -2452,10 +2504,10 @@ extern "C" int ptxfe_lex_device_noalloc(int device, const void* d_text_v, uint64
         else lx_chunk(PtxGlobalReader{text, me}, text, 0u, me, cs, cs + PTX_CHUNK, state, sink);
         cnt[c + 1] = PtxPair{sink.n_tokens, sink.n_errors};
     });
-    scan_kernel<PtxPair><<<(n_chunks + 1 + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, stream>>>(
+    launch_scan<PtxPair>(true, (n_chunks + 1 + SCAN_TILE - 1) / SCAN_TILE, stream,
         LaunchCount{(size_t)n_chunks + 1, &s->serial, nullptr, 1}, [=] __device__(size_t i) { return i ? cnt[i] : PtxPair{0, 0}; }, ArrayStore<PtxPair>{cnt},
         PairAddOp(), PtxPair{0, 0}, s->serial_desc, s->ctl + 2 * (PTXFE_NOALLOC_MAX_SEGS + 1), &s->aborted);
-    pf_kernel<<<walk_blocks, 256, 0, stream>>>(chunks, [=] __device__(size_t c) {
+    launch_pf(true, walk_blocks, stream, chunks, [=] __device__(size_t c) {
         const uint32_t cs = (uint32_t)c * PTX_CHUNK;
         int state = c == 0 ? CX_CODE : (int)(vec[c - 1] & 7u);
         LexCapSink sink;
