@@ -942,10 +942,10 @@ struct PtxDecodeListStep {
         PtxErrRec errs[PTX_UNIT_ERRS];
         bool as_is = true, bulk_used = false;      // as_is: the record depends on nothing that a tag cannot express
         PtxFast fast{text, (const PtxTokenWord*)(tokens + start), sc.win, nwin, sc.win_stride, end - start, out_words, out_tags, out_stride, out_cap};
-        if (!(dp >> 31) && (depth ? fast.instruction() : fast.kernel_header())) {
+        if (!(dp >> 31) && (depth ? fast.statement(depth) : fast.directive())) {
             r.end = end;
             r.status = US_OK;
-            r.kind = depth ? U_INSTR : U_FUNC;
+            r.kind = depth ? U_INSTR : fast.is_func ? U_FUNC : U_MODVAR;
             r.name_tok = start + fast.name_tok;
             r.n_rets = 0;
             r.n_inputs = fast.n_inputs;
