@@ -1780,6 +1780,9 @@ static uint64_t slice_target(uint64_t total, uint64_t done) {
     return t < PTXFE_SLICE_LEAST ? PTXFE_SLICE_LEAST : t;
 }
 
+// Module rows of a slice: up to this many are written to the host by the step that finishes them (17 ns a row: one thread
+// each, over the bus word by word), more travel as one copy behind the records (a few microseconds whatever their number).
+#define PTXFE_ROWS_OUT 512u
 int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* lens, uint32_t n, uint32_t mode, ptxfe_batch** out) {
     if (!out) return PTXFE_ERR_BAD_ARG;
     *out = nullptr;
@@ -1976,7 +1979,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
         r.raw = way[k] == UPLOAD_RUNS ? ctx->d_raw + raw_base[k] : nullptr;
         r.first = k < PTXFE_ARENAS;
         r.ahead = ns == 1 && total <= PTXFE_AHEAD_BYTES;
-        r.results_out = (PtxModuleResult*)ctx->h_results + sl.m0;
+        r.results_out = r.n <= PTXFE_ROWS_OUT ? (PtxModuleResult*)ctx->h_results + sl.m0 : nullptr;
         if (ns == 1 && total <= PTXFE_DIRECT_OUT_BYTES) {
             r.words_out = (uint32_t*)ctx->h_words;
             r.words_out_cap = (uint32_t)(ctx->h_words_cap / 4 - 4);
@@ -2018,12 +2021,14 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
             if ((rc = grow_pinned(ctx, &ctx->h_lexerrs, &ctx->h_lexerrs_cap, (size_t)((lexerrs_done + nl) * scale) * 8 + 4096, lexerrs_done * 8)) != PTXFE_OK) return drain(rc);
         }
         // the kernels of this slice have finished
-        const bool nothing_to_send = small && words_there && !ne && !nl;
+        const bool rows_there = runs[k].results_out != nullptr;
+        const bool nothing_to_send = small && words_there && rows_there && !ne && !nl;
         sent_back = sent_back || !nothing_to_send;
         if (!nothing_to_send) DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 3], ctx->s_out));
         if (nw && !words_there) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_words + words_done, w.words, nw * 4, cudaMemcpyDeviceToHost, ctx->s_out));
         if (ne) DRAIN_TRY(cudaMemcpyAsync((PtxErrRec*)ctx->h_errs + errs_done, w.errs, ne * sizeof(PtxErrRec), cudaMemcpyDeviceToHost, ctx->s_out));
         if (nl) DRAIN_TRY(cudaMemcpyAsync((uint32_t*)ctx->h_lexerrs + 2 * lexerrs_done, w.lexerrs, nl * 8, cudaMemcpyDeviceToHost, ctx->s_out));
+        if (!rows_there) DRAIN_TRY(cudaMemcpyAsync((PtxModuleResult*)ctx->h_results + sl.m0, w.results, sizeof(PtxModuleResult) * (size_t)runs[k].n, cudaMemcpyDeviceToHost, ctx->s_out));
         if (!nothing_to_send) DRAIN_TRY(cudaEventRecord(ctx->slice_ev[5 * k + 4], ctx->s_out));
         if (words_done + nw > 0xFFFFFFFFull) return drain(PTXFE_ERR_TOO_LARGE);   // module results index words with 32 bits
         base_w[k] = words_done; base_e[k] = errs_done; base_l[k] = lexerrs_done;
