@@ -1481,9 +1481,12 @@ struct SliceRun {
 #define PTXFE_DIRECT_OUT_BYTES (1u << 20)
 #define PTXFE_COUNTERS_SLOT(ctx, arena) ((PtxCounters*)((char*)(ctx)->h_counters + 2048 + 512 * (arena)))
 
-// Up to this much text every unit is decoded on its own (PtxWork::direct): there are then no more units than the device holds
-// warps that decode one each (some 3,500).
-#define PTXFE_DIRECT_BYTES (96u << 10)
+// Up to this much text every unit is decoded on its own (PtxWork::direct), which saves the four steps of keys, classes and
+// templates; beyond it the units are so many more than the warps the device holds (some 3,500) that the classes pay.  Parsing
+// one module with classes and without: 100 KB 190 and 156 us, 131 KB 200 and 160, 200 KB 205 and 179, 300 KB 220 and 205,
+// 450 KB 277 and 281, 600 KB 295 and 307.  The line stays under the 150 KB from which on the tests hold literals to the values
+// that a template gives them.
+#define PTXFE_DIRECT_BYTES (144u << 10)
 // capacities of a slice that runs with deferred counts: `bytes` of padded text
 static void deferred_caps(const ptxfe_ctx* ctx, uint64_t bytes, PtxWork& w) {
     auto cap = [&](double per_byte, uint64_t least, uint64_t most) -> uint32_t {
@@ -1764,8 +1767,8 @@ int ptxfe_fetch(ptxfe_ctx* ctx, ptxfe_batch** out) {
 }
 
 // One call, host text in, host records out.  The batch is cut into slices of whole modules; the text of slice k+1
-// travels to the device and the records of slice k-1 travel back while the kernels of slice k run (three streams,
-// two working arenas).  Text offsets inside the records are relative to the slice, as ptxfe_module_records reports.
+// travels to the device and the records of slice k-1 travel back while the kernels of slice k run (one stream
+// and one working arena for each of the slices in flight).  Text offsets inside the records are relative to the slice, as ptxfe_module_records reports.
 // How much text the next slice takes, `done` bytes into a batch of `total`.  Slices grow from 8 MiB and shrink to it again:
 // the first text copy and the last result copy overlap with nothing.  Below 16 MiB in all a batch is one slice, as a slice
 // is a chain of some fifteen short steps (0.25 ms) whatever its size; above 128 MiB a slice gains nothing.  Measured on
@@ -1799,7 +1802,7 @@ int ptxfe_parse_batch(ptxfe_ctx* ctx, const char* const* texts, const uint64_t* 
     ctx->layout.resize(n);
     // ---- slices
     // Small slices at both ends (the first text copy and the last result copy overlap with nothing), large ones in
-    // between (every slice costs a few host synchronisations and ~70 launches).  PTXFE_SLICE_BYTES forces one size.
+    // between (every slice costs 15 launches and a wait of the host).  PTXFE_SLICE_BYTES forces one size.
     uint64_t grand_total = 0;
     for (uint32_t m = 0; m < n; m++) grand_total += lens[m];
     uint64_t edge = (uint64_t)32 << 20, div = 8;
